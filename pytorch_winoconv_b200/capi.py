@@ -42,7 +42,7 @@ class Desc(Structure):
 class PlanInfo(Structure):
     _fields_ = [("out_size", c_int32 * 3), ("conv_out_size", c_int32 * 3), ("tile_m", c_int32 * 3),
                 ("tiles_per_dim", c_int32 * 3), ("n_pieces", c_int32), ("positions", c_int32), ("c_pad", c_int32),
-                ("gemm_engine", c_int32), ("algo", c_int32), ("reserved0", c_int32), ("tiles", c_int64), ("filter_bytes", c_uint64),
+                ("gemm_engine", c_int32), ("algo", c_int32), ("direct", c_int32), ("tiles", c_int64), ("filter_bytes", c_uint64),
                 ("input_ws_bytes", c_uint64), ("product_ws_bytes", c_uint64), ("input_ws_bytes_min", c_uint64),
                 ("product_ws_bytes_min", c_uint64), ("block_tiles", c_int64), ("direct_flops", c_double),
                 ("gemm_flops", c_double), ("algorithmic_bytes", c_double)]

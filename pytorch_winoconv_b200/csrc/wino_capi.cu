@@ -45,6 +45,9 @@ struct Plan {
   bool row;      // row-piece kernel
   RowDesc rd;
   RowPlan rp;
+  bool direct;   // AUTO: the direct-tap kernel runs the layer
+  DirectDesc dd;
+  DirectPlan dp;
   winoconv_plan_info_t info;
   int dtype, product_dtype, engine;
 };
@@ -252,6 +255,20 @@ int build_plan(const winoconv_desc_t *d, Plan *plan) {
     }
   }
 
+  // AUTO with no tile size asked for: the direct-tap kernel
+  plan->direct = false;
+  static const int direct_env = [] { const char *v = getenv("WINOCONV_DIRECT"); return v && *v ? atoi(v) : 1; }();
+  if (d->algo == WINOCONV_ALGO_AUTO && d->tile_m == 0 && d->gemm_engine == WINOCONV_GEMM_AUTO && pdt == WINOCONV_F32 && direct_env != 0 &&
+      (plan->row || (d->dtype == WINOCONV_F32 && direct_env == 2))) {
+    DirectDesc &q = plan->dd;
+    std::memset(&q, 0, sizeof q);
+    q.dtype = d->dtype; q.N = g.N; q.C = g.C; q.K = g.K; q.D = g.D; q.H = g.H; q.W = g.W;
+    q.oD = g.oD; q.oH = g.oH; q.oW = g.oW; q.yH = g.yH; q.yW = g.yW;
+    q.sD = g.sD; q.sH = g.sH; q.sW = g.sW; q.pD = g.pD; q.pH = g.pH; q.pW = g.pW; q.kD = g.kD; q.kH = g.kH; q.kW = g.kW;
+    q.epilogue = g.epilogue; q.weight_layout = g.weight_layout;
+    plan->direct = direct_plan(q, &plan->dp);
+  }
+
   winoconv_plan_info_t &I = plan->info;
   for (int i = 0; i < 3; ++i) { I.conv_out_size[i] = out[i]; I.tile_m[i] = m[i]; I.tiles_per_dim[i] = nt[i]; }
   I.out_size[0] = g.yD; I.out_size[1] = g.yH; I.out_size[2] = g.yW;
@@ -292,6 +309,10 @@ int build_plan(const winoconv_desc_t *d, Plan *plan) {
         ((rd.phases > 1 || rp.Cp != g.C) && !rp.raw_c && !rp.s2_chunks) ? (unsigned long long)rd.N * rd.D * rd.H * rd.W * rp.Cp * esz : 0ull;
     I.product_ws_bytes = I.product_ws_bytes_min = 0;
     I.block_tiles = I.tiles;
+  }
+  if (plan->direct) {
+    I.direct = 1;
+    I.filter_bytes = std::max<unsigned long long>(I.filter_bytes, (unsigned long long)plan->dp.filter_elems * esz);
   }
   I.direct_flops = 2.0 * g.N * g.K * g.C * (double)ks[0] * ks[1] * ks[2] * (double)out[0] * out[1] * out[2];
   I.gemm_flops = plan->fused ? 2.0 * 16 * (double)plan->fg.T * plan->fg.P * g.C * g.K : 2.0 * pos * (double)g.T * g.C * g.K;
@@ -395,7 +416,8 @@ int winoconv_filter_transform(const winoconv_desc_t *desc, const void *weights, 
   if (st != WINOCONV_OK) return st;
   if (!weights || !u) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "null weights or u");
   if ((st = winoconv_device_check()) != WINOCONV_OK) return st;
-  cudaError_t e = plan.row     ? launch_rowfused_filter_transform(plan.rd, plan.rp, plan.dtype, weights, u, (cudaStream_t)stream)
+  cudaError_t e = plan.direct  ? launch_direct_filter_transform(plan.dd, plan.dp, plan.dtype, weights, u, (cudaStream_t)stream)
+                  : plan.row   ? launch_rowfused_filter_transform(plan.rd, plan.rp, plan.dtype, weights, u, (cudaStream_t)stream)
                   : plan.fused ? launch_fused_filter_transform(plan.fg, plan.dtype, weights, u, (cudaStream_t)stream)
                                : launch_filter_transform(plan.g, plan.dtype, weights, u, (cudaStream_t)stream);
   if (e != cudaSuccess) return cuda_fail(e, "filter transform launch");
@@ -411,13 +433,13 @@ static int forward_impl(const winoconv_desc_t *desc, const void *x, const void *
   if (!x || !u || !y) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "null tensor pointer");
   if ((desc->epilogue & WINOCONV_EPI_BIAS) && !bias) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "EPI_BIAS set but bias is null");
   if (!aligned16(x) || !aligned16(u) || !aligned16(y)) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "tensors must be 16-byte aligned");
-  if (plan.row && plan.info.input_ws_bytes_min > 0) {
+  if (plan.row && !plan.direct && plan.info.input_ws_bytes_min > 0) {
     if (!v_ws || !aligned16(v_ws)) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "channel-padding scratch (v_ws) must be a 16-byte aligned pointer");
     if (v_ws_bytes < plan.info.input_ws_bytes_min)
       return fail(WINOCONV_ERR_WORKSPACE, "v_ws holds " + std::to_string(v_ws_bytes) + " bytes; padding the input channels needs " +
                                               std::to_string(plan.info.input_ws_bytes_min));
   }
-  if (plan.fused || plan.row) {   // one kernel, no V / M scratch
+  if (plan.fused || plan.row || plan.direct) {   // one kernel, no V / M scratch
     if ((st = winoconv_device_check()) != WINOCONV_OK) return st;
     cudaStream_t fs = (cudaStream_t)stream;
     struct EventPair {   // destroyed on every way out
@@ -433,10 +455,11 @@ static int forward_impl(const winoconv_desc_t *desc, const void *x, const void *
       if (e != cudaSuccess) return cuda_fail(e, "event record");
     }
     const char *detail = "";
-    e = plan.row ? launch_rowfused_forward(plan.rd, plan.rp, plan.dtype, x, u, bias, y, v_ws, fs, &detail)
+    e = plan.direct ? launch_direct_forward(plan.dd, plan.dp, x, u, bias, y, fs, &detail)
+        : plan.row ? launch_rowfused_forward(plan.rd, plan.rp, plan.dtype, x, u, bias, y, v_ws, fs, &detail)
                  : launch_fused_forward(plan.fg, plan.dtype, x, u, bias, y, fs, &detail);
     if (e != cudaSuccess) return cuda_fail(e, "fused forward launch", detail);
-    if (launches) *launches = (plan.row && plan.info.input_ws_bytes_min > 0) ? 2 : 1;
+    if (launches) *launches = (plan.row && !plan.direct && plan.info.input_ws_bytes_min > 0) ? 2 : 1;
     if (stage_ms) {
       stage_ms[0] = stage_ms[2] = 0.f;
       e = cudaEventRecord(e1, fs);
@@ -659,11 +682,12 @@ int winoconv_read_device_error(void *stream, uint32_t *code) {
   if (!code) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "null code");
   unsigned int host = 0, host2 = 0;
   cudaError_t e = read_and_clear_device_error((cudaStream_t)stream, &host);
-  unsigned int host3 = 0;
+  unsigned int host3 = 0, host4 = 0;
   if (e == cudaSuccess) e = read_and_clear_fused_error((cudaStream_t)stream, &host2);
   if (e == cudaSuccess) e = read_and_clear_row_error((cudaStream_t)stream, &host3);
+  if (e == cudaSuccess) e = read_and_clear_direct_error((cudaStream_t)stream, &host4);
   if (e != cudaSuccess) return cuda_fail(e, "reading the device error word");
-  if (host == 0) host = host2 ? host2 : host3;
+  if (host == 0) host = host2 ? host2 : host3 ? host3 : host4;
   *code = host;
   if (host != 0) return fail(WINOCONV_ERR_TIMEOUT, "a bounded device wait gave up, code 0x" + [&] { char b[16]; snprintf(b, sizeof b, "%x", host); return std::string(b); }());
   return WINOCONV_OK;

@@ -1,0 +1,921 @@
+// Direct-tap forward convolution on the tensor cores (sm_100a): every kernel tap is one K-major slice of the reduction,
+//
+//     y[n, o, k] = sum over taps t and channels c of x[n, s * o + t - p, c] * U[t][k][c]
+//
+// with the x operand of *all* taps read from one shared-memory slab.  A 128-row tile is 16 groups of 8 pixels along W (the
+// groups run over output rows, or over rows and images where the image is small); its slab holds those pixels and the halo
+// of the kernel, [rows][images][8 + kW - 1 pixels][64 channels] as TMA writes it with the 128-byte swizzle.  The swizzle is a
+// function of the absolute address, so a tcgen05 operand may start at any pixel of the slab: tap (kh, kw) is the same slab
+// read from kh rows and kw pixels further on, with a group stride of one slab row.  No im2col copy, no transform, nothing
+// but the filter is reloaded per tap.
+//
+// What bounds it: the tensor pipe needs N / 2 clocks per (M = 128, N, K = 16) instruction, shared memory delivers 128 B per
+// clock.  Per tap and 64 channels of a 256-column tile of a CTA pair an SM reads 4 x (4 KB of A + 4 KB of B) and TMA writes
+// 16 KB of filter and about 2.6 KB of slab: 50 KB in the 512 clocks the MMAs take, where a kernel that loads its A operand
+// tap by tap moves 64 KB.  F(2,3) row pieces do two thirds of the multiplies but move 74 KB per 256 columns' worth of work
+// and spend an epilogue and a producer pass on the transforms.
+//
+// Roles of a CTA: warp 0 TMA slabs, warp 1 TMA filter tiles, warps 2-3 MMA issue (one per 128-row block; warp 2 owns the
+// tensor memory), warps 4-11 epilogue (lane quarter x alternate 128-byte column chunks: bias, ReLU, 2x2 pool, TMA stores),
+// for fp32 also warps 12-15, which split every landed slab into a tf32 part and its remainder (three products per multiply,
+// the filter comes split from its transform).
+// Small problems run with one item per cluster of 2, 4 or 8 CTAs that share its reduction and add their accumulators through
+// distributed shared memory.  Every mbarrier wait is bounded and reports through the error word.
+//
+// Stands in for the chain of src/base_conv_launchers.cu:338-381 where no output tile larger than 1 is worth its transforms.
+#include <algorithm>
+#include <cstdlib>
+#include <cstring>
+#include <cstdio>
+#include <map>
+#include <mutex>
+#include <type_traits>
+
+#include "wino_launch.h"
+#include "wino_sm100.cuh"
+
+namespace wino {
+
+__device__ unsigned int g_direct_error = 0;
+
+namespace dconv {
+
+using namespace sm100;
+
+constexpr int BM = 128;
+constexpr int EPI_WARP0 = 4, EPI_WARPS = 8, SPLIT_WARP0 = 12, SPLIT_WARPS = 4;
+constexpr int STAGE_BYTES = 4096;      // epilogue staging per warp: 32 rows of 128 bytes
+constexpr int MAX_TAPS = 100;
+constexpr int BAR_BYTES = 512;
+
+enum ErrCode : unsigned { ERR_A_EMPTY = 0x401, ERR_B_EMPTY = 0x402, ERR_ACC = 0x403, ERR_A = 0x404, ERR_B = 0x405, ERR_EPI = 0x406, ERR_SPLIT = 0x407 };
+
+struct DGeom {
+  int N, K, oD, oH, oW, yH, yW;
+  int sD, sH, sW, pD, pH, pW, kD;
+  int TN, tn_shift, TH, PW;          // images and output rows of a block (TH * TN == 16), pixels of a slab row
+  int n_wb, n_hb, n_tiles, n_kb, n_items;
+  int n_ph, ph_h[4], ph_w[4], taps[4], tap0[4], T_hw;
+  int n_chunks, ch_el, k_full, k_tail;   // channel chunks, channels per chunk, MMA K steps of a full and of the last chunk
+  int units;                         // kD * T_hw * n_chunks: (tap, chunk) pairs of the whole reduction
+  int G, split;
+  unsigned epilogue;
+  int y_tma, bias_vec;
+  uint32_t a_hi, b_hi;               // high descriptor words
+  int mb_off16;                      // slab offset of the second row block (16-byte units)
+  uint16_t tap_off[MAX_TAPS + 1];    // offset of each tap's first pixel in the slab (16-byte units), phase by phase
+};
+struct DSmem {
+  int slab_bytes, a_bytes, lo_off;   // bytes TMA delivers, bytes of a stage, offset of the remainder copy (fp32)
+  int b_tile, b_lo, b_bytes, n_a, n_b;   // bytes of one tap's filter tile (hi part, and lo part for fp32), of a stage
+  int off_b, off_stage, off_bars, total;
+};
+
+template <typename T> struct OutWord {   // one 32-bit word of output: a 16-bit pair
+  static constexpr int COLS = 64;
+  static __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) { return Pair16<T>::max2(a, b); }
+};
+template <> struct OutWord<float> {
+  static constexpr int COLS = 32;
+  static __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) { return __float_as_uint(fmaxf(__uint_as_float(a), __uint_as_float(b))); }
+};
+
+// 8 (16-bit) or 4 (fp32) bias values from k on
+template <typename T> __device__ __forceinline__ void load_bias16(const T *bias, int k, int K, int vec, float *b) {
+  constexpr int V = 16 / (int)sizeof(T);
+  if (vec && k + V <= K) {
+    const uint4 q = *reinterpret_cast<const uint4 *>(bias + k);
+    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if constexpr (sizeof(T) == 4) b[i] = __uint_as_float(w[i]);
+      else { const float2 f = Pair16<T>::unpack(w[i]); b[2 * i] = f.x; b[2 * i + 1] = f.y; }
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < V; ++i) b[i] = k + i < K ? Elem<T>::load(bias + k + i) : 0.f;
+  }
+}
+
+struct Tile { int n0, od, oh0, ow0; bool valid; };
+template <int MB> __device__ __forceinline__ Tile decode(const DGeom &g, unsigned tile) {
+  Tile t;
+  t.valid = tile < (unsigned)g.n_tiles;
+  unsigned q = tile / (unsigned)g.n_wb;
+  t.ow0 = (int)(tile - q * (unsigned)g.n_wb) * 8;
+  unsigned r = q / (unsigned)g.n_hb;
+  t.oh0 = (int)(q - r * (unsigned)g.n_hb) * (MB * g.TH);
+  q = r / (unsigned)g.oD;
+  t.od = (int)(r - q * (unsigned)g.oD);
+  t.n0 = (int)q * g.TN;              // a tile past the end starts at an image past the end: TMA fills zeros
+  return t;
+}
+
+// Calls body(kd, p, ch, t0, t1) for the steps (depth tap, polyphase part, channel chunk) whose taps [t0, t1) fall into this
+// CTA's share [u0, u1) of the reduction, until it returns false; returns whether all of them ran.
+template <typename F> __device__ __forceinline__ bool for_steps(const DGeom &g, int u0, int u1, F &&body) {
+  int s0 = 0;
+  for (int kd = 0; kd < g.kD; ++kd)
+    for (int p = 0; p < g.n_ph; ++p) {
+      const int tp = g.taps[p];
+      for (int ch = 0; ch < g.n_chunks; ++ch, s0 += tp) {
+        const int t0 = max(0, u0 - s0), t1 = min(tp, u1 - s0);
+        if (t0 < t1 && !body(kd, p, ch, t0, t1)) return false;
+      }
+    }
+  return true;
+}
+
+template <typename T, int BN, int MB, bool PAIR>
+__global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
+    direct_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_u,
+                  const __grid_constant__ CUtensorMap map_y, T *__restrict__ y, const T *__restrict__ bias,
+                  const __grid_constant__ DGeom g, const __grid_constant__ DSmem sl, uint32_t idesc) {
+  constexpr bool F32 = std::is_same<T, float>::value;
+  constexpr int COLS = OutWord<T>::COLS;            // output columns of one 128-byte staging row
+  constexpr int ACC = MB * BN;                      // accumulator columns of a buffer
+  constexpr int N_ISSUE = MB >= 2 ? 2 : 1;
+  constexpr int BNH = PAIR ? BN / 2 : BN;           // filter rows this CTA loads
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw);
+  const uint32_t base = (raw + 1023u) & ~1023u;
+  uint8_t *base_ptr = smem_raw + (base - raw);
+  const uint32_t bars = base + sl.off_bars;         // a_full[8] a_empty[8] b_full[8] b_empty[8] a_split[8] acc_full[2] acc_empty[2]
+  auto a_full = [&](int i) { return bars + 8u * i; };
+  auto a_empty = [&](int i) { return bars + 64u + 8u * i; };
+  auto b_full = [&](int i) { return bars + 128u + 8u * i; };
+  auto b_empty = [&](int i) { return bars + 192u + 8u * i; };
+  auto a_split = [&](int i) { return bars + 256u + 8u * i; };
+  auto acc_full = [&](int i) { return bars + 320u + 8u * i; };
+  auto acc_empty = [&](int i) { return bars + 336u + 8u * i; };
+  volatile unsigned *abort_word = reinterpret_cast<volatile unsigned *>(base_ptr + sl.off_bars + 384);
+  const uint32_t tmem_slot = bars + 388u;
+  unsigned *err = &g_direct_error;
+
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // the warp index in a uniform register
+  if (threadIdx.x == 0) {
+    for (int i = 0; i < sl.n_a; ++i) { mbar_init(a_full(i), 1); mbar_init(a_empty(i), N_ISSUE); mbar_init(a_split(i), SPLIT_WARPS); }
+    for (int i = 0; i < sl.n_b; ++i) { mbar_init(b_full(i), 1); mbar_init(b_empty(i), N_ISSUE); }
+    for (int i = 0; i < 2; ++i) { mbar_init(acc_full(i), N_ISSUE); mbar_init(acc_empty(i), PAIR ? 2 * EPI_WARPS : EPI_WARPS); }
+    *abort_word = 0u;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    prefetch_map(&map_x); prefetch_map(&map_u); prefetch_map(&map_y);
+  }
+  const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
+  if (PAIR) { __syncthreads(); cluster_sync_all(); }
+  if (warp == 2) tmem_alloc<PAIR>(tmem_slot, 2 * ACC);
+  tc_fence_before();
+  __syncthreads();
+  if (PAIR) cluster_sync_all();
+  tc_fence_after();
+  uint32_t tmem;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot));
+  tmem = __shfl_sync(0xffffffffu, tmem, 0);
+  grid_launch_dependents();
+  grid_dependency_wait();
+
+  // work of this CTA: items item0, item0 + step, ... and the share [u0, u1) of each one's reduction
+  int item0, item_step, u0 = 0, u1 = g.units;
+  uint32_t part = 0;
+  if (PAIR) { item0 = (int)(blockIdx.x >> 1); item_step = (int)(gridDim.x >> 1); }
+  else if (g.split > 1) {
+    item0 = (int)blockIdx.x / g.split;
+    item_step = g.n_items;
+    part = (uint32_t)((int)blockIdx.x - item0 * g.split);
+    u0 = (int)((long long)g.units * part / g.split);
+    u1 = (int)((long long)g.units * (part + 1) / g.split);
+  } else { item0 = (int)blockIdx.x; item_step = (int)gridDim.x; }
+  // one channel block whose whole filter fits the ring: loaded once, its stages are never handed back
+  const bool resident = g.n_kb == 1 && g.split == 1 && g.kD * g.n_ph * g.n_chunks * ((g.taps[0] + g.G - 1) / g.G) <= sl.n_b;
+  bool alive = true;
+
+  if (warp == 0) {
+    // ---------------------------------------------------------------- slabs
+    int s = 0;
+    uint32_t ph = 1;
+    for (int item = item0; item < g.n_items && alive; item += item_step) {
+      const unsigned tb = (unsigned)item / (unsigned)g.n_kb;
+      const Tile t = decode<MB>(g, PAIR ? 2u * tb + rank : tb);
+      alive = for_steps(g, u0, u1, [&](int kd, int p, int ch, int t0, int t1) -> bool {
+        (void)t0; (void)t1;
+        if (!mbar_wait_warp(a_empty(s), ph, abort_word, err, ERR_A_EMPTY)) return false;
+        if (lane == 0) {
+          const uint32_t dst = base + (uint32_t)(s * sl.a_bytes);
+          const int cw = g.sW * t.ow0 + g.ph_w[p] - g.pW, chh = g.sH * t.oh0 + g.ph_h[p] - g.pH, cd = g.sD * t.od + kd - g.pD;
+          if (PAIR) {
+            if (rank == 0) mbar_expect_tx(a_full(s), 2u * (uint32_t)sl.slab_bytes);
+            tma_load_5d_pair(dst, &map_x, a_full(s), ch * g.ch_el, cw, t.n0, chh, cd);
+          } else {
+            mbar_expect_tx(a_full(s), (uint32_t)sl.slab_bytes);
+            tma_load_5d(dst, &map_x, a_full(s), ch * g.ch_el, cw, t.n0, chh, cd);
+          }
+        }
+        if (++s == sl.n_a) { s = 0; ph ^= 1u; }
+        return true;
+      });
+    }
+    if (*abort_word != 0u) {   // loads in flight must land before the shared memory goes away
+      const long long start = clock64();
+      while (clock64() - start < 2000000LL) { }
+    }
+  } else if (warp == 1) {
+    // ---------------------------------------------------------------- filter tiles
+    int s = 0;
+    uint32_t ph = 1;
+    for (int item = item0; item < g.n_items && alive; item += item_step) {
+      if (resident && item != item0) break;
+      const int kb = item - (int)((unsigned)item / (unsigned)g.n_kb) * g.n_kb;
+      const int row = kb * BN + (PAIR ? (int)rank * BNH : 0);
+      alive = for_steps(g, u0, u1, [&](int kd, int p, int ch, int t0, int t1) -> bool {
+        const int tap = kd * g.T_hw + g.tap0[p];
+        for (int t = t0; t < t1; t += g.G) {
+          if (!mbar_wait_warp(b_empty(s), ph, abort_word, err, ERR_B_EMPTY)) return false;
+          const int n = min(g.G, t1 - t);
+          if (lane == 0) {
+            const uint32_t bytes = (uint32_t)(n * sl.b_tile);
+            if (!PAIR || rank == 0) mbar_expect_tx(b_full(s), PAIR ? 2u * bytes : bytes);
+            uint32_t dst = base + (uint32_t)(sl.off_b + s * sl.b_bytes);
+            for (int j = 0; j < n; ++j, dst += (uint32_t)sl.b_tile) {
+              if (F32) {     // [tap][hi / lo][K][C]
+                tma_load_3d(dst, &map_u, b_full(s), ch * g.ch_el, row, 2 * (tap + t + j));
+                tma_load_3d(dst + (uint32_t)sl.b_lo, &map_u, b_full(s), ch * g.ch_el, row, 2 * (tap + t + j) + 1);
+              } else if (PAIR) {
+                tma_load_3d_pair(dst, &map_u, b_full(s), ch * g.ch_el, row, tap + t + j);
+              } else {
+                tma_load_3d(dst, &map_u, b_full(s), ch * g.ch_el, row, tap + t + j);
+              }
+            }
+          }
+          if (++s == sl.n_b) { s = 0; ph ^= 1u; }
+        }
+        return true;
+      });
+    }
+    if (*abort_word != 0u) {
+      const long long start = clock64();
+      while (clock64() - start < 2000000LL) { }
+    }
+  } else if (warp < 2 + N_ISSUE) {
+    // ---------------------------------------------------------------- MMA issue (rank 0 of a pair issues for both CTAs)
+    if (rank == 0) {
+      const int me = warp - 2;
+      int as = 0, bs = 0;
+      uint32_t a_ph = 0, b_ph = 0, n_done = 0;
+      for (int item = item0; item < g.n_items && alive; item += item_step, ++n_done) {
+        const int buf = (int)(n_done & 1u);
+        if (!mbar_wait_warp(acc_empty(buf), ((n_done >> 1) & 1u) ^ 1u, abort_word, err, ERR_ACC)) { alive = false; break; }
+        tc_fence_after();
+        const uint32_t d0 = tmem + (uint32_t)(buf * ACC + me * BN);
+        uint32_t acc = 0;
+        const bool loaded = resident && n_done > 0;
+        if (resident) { bs = 0; }
+        alive = for_steps(g, u0, u1, [&](int kd, int p, int ch, int t0, int t1) -> bool {
+          if (!mbar_wait_warp(F32 ? a_split(as) : a_full(as), a_ph, abort_word, err, ERR_A)) return false;
+          tc_fence_after();
+          const uint32_t a_lo = desc_lo(base + (uint32_t)(as * sl.a_bytes)) + (uint32_t)(me * g.mb_off16);
+          const int nk = ch == g.n_chunks - 1 ? g.k_tail : g.k_full;
+          const uint16_t *rows = g.tap_off + g.tap0[p];
+          for (int t = t0; t < t1; t += g.G) {
+            if (!loaded) {
+              if (!mbar_wait_warp(b_full(bs), b_ph, abort_word, err, ERR_B)) return false;
+              tc_fence_after();
+            }
+            const int n = min(g.G, t1 - t);
+            uint32_t b_lo = desc_lo(base + (uint32_t)(sl.off_b + bs * sl.b_bytes));
+            auto k_step = [&](uint32_t a_t, int k, uint32_t keep) {
+#pragma unroll
+              for (int mb = 0; mb < MB; mb += N_ISSUE) {   // blocks me, me + 2, ...
+                const uint32_t a_k = a_t + (uint32_t)(mb * g.mb_off16) + 2u * k, b_k = b_lo + 2u * k, d = d0 + (uint32_t)(mb * BN);
+                if (F32) {
+                  const uint32_t al = a_k + (uint32_t)(sl.lo_off >> 4), bl = b_k + (uint32_t)(sl.b_lo >> 4);
+                  umma<PAIR, F32>(d, al, g.a_hi, b_k, g.b_hi, idesc, keep);
+                  umma<PAIR, F32>(d, a_k, g.a_hi, bl, g.b_hi, idesc, 1u);
+                  umma<PAIR, F32>(d, a_k, g.a_hi, b_k, g.b_hi, idesc, 1u);
+                } else {
+                  umma<PAIR, F32>(d, a_k, g.a_hi, b_k, g.b_hi, idesc, keep);
+                }
+              }
+            };
+            if (elect_one()) {
+              if (nk == 4) {     // whole 128-byte rows: straight-line code, the offset of the next tap read ahead
+                uint32_t off = rows[t];
+                for (int j = 0; j < n; ++j, b_lo += (uint32_t)(sl.b_tile >> 4)) {
+                  const uint32_t a_t = a_lo + off;
+                  off = rows[t + j + 1];
+                  k_step(a_t, 0, acc); k_step(a_t, 1, 1u); k_step(a_t, 2, 1u); k_step(a_t, 3, 1u);
+                  acc = 1u;
+                }
+              } else {
+                for (int j = 0; j < n; ++j, b_lo += (uint32_t)(sl.b_tile >> 4)) {
+                  const uint32_t a_t = a_lo + rows[t + j];
+                  for (int k = 0; k < nk; ++k, acc = 1u) k_step(a_t, k, acc);
+                }
+              }
+            }
+            acc = 1u;
+            if (!resident && elect_one()) umma_commit<PAIR>(b_empty(bs));
+            if (++bs == sl.n_b) { bs = 0; b_ph ^= 1u; }
+          }
+          if (elect_one()) umma_commit<PAIR>(a_empty(as));
+          if (++as == sl.n_a) { as = 0; a_ph ^= 1u; }
+          return true;
+      });
+        if (resident) b_ph = 0;
+        if (elect_one()) umma_commit<PAIR>(acc_full(buf));
+      }
+    }
+  } else if (F32 && warp >= SPLIT_WARP0) {
+    // ---------------------------------------------------------------- fp32: slab -> tf32 part in place, remainder beside it
+    int s = 0;
+    uint32_t ph = 0;
+    const int st = threadIdx.x - SPLIT_WARP0 * 32;
+    for (int item = item0; item < g.n_items && alive; item += item_step) {
+      alive = for_steps(g, u0, u1, [&](int kd, int p, int ch, int t0, int t1) -> bool {
+        (void)kd; (void)p; (void)ch; (void)t0; (void)t1;
+        if (!mbar_wait_warp(a_full(s), ph, abort_word, err, ERR_SPLIT)) return false;
+        float4 *hi = reinterpret_cast<float4 *>(base_ptr + s * sl.a_bytes);
+        float4 *lo = reinterpret_cast<float4 *>(base_ptr + s * sl.a_bytes + sl.lo_off);
+#pragma unroll 4
+        for (int i = st; i < sl.slab_bytes / 16; i += SPLIT_WARPS * 32) {
+          const float4 v = hi[i];
+          float4 h;
+          h.x = tf32_round(v.x); h.y = tf32_round(v.y); h.z = tf32_round(v.z); h.w = tf32_round(v.w);
+          hi[i] = h;
+          lo[i] = make_float4(v.x - h.x, v.y - h.y, v.z - h.z, v.w - h.w);
+        }
+        fence_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(a_split(s));
+        if (++s == sl.n_a) { s = 0; ph ^= 1u; }
+        return true;
+      });
+    }
+  } else if (warp >= EPI_WARP0 && warp < EPI_WARP0 + EPI_WARPS && g.split == 1) {
+    // ---------------------------------------------------------------- epilogue
+    const int q = warp & 3, half = (warp - EPI_WARP0) >> 2;
+    const uint32_t stage = base + (uint32_t)(sl.off_stage + (warp - EPI_WARP0) * STAGE_BYTES);
+    const uint8_t *stage_ptr = base_ptr + sl.off_stage + (warp - EPI_WARP0) * STAGE_BYTES;
+    const bool relu = (g.epilogue & WINOCONV_EPI_RELU) != 0, has_bias = (g.epilogue & WINOCONV_EPI_BIAS) != 0;
+    const bool pool = (g.epilogue & WINOCONV_EPI_POOL2) != 0;
+    constexpr int CH_PER_MB = BN / COLS, N_CH = MB * CH_PER_MB;
+    const int tnm = g.TN - 1;
+    // this lane's pixel within the block, and the staging row its output goes to (-1: none)
+    const int grp = q * 4 + (lane >> 3), h_l = grp >> g.tn_shift, n_l = grp & tnm, w_l = lane & 7;
+    int srow = lane;
+    if (pool) srow = ((h_l | w_l) & 1) ? -1 : (g.TN == 1 ? ((lane >> 4) << 2) + (w_l >> 1) : (n_l << 2) + (w_l >> 1));
+    uint32_t n_done = 0;
+    for (int item = item0; item < g.n_items; item += item_step, ++n_done) {
+      const unsigned tb = (unsigned)item / (unsigned)g.n_kb;
+      const int kb = item - (int)tb * g.n_kb;
+      const Tile t = decode<MB>(g, PAIR ? 2u * tb + rank : tb);
+      const int buf = (int)(n_done & 1u);
+      if (!mbar_wait_warp(acc_full(buf), (n_done >> 1) & 1u, abort_word, err, ERR_EPI)) { alive = false; break; }
+      if (*abort_word != 0u) { alive = false; break; }
+      tc_fence_after();
+      bool handed = false;
+#pragma unroll 1
+      for (int ci = half; ci < N_CH; ci += 2) {
+        const int mb = ci / CH_PER_MB, c0 = (ci - mb * CH_PER_MB) * COLS;
+        const int k0 = kb * BN + c0;
+        const int oh_b = t.oh0 + mb * g.TH;
+        const bool wanted = k0 < g.K && t.valid && oh_b < g.oH;
+        uint32_t r[COLS];
+        if (wanted) {
+          const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * ACC + mb * BN + c0);
+          tmem_ld_x32(ta, r);
+          if (COLS == 64) tmem_ld_x32(ta + 32u, r + 32 % COLS);
+          tmem_wait_ld_x32(r);
+          if (COLS == 64) tmem_wait_ld_x32(r + 32 % COLS);
+        }
+        if (ci + 2 >= N_CH) {      // this warp's last columns are in registers: its share of the hand-back
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) { if (PAIR) mbar_arrive_rank0(acc_empty(buf)); else mbar_arrive(acc_empty(buf)); }
+          handed = true;
+        }
+        if (!wanted) continue;
+        uint32_t o[32];
+#pragma unroll
+        for (int v = 0; v < 8; ++v) {          // one 16-byte vector of output
+          constexpr int V = 16 / (int)sizeof(T);
+          float f[V], b[V];
+#pragma unroll
+          for (int i = 0; i < V; ++i) f[i] = __uint_as_float(r[v * V + i]);
+          if (has_bias) {
+            load_bias16<T>(bias, k0 + v * V, g.K, g.bias_vec, b);
+#pragma unroll
+            for (int i = 0; i < V; ++i) f[i] += b[i];
+          }
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            if constexpr (F32) o[v * 4 + i] = __float_as_uint(f[i]);
+            else o[v * 4 + i] = Pair16<T>::round(f[2 * i], f[2 * i + 1]);
+          }
+        }
+        if (pool) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) {
+            o[i] = OutWord<T>::max2(o[i], __shfl_xor_sync(0xffffffffu, o[i], 1));
+            o[i] = OutWord<T>::max2(o[i], __shfl_xor_sync(0xffffffffu, o[i], 8 << g.tn_shift));
+          }
+        }
+        if (relu) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) o[i] = OutWord<T>::max2(o[i], 0u);
+        }
+        if (lane == 0) bulk_wait_read();       // the previous store has read the staging rows
+        __syncwarp();
+        if (srow >= 0) {
+          const uint32_t dst = stage + (uint32_t)srow * 128u;
+#pragma unroll
+          for (int v = 0; v < 8; ++v)
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (uint32_t)((v ^ (srow & 7)) << 4)), "r"(o[4 * v]),
+                         "r"(o[4 * v + 1]), "r"(o[4 * v + 2]), "r"(o[4 * v + 3]) : "memory");
+        }
+        // first pixel of this warp's rows
+        const int g0 = q * 4, h0 = g0 >> g.tn_shift, n0 = g0 & tnm;
+        if (g.y_tma) {
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0 && (pool ? (oh_b + h0) >> 1 : oh_b + h0) < g.yH && t.n0 + n0 < g.N && (pool ? t.ow0 >> 1 : t.ow0) < g.yW) {
+            if (pool) tma_store_5d(&map_y, stage, k0, t.ow0 >> 1, t.n0 + n0, (oh_b + h0) >> 1, t.od);
+            else tma_store_5d(&map_y, stage, k0, t.ow0, t.n0 + n0, oh_b + h0, t.od);
+            bulk_commit();
+          }
+        } else {            // rows of y are not 16-byte aligned: a row of the staging tile per step, consecutive lanes, consecutive channels
+          __syncwarp();
+          constexpr int E = 4 / (int)sizeof(T);
+          const int rows_out = pool ? 8 : 32;
+          for (int rr = 0; rr < rows_out; ++rr) {
+            int oh, ow, n;
+            if (pool) {
+              const int a = rr >> 2;
+              ow = (t.ow0 >> 1) + (rr & 3);
+              oh = ((oh_b + h0) >> 1) + (g.TN == 1 ? a : 0);
+              n = t.n0 + (g.TN == 1 ? 0 : a);
+            } else {
+              const int gg = g0 + (rr >> 3);
+              oh = oh_b + (gg >> g.tn_shift); n = t.n0 + (gg & tnm); ow = t.ow0 + (rr & 7);
+            }
+            if (oh >= g.yH || ow >= g.yW || n >= g.N) continue;
+            const T *src = reinterpret_cast<const T *>(stage_ptr + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) + (lane & 3) * 4);
+            T *dst = y + ((((long long)n * g.oD + t.od) * g.yH + oh) * g.yW + ow) * g.K + k0 + lane * E;
+#pragma unroll
+            for (int e = 0; e < E; ++e)
+              if (k0 + lane * E + e < g.K) dst[e] = src[e];
+          }
+          __syncwarp();
+        }
+      }
+      if (!handed && lane == 0) { if (PAIR) mbar_arrive_rank0(acc_empty(buf)); else mbar_arrive(acc_empty(buf)); }
+    }
+    if (lane == 0) bulk_wait_all();
+  }
+  if (!PAIR && g.split > 1) {
+    // ---------------------------------------------------------------- the cluster's shares of one item added up
+    // Every CTA puts its accumulator into its own shared memory (the operand rings are idle by then) and finishes 1 / split
+    // of the rows from all of them.
+    constexpr int ROW_F = BN + 4;                  // floats per row: 16-byte accesses of neighbouring rows hit other banks
+    const bool epi = warp >= EPI_WARP0 && warp < EPI_WARP0 + EPI_WARPS;
+    __syncthreads();
+    if (epi && item0 < g.n_items) {
+      const int q = warp & 3, half = (warp - EPI_WARP0) >> 2;
+      if (mbar_wait_warp(acc_full(0), 0u, abort_word, err, ERR_EPI)) {
+        tc_fence_after();
+        for (int c0 = half * 32; c0 < ACC; c0 += 64) {
+          uint32_t r[32];
+          tmem_ld_x32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
+          tmem_wait_ld_x32(r);
+          const int mb = c0 / BN;
+          float4 *dst = reinterpret_cast<float4 *>(base_ptr) + ((mb * BM + q * 32 + lane) * ROW_F + (c0 - mb * BN)) / 4;
+#pragma unroll
+          for (int v = 0; v < 8; ++v)
+            dst[v] = make_float4(__uint_as_float(r[4 * v]), __uint_as_float(r[4 * v + 1]), __uint_as_float(r[4 * v + 2]), __uint_as_float(r[4 * v + 3]));
+        }
+        tc_fence_before();
+      }
+    }
+    cluster_sync_all();
+    if (epi && *abort_word == 0u) {
+      const unsigned tb = (unsigned)item0 / (unsigned)g.n_kb;
+      const int kb = item0 - (int)tb * g.n_kb;
+      const Tile t = decode<MB>(g, tb);
+      const bool relu = (g.epilogue & WINOCONV_EPI_RELU) != 0, has_bias = (g.epilogue & WINOCONV_EPI_BIAS) != 0;
+      const bool pool = (g.epilogue & WINOCONV_EPI_POOL2) != 0;
+      constexpr int V = 16 / (int)sizeof(T);       // outputs of one 16-byte vector
+      const int rows = MB * BM / g.split, tid = threadIdx.x - EPI_WARP0 * 32;
+      const int work = (pool ? rows / 4 : rows) * (BN / V);
+      for (int i = tid; i < work; i += EPI_WARPS * 32) {
+        const int rr = i / (BN / V), c = (i - rr * (BN / V)) * V;
+        const int k = kb * BN + c;
+        if (k >= g.K) continue;
+        float best[V];
+        int oh = 0, ow = 0, n = 0;
+        const int n_src = pool ? 4 : 1;
+        for (int a = 0; a < n_src; ++a) {
+          int row = (int)part * rows;
+          if (pool) {    // pooled pixel rr: image, row pair and column pair within this CTA's rows
+            const int wp = rr & 3, np = (rr >> 2) & (g.TN - 1), hp = rr >> (2 + g.tn_shift);
+            row += (((2 * hp + (a >> 1)) << g.tn_shift) + np) * 8 + 2 * wp + (a & 1);
+          } else row += rr;
+          float f[V];
+#pragma unroll
+          for (int v = 0; v < V; ++v) f[v] = 0.f;
+          const uint32_t src = base + (uint32_t)((row * ROW_F + c) * 4);
+          for (int pr = 0; pr < g.split; ++pr) {
+            const uint32_t rs = map_to_rank(src, (uint32_t)pr);
+#pragma unroll
+            for (int v = 0; v < V; v += 4) {
+              const float4 u = ld_cluster_f4(rs + v * 4);
+              f[v] += u.x; f[v + 1] += u.y; f[v + 2] += u.z; f[v + 3] += u.w;
+            }
+          }
+          if (a == 0) {
+            const int mb = row >> 7, grp = (row & 127) >> 3;
+            oh = t.oh0 + mb * g.TH + (grp >> g.tn_shift); n = t.n0 + (grp & (g.TN - 1)); ow = t.ow0 + (row & 7);
+          }
+#pragma unroll
+          for (int v = 0; v < V; ++v) best[v] = a == 0 ? f[v] : fmaxf(best[v], f[v]);
+        }
+        if (pool) { oh >>= 1; ow >>= 1; }
+        if (oh >= g.yH || ow >= g.yW || n >= g.N) continue;
+        if (has_bias) {
+          float b[V];
+          load_bias16<T>(bias, k, g.K, g.bias_vec, b);
+#pragma unroll
+          for (int v = 0; v < V; ++v) best[v] += b[v];
+        }
+        uint32_t o[4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          if constexpr (F32) o[v] = __float_as_uint(best[v]);
+          else o[v] = Pair16<T>::round(best[2 * v], best[2 * v + 1]);
+          if (relu) o[v] = OutWord<T>::max2(o[v], 0u);
+        }
+        T *dst = y + ((((long long)n * g.oD + t.od) * g.yH + oh) * g.yW + ow) * g.K + k;
+        if (g.y_tma) *reinterpret_cast<uint4 *>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+        else {
+#pragma unroll
+          for (int v = 0; v < V; ++v)
+            if (k + v < g.K) {
+              if constexpr (F32) dst[v] = __uint_as_float(o[v]);
+              else *reinterpret_cast<unsigned short *>(dst + v) = (unsigned short)(o[v >> 1] >> ((v & 1) * 16));
+            }
+        }
+      }
+    }
+    cluster_sync_all();      // no CTA leaves while another reads its shared memory
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (PAIR) cluster_sync_all();
+  if (warp == 2) {
+    tc_fence_after();
+    tmem_free<PAIR>(tmem, 2 * ACC);
+  }
+}
+
+// U[tap][o][i] = w[o, i, tap] in the order the kernel walks the taps, rounded once to T; fp32 as [tap][tf32 part, remainder][o][i].
+// The weights are read through strides, so a data gradient's filter (channels exchanged, taps mirrored) is the same kernel.
+struct FGeomD {
+  int O, I, Ip, kD, n_hw;
+  long long s_o, s_i, s_d;
+  int off_hw[MAX_TAPS];       // element offset of each (h, w) tap in walking order
+};
+template <typename TW, typename T>
+__global__ void __launch_bounds__(256) direct_filter_kernel(const TW *__restrict__ w, T *__restrict__ u, const __grid_constant__ FGeomD f) {
+  const unsigned idx = blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned total = (unsigned)f.O * (unsigned)f.Ip;
+  if (idx >= total) return;
+  const int o = (int)(idx / (unsigned)f.Ip), i = (int)(idx - (unsigned)o * (unsigned)f.Ip);
+  const TW *src = w + o * f.s_o + i * f.s_i;
+  const bool real = i < f.I;
+  const int kd = blockIdx.y;
+  for (int t = blockIdx.z; t < f.n_hw; t += gridDim.z) {
+    const float v = real ? Elem<TW>::load(src + kd * f.s_d + f.off_hw[t]) : 0.f;
+    const long long tap = (long long)kd * f.n_hw + t;
+    if constexpr (std::is_same<T, float>::value) {
+      const float h = tf32_round(v);
+      u[2 * tap * total + idx] = h;
+      u[(2 * tap + 1) * total + idx] = v - h;
+    } else {
+      Elem<T>::store(u + tap * total + idx, v);
+    }
+  }
+}
+
+static int sm_count_of_current_device() {
+  static std::mutex mu;
+  static std::map<int, int> cache;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+  std::lock_guard<std::mutex> lock(mu);
+  auto f = cache.find(dev);
+  if (f != cache.end()) return f->second;
+  int n = 0;
+  if (cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) n = 0;
+  return cache[dev] = n;
+}
+
+}  // namespace dconv
+
+using namespace dconv;
+
+// Estimated clocks of a launch with this configuration on 148 SMs, from the per-instruction clocks of the rate probe (an
+// instruction of N columns: 48 / 65 / 129 clocks for N = 64 / 128 / 256) and 128 B of shared memory per clock.
+static double estimate(const DirectPlan &p, double k_steps, int n_steps, int tiles, int n_kb, bool f32) {
+  const double t_mma = p.BN == 256 ? 129 : p.BN == 128 ? 65 : 48;
+  const double mma = k_steps * p.MB * t_mma * (f32 ? 3 : 1);
+  const double bytes = k_steps * p.MB * (f32 ? 3 : 1) * (4096.0 + (p.pair ? p.BN / 2 : p.BN) * 32.0) +
+                       n_steps * (double)p.slab_bytes * (f32 ? 4 : 1) + k_steps * (p.pair ? p.BN / 2 : p.BN) * 32.0 * (f32 ? 2 : 1);
+  const double item = std::max(mma, bytes / 128.0);
+  const int slots = p.pair ? 74 : 148 / p.split;
+  const int items = (p.pair ? (tiles + 1) / 2 : tiles) * n_kb;
+  const double waves = (items + slots - 1) / slots;
+  const double epi = 400.0 + 350.0 * p.MB * p.BN / 64;
+  const double fill = 3000.0;
+  if (p.split > 1) return fill + waves * (item / p.split + 3000.0 + (waves > 1 ? fill : 0.0));
+  return fill + waves * std::max(item + 200.0, epi) + epi;
+}
+
+bool direct_plan(const DirectDesc &d, DirectPlan *out) {
+  const bool f32 = d.dtype == WINOCONV_F32;
+  const int esz = f32 ? 4 : 2, vec = 16 / esz;
+  if (d.C % vec != 0) return false;
+  if (d.sH > 2 || d.sW > 2 || d.sD > 2 || d.kH * d.kW > MAX_TAPS || d.pH > 64 || d.pW > 64) return false;
+  const bool pool = (d.epilogue & WINOCONV_EPI_POOL2) != 0;
+  DirectPlan p;
+  std::memset(&p, 0, sizeof p);
+  // channels per slab row: 128-byte rows, or 64 / 32-byte rows where the channels fit them
+  const int cap = 128 / esz;
+  p.ch_el = d.C > cap / 2 ? cap : d.C > cap / 4 ? cap / 2 : cap / 4;
+  p.rb = p.ch_el * esz;
+  p.n_chunks = (d.C + p.ch_el - 1) / p.ch_el;
+  const int k_el = 32 / esz;                 // channels of one MMA K step
+  p.k_full = p.ch_el / k_el;
+  p.k_tail = (d.C - (p.n_chunks - 1) * p.ch_el + k_el - 1) / k_el;
+  // polyphase parts along H and W and their taps
+  const int Th = (d.kH + d.sH - 1) / d.sH, Tw = (d.kW + d.sW - 1) / d.sW;   // of part 0, the largest
+  p.PW = 8 + Tw - 1;
+  int n_taps = 0;
+  for (int a = 0; a < d.sH; ++a)
+    for (int b = 0; b < d.sW; ++b) {
+      const int th = (d.kH - a + d.sH - 1) / d.sH, tw = (d.kW - b + d.sW - 1) / d.sW;
+      if (th <= 0 || tw <= 0) continue;
+      p.ph_h[p.n_ph] = a; p.ph_w[p.n_ph] = b; p.ph_tw[p.n_ph] = tw;
+      p.taps[p.n_ph] = th * tw; p.tap0[p.n_ph] = n_taps;
+      n_taps += th * tw;
+      ++p.n_ph;
+    }
+  p.n_taps = n_taps;
+  p.filter_elems = (long long)d.kD * n_taps * d.K * d.C * (f32 ? 2 : 1);
+  p.units = d.kD * n_taps * p.n_chunks;
+  const double k_steps = (double)d.kD * n_taps * ((p.n_chunks - 1) * p.k_full + p.k_tail);
+  const int n_steps = d.kD * p.n_ph * p.n_chunks;
+  const int budget = 227 * 1024 - 2048 - BAR_BYTES - EPI_WARPS * STAGE_BYTES;
+
+  struct Cfg { int BN, MB, pair; };
+  static const Cfg cfgs16[] = {{256, 1, 1}, {128, 2, 1}, {128, 1, 1}, {64, 2, 1}, {128, 1, 0}, {64, 1, 0}, {64, 2, 0}};
+  static const Cfg cfgs32[] = {{128, 1, 0}, {64, 1, 0}};
+  const Cfg *cfgs = f32 ? cfgs32 : cfgs16;
+  const int n_cfgs = f32 ? 2 : 7;
+  const int force = [] { const char *v = getenv("WINOCONV_DIRECT_CFG"); return v && *v ? atoi(v) : -1; }();
+  const int force_split = [] { const char *v = getenv("WINOCONV_DIRECT_SPLIT"); return v && *v ? atoi(v) : 0; }();
+  double best = 1e30;
+  bool found = false;
+  for (int ci = 0; ci < n_cfgs; ++ci) {
+    const Cfg &c = cfgs[ci];
+    if (!f32 && force >= 0 && force != ci) continue;
+    if (c.BN > 64 && d.K <= c.BN / 2 && force < 0) continue;
+    const int n_kb = (d.K + c.BN - 1) / c.BN;
+    for (int tn = 1; tn <= 16; tn *= 2) {
+      if (pool && tn > 2) break;
+      if (tn > 1 && tn / 2 >= d.N) break;
+      DirectPlan q = p;
+      q.BN = c.BN; q.MB = c.MB; q.pair = c.pair; q.TN = tn; q.TH = 16 / tn;
+      const int rows_h = c.MB * q.TH + Th - 1;
+      if (q.PW * d.sW > 256 || rows_h * d.sH > 256) continue;
+      q.slab_rows_h = rows_h;
+      q.slab_bytes = rows_h * tn * q.PW * q.rb;
+      const int a1 = (q.slab_bytes + 1023) / 1024 * 1024;
+      q.a_bytes = f32 ? 2 * a1 : a1;
+      q.lo_off = a1;
+      q.b_lo = (c.pair ? c.BN / 2 : c.BN) * q.rb;
+      q.b_tile = q.b_lo * (f32 ? 2 : 1);
+      q.n_wb = (d.oW + 7) / 8; q.n_hb = (d.oH + c.MB * q.TH - 1) / (c.MB * q.TH);
+      const long long tiles = (long long)q.n_wb * q.n_hb * d.oD * ((d.N + tn - 1) / tn);
+      if (tiles * n_kb > 0x3fffffffLL) continue;
+      q.n_tiles = (int)tiles; q.n_kb = n_kb;
+      q.n_items = (int)((c.pair ? (tiles + 1) / 2 : tiles) * n_kb);
+      // taps per filter stage: enough that a stage is worth its barrier round trip
+      int G = std::max(1, std::min(p.taps[0], 24 * 1024 / q.b_tile));
+      q.n_a = 0;
+      for (; G >= 1; --G) {
+        q.G = G;
+        q.b_bytes = (G * q.b_tile + 1023) / 1024 * 1024;
+        int na = 2, nb = 2;
+        const double groups = (p.taps[0] + G - 1) / G;
+        if (2 * q.a_bytes + 2 * q.b_bytes > budget) {
+          na = 1;
+          if (q.a_bytes + 2 * q.b_bytes > budget) continue;
+        }
+        // deepen whichever ring looks less far ahead
+        for (bool grew = true; grew;) {
+          grew = false;
+          const bool want_b = nb / groups <= na;
+          for (int turn = 0; turn < 2 && !grew; ++turn) {
+            const bool b = turn == 0 ? want_b : !want_b;
+            if (b && nb < 8 && na * q.a_bytes + (nb + 1) * q.b_bytes <= budget) { ++nb; grew = true; }
+            if (!b && na < 8 && (na + 1) * q.a_bytes + nb * q.b_bytes <= budget) { ++na; grew = true; }
+          }
+        }
+        q.n_a = na; q.n_b = nb;
+        break;
+      }
+      if (q.n_a == 0) continue;
+      for (int split = 1; split <= 8; split *= 2) {
+        if (split > 1 && (c.pair || q.n_items * split > 148 || split > q.units)) break;
+        if (split > 1 && pool && c.MB * BM / split < 16 * tn) break;
+        if (split > 1 && c.MB * BM * (c.BN + 4) * 4 > q.n_a * q.a_bytes + q.n_b * q.b_bytes) break;
+        if (force_split > 0 && split != force_split && !c.pair) continue;
+        q.split = split;
+        const double e = estimate(q, k_steps, n_steps, q.n_tiles, n_kb, f32);
+        if (e < best) { best = e; *out = q; found = true; }
+      }
+    }
+  }
+  if (!found) return false;
+  if (getenv("WINOCONV_DIRECT_DEBUG")) fprintf(stderr, "[direct] BN%d MB%d pair%d split%d TN%d tiles%d items%d na%d nb%d G%d slab%d est %.1f us\n", out->BN, out->MB, out->pair, out->split, out->TN, out->n_tiles, out->n_items, out->n_a, out->n_b, out->G, out->slab_bytes, best/1.9e3);
+  out->estimate = best;
+  out->smem = 1024 + out->n_a * out->a_bytes + out->n_b * out->b_bytes + EPI_WARPS * STAGE_BYTES + BAR_BYTES;
+  return true;
+}
+
+cudaError_t launch_direct_filter_transform(const DirectDesc &d, const DirectPlan &p, int w_dtype, const void *w, void *u, cudaStream_t s) {
+  FGeomD f;
+  std::memset(&f, 0, sizeof f);
+  f.O = d.K; f.I = d.C; f.Ip = d.C; f.kD = d.kD; f.n_hw = p.n_taps;
+  const bool kcrs = d.weight_layout == WINOCONV_W_KCRS;
+  const long long hw = (long long)d.kH * d.kW;
+  const long long tap_stride = kcrs ? 1 : (long long)d.C * d.K;
+  f.s_o = kcrs ? d.C * d.kD * hw : 1;
+  f.s_i = kcrs ? d.kD * hw : d.K;
+  f.s_d = hw * tap_stride;
+  for (int q = 0; q < p.n_ph; ++q)
+    for (int t = 0; t < p.taps[q]; ++t) {
+      const int th = t / p.ph_tw[q], tw = t - th * p.ph_tw[q];
+      f.off_hw[p.tap0[q] + t] = (int)(((d.sH * th + p.ph_h[q]) * d.kW + d.sW * tw + p.ph_w[q]) * tap_stride);
+    }
+  const unsigned blocks = (unsigned)(((long long)f.O * f.Ip + 255) / 256);
+  const dim3 grid(blocks, d.kD, blocks >= 296 ? 1 : std::min(p.n_taps, (int)(592 / blocks) + 1));
+#define WINO_FILT(TW, T) direct_filter_kernel<TW, T><<<grid, 256, 0, s>>>((const TW *)w, (T *)u, f)
+  if (d.dtype == WINOCONV_F32) WINO_FILT(float, float);
+  else if (d.dtype == WINOCONV_F16) { if (w_dtype == WINOCONV_F32) WINO_FILT(float, __half); else WINO_FILT(__half, __half); }
+  else { if (w_dtype == WINOCONV_F32) WINO_FILT(float, __nv_bfloat16); else WINO_FILT(__nv_bfloat16, __nv_bfloat16); }
+#undef WINO_FILT
+  return cudaGetLastError();
+}
+
+template <typename T, int BN, int MB, bool PAIR>
+static cudaError_t launch_one(const DirectPlan &p, const CUtensorMap &mx, const CUtensorMap &mu, const CUtensorMap &my, void *y,
+                              const void *bias, const DGeom &g, const DSmem &sl, uint32_t idesc, int sms, cudaStream_t s) {
+  auto kern = direct_kernel<T, BN, MB, PAIR>;
+  static std::mutex mu_;
+  static std::map<int, int> pairs_of;     // device -> resident CTA pairs (0: attribute set, not asked)
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.blockDim = dim3(std::is_same<T, float>::value ? 512 : 384, 1, 1);
+  cfg.dynamicSmemBytes = (size_t)p.smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = PAIR ? 2 : (unsigned)p.split; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = (PAIR || p.split > 1) ? 2 : 1;
+  int pairs = 0;
+  {
+    std::lock_guard<std::mutex> lock(mu_);
+    auto f = pairs_of.find(dev);
+    if (f == pairs_of.end()) {
+      e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024);
+      if (e != cudaSuccess) return e;
+      f = pairs_of.emplace(dev, 0).first;
+      if (PAIR) {
+        cfg.gridDim = dim3(2, 1, 1);
+        cfg.dynamicSmemBytes = 227 * 1024;
+        if (cudaOccupancyMaxActiveClusters(&f->second, kern, &cfg) != cudaSuccess || f->second <= 0) f->second = sms / 2;
+        cfg.dynamicSmemBytes = (size_t)p.smem;
+      }
+    }
+    pairs = f->second;
+  }
+  if (PAIR) cfg.gridDim = dim3((unsigned)(2 * std::min(p.n_items, std::min(pairs, sms / 2))), 1, 1);
+  else if (p.split > 1) cfg.gridDim = dim3((unsigned)(p.n_items * p.split), 1, 1);
+  else cfg.gridDim = dim3((unsigned)std::min(p.n_items, sms), 1, 1);
+  return cudaLaunchKernelEx(&cfg, kern, mx, mu, my, (T *)y, (const T *)bias, g, sl, idesc);
+}
+
+cudaError_t launch_direct_forward(const DirectDesc &d, const DirectPlan &p, const void *x, const void *u, const void *bias, void *y,
+                                  cudaStream_t s, const char **detail) {
+  *detail = "";
+  EncodeTiledFn enc = encode_tiled_fn();
+  if (!enc) { *detail = "cuTensorMapEncodeTiled unavailable"; return cudaErrorNotSupported; }
+  const bool f32 = d.dtype == WINOCONV_F32, pool = (d.epilogue & WINOCONV_EPI_POOL2) != 0;
+  const cuuint64_t esz = f32 ? 4 : 2;
+  const CUtensorMapDataType dt = map_dtype(d.dtype);
+  const CUtensorMapSwizzle swz = p.rb == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : p.rb == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
+  const uint32_t swz_code = p.rb == 128 ? 2u : p.rb == 64 ? 4u : 6u;
+  CUtensorMap mx, mu, my;
+  {   // x as [D][H][N][W][C]: a slab is rows x images x pixels x channels; H and W walked with the layer's stride
+    const cuuint64_t dims[5] = {(cuuint64_t)d.C, (cuuint64_t)d.W, (cuuint64_t)d.N, (cuuint64_t)d.H, (cuuint64_t)d.D};
+    const cuuint64_t w_ = (cuuint64_t)d.C * esz, h_ = w_ * d.W, d_ = h_ * d.H, n_ = d_ * d.D;
+    const cuuint64_t st[4] = {w_, n_, h_, d_};
+    const cuuint32_t box[5] = {(cuuint32_t)p.ch_el, (cuuint32_t)(p.PW * d.sW), (cuuint32_t)p.TN, (cuuint32_t)(p.slab_rows_h * d.sH), 1u};
+    const cuuint32_t es[5] = {1u, (cuuint32_t)d.sW, 1u, (cuuint32_t)d.sH, 1u};
+    if (enc(&mx, dt, 5, const_cast<void *>(x), dims, st, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) { *detail = "cuTensorMapEncodeTiled failed for the input"; return cudaErrorInvalidValue; }
+  }
+  {   // filter tiles [tap][K][C] (fp32: two per tap)
+    const cuuint64_t dims[3] = {(cuuint64_t)d.C, (cuuint64_t)d.K, (cuuint64_t)d.kD * p.n_taps * (f32 ? 2 : 1)};
+    const cuuint64_t st[2] = {(cuuint64_t)d.C * esz, (cuuint64_t)d.C * esz * d.K};
+    const cuuint32_t box[3] = {(cuuint32_t)p.ch_el, (cuuint32_t)(p.pair ? p.BN / 2 : p.BN), 1u};
+    const cuuint32_t es[3] = {1u, 1u, 1u};
+    if (enc(&mu, dt, 3, const_cast<void *>(u), dims, st, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) { *detail = "cuTensorMapEncodeTiled failed for the filter"; return cudaErrorInvalidValue; }
+  }
+  const bool y_tma = ((cuuint64_t)d.K * esz) % 16 == 0;
+  if (y_tma) {   // one epilogue warp's 32 pixels (8 when pooled) x 128 bytes of channels
+    const cuuint64_t dims[5] = {(cuuint64_t)d.K, (cuuint64_t)d.yW, (cuuint64_t)d.N, (cuuint64_t)d.yH, (cuuint64_t)d.oD};
+    const cuuint64_t w_ = (cuuint64_t)d.K * esz, h_ = w_ * d.yW, d_ = h_ * d.yH, n_ = d_ * d.oD;
+    const cuuint64_t st[4] = {w_, n_, h_, d_};
+    const cuuint32_t sn = (cuuint32_t)std::min(p.TN, 4), sh = 4u / sn;
+    const cuuint32_t box[5] = {(cuuint32_t)(128 / esz), pool ? 4u : 8u, sn, pool ? sh / 2 : sh, 1u};
+    const cuuint32_t es[5] = {1u, 1u, 1u, 1u, 1u};
+    if (enc(&my, dt, 5, y, dims, st, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) { *detail = "cuTensorMapEncodeTiled failed for the output"; return cudaErrorInvalidValue; }
+  } else my = mx;
+  DGeom g;
+  std::memset(&g, 0, sizeof g);
+  g.N = d.N; g.K = d.K; g.oD = d.oD; g.oH = d.oH; g.oW = d.oW; g.yH = d.yH; g.yW = d.yW;
+  g.sD = d.sD; g.sH = d.sH; g.sW = d.sW; g.pD = d.pD; g.pH = d.pH; g.pW = d.pW; g.kD = d.kD;
+  g.TN = p.TN; g.TH = p.TH; g.PW = p.PW;
+  while ((1 << g.tn_shift) < p.TN) ++g.tn_shift;
+  g.n_wb = p.n_wb; g.n_hb = p.n_hb; g.n_tiles = p.n_tiles; g.n_kb = p.n_kb; g.n_items = p.n_items;
+  g.n_ph = p.n_ph; g.T_hw = p.n_taps;
+  for (int q = 0; q < p.n_ph; ++q) {
+    g.ph_h[q] = p.ph_h[q]; g.ph_w[q] = p.ph_w[q]; g.taps[q] = p.taps[q]; g.tap0[q] = p.tap0[q];
+    for (int t = 0; t < p.taps[q]; ++t) {
+      const int th = t / p.ph_tw[q], tw = t - th * p.ph_tw[q];
+      g.tap_off[p.tap0[q] + t] = (uint16_t)((th * p.TN * p.PW + tw) * (p.rb / 16));
+    }
+  }
+  g.n_chunks = p.n_chunks; g.ch_el = p.ch_el; g.k_full = p.k_full; g.k_tail = p.k_tail; g.units = p.units;
+  g.G = p.G; g.split = p.split; g.epilogue = d.epilogue;
+  g.y_tma = y_tma; g.bias_vec = y_tma && (reinterpret_cast<uintptr_t>(bias) & 15u) == 0;
+  g.a_hi = desc_hi((uint32_t)(p.PW * p.rb), swz_code);
+  g.b_hi = desc_hi((uint32_t)(8 * p.rb), swz_code);
+  g.mb_off16 = p.TH * p.TN * p.PW * p.rb / 16;
+  DSmem sl;
+  sl.slab_bytes = p.slab_bytes; sl.a_bytes = p.a_bytes; sl.lo_off = p.lo_off;
+  sl.b_tile = p.b_tile; sl.b_lo = p.b_lo; sl.b_bytes = p.b_bytes; sl.n_a = p.n_a; sl.n_b = p.n_b;
+  sl.off_b = p.n_a * p.a_bytes; sl.off_stage = sl.off_b + p.n_b * p.b_bytes;
+  sl.off_bars = sl.off_stage + EPI_WARPS * STAGE_BYTES; sl.total = p.smem;
+  const int sms = sm_count_of_current_device();
+  if (sms <= 0) { *detail = "no device"; return cudaErrorNoDevice; }
+  const uint32_t fmt = f32 ? 2u : d.dtype == WINOCONV_F16 ? 0u : 1u;
+  const uint32_t m_rows = p.pair ? 2u * BM : (uint32_t)BM;
+  const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.BN >> 3) << 17) | ((m_rows >> 4) << 24);
+#define WINO_GO(T, BN_, MB_, P_) return launch_one<T, BN_, MB_, P_>(p, mx, mu, my, y, bias, g, sl, idesc, sms, s)
+#define WINO_PICK(T)                                                             \
+  do {                                                                           \
+    if (p.pair) {                                                                \
+      if (p.BN == 256) WINO_GO(T, 256, 1, true);                                 \
+      if (p.BN == 128) { if (p.MB == 2) WINO_GO(T, 128, 2, true); WINO_GO(T, 128, 1, true); } \
+      WINO_GO(T, 64, 2, true);                                                   \
+    }                                                                            \
+    if (p.BN == 128) WINO_GO(T, 128, 1, false);                                  \
+    if (p.MB == 2) WINO_GO(T, 64, 2, false);                                     \
+    WINO_GO(T, 64, 1, false);                                                    \
+  } while (0)
+  if (d.dtype == WINOCONV_F16) WINO_PICK(__half);
+  if (d.dtype == WINOCONV_BF16) WINO_PICK(__nv_bfloat16);
+  if (p.BN == 128) WINO_GO(float, 128, 1, false);
+  WINO_GO(float, 64, 1, false);
+#undef WINO_PICK
+#undef WINO_GO
+}
+
+cudaError_t read_and_clear_direct_error(cudaStream_t s, unsigned int *code) {
+  unsigned int host = 0, zero = 0;
+  cudaError_t e = cudaMemcpyFromSymbolAsync(&host, g_direct_error, sizeof(host), 0, cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaMemcpyToSymbolAsync(g_direct_error, &zero, sizeof(zero), 0, cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  *code = host;
+  return e;
+}
+
+}  // namespace wino

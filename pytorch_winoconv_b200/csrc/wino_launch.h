@@ -77,6 +77,29 @@ cudaError_t launch_rowfused_forward(const RowDesc &d, const RowPlan &p, int dtyp
                                     const void *bias, void *y, void *pad_ws, cudaStream_t s, const char **detail);
 cudaError_t read_and_clear_row_error(cudaStream_t s, unsigned int *code);
 
+// Direct-tap kernel (wino_direct.cu): 16-bit layers, and fp32 layers with three tf32 products per multiply.
+struct DirectDesc {
+  int dtype, N, C, K, D, H, W, oD, oH, oW, yH, yW;
+  int sD, sH, sW, pD, pH, pW, kD, kH, kW;
+  unsigned epilogue;
+  int weight_layout;
+};
+struct DirectPlan {
+  int BN, MB, pair, split;           // columns and row blocks of an item, CTA pairs, CTAs that share an item's reduction
+  int TN, TH, PW, slab_rows_h;       // images and output rows of a row block, pixels of a slab row, slab rows
+  int ch_el, rb, n_chunks, k_full, k_tail;
+  int n_ph, ph_h[4], ph_w[4], ph_tw[4], taps[4], tap0[4], n_taps, units;
+  int n_wb, n_hb, n_tiles, n_kb, n_items;
+  int slab_bytes, a_bytes, lo_off, b_tile, b_lo, b_bytes, G, n_a, n_b, smem;
+  long long filter_elems;
+  double estimate;                   // clocks
+};
+bool direct_plan(const DirectDesc &d, DirectPlan *out);
+cudaError_t launch_direct_filter_transform(const DirectDesc &d, const DirectPlan &p, int w_dtype, const void *w, void *u, cudaStream_t s);
+cudaError_t launch_direct_forward(const DirectDesc &d, const DirectPlan &p, const void *x, const void *u, const void *bias, void *y,
+                                  cudaStream_t s, const char **detail);
+cudaError_t read_and_clear_direct_error(cudaStream_t s, unsigned int *code);
+
 // Reads the error word of the bounded device waits, clears it and synchronises the stream.
 cudaError_t read_and_clear_device_error(cudaStream_t s, unsigned int *code);
 
