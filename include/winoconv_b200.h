@@ -159,6 +159,12 @@ WINOCONV_API int winoconv_plan_pieces(const winoconv_desc_t *desc, int32_t *piec
 WINOCONV_API int winoconv_filter_transform(const winoconv_desc_t *desc, const void *weights, void *u, void *stream);
 
 /*
+ * The same from weights of another dtype: f32 weights (a training loop's master copy) for a 16-bit layer that runs on the
+ * direct-tap kernel; rounded once.
+ */
+WINOCONV_API int winoconv_filter_transform_from(const winoconv_desc_t *desc, const void *weights, int w_dtype, void *u, void *stream);
+
+/*
  * y = conv(x, w) by the algorithm the plan names (winoconv_plan_info_t.algo):
  *   ROW / FUSED  one kernel: input tiles are transformed in shared memory, multiplied on the tensor
  *                cores with the DWM pieces summed in the accumulator, and written through the output
@@ -215,6 +221,27 @@ WINOCONV_API int winoconv_forward_timed(const winoconv_desc_t *desc, const void 
 #define WINOCONV_STATIC_SCRATCH_BYTES (32u << 20)
 WINOCONV_API int winoconv_forward_static(const winoconv_desc_t *desc, const void *x, const void *u, const void *bias,
                                          void *y, void *stream);
+
+/*
+ * Gradients of a 16-bit layer on the tensor cores (desc: the forward layer; EPI_BIAS asks for the bias gradient too, the
+ * other epilogue bits are ignored).  x and gy are channels last with channel strides c_stride and k_stride (C and K rounded
+ * up to a multiple of 8, the extra channels zero); gx has C channels; dw is [K, C, kD, kH, kW] in dw_dtype, accumulated in fp32.
+ *   data:   gx = conv(gy, mirrored w with K and C exchanged), strided layers a launch over the polyphase parts of gx;
+ *           u from winoconv_backward_filter_transform (data_filter_bytes).
+ *   weight: dw = sum over images and output pixels of gy x^T per tap, dbias = sum of gy; ws: weight_ws_bytes of scratch.
+ * data_ok / weight_ok say whether the layer is covered (f32 layers and kernels of more than 400 taps are not).
+ * The reference left traces of a backward only (include/splitstrideone/split_functions_grad.h:1-7, src/back/utils.cu:16).
+ */
+typedef struct winoconv_backward_info {
+  int32_t data_ok, weight_ok;
+  int32_t c_stride, k_stride;
+  uint64_t data_filter_bytes, weight_ws_bytes;
+} winoconv_backward_info_t;
+WINOCONV_API int winoconv_backward_plan(const winoconv_desc_t *desc, winoconv_backward_info_t *info);
+WINOCONV_API int winoconv_backward_filter_transform(const winoconv_desc_t *desc, const void *weights, int w_dtype, void *u, void *stream);
+WINOCONV_API int winoconv_backward_data(const winoconv_desc_t *desc, const void *gy, const void *u, void *gx, void *stream);
+WINOCONV_API int winoconv_backward_weight(const winoconv_desc_t *desc, const void *x, const void *gy, void *dw, int dw_dtype,
+                                          float *dbias, void *ws, size_t ws_bytes, void *stream);
 
 /*
  * The per-position batched GEMM on its own: m[p][t][k] = sum_c v[p][t][c] * u[p][k][c],

@@ -31,13 +31,14 @@ from __future__ import annotations
 
 import itertools
 import math
+import types
 from typing import Optional, Tuple
 
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
 
-from . import capi, engine
+from . import _backend, capi, engine
 
 __all__ = ["Conv2d", "Conv3d"]
 
@@ -64,10 +65,60 @@ class _WinoConvMixin:
         self.pool = 2 if pool == 2 else None
         self.tile_m = int(tile_m)
         self.algo = int(algo)
-        self._plans = {}          # input shape (or backward key) -> engine.WinoConv, most recently used last
-        self._weight_key = None   # identity of the weight the cached plans were built from
+        self._reset_plans()
 
-    # -- cache -------------------------------------------------------------------------------------
+    # -- native path -------------------------------------------------------------------------------
+    # The forward and the autograd node are native (csrc/conv_module.cpp): plan lookup, filter transform, layout, allocation
+    # and launch cost about 6 us a call where the same steps in Python cost 24.  What it does not take (an argument to
+    # refuse, fp32 gradients) returns None and runs below.
+    _CONFIG = frozenset(("compute_dtype", "activation", "pool", "tile_m", "algo", "stride", "padding"))
+
+    def _reset_plans(self):
+        d = self.__dict__
+        d["_runner"] = None        # native runner, made on the first call
+        d["_views"] = {}           # what _plans shows of the runner's entries
+        d["_py_plans"] = {}        # input shape (or backward key) -> engine.WinoConv of the Python path, most recently used last
+        d["_weight_key"] = None    # identity of the weight the Python path's plans were built from
+
+    def __setattr__(self, name, value):
+        super().__setattr__(name, value)
+        if name in _WinoConvMixin._CONFIG and "_runner" in self.__dict__:
+            self._reset_plans()
+
+    def __getstate__(self):        # plans and runners stay behind when a module is copied or pickled
+        state = dict(self.__dict__)
+        for name in ("_runner", "_views", "_py_plans", "_weight_key"):
+            state.pop(name, None)
+        return state
+
+    def __setstate__(self, state):
+        super().__setstate__(state)
+        self._reset_plans()
+
+    def _make_runner(self):
+        code = -1 if self.compute_dtype is None else engine.dtype_code(self.compute_dtype)
+        self.__dict__["_runner"] = _backend.load().ConvRunner(
+            self._nd, [int(s) for s in self.stride], [int(p) for p in self.padding], self.tile_m, self.algo,
+            self.activation == "relu", self.pool == 2, code, self.MAX_CACHED_PLANS)
+        return self._runner
+
+    @property
+    def _plans(self):
+        """Input shape (channels last) -> plan of every shape whose filter is transformed from the current weights."""
+        out = {}
+        if self._runner is not None:
+            views = {}
+            for shape, dtype, device, u, serial, info in self._runner.entries():
+                key = (tuple(shape), dtype, device)
+                view = self._views.get(key)
+                if view is None or view.serial != serial:
+                    view = types.SimpleNamespace(u=u, serial=serial, info=capi.PlanInfo.from_buffer_copy(info))
+                views[key] = out[tuple(shape)] = view
+            self.__dict__["_views"] = views
+        out.update(self._py_plans)
+        return out
+
+    # -- cache of the Python path ------------------------------------------------------------------
     def _current_weight_key(self, dtype, device):
         w, b = self.weight, self.bias
         return (w.data_ptr(), w._version, None if b is None else (b.data_ptr(), b._version), dtype, device)
@@ -75,24 +126,31 @@ class _WinoConvMixin:
     def _plan_for(self, in_shape_cl: Tuple[int, ...], dtype, device) -> engine.WinoConv:
         key = self._current_weight_key(dtype, device)
         if key != self._weight_key:            # the parameters changed: every cached filter transform is stale
-            self._plans.clear()
+            self._py_plans.clear()
             self._weight_key = key
-        plan = self._plans.pop(in_shape_cl, None)
+        plan = self._py_plans.pop(in_shape_cl, None)
         if plan is not None:
-            self._plans[in_shape_cl] = plan            # most recently used last
+            self._py_plans[in_shape_cl] = plan            # most recently used last
         if plan is None:
             w = self.weight.detach().to(device=device, dtype=dtype)
             b = None if self.bias is None else self.bias.detach().to(device=device, dtype=dtype)
             plan = engine.WinoConv(in_shape_cl, w, stride=tuple(int(s) for s in self.stride),
                                    padding=tuple(int(p) for p in self.padding), tile_m=self.tile_m, bias=b,
                                    relu=self.activation == "relu", pool2=self.pool == 2, algo=self.algo)
-            self._plans[in_shape_cl] = plan
-            while len(self._plans) > self.MAX_CACHED_PLANS:      # each plan holds its own transformed filter
-                self._plans.pop(next(iter(self._plans)))
+            self._py_plans[in_shape_cl] = plan
+            while len(self._py_plans) > self.MAX_CACHED_PLANS:   # each plan holds its own transformed filter
+                self._py_plans.pop(next(iter(self._py_plans)))
         return plan
 
     # -- forward -----------------------------------------------------------------------------------
     def forward(self, input: torch.Tensor) -> torch.Tensor:      # noqa: A002  (torch's argument name)
+        params = self._parameters
+        if "weight" not in params or "bias" not in params:      # a parametrised module computes them
+            params = {"weight": self.weight, "bias": self.bias}
+        y = (self._runner or self._make_runner()).forward(input, params["weight"], params["bias"], self.training)
+        return y if y is not None else self._forward_python(input)
+
+    def _forward_python(self, input: torch.Tensor) -> torch.Tensor:      # noqa: A002
         nd = self._nd
         if input.dim() != nd + 2:
             raise ValueError(f"expected a {nd + 2}-D input [N, C, {'D, ' if nd == 3 else ''}H, W]")
@@ -148,13 +206,13 @@ class _WinoConvMixin:
         key = ("bwd", tuple(z.shape), z.dtype, z.device)
         wkey = self._current_weight_key(z.dtype, z.device)
         if wkey != self._weight_key:
-            self._plans.clear()
+            self._py_plans.clear()
             self._weight_key = wkey
-        plan = self._plans.get(key)
+        plan = self._py_plans.get(key)
         if plan is None:
             wt = self.weight.detach().to(device=z.device, dtype=z.dtype).flip(*range(2, 2 + nd)).transpose(0, 1).contiguous()
             plan = engine.WinoConv(tuple(z.shape), wt, stride=1, padding=pad_arg)
-            self._plans[key] = plan
+            self._py_plans[key] = plan
         gx = plan(z)
         assert tuple(gx.shape) == tuple(in_shape_cl), (gx.shape, in_shape_cl)
         return gx
@@ -207,7 +265,7 @@ class _WinoConvMixin:
 
 
 class _WinoConvFn(torch.autograd.Function):
-    """Autograd node of the module forward: every arithmetic kernel of the three gradients is the engine's."""
+    """Autograd node of the Python path (fp32 layers, kernels the native gradients do not cover): every arithmetic kernel of the three gradients is the engine's."""
 
     @staticmethod
     def forward(ctx, module, x, weight, bias):

@@ -1,0 +1,291 @@
+#include "conv_module.h"
+
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+
+#include <cstring>
+
+namespace {
+
+int code_of(at::ScalarType t) {
+  switch (t) {
+    case at::kFloat: return WINOCONV_F32;
+    case at::kHalf: return WINOCONV_F16;
+    case at::kBFloat16: return WINOCONV_BF16;
+    default: return -1;
+  }
+}
+at::ScalarType type_of(int code) { return code == WINOCONV_F32 ? at::kFloat : code == WINOCONV_F16 ? at::kHalf : at::kBFloat16; }
+
+void check_abi(int st, const char *what) {
+  if (st == WINOCONV_OK) return;
+  char buf[1024];
+  winoconv_last_error(buf, sizeof buf);
+  TORCH_CHECK(false, what, " failed (", winoconv_status_string(st), "): ", buf);
+}
+void *stream_of() { return (void *)at::cuda::getCurrentCUDAStream().stream(); }
+
+ConvRunner::Stamp stamp_of(const at::Tensor &w, const std::optional<at::Tensor> &b) {
+  ConvRunner::Stamp s;
+  s.w = w.data_ptr();
+  s.w_version = w.is_inference() ? 0 : (int64_t)w._version();
+  s.w_dtype = (int)w.scalar_type();
+  if (b) {
+    s.b = b->data_ptr();
+    s.b_version = b->is_inference() ? 0 : (int64_t)b->_version();
+  }
+  return s;
+}
+
+// Whether an [N, C, spatial...] tensor lies channels last in memory (dimensions of one element may have any stride).
+bool lies_channels_last(const at::Tensor &t) {
+  const auto sizes = t.sizes(), strides = t.strides();
+  const int nd = (int)sizes.size();
+  int64_t want = 1;
+  auto ok = [&](int d) {
+    if (sizes[d] != 1 && strides[d] != want) return false;
+    want *= sizes[d];
+    return true;
+  };
+  if (!ok(1)) return false;
+  for (int d = nd - 1; d >= 2; --d)
+    if (!ok(d)) return false;
+  return ok(0);
+}
+
+at::Tensor empty_bytes(uint64_t bytes, const at::Tensor &like) {
+  return at::empty({(int64_t)bytes}, like.options().dtype(at::kByte).requires_grad(false));
+}
+
+// The last dimension of a channels-last buffer zero-extended to `c` channels; the tensor itself where it has them.
+at::Tensor pad_channels(const at::Tensor &t, int64_t c) {
+  const int nd = (int)t.dim();
+  if (t.size(1) == c) return t;
+  at::Tensor cl = t.movedim(1, nd - 1);
+  return at::constant_pad_nd(cl, {0, c - t.size(1)}).contiguous().movedim(nd - 1, 1);
+}
+
+struct ConvFn : public torch::autograd::Function<ConvFn> {
+  static at::Tensor forward(torch::autograd::AutogradContext *ctx, const c10::intrusive_ptr<ConvRunner> &runner, const at::Tensor &x,
+                            const at::Tensor &x_cl, const std::shared_ptr<ConvRunner::Entry> &entry, const at::Tensor &weight,
+                            const std::optional<at::Tensor> &bias, bool relu) {
+    at::Tensor y = runner->run(*entry, x_cl, weight, bias);
+    ctx->save_for_backward({x, relu ? y : at::Tensor()});
+    ctx->saved_data["runner"] = c10::IValue::make_capsule(runner);
+    ctx->saved_data["weight"] = weight;
+    if (bias) ctx->saved_data["bias"] = *bias;
+    return y;
+  }
+  static torch::autograd::variable_list backward(torch::autograd::AutogradContext *ctx, torch::autograd::variable_list grads) {
+    torch::autograd::variable_list out(7);
+    if (!grads[0].defined()) return out;
+    auto saved = ctx->get_saved_variables();
+    auto runner = c10::static_intrusive_pointer_cast<ConvRunner>(ctx->saved_data["runner"].toCapsule());
+    const at::Tensor weight = ctx->saved_data["weight"].toTensor();
+    std::optional<at::Tensor> bias;
+    auto b = ctx->saved_data.find("bias");
+    if (b != ctx->saved_data.end()) bias = b->second.toTensor();
+    // numbered by the tensors among the arguments of apply: x, x_cl, weight, bias
+    const bool nx = ctx->needs_input_grad(0), nw = ctx->needs_input_grad(2), nb = bias && ctx->needs_input_grad(3);
+    auto g = runner->backward(grads[0], saved[0], saved[1], weight, bias, nx, nw, nb);
+    out[1] = g[0];
+    out[4] = g[1];
+    out[5] = g[2];
+    return out;
+  }
+};
+
+}  // namespace
+
+ConvRunner::ConvRunner(int64_t nd, std::vector<int64_t> stride, std::vector<int64_t> padding, int64_t tile_m, int64_t algo, bool relu,
+                       bool pool, int64_t compute, int64_t max_plans)
+    : nd_((int)nd), tile_m_((int)tile_m), algo_((int)algo), compute_((int)compute), relu_(relu), pool_(pool), max_plans_((size_t)max_plans) {
+  TORCH_CHECK((nd == 2 || nd == 3) && (int64_t)stride.size() == nd && (int64_t)padding.size() == nd, "ConvRunner: bad rank");
+  for (int i = 0; i < 3; ++i) { stride_[i] = 1; pad_[i] = 0; }
+  for (int i = 0; i < nd; ++i) { stride_[3 - nd + i] = (int)stride[i]; pad_[3 - nd + i] = (int)padding[i]; }
+}
+
+at::Tensor ConvRunner::channels_last(const at::Tensor &t, at::ScalarType type) const {
+  if (t.scalar_type() == type && lies_channels_last(t)) return t;
+  return t.to(t.options().dtype(type), false, false, nd_ == 2 ? at::MemoryFormat::ChannelsLast : at::MemoryFormat::ChannelsLast3d);
+}
+
+std::shared_ptr<ConvRunner::Entry> ConvRunner::entry_for(const at::Tensor &x, const at::Tensor &weight, const std::optional<at::Tensor> &bias,
+                                                         int dtype) {
+  int64_t shape[5] = {x.size(0), 1, 1, 1, x.size(1)};
+  for (int i = 0; i < nd_; ++i) shape[4 - nd_ + i] = x.size(2 + i);
+  const int device = x.get_device();
+  std::lock_guard<std::mutex> lock(mu_);
+  for (size_t i = entries_.size(); i-- > 0;) {
+    Entry &e = *entries_[i];
+    if (e.dtype == dtype && e.device == device && std::memcmp(e.shape, shape, sizeof shape) == 0) {
+      auto hit = entries_[i];
+      if (i + 1 != entries_.size()) {
+        entries_.erase(entries_.begin() + i);
+        entries_.push_back(hit);
+      }
+      return hit;
+    }
+  }
+  auto e = std::make_shared<Entry>();
+  std::memcpy(e->shape, shape, sizeof shape);
+  e->dtype = dtype;
+  e->device = device;
+  winoconv_desc_t &d = e->desc;
+  std::memset(&d, 0, sizeof d);
+  d.ndim = nd_;
+  for (int64_t s : {shape[0], shape[1], shape[2], shape[3], shape[4], weight.size(0)})
+    if (s <= 0 || s > 0x7fffffffLL) return nullptr;
+  d.batch = (int)shape[0]; d.c_in = (int)shape[4]; d.k_out = (int)weight.size(0);
+  for (int i = 0; i < 3; ++i) {
+    d.in_size[i] = (int)shape[1 + i];
+    d.ker_size[i] = i < 3 - nd_ ? 1 : (int)weight.size(2 + i - (3 - nd_));
+    d.stride[i] = stride_[i];
+    d.pad[i] = pad_[i];
+  }
+  d.tile_m = tile_m_;
+  d.dtype = dtype;
+  d.epilogue = (bias ? WINOCONV_EPI_BIAS : 0u) | (relu_ ? WINOCONV_EPI_RELU : 0u) | (pool_ ? WINOCONV_EPI_POOL2 : 0u);
+  d.algo = algo_;
+  if (winoconv_plan(&d, &e->info) != WINOCONV_OK) return nullptr;
+  entries_.push_back(e);
+  while (entries_.size() > max_plans_) entries_.erase(entries_.begin());      // each entry holds its own transformed filter
+  return e;
+}
+
+at::Tensor ConvRunner::run(Entry &e, const at::Tensor &x, const at::Tensor &weight, const std::optional<at::Tensor> &bias) {
+  const at::ScalarType type = type_of(e.dtype);
+  void *s = stream_of();
+  const Stamp now = stamp_of(weight, bias);
+  at::Tensor u, b;
+  {
+    std::lock_guard<std::mutex> lock(mu_);
+    if (!(e.stamp == now) || !e.u.defined()) {
+      at::AutoDispatchBelowADInplaceOrView guard;
+      // a new buffer, not the old one: launches that read it may still be queued on another stream
+      e.u = empty_bytes(e.info.filter_bytes, weight);
+      at::Tensor w = weight.is_contiguous() ? weight : weight.contiguous();
+      if (winoconv_filter_transform_from(&e.desc, w.data_ptr(), code_of(w.scalar_type()), e.u.data_ptr(), s) != WINOCONV_OK) {
+        w = w.to(type);
+        check_abi(winoconv_filter_transform(&e.desc, w.data_ptr(), e.u.data_ptr(), s), "winoconv_filter_transform");
+      }
+      e.bias = bias ? bias->to(type).contiguous() : at::Tensor();
+      e.stamp = now;
+      e.serial = ++serial_;
+      newest_ = now;
+    }
+    u = e.u;
+    b = e.bias;
+  }
+  int64_t sizes[5] = {e.shape[0], (int64_t)e.desc.k_out, 0, 0, 0};
+  for (int i = 0; i < nd_; ++i) sizes[2 + i] = e.info.out_size[3 - nd_ + i];
+  at::Tensor y = at::empty(at::IntArrayRef(sizes, nd_ + 2), x.options().dtype(type).requires_grad(false),
+                           nd_ == 2 ? at::MemoryFormat::ChannelsLast : at::MemoryFormat::ChannelsLast3d);
+  at::Tensor v, m;
+  if (!e.info.direct) {
+    if (e.info.input_ws_bytes) v = empty_bytes(e.info.input_ws_bytes, x);
+    if (e.info.product_ws_bytes) m = empty_bytes(e.info.product_ws_bytes, x);
+  }
+  check_abi(winoconv_forward(&e.desc, x.data_ptr(), u.data_ptr(), b.defined() ? b.data_ptr() : nullptr, y.data_ptr(),
+                             v.defined() ? v.data_ptr() : nullptr, e.info.input_ws_bytes, m.defined() ? m.data_ptr() : nullptr,
+                             e.info.product_ws_bytes, s),
+            "winoconv_forward");
+  return y;
+}
+
+std::optional<at::Tensor> ConvRunner::forward(const at::Tensor &x, const at::Tensor &weight, const std::optional<at::Tensor> &bias, bool training) {
+  if (!x.is_cuda() || x.dim() != nd_ + 2 || weight.dim() != nd_ + 2 || !weight.is_cuda() || weight.get_device() != x.get_device() ||
+      x.size(1) != weight.size(1) || x.numel() == 0 || (bias && !bias->is_cuda()) || code_of(weight.scalar_type()) < 0)
+    return std::nullopt;
+  const int dtype = compute_ >= 0 ? compute_ : code_of(x.scalar_type());
+  if (dtype < 0) return std::nullopt;
+  const bool grad = at::GradMode::is_enabled() && (x.requires_grad() || (weight.requires_grad() && training));
+  if (grad && (pool_ || dtype == WINOCONV_F32)) return std::nullopt;
+  c10::cuda::CUDAGuard guard(x.device());
+  std::shared_ptr<Entry> e = entry_for(x, weight, bias, dtype);
+  if (!e) return std::nullopt;
+  if (!grad) {
+    at::AutoDispatchBelowADInplaceOrView no_graph;
+    return run(*e, channels_last(x, type_of(dtype)), weight, bias);
+  }
+  if (!e->back_known) {
+    winoconv_backward_info_t info;
+    e->back_ok = winoconv_backward_plan(&e->desc, &info) == WINOCONV_OK && info.data_ok && info.weight_ok;
+    e->back_known = true;
+  }
+  if (!e->back_ok) return std::nullopt;
+  at::Tensor x_cl;
+  {
+    at::AutoDispatchBelowADInplaceOrView no_graph;
+    x_cl = channels_last(x, type_of(dtype));
+    if (x_cl.is_same(x)) x_cl = x.detach();
+  }
+  return ConvFn::apply(c10::intrusive_ptr<ConvRunner>::reclaim_copy(this), x, x_cl, e, weight, bias, relu_);
+}
+
+std::vector<at::Tensor> ConvRunner::backward(const at::Tensor &gy_in, const at::Tensor &x_in, const at::Tensor &y, const at::Tensor &weight,
+                                             const std::optional<at::Tensor> &bias, bool need_x, bool need_w, bool need_b) {
+  at::AutoDispatchBelowADInplaceOrView no_graph;
+  c10::cuda::CUDAGuard guard(x_in.device());
+  const int dtype = compute_ >= 0 ? compute_ : code_of(x_in.scalar_type());
+  const at::ScalarType type = type_of(dtype);
+  std::shared_ptr<Entry> e = entry_for(x_in, weight, bias, dtype);
+  TORCH_CHECK(e, "winoconv backward: no plan");
+  void *s = stream_of();
+  at::Tensor gy = gy_in;
+  if (y.defined()) gy = gy * (y > 0).to(gy.scalar_type());
+  gy = channels_last(gy, type);
+  winoconv_desc_t d = e->desc;
+  d.epilogue = need_b ? WINOCONV_EPI_BIAS : 0u;
+  winoconv_backward_info_t info;
+  check_abi(winoconv_backward_plan(&d, &info), "winoconv_backward_plan");
+  const at::Tensor gyp = pad_channels(gy, info.k_stride);
+  at::Tensor gx, gw, gb;
+  const at::Tensor w = weight.is_contiguous() ? weight : weight.contiguous();
+  if (need_x) {
+    at::Tensor u;
+    const Stamp now = stamp_of(weight, std::nullopt);
+    {
+      std::lock_guard<std::mutex> lock(mu_);
+      if (!(e->back_stamp == now) || !e->u_back.defined()) {
+        e->u_back = empty_bytes(std::max<uint64_t>(info.data_filter_bytes, 16), w);
+        at::Tensor wt = w;
+        if (code_of(w.scalar_type()) != WINOCONV_F32 && code_of(w.scalar_type()) != dtype) wt = w.to(type);
+        check_abi(winoconv_backward_filter_transform(&d, wt.data_ptr(), code_of(wt.scalar_type()), e->u_back.data_ptr(), s),
+                  "winoconv_backward_filter_transform");
+        e->back_stamp = now;
+      }
+      u = e->u_back;
+    }
+    gx = at::empty(x_in.sizes(), x_in.options().dtype(type).requires_grad(false), nd_ == 2 ? at::MemoryFormat::ChannelsLast : at::MemoryFormat::ChannelsLast3d);
+    check_abi(winoconv_backward_data(&d, gyp.data_ptr(), u.data_ptr(), gx.data_ptr(), s), "winoconv_backward_data");
+    if (x_in.scalar_type() != type) gx = gx.to(x_in.scalar_type());
+  }
+  if (need_w) {
+    const at::Tensor xp = pad_channels(channels_last(x_in, type), info.c_stride);
+    gw = at::empty(weight.sizes(), weight.options().requires_grad(false));
+    if (need_b) gb = at::empty({weight.size(0)}, weight.options().dtype(at::kFloat).requires_grad(false));
+    const at::Tensor ws = empty_bytes(info.weight_ws_bytes, w);
+    check_abi(winoconv_backward_weight(&d, xp.data_ptr(), gyp.data_ptr(), gw.data_ptr(), code_of(gw.scalar_type()),
+                                       need_b ? gb.data_ptr<float>() : nullptr, ws.data_ptr(), info.weight_ws_bytes, s),
+              "winoconv_backward_weight");
+  } else if (need_b) {
+    std::vector<int64_t> dims{0};
+    for (int i = 0; i < nd_; ++i) dims.push_back(2 + i);
+    gb = gy.to(at::kFloat).sum(dims);
+  }
+  if (gb.defined() && gb.scalar_type() != bias->scalar_type()) gb = gb.to(bias->scalar_type());
+  return {gx, gw, gb};
+}
+
+std::vector<std::tuple<std::vector<int64_t>, int64_t, int64_t, at::Tensor, int64_t, std::string>> ConvRunner::entries() {
+  std::lock_guard<std::mutex> lock(mu_);
+  std::vector<std::tuple<std::vector<int64_t>, int64_t, int64_t, at::Tensor, int64_t, std::string>> out;
+  for (auto &e : entries_) {
+    if (!e->u.defined() || !(e->stamp == newest_)) continue;
+    std::vector<int64_t> shape{e->shape[0]};
+    for (int i = 4 - nd_; i < 5; ++i) shape.push_back(e->shape[i]);
+    out.emplace_back(shape, e->dtype, e->device, e->u, e->serial, std::string(reinterpret_cast<const char *>(&e->info), sizeof e->info));
+  }
+  return out;
+}

@@ -1,0 +1,67 @@
+// Native forward and backward of the convolution modules (conv.py): plan and filter cache, layout, launches and the autograd
+// node without a trip through Python per call.
+#pragma once
+
+#include <cstdint>
+#include <memory>
+#include <mutex>
+#include <optional>
+#include <string>
+#include <vector>
+
+#include <torch/extension.h>
+
+#include "winoconv_b200.h"
+
+// One per module.  Every entry is the plan of an input shape with its transformed filters; they follow the weights (storage,
+// version, dtype), and the least recently used one goes when there are more than `max_plans`.
+class ConvRunner : public torch::CustomClassHolder {
+ public:
+  ConvRunner(int64_t nd, std::vector<int64_t> stride, std::vector<int64_t> padding, int64_t tile_m, int64_t algo, bool relu, bool pool,
+             int64_t compute, int64_t max_plans);
+
+  // The module's forward, or nothing where the Python path has to decide (an error to raise, a gradient the kernels do not cover).
+  std::optional<at::Tensor> forward(const at::Tensor &x, const at::Tensor &weight, const std::optional<at::Tensor> &bias, bool training);
+
+  // (input shape channels last, dtype code, device index, transformed filter, serial of its transform, plan bytes) of every entry
+  // whose filter belongs to the newest weights, least recently used first
+  std::vector<std::tuple<std::vector<int64_t>, int64_t, int64_t, at::Tensor, int64_t, std::string>> entries();
+
+  struct Stamp {        // what a transformed filter was made from
+    const void *w = nullptr, *b = nullptr;
+    int64_t w_version = -1, b_version = -1;
+    int w_dtype = -1;
+    bool operator==(const Stamp &o) const {
+      return w == o.w && b == o.b && w_version == o.w_version && b_version == o.b_version && w_dtype == o.w_dtype;
+    }
+  };
+  struct Entry {
+    int64_t shape[5] = {0, 0, 0, 0, 0};      // N, D, H, W, C of the input
+    int dtype = -1, device = -1;
+    winoconv_desc_t desc;
+    winoconv_plan_info_t info;
+    at::Tensor u, bias;                      // transformed filter, bias in the compute dtype
+    Stamp stamp;
+    int64_t serial = 0;
+    at::Tensor u_back;                       // filter of the data gradient
+    Stamp back_stamp;
+    bool back_known = false, back_ok = false;
+  };
+
+  at::Tensor run(Entry &e, const at::Tensor &x_cl, const at::Tensor &weight, const std::optional<at::Tensor> &bias);
+  // Gradients of one layer call; undefined where not asked for.
+  std::vector<at::Tensor> backward(const at::Tensor &gy, const at::Tensor &x, const at::Tensor &y, const at::Tensor &weight,
+                                   const std::optional<at::Tensor> &bias, bool need_x, bool need_w, bool need_b);
+
+ private:
+  std::shared_ptr<Entry> entry_for(const at::Tensor &x, const at::Tensor &weight, const std::optional<at::Tensor> &bias, int dtype);
+  at::Tensor channels_last(const at::Tensor &t, at::ScalarType type) const;
+
+  int nd_, stride_[3], pad_[3], tile_m_, algo_, compute_;
+  bool relu_, pool_;
+  size_t max_plans_;
+  std::mutex mu_;
+  std::vector<std::shared_ptr<Entry>> entries_;     // most recently used last
+  Stamp newest_;
+  int64_t serial_ = 0;
+};

@@ -4,6 +4,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -261,11 +262,7 @@ int build_plan(const winoconv_desc_t *d, Plan *plan) {
   if (d->algo == WINOCONV_ALGO_AUTO && d->tile_m == 0 && d->gemm_engine == WINOCONV_GEMM_AUTO && pdt == WINOCONV_F32 && direct_env != 0 &&
       (plan->row || (d->dtype == WINOCONV_F32 && direct_env == 2))) {
     DirectDesc &q = plan->dd;
-    std::memset(&q, 0, sizeof q);
-    q.dtype = d->dtype; q.N = g.N; q.C = g.C; q.K = g.K; q.D = g.D; q.H = g.H; q.W = g.W;
-    q.oD = g.oD; q.oH = g.oH; q.oW = g.oW; q.yH = g.yH; q.yW = g.yW;
-    q.sD = g.sD; q.sH = g.sH; q.sW = g.sW; q.pD = g.pD; q.pH = g.pH; q.pW = g.pW; q.kD = g.kD; q.kH = g.kH; q.kW = g.kW;
-    q.epilogue = g.epilogue; q.weight_layout = g.weight_layout;
+    direct_forward_desc(&q, d->dtype, g.N, g.C, g.K, in, ks, st, pd, out, g.yH, g.yW, g.epilogue, g.weight_layout);
     plan->direct = direct_plan(q, &plan->dp);
   }
 
@@ -319,6 +316,75 @@ int build_plan(const winoconv_desc_t *d, Plan *plan) {
   if (plan->row) I.gemm_flops = 2.0 * 4 * (double)I.tiles * I.n_pieces * plan->rd.C * g.K;
   I.algorithmic_bytes = (double)esz * ((double)g.N * g.D * g.H * g.W * g.C + (double)g.K * g.C * ks[0] * ks[1] * ks[2] +
                                        (double)g.N * g.yD * g.yH * g.yW * g.K);
+  return WINOCONV_OK;
+}
+
+// Plans are functions of the descriptor alone; a caller runs the same few descriptors over and over, so each thread keeps the
+// last ones (direct mapped by a hash of the descriptor; a planner pass costs tens of microseconds).
+template <typename P> struct PlanSlot { winoconv_desc_t desc; std::unique_ptr<P> plan; };
+constexpr unsigned kPlanSlots = 64;
+template <typename P>
+int plan_of(const winoconv_desc_t *d, int (*build)(const winoconv_desc_t *, P *), const P **out) {
+  static thread_local PlanSlot<P> slots[kPlanSlots];
+  if (!d) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "null descriptor");
+  const uint32_t *w = reinterpret_cast<const uint32_t *>(d);
+  uint32_t h = 2166136261u;
+  for (size_t i = 0; i < sizeof(*d) / 4; ++i) h = (h ^ w[i]) * 16777619u;
+  PlanSlot<P> &s = slots[(h ^ (h >> 15)) % kPlanSlots];
+  if (!s.plan || std::memcmp(&s.desc, d, sizeof(*d)) != 0) {
+    std::unique_ptr<P> fresh(new P());
+    const int st = build(d, fresh.get());
+    if (st != WINOCONV_OK) return st;
+    s.desc = *d;
+    s.plan = std::move(fresh);
+  }
+  *out = s.plan.get();
+  return WINOCONV_OK;
+}
+
+// Gradients of a 16-bit layer: the data gradient on the direct-tap kernel (a launch per depth parity), the weight gradient on
+// its own kernel.  x and gy have channel strides rounded up to a multiple of 8.
+struct BackPlan {
+  DirectDesc dd[2];
+  DirectPlan dp[2];
+  int n_data;
+  bool data_ok, weight_ok, zero_fill;
+  unsigned long long u_off[3];
+  WgradDesc wd;
+  WgradPlan wp;
+  size_t gx_bytes;
+};
+int build_back_plan(const winoconv_desc_t *d, BackPlan *b) {
+  winoconv_desc_t f = *d;     // the forward layer's shape, whatever algorithm and epilogue it runs with
+  f.algo = WINOCONV_ALGO_AUTO; f.tile_m = 0; f.gemm_engine = WINOCONV_GEMM_AUTO; f.product_dtype = WINOCONV_F32; f.epilogue = 0;
+  const Plan *p = nullptr;
+  const int st = plan_of<Plan>(&f, build_plan, &p);
+  if (st != WINOCONV_OK) return st;
+  const Geom &g = p->g;
+  b->n_data = 0; b->data_ok = b->weight_ok = b->zero_fill = false;
+  if (d->dtype == WINOCONV_F32) return WINOCONV_OK;
+  const int in[3] = {g.D, g.H, g.W}, ker[3] = {g.kD, g.kH, g.kW}, str[3] = {g.sD, g.sH, g.sW}, pad[3] = {g.pD, g.pH, g.pW};
+  const int out[3] = {g.oD, g.oH, g.oW};
+  const int Cm = (g.C + 7) / 8 * 8, Km = (g.K + 7) / 8 * 8;
+  b->data_ok = true;
+  b->u_off[0] = 0;
+  for (int e = 0; e < g.sD && b->data_ok; ++e) {
+    DirectDesc &q = b->dd[b->n_data];
+    direct_grad_desc(&q, d->dtype, g.N, g.C, g.K, Km, in, ker, str, pad, out, d->weight_layout, e, &b->zero_fill);
+    if (q.n_parts == 0) continue;
+    b->data_ok = direct_plan(q, &b->dp[b->n_data]);
+    if (b->data_ok) {
+      b->u_off[b->n_data + 1] = b->u_off[b->n_data] + ((unsigned long long)b->dp[b->n_data].filter_elems * 2 + 255) / 256 * 256;
+      ++b->n_data;
+    }
+  }
+  b->gx_bytes = (size_t)g.N * g.D * g.H * g.W * g.C * 2;
+  WgradDesc &w = b->wd;
+  std::memset(&w, 0, sizeof w);
+  w.dtype = d->dtype; w.N = g.N; w.C = g.C; w.K = g.K; w.Cm = Cm; w.Km = Km; w.D = g.D; w.H = g.H; w.W = g.W;
+  w.oD = g.oD; w.oH = g.oH; w.oW = g.oW; w.sD = g.sD; w.sH = g.sH; w.sW = g.sW; w.pD = g.pD; w.pH = g.pH; w.pW = g.pW;
+  w.kD = g.kD; w.kH = g.kH; w.kW = g.kW; w.bias = (d->epilogue & WINOCONV_EPI_BIAS) ? 1 : 0;
+  b->weight_ok = d->weight_layout == WINOCONV_W_KCRS && wgrad_plan(w, &b->wp);
   return WINOCONV_OK;
 }
 
@@ -387,10 +453,10 @@ int winoconv_device_check(void) {
 
 int winoconv_plan(const winoconv_desc_t *desc, winoconv_plan_info_t *info) {
   if (!info) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "null info");
-  Plan plan;
-  const int st = build_plan(desc, &plan);
+  const Plan *plan = nullptr;
+  const int st = plan_of<Plan>(desc, build_plan, &plan);
   if (st != WINOCONV_OK) return st;
-  *info = plan.info;
+  *info = plan->info;
   return WINOCONV_OK;
 }
 
@@ -411,12 +477,19 @@ int winoconv_plan_pieces(const winoconv_desc_t *desc, int32_t *pieces, int32_t m
 }
 
 int winoconv_filter_transform(const winoconv_desc_t *desc, const void *weights, void *u, void *stream) {
-  Plan plan;
-  int st = build_plan(desc, &plan);
+  return desc ? winoconv_filter_transform_from(desc, weights, desc->dtype, u, stream) : fail(WINOCONV_ERR_INVALID_ARGUMENT, "null descriptor");
+}
+
+int winoconv_filter_transform_from(const winoconv_desc_t *desc, const void *weights, int w_dtype, void *u, void *stream) {
+  const Plan *plan_p = nullptr;
+  int st = plan_of<Plan>(desc, build_plan, &plan_p);
   if (st != WINOCONV_OK) return st;
+  const Plan &plan = *plan_p;
   if (!weights || !u) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "null weights or u");
   if ((st = winoconv_device_check()) != WINOCONV_OK) return st;
-  cudaError_t e = plan.direct  ? launch_direct_filter_transform(plan.dd, plan.dp, plan.dtype, weights, u, (cudaStream_t)stream)
+  if (w_dtype != plan.dtype && !(w_dtype == WINOCONV_F32 && plan.direct))
+    return fail(WINOCONV_ERR_UNSUPPORTED, "this layer's filter transform takes weights of its own dtype");
+  cudaError_t e = plan.direct  ? launch_direct_filter_transform(plan.dd, plan.dp, w_dtype, weights, u, (cudaStream_t)stream)
                   : plan.row   ? launch_rowfused_filter_transform(plan.rd, plan.rp, plan.dtype, weights, u, (cudaStream_t)stream)
                   : plan.fused ? launch_fused_filter_transform(plan.fg, plan.dtype, weights, u, (cudaStream_t)stream)
                                : launch_filter_transform(plan.g, plan.dtype, weights, u, (cudaStream_t)stream);
@@ -427,9 +500,10 @@ int winoconv_filter_transform(const winoconv_desc_t *desc, const void *weights, 
 static int forward_impl(const winoconv_desc_t *desc, const void *x, const void *u, const void *bias, void *y,
                         void *v_ws, size_t v_ws_bytes, void *m_ws, size_t m_ws_bytes, void *stream, float *stage_ms,
                         int32_t *launches) {
-  Plan plan;
-  int st = build_plan(desc, &plan);
+  const Plan *plan_p = nullptr;
+  int st = plan_of<Plan>(desc, build_plan, &plan_p);
   if (st != WINOCONV_OK) return st;
+  const Plan &plan = *plan_p;
   if (!x || !u || !y) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "null tensor pointer");
   if ((desc->epilogue & WINOCONV_EPI_BIAS) && !bias) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "EPI_BIAS set but bias is null");
   if (!aligned16(x) || !aligned16(u) || !aligned16(y)) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "tensors must be 16-byte aligned");
@@ -582,9 +656,10 @@ static int static_scratch_of_current_device(unsigned char **out) {
 
 int winoconv_forward_static(const winoconv_desc_t *desc, const void *x, const void *u, const void *bias, void *y,
                             void *stream) {
-  Plan plan;
-  int st = build_plan(desc, &plan);
+  const Plan *plan_p = nullptr;
+  int st = plan_of<Plan>(desc, build_plan, &plan_p);
   if (st != WINOCONV_OK) return st;
+  const Plan &plan = *plan_p;
   if ((st = winoconv_device_check()) != WINOCONV_OK) return st;
   const winoconv_plan_info_t &I = plan.info;
   if (plan.fused || (plan.row && I.input_ws_bytes_min == 0))
@@ -615,6 +690,72 @@ int winoconv_forward_static(const winoconv_desc_t *desc, const void *x, const vo
   if ((st = static_scratch_of_current_device(&base)) != WINOCONV_OK) return st;
   return forward_impl(desc, x, u, bias, y, base, v_bytes, base + v_bytes, WINOCONV_STATIC_SCRATCH_BYTES - v_bytes, stream,
                       nullptr, nullptr);
+}
+
+int winoconv_backward_plan(const winoconv_desc_t *desc, winoconv_backward_info_t *info) {
+  if (!info) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "null info");
+  const BackPlan *b = nullptr;
+  const int st = plan_of<BackPlan>(desc, build_back_plan, &b);
+  if (st != WINOCONV_OK) return st;
+  std::memset(info, 0, sizeof *info);
+  info->data_ok = b->data_ok; info->weight_ok = b->weight_ok;
+  info->c_stride = (desc->c_in + 7) / 8 * 8; info->k_stride = (desc->k_out + 7) / 8 * 8;
+  if (b->data_ok) info->data_filter_bytes = b->u_off[b->n_data];
+  if (b->weight_ok) info->weight_ws_bytes = b->wp.ws_bytes;
+  return WINOCONV_OK;
+}
+
+int winoconv_backward_filter_transform(const winoconv_desc_t *desc, const void *weights, int w_dtype, void *u, void *stream) {
+  const BackPlan *b = nullptr;
+  int st = plan_of<BackPlan>(desc, build_back_plan, &b);
+  if (st != WINOCONV_OK) return st;
+  if (!b->data_ok) return fail(WINOCONV_ERR_UNSUPPORTED, "no data-gradient kernel for this layer");
+  if (!weights || (!u && b->n_data > 0)) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "null weights or u");
+  if (w_dtype != WINOCONV_F32 && w_dtype != desc->dtype) return fail(WINOCONV_ERR_UNSUPPORTED, "weights must be f32 or of the layer's dtype");
+  if ((st = winoconv_device_check()) != WINOCONV_OK) return st;
+  for (int i = 0; i < b->n_data; ++i) {
+    const cudaError_t e = launch_direct_filter_transform(b->dd[i], b->dp[i], w_dtype, weights, (uint8_t *)u + b->u_off[i], (cudaStream_t)stream);
+    if (e != cudaSuccess) return cuda_fail(e, "data-gradient filter transform launch");
+  }
+  return WINOCONV_OK;
+}
+
+int winoconv_backward_data(const winoconv_desc_t *desc, const void *gy, const void *u, void *gx, void *stream) {
+  const BackPlan *b = nullptr;
+  int st = plan_of<BackPlan>(desc, build_back_plan, &b);
+  if (st != WINOCONV_OK) return st;
+  if (!b->data_ok) return fail(WINOCONV_ERR_UNSUPPORTED, "no data-gradient kernel for this layer");
+  if (!gy || !gx || (!u && b->n_data > 0)) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "null tensor pointer");
+  if (!aligned16(gy) || !aligned16(u) || !aligned16(gx)) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "tensors must be 16-byte aligned");
+  if ((st = winoconv_device_check()) != WINOCONV_OK) return st;
+  if (b->zero_fill) {
+    const cudaError_t e = cudaMemsetAsync(gx, 0, b->gx_bytes, (cudaStream_t)stream);
+    if (e != cudaSuccess) return cuda_fail(e, "clearing the data gradient");
+  }
+  for (int i = 0; i < b->n_data; ++i) {
+    const char *detail = "";
+    const cudaError_t e = launch_direct_forward(b->dd[i], b->dp[i], gy, (const uint8_t *)u + b->u_off[i], nullptr, gx, (cudaStream_t)stream, &detail);
+    if (e != cudaSuccess) return cuda_fail(e, "data gradient launch", detail);
+  }
+  return WINOCONV_OK;
+}
+
+int winoconv_backward_weight(const winoconv_desc_t *desc, const void *x, const void *gy, void *dw, int dw_dtype, float *dbias, void *ws,
+                             size_t ws_bytes, void *stream) {
+  const BackPlan *b = nullptr;
+  int st = plan_of<BackPlan>(desc, build_back_plan, &b);
+  if (st != WINOCONV_OK) return st;
+  if (!b->weight_ok) return fail(WINOCONV_ERR_UNSUPPORTED, "no weight-gradient kernel for this layer");
+  if (!x || !gy || !dw || !ws) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "null tensor pointer");
+  if ((desc->epilogue & WINOCONV_EPI_BIAS) && !dbias) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "EPI_BIAS set but dbias is null");
+  if (!aligned16(x) || !aligned16(gy) || !aligned16(ws)) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "tensors must be 16-byte aligned");
+  if (ws_bytes < b->wp.ws_bytes) return fail(WINOCONV_ERR_WORKSPACE, "weight-gradient scratch holds " + std::to_string(ws_bytes) + " bytes; needs " + std::to_string(b->wp.ws_bytes));
+  if (dw_dtype != WINOCONV_F32 && dw_dtype != WINOCONV_F16 && dw_dtype != WINOCONV_BF16) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "bad dw_dtype");
+  if ((st = winoconv_device_check()) != WINOCONV_OK) return st;
+  const char *detail = "";
+  const cudaError_t e = launch_wgrad(b->wd, b->wp, x, gy, dw, dw_dtype, dbias, ws, (cudaStream_t)stream, &detail);
+  if (e != cudaSuccess) return cuda_fail(e, "weight gradient launch", detail);
+  return WINOCONV_OK;
 }
 
 int winoconv_gemm_batched(int dtype, int product_dtype, int gemm_engine, int positions, int64_t tiles, int c_pad,
@@ -682,12 +823,13 @@ int winoconv_read_device_error(void *stream, uint32_t *code) {
   if (!code) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "null code");
   unsigned int host = 0, host2 = 0;
   cudaError_t e = read_and_clear_device_error((cudaStream_t)stream, &host);
-  unsigned int host3 = 0, host4 = 0;
+  unsigned int host3 = 0, host4 = 0, host5 = 0;
   if (e == cudaSuccess) e = read_and_clear_fused_error((cudaStream_t)stream, &host2);
   if (e == cudaSuccess) e = read_and_clear_row_error((cudaStream_t)stream, &host3);
   if (e == cudaSuccess) e = read_and_clear_direct_error((cudaStream_t)stream, &host4);
+  if (e == cudaSuccess) e = read_and_clear_wgrad_error((cudaStream_t)stream, &host5);
   if (e != cudaSuccess) return cuda_fail(e, "reading the device error word");
-  if (host == 0) host = host2 ? host2 : host3 ? host3 : host4;
+  if (host == 0) host = host2 ? host2 : host3 ? host3 : host4 ? host4 : host5;
   *code = host;
   if (host != 0) return fail(WINOCONV_ERR_TIMEOUT, "a bounded device wait gave up, code 0x" + [&] { char b[16]; snprintf(b, sizeof b, "%x", host); return std::string(b); }());
   return WINOCONV_OK;

@@ -47,15 +47,21 @@ constexpr int EPI_WARP0 = 4, EPI_WARPS = 8, SPLIT_WARP0 = 12, SPLIT_WARPS = 4;
 constexpr int STAGE_BYTES = 4096;      // epilogue staging per warp: 32 rows of 128 bytes
 constexpr int MAX_TAPS = 100;
 constexpr int BAR_BYTES = 512;
+constexpr int FIXED_BYTES = 1024 /*alignment*/ + EPI_WARPS * STAGE_BYTES + BAR_BYTES;
 
 enum ErrCode : unsigned { ERR_A_EMPTY = 0x401, ERR_B_EMPTY = 0x402, ERR_ACC = 0x403, ERR_A = 0x404, ERR_B = 0x405, ERR_EPI = 0x406, ERR_SPLIT = 0x407 };
 
 struct DGeom {
-  int N, K, oD, oH, oW, yH, yW;
-  int sD, sH, sW, pD, pH, pW, kD;
-  int TN, tn_shift, TH, PW;          // images and output rows of a block (TH * TN == 16), pixels of a slab row
-  int n_wb, n_hb, n_tiles, n_kb, n_items;
-  int n_ph, ph_h[4], ph_w[4], taps[4], tap0[4], T_hw;
+  int N, K, oD, oH;
+  int sD, sH, sW, pD, kD;
+  int yH[4], yW[4];                  // stored extents (of each variant)
+  long long y_off[4], ys_n, ys_d, ys_h, ys_w;   // first element of each variant, element strides
+  // A block's 128 rows are 16 groups of 8, numbered (output row, image group) with TH * TN == 16; the 8 rows of a group are
+  // 8 / TI pixels along W of TI images, image innermost (TI > 1 where 8 pixels would not divide a small image).
+  int TN, tn_shift, TH, TI, ti_shift, PW;   // PW: pixels of a slab row
+  int map_mode;                      // order of the tensor maps' dimensions: see tile_load
+  int n_wb, n_hb, n_tiles, n_kb, n_items, var_items;   // n_items = var_items x variants
+  int n_ph, n_var, org_h[4], org_w[4], taps[4], tap0[4], T_hw;   // parts of the taps: all of them per item, or one (variants)
   int n_chunks, ch_el, k_full, k_tail;   // channel chunks, channels per chunk, MMA K steps of a full and of the last chunk
   int units;                         // kD * T_hw * n_chunks: (tap, chunk) pairs of the whole reduction
   int G, split;
@@ -97,26 +103,50 @@ template <typename T> __device__ __forceinline__ void load_bias16(const T *bias,
   }
 }
 
-struct Tile { int n0, od, oh0, ow0; bool valid; };
-template <int MB> __device__ __forceinline__ Tile decode(const DGeom &g, unsigned tile) {
+struct MapSet { CUtensorMap m[4]; };      // the output of each variant
+
+struct Tile { int var, kb, n0, od, oh0, ow0; bool valid; };
+// item -> variant, channel block and the tile (of this CTA: a pair's CTAs take neighbouring tiles)
+template <int MB, bool PAIR> __device__ __forceinline__ Tile decode(const DGeom &g, int item, uint32_t rank) {
   Tile t;
+  t.var = g.n_var > 1 ? item / g.var_items : 0;
+  const unsigned it = (unsigned)(item - t.var * g.var_items), tb = it / (unsigned)g.n_kb;
+  t.kb = (int)(it - tb * (unsigned)g.n_kb);
+  const unsigned tile = PAIR ? 2u * tb + rank : tb;
   t.valid = tile < (unsigned)g.n_tiles;
   unsigned q = tile / (unsigned)g.n_wb;
-  t.ow0 = (int)(tile - q * (unsigned)g.n_wb) * 8;
+  t.ow0 = (int)(tile - q * (unsigned)g.n_wb) * (8 >> g.ti_shift);
   unsigned r = q / (unsigned)g.n_hb;
   t.oh0 = (int)(q - r * (unsigned)g.n_hb) * (MB * g.TH);
   q = r / (unsigned)g.oD;
   t.od = (int)(r - q * (unsigned)g.oD);
-  t.n0 = (int)q * g.TN;              // a tile past the end starts at an image past the end: TMA fills zeros
+  t.n0 = (int)q * (g.TN * g.TI);     // a tile past the end starts at an image past the end: TMA fills zeros
   return t;
+}
+
+// The maps order a tensor's dimensions so that a box lands in the block's row order: mode 0 [channel, W, image, H, depth];
+// mode 1 (TI > 1, TN == 1) [channel, image, W, H, depth]; mode 2 (TI > 1 and TN > 1, 2-D, the batch a multiple of TI)
+// [channel, image within a group, W, image group, H].
+template <bool PAIR>
+__device__ __forceinline__ void tile_load(const DGeom &g, uint32_t dst, const CUtensorMap *map, uint32_t bar, int c, int w, int n, int h, int d) {
+  const int c1 = g.map_mode == 0 ? w : g.map_mode == 1 ? n : 0, c2 = g.map_mode == 0 ? n : w;
+  const int c3 = g.map_mode == 2 ? n >> g.ti_shift : h, c4 = g.map_mode == 2 ? h : d;
+  if (PAIR) tma_load_5d_pair(dst, map, bar, c, c1, c2, c3, c4);
+  else tma_load_5d(dst, map, bar, c, c1, c2, c3, c4);
+}
+__device__ __forceinline__ void tile_store(const DGeom &g, const CUtensorMap *map, uint32_t src, int k, int w, int n, int h, int d) {
+  const int c1 = g.map_mode == 0 ? w : g.map_mode == 1 ? n : 0, c2 = g.map_mode == 0 ? n : w;
+  const int c3 = g.map_mode == 2 ? n >> g.ti_shift : h, c4 = g.map_mode == 2 ? h : d;
+  tma_store_5d(map, src, k, c1, c2, c3, c4);
 }
 
 // Calls body(kd, p, ch, t0, t1) for the steps (depth tap, polyphase part, channel chunk) whose taps [t0, t1) fall into this
 // CTA's share [u0, u1) of the reduction, until it returns false; returns whether all of them ran.
-template <typename F> __device__ __forceinline__ bool for_steps(const DGeom &g, int u0, int u1, F &&body) {
+template <typename F> __device__ __forceinline__ bool for_steps(const DGeom &g, int var, int u0, int u1, F &&body) {
   int s0 = 0;
+  const int p0 = g.n_var > 1 ? var : 0, p1 = g.n_var > 1 ? var + 1 : g.n_ph;
   for (int kd = 0; kd < g.kD; ++kd)
-    for (int p = 0; p < g.n_ph; ++p) {
+    for (int p = p0; p < p1; ++p) {
       const int tp = g.taps[p];
       for (int ch = 0; ch < g.n_chunks; ++ch, s0 += tp) {
         const int t0 = max(0, u0 - s0), t1 = min(tp, u1 - s0);
@@ -129,7 +159,7 @@ template <typename F> __device__ __forceinline__ bool for_steps(const DGeom &g, 
 template <typename T, int BN, int MB, bool PAIR>
 __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
     direct_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_u,
-                  const __grid_constant__ CUtensorMap map_y, T *__restrict__ y, const T *__restrict__ bias,
+                  const __grid_constant__ MapSet maps_y, T *__restrict__ y, const T *__restrict__ bias,
                   const __grid_constant__ DGeom g, const __grid_constant__ DSmem sl, uint32_t idesc) {
   constexpr bool F32 = std::is_same<T, float>::value;
   constexpr int COLS = OutWord<T>::COLS;            // output columns of one 128-byte staging row
@@ -153,20 +183,28 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
   unsigned *err = &g_direct_error;
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;   // the warp index in a uniform register
-  if (threadIdx.x == 0) {
-    for (int i = 0; i < sl.n_a; ++i) { mbar_init(a_full(i), 1); mbar_init(a_empty(i), N_ISSUE); mbar_init(a_split(i), SPLIT_WARPS); }
-    for (int i = 0; i < sl.n_b; ++i) { mbar_init(b_full(i), 1); mbar_init(b_empty(i), N_ISSUE); }
-    for (int i = 0; i < 2; ++i) { mbar_init(acc_full(i), N_ISSUE); mbar_init(acc_empty(i), PAIR ? 2 * EPI_WARPS : EPI_WARPS); }
-    *abort_word = 0u;
+  // Set-up, spread over warps and lanes (it is a fifth of a one-wave launch): descriptors fetched, barriers initialised,
+  // tensor memory allocated.
+  if (warp == 1 && lane == 0) { prefetch_map(&map_x); prefetch_map(&map_u); prefetch_map(&maps_y.m[0]); }
+  if (warp == 0) {
+    if (lane < 8) {
+      mbar_init(a_full(lane), 1); mbar_init(a_empty(lane), N_ISSUE); mbar_init(a_split(lane), SPLIT_WARPS);
+    } else if (lane < 16) {
+      mbar_init(b_full(lane - 8), 1); mbar_init(b_empty(lane - 8), N_ISSUE);
+    } else if (lane < 18) {
+      mbar_init(acc_full(lane - 16), N_ISSUE); mbar_init(acc_empty(lane - 16), PAIR ? 2 * EPI_WARPS : EPI_WARPS);
+    } else if (lane == 18) {
+      *abort_word = 0u;
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    prefetch_map(&map_x); prefetch_map(&map_u); prefetch_map(&map_y);
   }
-  const uint32_t rank = PAIR ? cluster_ctarank() : 0u;
-  if (PAIR) { __syncthreads(); cluster_sync_all(); }
-  if (warp == 2) tmem_alloc<PAIR>(tmem_slot, 2 * ACC);
+  const uint32_t crank = PAIR ? cluster_ctarank() : 0u, rank = crank & 1u;   // rank within the pair
+  const bool leader = rank == 0;                   // issues the MMAs of the pair
+  const uint32_t tmem_cols = g.split > 1 ? ACC : 2 * ACC;      // a shared item needs one accumulator
+  if (warp == 2) tmem_alloc<PAIR>(tmem_slot, tmem_cols);
   tc_fence_before();
   __syncthreads();
-  if (PAIR) cluster_sync_all();
+  if (PAIR) cluster_sync_all();      // the barriers of both CTAs exist before either arrives at the other's
   tc_fence_after();
   uint32_t tmem;
   asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot));
@@ -177,16 +215,16 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
   // work of this CTA: items item0, item0 + step, ... and the share [u0, u1) of each one's reduction
   int item0, item_step, u0 = 0, u1 = g.units;
   uint32_t part = 0;
-  if (PAIR) { item0 = (int)(blockIdx.x >> 1); item_step = (int)(gridDim.x >> 1); }
-  else if (g.split > 1) {
-    item0 = (int)blockIdx.x / g.split;
+  const int unit_cta = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;     // a CTA, or a pair
+  if (g.split > 1) {
+    item0 = unit_cta / g.split;
     item_step = g.n_items;
-    part = (uint32_t)((int)blockIdx.x - item0 * g.split);
+    part = (uint32_t)(unit_cta - item0 * g.split);
     u0 = (int)((long long)g.units * part / g.split);
     u1 = (int)((long long)g.units * (part + 1) / g.split);
-  } else { item0 = (int)blockIdx.x; item_step = (int)gridDim.x; }
+  } else { item0 = unit_cta; item_step = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x; }
   // one channel block whose whole filter fits the ring: loaded once, its stages are never handed back
-  const bool resident = g.n_kb == 1 && g.split == 1 && g.kD * g.n_ph * g.n_chunks * ((g.taps[0] + g.G - 1) / g.G) <= sl.n_b;
+  const bool resident = g.n_kb == 1 && g.split == 1 && g.n_var == 1 && g.kD * g.n_ph * g.n_chunks * ((g.taps[0] + g.G - 1) / g.G) <= sl.n_b;
   bool alive = true;
 
   if (warp == 0) {
@@ -194,21 +232,15 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
     int s = 0;
     uint32_t ph = 1;
     for (int item = item0; item < g.n_items && alive; item += item_step) {
-      const unsigned tb = (unsigned)item / (unsigned)g.n_kb;
-      const Tile t = decode<MB>(g, PAIR ? 2u * tb + rank : tb);
-      alive = for_steps(g, u0, u1, [&](int kd, int p, int ch, int t0, int t1) -> bool {
+      const Tile t = decode<MB, PAIR>(g, item, rank);
+      alive = for_steps(g, t.var, u0, u1, [&](int kd, int p, int ch, int t0, int t1) -> bool {
         (void)t0; (void)t1;
         if (!mbar_wait_warp(a_empty(s), ph, abort_word, err, ERR_A_EMPTY)) return false;
         if (lane == 0) {
           const uint32_t dst = base + (uint32_t)(s * sl.a_bytes);
-          const int cw = g.sW * t.ow0 + g.ph_w[p] - g.pW, chh = g.sH * t.oh0 + g.ph_h[p] - g.pH, cd = g.sD * t.od + kd - g.pD;
-          if (PAIR) {
-            if (rank == 0) mbar_expect_tx(a_full(s), 2u * (uint32_t)sl.slab_bytes);
-            tma_load_5d_pair(dst, &map_x, a_full(s), ch * g.ch_el, cw, t.n0, chh, cd);
-          } else {
-            mbar_expect_tx(a_full(s), (uint32_t)sl.slab_bytes);
-            tma_load_5d(dst, &map_x, a_full(s), ch * g.ch_el, cw, t.n0, chh, cd);
-          }
+          const int cw = g.sW * t.ow0 + g.org_w[p], chh = g.sH * t.oh0 + g.org_h[p], cd = g.sD * t.od + kd - g.pD;
+          if (!PAIR || leader) mbar_expect_tx(a_full(s), (PAIR ? 2u : 1u) * (uint32_t)sl.slab_bytes);
+          tile_load<PAIR>(g, dst, &map_x, a_full(s), ch * g.ch_el, cw, t.n0, chh, cd);
         }
         if (++s == sl.n_a) { s = 0; ph ^= 1u; }
         return true;
@@ -224,16 +256,16 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
     uint32_t ph = 1;
     for (int item = item0; item < g.n_items && alive; item += item_step) {
       if (resident && item != item0) break;
-      const int kb = item - (int)((unsigned)item / (unsigned)g.n_kb) * g.n_kb;
-      const int row = kb * BN + (PAIR ? (int)rank * BNH : 0);
-      alive = for_steps(g, u0, u1, [&](int kd, int p, int ch, int t0, int t1) -> bool {
+      const Tile tl = decode<MB, PAIR>(g, item, rank);
+      const int row = tl.kb * BN + (PAIR ? (int)rank * BNH : 0);
+      alive = for_steps(g, tl.var, u0, u1, [&](int kd, int p, int ch, int t0, int t1) -> bool {
         const int tap = kd * g.T_hw + g.tap0[p];
         for (int t = t0; t < t1; t += g.G) {
           if (!mbar_wait_warp(b_empty(s), ph, abort_word, err, ERR_B_EMPTY)) return false;
           const int n = min(g.G, t1 - t);
           if (lane == 0) {
             const uint32_t bytes = (uint32_t)(n * sl.b_tile);
-            if (!PAIR || rank == 0) mbar_expect_tx(b_full(s), PAIR ? 2u * bytes : bytes);
+            if (!PAIR || leader) mbar_expect_tx(b_full(s), PAIR ? 2u * bytes : bytes);
             uint32_t dst = base + (uint32_t)(sl.off_b + s * sl.b_bytes);
             for (int j = 0; j < n; ++j, dst += (uint32_t)sl.b_tile) {
               if (F32) {     // [tap][hi / lo][K][C]
@@ -257,8 +289,9 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
     }
   } else if (warp < 2 + N_ISSUE) {
     // ---------------------------------------------------------------- MMA issue (rank 0 of a pair issues for both CTAs)
-    if (rank == 0) {
+    if (leader) {
       const int me = warp - 2;
+      const uint16_t pair_mask = (uint16_t)(3u << (crank & ~1u));
       int as = 0, bs = 0;
       uint32_t a_ph = 0, b_ph = 0, n_done = 0;
       for (int item = item0; item < g.n_items && alive; item += item_step, ++n_done) {
@@ -269,7 +302,7 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
         uint32_t acc = 0;
         const bool loaded = resident && n_done > 0;
         if (resident) { bs = 0; }
-        alive = for_steps(g, u0, u1, [&](int kd, int p, int ch, int t0, int t1) -> bool {
+        alive = for_steps(g, g.n_var > 1 ? item / g.var_items : 0, u0, u1, [&](int kd, int p, int ch, int t0, int t1) -> bool {
           if (!mbar_wait_warp(F32 ? a_split(as) : a_full(as), a_ph, abort_word, err, ERR_A)) return false;
           tc_fence_after();
           const uint32_t a_lo = desc_lo(base + (uint32_t)(as * sl.a_bytes)) + (uint32_t)(me * g.mb_off16);
@@ -313,15 +346,15 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
               }
             }
             acc = 1u;
-            if (!resident && elect_one()) umma_commit<PAIR>(b_empty(bs));
+            if (!resident && elect_one()) umma_commit<PAIR>(b_empty(bs), pair_mask);
             if (++bs == sl.n_b) { bs = 0; b_ph ^= 1u; }
           }
-          if (elect_one()) umma_commit<PAIR>(a_empty(as));
+          if (elect_one()) umma_commit<PAIR>(a_empty(as), pair_mask);
           if (++as == sl.n_a) { as = 0; a_ph ^= 1u; }
           return true;
       });
         if (resident) b_ph = 0;
-        if (elect_one()) umma_commit<PAIR>(acc_full(buf));
+        if (elect_one()) umma_commit<PAIR>(acc_full(buf), pair_mask);
       }
     }
   } else if (F32 && warp >= SPLIT_WARP0) {
@@ -330,7 +363,7 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
     uint32_t ph = 0;
     const int st = threadIdx.x - SPLIT_WARP0 * 32;
     for (int item = item0; item < g.n_items && alive; item += item_step) {
-      alive = for_steps(g, u0, u1, [&](int kd, int p, int ch, int t0, int t1) -> bool {
+      alive = for_steps(g, g.n_var > 1 ? item / g.var_items : 0, u0, u1, [&](int kd, int p, int ch, int t0, int t1) -> bool {
         (void)kd; (void)p; (void)ch; (void)t0; (void)t1;
         if (!mbar_wait_warp(a_full(s), ph, abort_word, err, ERR_SPLIT)) return false;
         float4 *hi = reinterpret_cast<float4 *>(base_ptr + s * sl.a_bytes);
@@ -360,14 +393,13 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
     constexpr int CH_PER_MB = BN / COLS, N_CH = MB * CH_PER_MB;
     const int tnm = g.TN - 1;
     // this lane's pixel within the block, and the staging row its output goes to (-1: none)
-    const int grp = q * 4 + (lane >> 3), h_l = grp >> g.tn_shift, n_l = grp & tnm, w_l = lane & 7;
+    const int grp = q * 4 + (lane >> 3), h_l = grp >> g.tn_shift, w_l = (lane & 7) >> g.ti_shift, i_l = lane & (g.TI - 1);
     int srow = lane;
-    if (pool) srow = ((h_l | w_l) & 1) ? -1 : (g.TN == 1 ? ((lane >> 4) << 2) + (w_l >> 1) : (n_l << 2) + (w_l >> 1));
+    if (pool) srow = ((h_l | w_l) & 1) ? -1 : ((g.TN == 1 ? lane >> 4 : grp & tnm) << 2) + ((w_l >> 1) << g.ti_shift) + i_l;
     uint32_t n_done = 0;
     for (int item = item0; item < g.n_items; item += item_step, ++n_done) {
-      const unsigned tb = (unsigned)item / (unsigned)g.n_kb;
-      const int kb = item - (int)tb * g.n_kb;
-      const Tile t = decode<MB>(g, PAIR ? 2u * tb + rank : tb);
+      const Tile t = decode<MB, PAIR>(g, item, rank);
+      const int kb = t.kb, yH = g.yH[t.var], yW = g.yW[t.var];
       const int buf = (int)(n_done & 1u);
       if (!mbar_wait_warp(acc_full(buf), (n_done >> 1) & 1u, abort_word, err, ERR_EPI)) { alive = false; break; }
       if (*abort_word != 0u) { alive = false; break; }
@@ -415,7 +447,7 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
         if (pool) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
-            o[i] = OutWord<T>::max2(o[i], __shfl_xor_sync(0xffffffffu, o[i], 1));
+            o[i] = OutWord<T>::max2(o[i], __shfl_xor_sync(0xffffffffu, o[i], g.TI));
             o[i] = OutWord<T>::max2(o[i], __shfl_xor_sync(0xffffffffu, o[i], 8 << g.tn_shift));
           }
         }
@@ -433,13 +465,13 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
                          "r"(o[4 * v + 1]), "r"(o[4 * v + 2]), "r"(o[4 * v + 3]) : "memory");
         }
         // first pixel of this warp's rows
-        const int g0 = q * 4, h0 = g0 >> g.tn_shift, n0 = g0 & tnm;
+        const int g0 = q * 4, h0 = g0 >> g.tn_shift, n0 = (g0 & tnm) << g.ti_shift;
         if (g.y_tma) {
           fence_async_smem();
           __syncwarp();
-          if (lane == 0 && (pool ? (oh_b + h0) >> 1 : oh_b + h0) < g.yH && t.n0 + n0 < g.N && (pool ? t.ow0 >> 1 : t.ow0) < g.yW) {
-            if (pool) tma_store_5d(&map_y, stage, k0, t.ow0 >> 1, t.n0 + n0, (oh_b + h0) >> 1, t.od);
-            else tma_store_5d(&map_y, stage, k0, t.ow0, t.n0 + n0, oh_b + h0, t.od);
+          if (lane == 0 && (pool ? (oh_b + h0) >> 1 : oh_b + h0) < yH && t.n0 + n0 < g.N && (pool ? t.ow0 >> 1 : t.ow0) < yW) {
+            if (pool) tile_store(g, &maps_y.m[t.var], stage, k0, t.ow0 >> 1, t.n0 + n0, (oh_b + h0) >> 1, t.od);
+            else tile_store(g, &maps_y.m[t.var], stage, k0, t.ow0, t.n0 + n0, oh_b + h0, t.od);
             bulk_commit();
           }
         } else {            // rows of y are not 16-byte aligned: a row of the staging tile per step, consecutive lanes, consecutive channels
@@ -450,16 +482,16 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
             int oh, ow, n;
             if (pool) {
               const int a = rr >> 2;
-              ow = (t.ow0 >> 1) + (rr & 3);
+              ow = (t.ow0 >> 1) + ((rr & 3) >> g.ti_shift);
               oh = ((oh_b + h0) >> 1) + (g.TN == 1 ? a : 0);
-              n = t.n0 + (g.TN == 1 ? 0 : a);
+              n = t.n0 + ((g.TN == 1 ? 0 : a) << g.ti_shift) + (rr & (g.TI - 1));
             } else {
               const int gg = g0 + (rr >> 3);
-              oh = oh_b + (gg >> g.tn_shift); n = t.n0 + (gg & tnm); ow = t.ow0 + (rr & 7);
+              oh = oh_b + (gg >> g.tn_shift); n = t.n0 + ((gg & tnm) << g.ti_shift) + (rr & (g.TI - 1)); ow = t.ow0 + ((rr & 7) >> g.ti_shift);
             }
-            if (oh >= g.yH || ow >= g.yW || n >= g.N) continue;
+            if (oh >= yH || ow >= yW || n >= g.N) continue;
             const T *src = reinterpret_cast<const T *>(stage_ptr + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) + (lane & 3) * 4);
-            T *dst = y + ((((long long)n * g.oD + t.od) * g.yH + oh) * g.yW + ow) * g.K + k0 + lane * E;
+            T *dst = y + g.y_off[t.var] + n * g.ys_n + t.od * g.ys_d + oh * g.ys_h + ow * g.ys_w + k0 + lane * E;
 #pragma unroll
             for (int e = 0; e < E; ++e)
               if (k0 + lane * E + e < g.K) dst[e] = src[e];
@@ -469,9 +501,9 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
       }
       if (!handed && lane == 0) { if (PAIR) mbar_arrive_rank0(acc_empty(buf)); else mbar_arrive(acc_empty(buf)); }
     }
-    if (lane == 0) bulk_wait_all();
+    if (lane == 0) bulk_wait_read();     // the staging rows are read before the CTA's shared memory goes
   }
-  if (!PAIR && g.split > 1) {
+  if (g.split > 1) {
     // ---------------------------------------------------------------- the cluster's shares of one item added up
     // Every CTA puts its accumulator into its own shared memory (the operand rings are idle by then) and finishes 1 / split
     // of the rows from all of them.
@@ -497,12 +529,11 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
     }
     cluster_sync_all();
     if (epi && *abort_word == 0u) {
-      const unsigned tb = (unsigned)item0 / (unsigned)g.n_kb;
-      const int kb = item0 - (int)tb * g.n_kb;
-      const Tile t = decode<MB>(g, tb);
+      const Tile t = decode<MB, PAIR>(g, item0, rank);
+      const int kb = t.kb;
       const bool relu = (g.epilogue & WINOCONV_EPI_RELU) != 0, has_bias = (g.epilogue & WINOCONV_EPI_BIAS) != 0;
       const bool pool = (g.epilogue & WINOCONV_EPI_POOL2) != 0;
-      constexpr int V = 16 / (int)sizeof(T);       // outputs of one 16-byte vector
+      constexpr int V = 4;                         // a warp reads 512 consecutive bytes of a row of each peer
       const int rows = MB * BM / g.split, tid = threadIdx.x - EPI_WARP0 * 32;
       const int work = (pool ? rows / 4 : rows) * (BN / V);
       for (int i = tid; i < work; i += EPI_WARPS * 32) {
@@ -514,53 +545,53 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
         const int n_src = pool ? 4 : 1;
         for (int a = 0; a < n_src; ++a) {
           int row = (int)part * rows;
-          if (pool) {    // pooled pixel rr: image, row pair and column pair within this CTA's rows
-            const int wp = rr & 3, np = (rr >> 2) & (g.TN - 1), hp = rr >> (2 + g.tn_shift);
-            row += (((2 * hp + (a >> 1)) << g.tn_shift) + np) * 8 + 2 * wp + (a & 1);
+          if (pool) {    // pooled pixel rr: row pair, image group, column pair and image within this CTA's rows
+            const int wp = (rr & 3) >> g.ti_shift, np = (rr >> 2) & (g.TN - 1), hp = rr >> (2 + g.tn_shift);
+            row += (((2 * hp + (a >> 1)) << g.tn_shift) + np) * 8 + ((2 * wp + (a & 1)) << g.ti_shift) + (rr & (g.TI - 1));
           } else row += rr;
           float f[V];
 #pragma unroll
           for (int v = 0; v < V; ++v) f[v] = 0.f;
           const uint32_t src = base + (uint32_t)((row * ROW_F + c) * 4);
-          for (int pr = 0; pr < g.split; ++pr) {
-            const uint32_t rs = map_to_rank(src, (uint32_t)pr);
+          // all peers' values in flight at once: one remote read takes as long as eight
+          auto add_peers = [&](auto n_peers) {
+            constexpr int S = decltype(n_peers)::value;
+            float4 u[S];
 #pragma unroll
-            for (int v = 0; v < V; v += 4) {
-              const float4 u = ld_cluster_f4(rs + v * 4);
-              f[v] += u.x; f[v + 1] += u.y; f[v + 2] += u.z; f[v + 3] += u.w;
+            for (int i2 = 0; i2 < S; ++i2) {
+              const uint32_t pr = ((uint32_t)i2 + part) & (uint32_t)(S - 1);     // every CTA starts at another peer
+              u[i2] = ld_cluster_f4(map_to_rank(src, PAIR ? 2u * pr + rank : pr));   // (of a pair's, those with the same pixels)
             }
-          }
+#pragma unroll
+            for (int i2 = 0; i2 < S; ++i2) { f[0] += u[i2].x; f[1] += u[i2].y; f[2] += u[i2].z; f[3] += u[i2].w; }
+          };
+          if (g.split == 2) add_peers(std::integral_constant<int, 2>());
+          else if (g.split == 4) add_peers(std::integral_constant<int, 4>());
+          else add_peers(std::integral_constant<int, 8>());
           if (a == 0) {
             const int mb = row >> 7, grp = (row & 127) >> 3;
-            oh = t.oh0 + mb * g.TH + (grp >> g.tn_shift); n = t.n0 + (grp & (g.TN - 1)); ow = t.ow0 + (row & 7);
+            oh = t.oh0 + mb * g.TH + (grp >> g.tn_shift); n = t.n0 + ((grp & (g.TN - 1)) << g.ti_shift) + (row & (g.TI - 1));
+            ow = t.ow0 + ((row & 7) >> g.ti_shift);
           }
 #pragma unroll
           for (int v = 0; v < V; ++v) best[v] = a == 0 ? f[v] : fmaxf(best[v], f[v]);
         }
         if (pool) { oh >>= 1; ow >>= 1; }
-        if (oh >= g.yH || ow >= g.yW || n >= g.N) continue;
+        if (oh >= g.yH[t.var] || ow >= g.yW[t.var] || n >= g.N || !t.valid) continue;
         if (has_bias) {
-          float b[V];
-          load_bias16<T>(bias, k, g.K, g.bias_vec, b);
 #pragma unroll
-          for (int v = 0; v < V; ++v) best[v] += b[v];
+          for (int v = 0; v < V; ++v) best[v] += k + v < g.K ? Elem<T>::load(bias + k + v) : 0.f;
         }
-        uint32_t o[4];
+        if (relu) {
 #pragma unroll
-        for (int v = 0; v < 4; ++v) {
-          if constexpr (F32) o[v] = __float_as_uint(best[v]);
-          else o[v] = Pair16<T>::round(best[2 * v], best[2 * v + 1]);
-          if (relu) o[v] = OutWord<T>::max2(o[v], 0u);
+          for (int v = 0; v < V; ++v) best[v] = fmaxf(best[v], 0.f);
         }
-        T *dst = y + ((((long long)n * g.oD + t.od) * g.yH + oh) * g.yW + ow) * g.K + k;
-        if (g.y_tma) *reinterpret_cast<uint4 *>(dst) = make_uint4(o[0], o[1], o[2], o[3]);
+        T *dst = y + g.y_off[t.var] + n * g.ys_n + t.od * g.ys_d + oh * g.ys_h + ow * g.ys_w + k;
+        if (g.y_tma) VecIO<T, 4>::store(dst, best);       // K a multiple of 8 (4): whole, aligned vectors
         else {
 #pragma unroll
           for (int v = 0; v < V; ++v)
-            if (k + v < g.K) {
-              if constexpr (F32) dst[v] = __uint_as_float(o[v]);
-              else *reinterpret_cast<unsigned short *>(dst + v) = (unsigned short)(o[v >> 1] >> ((v & 1) * 16));
-            }
+            if (k + v < g.K) Elem<T>::store(dst + v, best[v]);
         }
       }
     }
@@ -571,7 +602,7 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
   if (PAIR) cluster_sync_all();
   if (warp == 2) {
     tc_fence_after();
-    tmem_free<PAIR>(tmem, 2 * ACC);
+    tmem_free<PAIR>(tmem, tmem_cols);
   }
 }
 
@@ -579,7 +610,7 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
 // The weights are read through strides, so a data gradient's filter (channels exchanged, taps mirrored) is the same kernel.
 struct FGeomD {
   int O, I, Ip, kD, n_hw;
-  long long s_o, s_i, s_d;
+  long long s_o, s_i, s_d, off_d;
   int off_hw[MAX_TAPS];       // element offset of each (h, w) tap in walking order
 };
 template <typename TW, typename T>
@@ -592,7 +623,7 @@ __global__ void __launch_bounds__(256) direct_filter_kernel(const TW *__restrict
   const bool real = i < f.I;
   const int kd = blockIdx.y;
   for (int t = blockIdx.z; t < f.n_hw; t += gridDim.z) {
-    const float v = real ? Elem<TW>::load(src + kd * f.s_d + f.off_hw[t]) : 0.f;
+    const float v = real ? Elem<TW>::load(src + f.off_d + kd * f.s_d + f.off_hw[t]) : 0.f;
     const long long tap = (long long)kd * f.n_hw + t;
     if constexpr (std::is_same<T, float>::value) {
       const float h = tf32_round(v);
@@ -621,28 +652,129 @@ static int sm_count_of_current_device() {
 
 using namespace dconv;
 
-// Estimated clocks of a launch with this configuration on 148 SMs, from the per-instruction clocks of the rate probe (an
-// instruction of N columns: 48 / 65 / 129 clocks for N = 64 / 128 / 256) and 128 B of shared memory per clock.
-static double estimate(const DirectPlan &p, double k_steps, int n_steps, int tiles, int n_kb, bool f32) {
-  const double t_mma = p.BN == 256 ? 129 : p.BN == 128 ? 65 : 48;
+// Clusters of this many CTAs that 148 SMs hold at once, one CTA per SM (cudaOccupancyMaxActiveClusters on B200: clusters of 4
+// and 8 do not fill every GPC).
+static int clusters_at_once(int width) { return width == 1 ? 148 : width == 2 ? 74 : width == 4 ? 33 : 15; }
+
+// Estimated clocks of a launch with this configuration on 148 SMs.  An item takes as long as its MMAs (66 / 130 clocks an
+// instruction of 128 / 256 columns; of 64 columns 60 from one issuing thread, 48 from two), its shared-memory traffic at 128 B
+// per clock, or its loads: about 28 B per clock and SM from L2 when all SMs load, at most 60 for one.  Set-up, first loads
+// and drain of a launch were measured at about 8000 clocks, 800 more for a pair, 4600 for a cluster's exchange of partial sums.
+static double estimate(const DirectPlan &p, double k_steps, int n_steps, int n_var, bool f32) {
+  const double t_mma = p.BN == 256 ? 130 : p.BN == 128 ? 66 : p.MB >= 2 ? 48 : 60;
+  const int bn_own = p.pair ? p.BN / 2 : p.BN;
   const double mma = k_steps * p.MB * t_mma * (f32 ? 3 : 1);
-  const double bytes = k_steps * p.MB * (f32 ? 3 : 1) * (4096.0 + (p.pair ? p.BN / 2 : p.BN) * 32.0) +
-                       n_steps * (double)p.slab_bytes * (f32 ? 4 : 1) + k_steps * (p.pair ? p.BN / 2 : p.BN) * 32.0 * (f32 ? 2 : 1);
-  const double item = std::max(mma, bytes / 128.0);
-  const int slots = p.pair ? 74 : 148 / p.split;
-  const int items = (p.pair ? (tiles + 1) / 2 : tiles) * n_kb;
-  const double waves = (items + slots - 1) / slots;
+  const double loads = n_steps * (double)p.slab_bytes + k_steps * bn_own * 32.0 * (f32 ? 2 : 1);
+  const double smem = k_steps * p.MB * (f32 ? 3 : 1) * (4096.0 + bn_own * 32.0) + loads + (f32 ? 3.0 * n_steps * p.slab_bytes : 0.0);
+  const int width = (p.pair ? 2 : 1) * p.split;
+  const int slots = clusters_at_once(width);
+  const int n_items = p.n_items * n_var;
+  const double waves = (n_items + slots - 1) / slots;
+  const double active = std::min(148.0, (double)n_items * width);
+  const double l2 = loads / std::min(60.0, 28.0 * 148 / active);
+  const double item = std::max(mma, std::max(smem / 128.0, l2));
   const double epi = 400.0 + 350.0 * p.MB * p.BN / 64;
-  const double fill = 3000.0;
-  if (p.split > 1) return fill + waves * (item / p.split + 3000.0 + (waves > 1 ? fill : 0.0));
-  return fill + waves * std::max(item + 200.0, epi) + epi;
+  const double tail = 1500.0 * ((p.MB * p.BN / (f32 ? 32 : 64) + 1) / 2 - 1);     // the last epilogue
+  if (p.split > 1) return 8000.0 + (p.pair ? 800.0 : 0.0) + item / p.split + 4000.0 + 10.0 * p.BN * p.MB;
+  return 8000.0 + (p.pair ? 800.0 : 0.0) + waves * std::max(item + 200.0, epi) + tail;
+}
+
+// Stages of the slab and filter rings within `budget` bytes, the ring that looks less far ahead growing first; taps per filter
+// stage (G) so that a stage is worth its barrier round trip.
+static bool ring_depths(DirectPlan &q, int taps, int budget) {
+  for (int G = std::max(1, std::min(taps, 24 * 1024 / q.b_tile)); G >= 1; --G) {
+    q.G = G;
+    q.b_bytes = (G * q.b_tile + 1023) / 1024 * 1024;
+    int na = 2, nb = 2;
+    if (2 * q.a_bytes + 2 * q.b_bytes > budget) {
+      na = 1;
+      if (q.a_bytes + 2 * q.b_bytes > budget) continue;
+    }
+    const double groups = (taps + G - 1) / G;
+    for (bool grew = true; grew;) {
+      grew = false;
+      const bool want_b = nb / groups <= na;
+      for (int turn = 0; turn < 2 && !grew; ++turn) {
+        const bool b = turn == 0 ? want_b : !want_b;
+        if (b && nb < 8 && na * q.a_bytes + (nb + 1) * q.b_bytes <= budget) { ++nb; grew = true; }
+        if (!b && na < 8 && (na + 1) * q.a_bytes + nb * q.b_bytes <= budget) { ++na; grew = true; }
+      }
+    }
+    q.n_a = na; q.n_b = nb;
+    return true;
+  }
+  return false;
+}
+
+void direct_forward_desc(DirectDesc *q, int dtype, int N, int C, int K, const int in[3], const int ker[3], const int stride[3],
+                         const int pad[3], const int out[3], int yH, int yW, unsigned epilogue, int weight_layout) {
+  std::memset(q, 0, sizeof *q);
+  q->dtype = dtype; q->N = N; q->C = q->Cw = C; q->K = K; q->D = in[0]; q->H = in[1]; q->W = in[2];
+  q->oD = out[0]; q->oH = out[1]; q->oW = out[2]; q->yH = yH; q->yW = yW;
+  q->sD = stride[0]; q->sH = stride[1]; q->sW = stride[2]; q->pD = pad[0];
+  q->kD = q->kD_w = ker[0]; q->kH_w = ker[1]; q->kW_w = ker[2];
+  q->d0 = 0; q->ds = 1;
+  q->ys_w = K; q->ys_h = q->ys_w * yW; q->ys_d = q->ys_h * yH; q->ys_n = q->ys_d * out[0];
+  q->epilogue = epilogue; q->weight_layout = weight_layout;
+  for (int a = 0; a < stride[1]; ++a)
+    for (int b = 0; b < stride[2]; ++b) {
+      DirectPart p;
+      std::memset(&p, 0, sizeof p);
+      p.th = (ker[1] - a + stride[1] - 1) / stride[1]; p.tw = (ker[2] - b + stride[2] - 1) / stride[2];
+      if (p.th <= 0 || p.tw <= 0) continue;
+      p.org_h = a - pad[1]; p.org_w = b - pad[2];
+      p.t0_h = a; p.ts_h = stride[1]; p.t0_w = b; p.ts_w = stride[2];
+      q->parts[q->n_parts++] = p;
+    }
+}
+
+// grad_x[i] = sum over taps t with (i + p - t) divisible by s of grad_y[(i + p - t) / s] w[t].  For inputs i = s j + r these are
+// the taps t = t0 + s m, t0 = (r + p) mod s, and the gradient is a stride-1 convolution of grad_y over j with the taps m
+// mirrored: a part per residue (r_h, r_w), writing every s-th pixel.
+bool direct_grad_desc(DirectDesc *q, int dtype, int N, int C, int K, int Km, const int in[3], const int ker[3], const int stride[3],
+                      const int pad[3], const int out[3], int weight_layout, int e, bool *zero_fill) {
+  std::memset(q, 0, sizeof *q);
+  struct Axis { int r, m, org, t0, n; };       // residue, taps, first input of output 0, last tap (mirrored order starts there), outputs
+  auto axis = [&](int i, int r) {
+    Axis a;
+    const int s = stride[i], t0 = (r + pad[i]) % s;
+    a.r = r;
+    a.m = ker[i] > t0 ? (ker[i] - t0 + s - 1) / s : 0;
+    a.org = (r + pad[i] - t0) / s - (a.m - 1);
+    a.t0 = t0 + s * (a.m - 1);
+    a.n = (in[i] - r + s - 1) / s;
+    return a;
+  };
+  const Axis dz = axis(0, e);
+  q->dtype = dtype; q->N = N; q->C = Km; q->Cw = K; q->K = C; q->D = out[0]; q->H = out[1]; q->W = out[2];
+  q->oD = dz.n; q->sD = q->sH = q->sW = 1; q->pD = -dz.org; q->kD = dz.m; q->d0 = dz.t0; q->ds = -stride[0];
+  q->kD_w = ker[0]; q->kH_w = ker[1]; q->kW_w = ker[2];
+  const long long w_ = C, h_ = w_ * in[2], d_ = h_ * in[1], n_ = d_ * in[0];
+  q->ys_w = w_ * stride[2]; q->ys_h = h_ * stride[1]; q->ys_d = d_ * stride[0]; q->ys_n = n_;
+  q->weight_layout = weight_layout; q->transposed = 1; q->variants = 1;
+  if (dz.n <= 0) return true;                  // no input of this parity
+  for (int a = 0; a < stride[1]; ++a)
+    for (int b = 0; b < stride[2]; ++b) {
+      const Axis h = axis(1, a), w = axis(2, b);
+      if (h.n <= 0 || w.n <= 0) continue;
+      if (h.m == 0 || w.m == 0 || dz.m == 0) { *zero_fill = true; continue; }      // inputs that no output reads
+      DirectPart p;
+      p.org_h = h.org; p.org_w = w.org; p.th = h.m; p.tw = w.m;
+      p.t0_h = h.t0; p.ts_h = -stride[1]; p.t0_w = w.t0; p.ts_w = -stride[2];
+      p.oH = h.n; p.oW = w.n;
+      p.y_off = e * d_ + a * h_ + b * w_;
+      q->oH = std::max(q->oH, h.n); q->oW = std::max(q->oW, w.n);
+      q->parts[q->n_parts++] = p;
+    }
+  q->yH = q->oH; q->yW = q->oW;
+  return true;
 }
 
 bool direct_plan(const DirectDesc &d, DirectPlan *out) {
+  if (d.n_parts == 0) return false;
   const bool f32 = d.dtype == WINOCONV_F32;
   const int esz = f32 ? 4 : 2, vec = 16 / esz;
   if (d.C % vec != 0) return false;
-  if (d.sH > 2 || d.sW > 2 || d.sD > 2 || d.kH * d.kW > MAX_TAPS || d.pH > 64 || d.pW > 64) return false;
   const bool pool = (d.epilogue & WINOCONV_EPI_POOL2) != 0;
   DirectPlan p;
   std::memset(&p, 0, sizeof p);
@@ -654,25 +786,21 @@ bool direct_plan(const DirectDesc &d, DirectPlan *out) {
   const int k_el = 32 / esz;                 // channels of one MMA K step
   p.k_full = p.ch_el / k_el;
   p.k_tail = (d.C - (p.n_chunks - 1) * p.ch_el + k_el - 1) / k_el;
-  // polyphase parts along H and W and their taps
-  const int Th = (d.kH + d.sH - 1) / d.sH, Tw = (d.kW + d.sW - 1) / d.sW;   // of part 0, the largest
-  p.PW = 8 + Tw - 1;
-  int n_taps = 0;
-  for (int a = 0; a < d.sH; ++a)
-    for (int b = 0; b < d.sW; ++b) {
-      const int th = (d.kH - a + d.sH - 1) / d.sH, tw = (d.kW - b + d.sW - 1) / d.sW;
-      if (th <= 0 || tw <= 0) continue;
-      p.ph_h[p.n_ph] = a; p.ph_w[p.n_ph] = b; p.ph_tw[p.n_ph] = tw;
-      p.taps[p.n_ph] = th * tw; p.tap0[p.n_ph] = n_taps;
-      n_taps += th * tw;
-      ++p.n_ph;
-    }
+  int Th = 0, Tw = 0, n_taps = 0;            // largest part
+  for (int q = 0; q < d.n_parts; ++q) {
+    Th = std::max(Th, d.parts[q].th); Tw = std::max(Tw, d.parts[q].tw);
+    p.taps[q] = d.parts[q].th * d.parts[q].tw;
+    p.tap0[q] = n_taps;
+    n_taps += p.taps[q];
+    p.max_taps = std::max(p.max_taps, p.taps[q]);
+  }
+  if (n_taps == 0 || n_taps > MAX_TAPS) return false;
   p.n_taps = n_taps;
   p.filter_elems = (long long)d.kD * n_taps * d.K * d.C * (f32 ? 2 : 1);
-  p.units = d.kD * n_taps * p.n_chunks;
-  const double k_steps = (double)d.kD * n_taps * ((p.n_chunks - 1) * p.k_full + p.k_tail);
-  const int n_steps = d.kD * p.n_ph * p.n_chunks;
-  const int budget = 227 * 1024 - 2048 - BAR_BYTES - EPI_WARPS * STAGE_BYTES;
+  const int n_var = d.variants ? d.n_parts : 1, item_taps = d.variants ? p.max_taps : n_taps;
+  p.units = d.kD * item_taps * p.n_chunks;
+  const double k_steps = (double)d.kD * n_taps / n_var * ((p.n_chunks - 1) * p.k_full + p.k_tail);
+  const int n_steps = d.kD * (d.variants ? 1 : d.n_parts) * p.n_chunks;
 
   struct Cfg { int BN, MB, pair; };
   static const Cfg cfgs16[] = {{256, 1, 1}, {128, 2, 1}, {128, 1, 1}, {64, 2, 1}, {128, 1, 0}, {64, 1, 0}, {64, 2, 0}};
@@ -688,84 +816,68 @@ bool direct_plan(const DirectDesc &d, DirectPlan *out) {
     if (!f32 && force >= 0 && force != ci) continue;
     if (c.BN > 64 && d.K <= c.BN / 2 && force < 0) continue;
     const int n_kb = (d.K + c.BN - 1) / c.BN;
+    for (int ti = 1; ti <= 8; ti *= 2)
     for (int tn = 1; tn <= 16; tn *= 2) {
-      if (pool && tn > 2) break;
-      if (tn > 1 && tn / 2 >= d.N) break;
+      if (pool && (tn > 2 || ti > 4)) continue;
+      if (ti * tn > 1 && ti * tn / 2 >= d.N) continue;
+      if (ti > 1 && tn > 1 && (d.D != 1 || d.oD != 1 || d.kD != 1 || d.pD != 0 || d.N % ti != 0)) continue;
       DirectPlan q = p;
-      q.BN = c.BN; q.MB = c.MB; q.pair = c.pair; q.TN = tn; q.TH = 16 / tn;
+      q.BN = c.BN; q.MB = c.MB; q.pair = c.pair; q.TN = tn; q.TH = 16 / tn; q.TI = ti;
+      q.PW = 8 / ti + Tw - 1;
       const int rows_h = c.MB * q.TH + Th - 1;
       if (q.PW * d.sW > 256 || rows_h * d.sH > 256) continue;
       q.slab_rows_h = rows_h;
-      q.slab_bytes = rows_h * tn * q.PW * q.rb;
+      q.slab_bytes = rows_h * tn * q.PW * ti * q.rb;
       const int a1 = (q.slab_bytes + 1023) / 1024 * 1024;
       q.a_bytes = f32 ? 2 * a1 : a1;
       q.lo_off = a1;
       q.b_lo = (c.pair ? c.BN / 2 : c.BN) * q.rb;
       q.b_tile = q.b_lo * (f32 ? 2 : 1);
-      q.n_wb = (d.oW + 7) / 8; q.n_hb = (d.oH + c.MB * q.TH - 1) / (c.MB * q.TH);
-      const long long tiles = (long long)q.n_wb * q.n_hb * d.oD * ((d.N + tn - 1) / tn);
-      if (tiles * n_kb > 0x3fffffffLL) continue;
+      q.n_wb = (d.oW + 8 / ti - 1) / (8 / ti); q.n_hb = (d.oH + c.MB * q.TH - 1) / (c.MB * q.TH);
+      const long long tiles = (long long)q.n_wb * q.n_hb * d.oD * ((d.N + tn * ti - 1) / (tn * ti));
+      if (tiles * n_kb * n_var > 0x3fffffffLL) continue;
       q.n_tiles = (int)tiles; q.n_kb = n_kb;
       q.n_items = (int)((c.pair ? (tiles + 1) / 2 : tiles) * n_kb);
-      // taps per filter stage: enough that a stage is worth its barrier round trip
-      int G = std::max(1, std::min(p.taps[0], 24 * 1024 / q.b_tile));
-      q.n_a = 0;
-      for (; G >= 1; --G) {
-        q.G = G;
-        q.b_bytes = (G * q.b_tile + 1023) / 1024 * 1024;
-        int na = 2, nb = 2;
-        const double groups = (p.taps[0] + G - 1) / G;
-        if (2 * q.a_bytes + 2 * q.b_bytes > budget) {
-          na = 1;
-          if (q.a_bytes + 2 * q.b_bytes > budget) continue;
-        }
-        // deepen whichever ring looks less far ahead
-        for (bool grew = true; grew;) {
-          grew = false;
-          const bool want_b = nb / groups <= na;
-          for (int turn = 0; turn < 2 && !grew; ++turn) {
-            const bool b = turn == 0 ? want_b : !want_b;
-            if (b && nb < 8 && na * q.a_bytes + (nb + 1) * q.b_bytes <= budget) { ++nb; grew = true; }
-            if (!b && na < 8 && (na + 1) * q.a_bytes + nb * q.b_bytes <= budget) { ++na; grew = true; }
-          }
-        }
-        q.n_a = na; q.n_b = nb;
-        break;
-      }
-      if (q.n_a == 0) continue;
       for (int split = 1; split <= 8; split *= 2) {
-        if (split > 1 && (c.pair || q.n_items * split > 148 || split > q.units)) break;
+        const int width = split * (c.pair ? 2 : 1);
+        if (split > 1 && (width > 8 || d.variants || q.n_items > clusters_at_once(width) || split > q.units)) break;
         if (split > 1 && pool && c.MB * BM / split < 16 * tn) break;
-        if (split > 1 && c.MB * BM * (c.BN + 4) * 4 > q.n_a * q.a_bytes + q.n_b * q.b_bytes) break;
-        if (force_split > 0 && split != force_split && !c.pair) continue;
+        if (force_split > 0 && split != force_split) continue;
         q.split = split;
-        const double e = estimate(q, k_steps, n_steps, q.n_tiles, n_kb, f32);
+        if (!ring_depths(q, p.max_taps, 227 * 1024 - FIXED_BYTES)) continue;
+        if (split > 1 && c.MB * BM * (c.BN + 4) * 4 > q.n_a * q.a_bytes + q.n_b * q.b_bytes) continue;
+        const double e = estimate(q, k_steps, n_steps, n_var, f32);
         if (e < best) { best = e; *out = q; found = true; }
       }
     }
   }
   if (!found) return false;
-  if (getenv("WINOCONV_DIRECT_DEBUG")) fprintf(stderr, "[direct] BN%d MB%d pair%d split%d TN%d tiles%d items%d na%d nb%d G%d slab%d est %.1f us\n", out->BN, out->MB, out->pair, out->split, out->TN, out->n_tiles, out->n_items, out->n_a, out->n_b, out->G, out->slab_bytes, best/1.9e3);
+  if (getenv("WINOCONV_DIRECT_DEBUG")) fprintf(stderr, "[direct] BN%d MB%d pair%d split%d TI%d TN%d tiles%d items%d na%d nb%d G%d slab%d est %.1f us\n", out->BN, out->MB, out->pair, out->split, out->TI, out->TN, out->n_tiles, out->n_items, out->n_a, out->n_b, out->G, out->slab_bytes, best/1.9e3);
   out->estimate = best;
-  out->smem = 1024 + out->n_a * out->a_bytes + out->n_b * out->b_bytes + EPI_WARPS * STAGE_BYTES + BAR_BYTES;
+  out->smem = FIXED_BYTES + out->n_a * out->a_bytes + out->n_b * out->b_bytes;
   return true;
 }
 
 cudaError_t launch_direct_filter_transform(const DirectDesc &d, const DirectPlan &p, int w_dtype, const void *w, void *u, cudaStream_t s) {
   FGeomD f;
   std::memset(&f, 0, sizeof f);
-  f.O = d.K; f.I = d.C; f.Ip = d.C; f.kD = d.kD; f.n_hw = p.n_taps;
+  f.O = d.K; f.I = d.Cw; f.Ip = d.C; f.kD = d.kD; f.n_hw = p.n_taps;
+  // the weights' own channel counts: [Kw][Cw][taps] or [taps][Cw][Kw]
+  const long long Kw = d.transposed ? d.Cw : d.K, Cw = d.transposed ? d.K : d.Cw;
   const bool kcrs = d.weight_layout == WINOCONV_W_KCRS;
-  const long long hw = (long long)d.kH * d.kW;
-  const long long tap_stride = kcrs ? 1 : (long long)d.C * d.K;
-  f.s_o = kcrs ? d.C * d.kD * hw : 1;
-  f.s_i = kcrs ? d.kD * hw : d.K;
-  f.s_d = hw * tap_stride;
-  for (int q = 0; q < p.n_ph; ++q)
+  const long long hw = (long long)d.kH_w * d.kW_w, tap_stride = kcrs ? 1 : Cw * Kw;
+  const long long s_k = kcrs ? Cw * d.kD_w * hw : 1, s_c = kcrs ? d.kD_w * hw : Kw;
+  f.s_o = d.transposed ? s_c : s_k;
+  f.s_i = d.transposed ? s_k : s_c;
+  f.off_d = d.d0 * hw * tap_stride;
+  f.s_d = d.ds * hw * tap_stride;
+  for (int q = 0; q < d.n_parts; ++q) {
+    const DirectPart &a = d.parts[q];
     for (int t = 0; t < p.taps[q]; ++t) {
-      const int th = t / p.ph_tw[q], tw = t - th * p.ph_tw[q];
-      f.off_hw[p.tap0[q] + t] = (int)(((d.sH * th + p.ph_h[q]) * d.kW + d.sW * tw + p.ph_w[q]) * tap_stride);
+      const int th = t / a.tw, tw = t - th * a.tw;
+      f.off_hw[p.tap0[q] + t] = (int)(((a.t0_h + a.ts_h * th) * d.kW_w + a.t0_w + a.ts_w * tw) * tap_stride);
     }
+  }
   const unsigned blocks = (unsigned)(((long long)f.O * f.Ip + 255) / 256);
   const dim3 grid(blocks, d.kD, blocks >= 296 ? 1 : std::min(p.n_taps, (int)(592 / blocks) + 1));
 #define WINO_FILT(TW, T) direct_filter_kernel<TW, T><<<grid, 256, 0, s>>>((const TW *)w, (T *)u, f)
@@ -777,7 +889,7 @@ cudaError_t launch_direct_filter_transform(const DirectDesc &d, const DirectPlan
 }
 
 template <typename T, int BN, int MB, bool PAIR>
-static cudaError_t launch_one(const DirectPlan &p, const CUtensorMap &mx, const CUtensorMap &mu, const CUtensorMap &my, void *y,
+static cudaError_t launch_one(const DirectPlan &p, const CUtensorMap &mx, const CUtensorMap &mu, const MapSet &my, void *y,
                               const void *bias, const DGeom &g, const DSmem &sl, uint32_t idesc, int sms, cudaStream_t s) {
   auto kern = direct_kernel<T, BN, MB, PAIR>;
   static std::mutex mu_;
@@ -793,7 +905,7 @@ static cudaError_t launch_one(const DirectPlan &p, const CUtensorMap &mx, const 
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   attr[1].id = cudaLaunchAttributeClusterDimension;
-  attr[1].val.clusterDim.x = PAIR ? 2 : (unsigned)p.split; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
+  attr[1].val.clusterDim.x = (PAIR ? 2u : 1u) * (unsigned)p.split; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = (PAIR || p.split > 1) ? 2 : 1;
   int pairs = 0;
@@ -807,15 +919,17 @@ static cudaError_t launch_one(const DirectPlan &p, const CUtensorMap &mx, const 
       if (PAIR) {
         cfg.gridDim = dim3(2, 1, 1);
         cfg.dynamicSmemBytes = 227 * 1024;
+        attr[1].val.clusterDim.x = 2;
         if (cudaOccupancyMaxActiveClusters(&f->second, kern, &cfg) != cudaSuccess || f->second <= 0) f->second = sms / 2;
         cfg.dynamicSmemBytes = (size_t)p.smem;
+        attr[1].val.clusterDim.x = 2u * (unsigned)p.split;
       }
     }
     pairs = f->second;
   }
-  if (PAIR) cfg.gridDim = dim3((unsigned)(2 * std::min(p.n_items, std::min(pairs, sms / 2))), 1, 1);
-  else if (p.split > 1) cfg.gridDim = dim3((unsigned)(p.n_items * p.split), 1, 1);
-  else cfg.gridDim = dim3((unsigned)std::min(p.n_items, sms), 1, 1);
+  if (p.split > 1) cfg.gridDim = dim3((unsigned)(g.n_items * p.split) * (PAIR ? 2u : 1u), 1, 1);
+  else if (PAIR) cfg.gridDim = dim3((unsigned)(2 * std::min(g.n_items, std::min(pairs, sms / 2))), 1, 1);
+  else cfg.gridDim = dim3((unsigned)std::min(g.n_items, sms), 1, 1);
   return cudaLaunchKernelEx(&cfg, kern, mx, mu, my, (T *)y, (const T *)bias, g, sl, idesc);
 }
 
@@ -829,15 +943,37 @@ cudaError_t launch_direct_forward(const DirectDesc &d, const DirectPlan &p, cons
   const CUtensorMapDataType dt = map_dtype(d.dtype);
   const CUtensorMapSwizzle swz = p.rb == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : p.rb == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_32B;
   const uint32_t swz_code = p.rb == 128 ? 2u : p.rb == 64 ? 4u : 6u;
-  CUtensorMap mx, mu, my;
-  {   // x as [D][H][N][W][C]: a slab is rows x images x pixels x channels; H and W walked with the layer's stride
-    const cuuint64_t dims[5] = {(cuuint64_t)d.C, (cuuint64_t)d.W, (cuuint64_t)d.N, (cuuint64_t)d.H, (cuuint64_t)d.D};
-    const cuuint64_t w_ = (cuuint64_t)d.C * esz, h_ = w_ * d.W, d_ = h_ * d.H, n_ = d_ * d.D;
-    const cuuint64_t st[4] = {w_, n_, h_, d_};
-    const cuuint32_t box[5] = {(cuuint32_t)p.ch_el, (cuuint32_t)(p.PW * d.sW), (cuuint32_t)p.TN, (cuuint32_t)(p.slab_rows_h * d.sH), 1u};
-    const cuuint32_t es[5] = {1u, (cuuint32_t)d.sW, 1u, (cuuint32_t)d.sH, 1u};
-    if (enc(&mx, dt, 5, const_cast<void *>(x), dims, st, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) { *detail = "cuTensorMapEncodeTiled failed for the input"; return cudaErrorInvalidValue; }
+  CUtensorMap mx, mu;
+  MapSet my;
+  // order of the dimensions (see tile_load): dims / strides / box / element strides of channel, W, image, H, depth
+  const int mode = p.TI == 1 ? 0 : p.TN == 1 ? 1 : 2;
+  auto tile_map = [&](CUtensorMap *m, const void *ptr, cuuint64_t C_, cuuint64_t W_, cuuint64_t H_, cuuint64_t D_, cuuint64_t sw_, cuuint64_t sh_,
+                      cuuint64_t sd_, cuuint64_t sn_, cuuint32_t bc, cuuint32_t bw, cuuint32_t bn, cuuint32_t bh, cuuint32_t ew, cuuint32_t eh,
+                      CUtensorMapSwizzle sw) -> bool {     // byte strides of W, H, depth and image
+    const cuuint64_t N_ = (cuuint64_t)d.N, TI_ = (cuuint64_t)p.TI;
+    cuuint64_t dims[5], st[4];
+    cuuint32_t box[5], es[5] = {1u, 1u, 1u, 1u, 1u};
+    dims[0] = C_; box[0] = bc;
+    if (mode == 0) {
+      dims[1] = W_; dims[2] = N_; dims[3] = H_; dims[4] = D_;
+      st[0] = sw_; st[1] = sn_; st[2] = sh_; st[3] = sd_;
+      box[1] = bw; box[2] = bn; box[3] = bh; box[4] = 1u; es[1] = ew; es[3] = eh;
+    } else if (mode == 1) {
+      dims[1] = N_; dims[2] = W_; dims[3] = H_; dims[4] = D_;
+      st[0] = sn_; st[1] = sw_; st[2] = sh_; st[3] = sd_;
+      box[1] = (cuuint32_t)p.TI; box[2] = bw; box[3] = bh; box[4] = 1u; es[2] = ew; es[3] = eh;
+    } else {
+      dims[1] = TI_; dims[2] = W_; dims[3] = N_ / TI_; dims[4] = H_;
+      st[0] = sn_; st[1] = sw_; st[2] = sn_ * TI_; st[3] = sh_;
+      box[1] = (cuuint32_t)p.TI; box[2] = bw; box[3] = bn; box[4] = bh; es[2] = ew; es[4] = eh;
+    }
+    return enc(m, dt, 5, const_cast<void *>(ptr), dims, st, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+  };
+  const cuuint64_t xw = (cuuint64_t)d.C * esz, xh = xw * d.W, xd = xh * d.H, xn = xd * d.D;
+  if (!tile_map(&mx, x, d.C, d.W, d.H, d.D, xw, xh, xd, xn, p.ch_el, p.PW * d.sW, p.TN, p.slab_rows_h * d.sH, d.sW, d.sH, swz)) {
+    *detail = "cuTensorMapEncodeTiled failed for the input";
+    return cudaErrorInvalidValue;
   }
   {   // filter tiles [tap][K][C] (fp32: two per tap)
     const cuuint64_t dims[3] = {(cuuint64_t)d.C, (cuuint64_t)d.K, (cuuint64_t)d.kD * p.n_taps * (f32 ? 2 : 1)};
@@ -847,38 +983,47 @@ cudaError_t launch_direct_forward(const DirectDesc &d, const DirectPlan &p, cons
     if (enc(&mu, dt, 3, const_cast<void *>(u), dims, st, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) { *detail = "cuTensorMapEncodeTiled failed for the filter"; return cudaErrorInvalidValue; }
   }
+  const int n_var = d.variants ? d.n_parts : 1;
   const bool y_tma = ((cuuint64_t)d.K * esz) % 16 == 0;
   if (y_tma) {   // one epilogue warp's 32 pixels (8 when pooled) x 128 bytes of channels
-    const cuuint64_t dims[5] = {(cuuint64_t)d.K, (cuuint64_t)d.yW, (cuuint64_t)d.N, (cuuint64_t)d.yH, (cuuint64_t)d.oD};
-    const cuuint64_t w_ = (cuuint64_t)d.K * esz, h_ = w_ * d.yW, d_ = h_ * d.yH, n_ = d_ * d.oD;
-    const cuuint64_t st[4] = {w_, n_, h_, d_};
-    const cuuint32_t sn = (cuuint32_t)std::min(p.TN, 4), sh = 4u / sn;
-    const cuuint32_t box[5] = {(cuuint32_t)(128 / esz), pool ? 4u : 8u, sn, pool ? sh / 2 : sh, 1u};
-    const cuuint32_t es[5] = {1u, 1u, 1u, 1u, 1u};
-    if (enc(&my, dt, 5, y, dims, st, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) { *detail = "cuTensorMapEncodeTiled failed for the output"; return cudaErrorInvalidValue; }
-  } else my = mx;
+    const cuuint32_t sn = (cuuint32_t)std::min(p.TN, 4), sh = 4u / sn, w_px = (cuuint32_t)(8 / p.TI);
+    for (int v = 0; v < n_var; ++v) {
+      const DirectPart &a = d.parts[v];
+      const int yw = d.variants ? a.oW : d.yW, yh = d.variants ? a.oH : d.yH;
+      if (!tile_map(&my.m[v], (uint8_t *)y + (d.variants ? a.y_off : 0) * (long long)esz, d.K, yw, yh, d.oD, d.ys_w * esz, d.ys_h * esz, d.ys_d * esz, d.ys_n * esz,
+                    (cuuint32_t)(128 / esz), pool ? w_px / 2 : w_px, sn, pool ? sh / 2 : sh, 1u, 1u, CU_TENSOR_MAP_SWIZZLE_128B)) {
+        *detail = "cuTensorMapEncodeTiled failed for the output";
+        return cudaErrorInvalidValue;
+      }
+    }
+  } else my.m[0] = mx;
   DGeom g;
   std::memset(&g, 0, sizeof g);
-  g.N = d.N; g.K = d.K; g.oD = d.oD; g.oH = d.oH; g.oW = d.oW; g.yH = d.yH; g.yW = d.yW;
-  g.sD = d.sD; g.sH = d.sH; g.sW = d.sW; g.pD = d.pD; g.pH = d.pH; g.pW = d.pW; g.kD = d.kD;
-  g.TN = p.TN; g.TH = p.TH; g.PW = p.PW;
+  g.N = d.N; g.K = d.K; g.oD = d.oD; g.oH = d.oH;
+  g.sD = d.sD; g.sH = d.sH; g.sW = d.sW; g.pD = d.pD; g.kD = d.kD;
+  g.ys_n = d.ys_n; g.ys_d = d.ys_d; g.ys_h = d.ys_h; g.ys_w = d.ys_w;
+  for (int v = 0; v < n_var; ++v) {
+    g.yH[v] = d.variants ? d.parts[v].oH : d.yH; g.yW[v] = d.variants ? d.parts[v].oW : d.yW;
+    g.y_off[v] = d.variants ? d.parts[v].y_off : 0;
+  }
+  g.TN = p.TN; g.TH = p.TH; g.TI = p.TI; g.PW = p.PW; g.map_mode = mode;
   while ((1 << g.tn_shift) < p.TN) ++g.tn_shift;
-  g.n_wb = p.n_wb; g.n_hb = p.n_hb; g.n_tiles = p.n_tiles; g.n_kb = p.n_kb; g.n_items = p.n_items;
-  g.n_ph = p.n_ph; g.T_hw = p.n_taps;
-  for (int q = 0; q < p.n_ph; ++q) {
-    g.ph_h[q] = p.ph_h[q]; g.ph_w[q] = p.ph_w[q]; g.taps[q] = p.taps[q]; g.tap0[q] = p.tap0[q];
+  while ((1 << g.ti_shift) < p.TI) ++g.ti_shift;
+  g.n_wb = p.n_wb; g.n_hb = p.n_hb; g.n_tiles = p.n_tiles; g.n_kb = p.n_kb; g.var_items = p.n_items; g.n_items = p.n_items * n_var;
+  g.n_ph = d.n_parts; g.n_var = n_var; g.T_hw = p.n_taps;
+  for (int q = 0; q < d.n_parts; ++q) {
+    g.org_h[q] = d.parts[q].org_h; g.org_w[q] = d.parts[q].org_w; g.taps[q] = p.taps[q]; g.tap0[q] = p.tap0[q];
     for (int t = 0; t < p.taps[q]; ++t) {
-      const int th = t / p.ph_tw[q], tw = t - th * p.ph_tw[q];
-      g.tap_off[p.tap0[q] + t] = (uint16_t)((th * p.TN * p.PW + tw) * (p.rb / 16));
+      const int th = t / d.parts[q].tw, tw = t - th * d.parts[q].tw;
+      g.tap_off[p.tap0[q] + t] = (uint16_t)((th * p.TN * p.PW + tw) * p.TI * (p.rb / 16));
     }
   }
   g.n_chunks = p.n_chunks; g.ch_el = p.ch_el; g.k_full = p.k_full; g.k_tail = p.k_tail; g.units = p.units;
   g.G = p.G; g.split = p.split; g.epilogue = d.epilogue;
   g.y_tma = y_tma; g.bias_vec = y_tma && (reinterpret_cast<uintptr_t>(bias) & 15u) == 0;
-  g.a_hi = desc_hi((uint32_t)(p.PW * p.rb), swz_code);
+  g.a_hi = desc_hi((uint32_t)(p.PW * p.TI * p.rb), swz_code);
   g.b_hi = desc_hi((uint32_t)(8 * p.rb), swz_code);
-  g.mb_off16 = p.TH * p.TN * p.PW * p.rb / 16;
+  g.mb_off16 = p.TH * p.TN * p.PW * p.TI * p.rb / 16;
   DSmem sl;
   sl.slab_bytes = p.slab_bytes; sl.a_bytes = p.a_bytes; sl.lo_off = p.lo_off;
   sl.b_tile = p.b_tile; sl.b_lo = p.b_lo; sl.b_bytes = p.b_bytes; sl.n_a = p.n_a; sl.n_b = p.n_b;

@@ -78,18 +78,36 @@ cudaError_t launch_rowfused_forward(const RowDesc &d, const RowPlan &p, int dtyp
 cudaError_t read_and_clear_row_error(cudaStream_t s, unsigned int *code);
 
 // Direct-tap kernel (wino_direct.cu): 16-bit layers, and fp32 layers with three tf32 products per multiply.
-struct DirectDesc {
-  int dtype, N, C, K, D, H, W, oD, oH, oW, yH, yW;
-  int sD, sH, sW, pD, pH, pW, kD, kH, kW;
-  unsigned epilogue;
-  int weight_layout;
+// A polyphase part of the taps along H and W: tap (th, tw) of the part reads the input (stride * output + org + tap) and is
+// tap (t0 + ts * th, ...) of the weights.  A strided forward sums its parts; a strided data gradient writes each part's sums to
+// output pixels of its own ("variants").
+struct DirectPart {
+  int org_h, org_w, th, tw, t0_h, ts_h, t0_w, ts_w;
+  int oH, oW;                        // variants: output extents (before pooling)
+  long long y_off;                   // variants: first output element
 };
+struct DirectDesc {
+  int dtype, N, C, Cw, K, D, H, W;   // C: channels of the input tensor; Cw: of the weights (the rest are zeros)
+  int oD, oH, oW, yH, yW;            // output extents (the largest part's), stored extents after pooling
+  int sD, sH, sW, pD, kD, d0, ds;    // input step per output; depth taps kD, tap kd is depth d0 + ds * kd of the weights
+  int kD_w, kH_w, kW_w;              // kernel extents of the weights
+  int n_parts, variants;
+  DirectPart parts[4];
+  long long ys_n, ys_d, ys_h, ys_w;  // element strides of the output
+  unsigned epilogue;
+  int weight_layout, transposed;     // transposed: K and C exchanged in the weights (data gradient)
+};
+// A forward layer; and the part of a layer's data gradient with input depths of parity e (e < stride along depth).
+void direct_forward_desc(DirectDesc *q, int dtype, int N, int C, int K, const int in[3], const int ker[3], const int stride[3],
+                         const int pad[3], const int out[3], int yH, int yW, unsigned epilogue, int weight_layout);
+bool direct_grad_desc(DirectDesc *q, int dtype, int N, int C, int K, int Km, const int in[3], const int ker[3], const int stride[3],
+                      const int pad[3], const int out[3], int weight_layout, int e, bool *zero_fill);
 struct DirectPlan {
   int BN, MB, pair, split;           // columns and row blocks of an item, CTA pairs, CTAs that share an item's reduction
-  int TN, TH, PW, slab_rows_h;       // images and output rows of a row block, pixels of a slab row, slab rows
+  int TN, TH, TI, PW, slab_rows_h;   // a block's image groups and output rows, images within a group of 8 rows, pixels of a slab row, slab rows
   int ch_el, rb, n_chunks, k_full, k_tail;
-  int n_ph, ph_h[4], ph_w[4], ph_tw[4], taps[4], tap0[4], n_taps, units;
-  int n_wb, n_hb, n_tiles, n_kb, n_items;
+  int taps[4], tap0[4], max_taps, n_taps, units;
+  int n_wb, n_hb, n_tiles, n_kb, n_items;   // n_items: of one variant
   int slab_bytes, a_bytes, lo_off, b_tile, b_lo, b_bytes, G, n_a, n_b, smem;
   long long filter_elems;
   double estimate;                   // clocks
@@ -98,6 +116,22 @@ bool direct_plan(const DirectDesc &d, DirectPlan *out);
 cudaError_t launch_direct_filter_transform(const DirectDesc &d, const DirectPlan &p, int w_dtype, const void *w, void *u, cudaStream_t s);
 cudaError_t launch_direct_forward(const DirectDesc &d, const DirectPlan &p, const void *x, const void *u, const void *bias, void *y,
                                   cudaStream_t s, const char **detail);
+// Weight gradient (wino_wgrad.cu): 16-bit x and gy whose channel strides Cm, Km are multiples of 8; dW [K][C][taps] and the bias
+// sums from fp32 accumulators.
+struct WgradDesc {
+  int dtype, N, C, K, Cm, Km, D, H, W, oD, oH, oW;
+  int sD, sH, sW, pD, pH, pW, kD, kH, kW;
+  int bias;
+};
+struct WgradPlan {
+  alignas(8) unsigned char geom[2048];
+  int smem, slab_rows_h;
+  unsigned long long ws_bytes;
+};
+bool wgrad_plan(const WgradDesc &d, WgradPlan *out);
+cudaError_t launch_wgrad(const WgradDesc &d, const WgradPlan &p, const void *x, const void *gy, void *dw, int dw_dtype, float *dbias,
+                         void *ws, cudaStream_t s, const char **detail);
+cudaError_t read_and_clear_wgrad_error(cudaStream_t s, unsigned int *code);
 cudaError_t read_and_clear_direct_error(cudaStream_t s, unsigned int *code);
 
 // Reads the error word of the bounded device waits, clears it and synchronises the stream.

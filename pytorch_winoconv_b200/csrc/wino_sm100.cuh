@@ -165,10 +165,9 @@ __device__ __forceinline__ void umma(uint32_t d, uint32_t a_lo, uint32_t a_hi, u
   else { if constexpr (TF32) WINO_UMMA("1", "tf32"); else WINO_UMMA("1", "f16"); }
 #undef WINO_UMMA
 }
-// Arrives on `bar` (of both CTAs of a pair) when the MMAs issued so far by this thread have completed.
-template <bool PAIR> __device__ __forceinline__ void umma_commit(uint32_t bar) {
+// Arrives on `bar` (of both CTAs of a pair, given by their bits in `mask`) when the MMAs issued so far by this thread have completed.
+template <bool PAIR> __device__ __forceinline__ void umma_commit(uint32_t bar, uint16_t mask) {
   if (PAIR) {
-    const uint16_t mask = 3;
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                  ::"r"(bar), "h"(mask) : "memory");
   } else {
