@@ -88,7 +88,8 @@ typedef struct winoconv_desc {
   int32_t ker_size[3];   /* kD, kH, kW (each 1..10);  kD = 1 if ndim = 2                     */
   int32_t stride[3];     /* 1 or 2 per dimension                                             */
   int32_t pad[3];        /* symmetric zero padding per dimension, applied in-kernel          */
-  int32_t tile_m;        /* Winograd output block: 0 = auto (2 where a single-kernel path
+  int32_t tile_m;        /* Winograd output block: 1 = direct taps (one kernel, no transform; C a multiple of 16 bytes);
+                          * 0 = auto (2 where a single-kernel path
                           * takes the layer, else 4 for 2-D 3x3 stride 1), 2 = F(2,r),
                           * 4 = F(4x4,3x3), 6 = F(6x6,3x3) (f32 operands with the SIMT or
                           * TF32X3 engine only: 64 positions, 1.78 multiplies per output) */
@@ -253,6 +254,16 @@ WINOCONV_API int winoconv_backward_weight(const winoconv_desc_t *desc, const voi
  */
 WINOCONV_API int winoconv_gemm_batched(int dtype, int product_dtype, int gemm_engine, int positions, int64_t tiles, int c_pad,
                           int k_out, const void *v, const void *u, void *m, void *stream);
+
+/*
+ * Layout changes either side of the kernels, converting the element type on the way: x [N, C, P] -> y [N, P, c_stride]
+ * (zeros from channel C on), and x [N, P, C] -> y [N, C, P] (+ bias[c], f32, where bias is not NULL).
+ * Replace the permute / contiguous / type passes of dwm.py:129-144 and matrix_conv.py:70-107.
+ */
+WINOCONV_API int winoconv_to_channels_last(const void *x, int in_dtype, void *y, int out_dtype, int batch, int c, int64_t pixels,
+                                           int c_stride, void *stream);
+WINOCONV_API int winoconv_to_channels_first(const void *x, int in_dtype, void *y, int out_dtype, const float *bias, int batch,
+                                            int c, int64_t pixels, void *stream);
 
 /*
  * Overlapping-tile extraction and re-assembly, kept so the reference's torch-level route keeps

@@ -30,7 +30,7 @@ EXPORTED_SYMBOLS = (
     "winoconv_forward_timed", "winoconv_forward_static", "winoconv_gemm_batched", "winoconv_split",
     "winoconv_concat", "winoconv_add", "winoconv_read_device_error", "winoconv_probe_mma_rate",
     "winoconv_filter_transform_from", "winoconv_backward_plan", "winoconv_backward_filter_transform",
-    "winoconv_backward_data", "winoconv_backward_weight",
+    "winoconv_backward_data", "winoconv_backward_weight", "winoconv_to_channels_last", "winoconv_to_channels_first",
 )
 
 

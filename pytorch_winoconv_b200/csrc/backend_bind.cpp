@@ -18,6 +18,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("DWM", &DWM);
   m.def("set_dwm_output_block", &set_dwm_output_block);
   m.def("get_dwm_output_block", &get_dwm_output_block);
+  m.def("conv_call", &conv_call, py::call_guard<py::gil_scoped_release>());
   py::class_<ConvRunner, c10::intrusive_ptr<ConvRunner>>(m, "ConvRunner")
       .def(py::init<int64_t, std::vector<int64_t>, std::vector<int64_t>, int64_t, int64_t, bool, bool, int64_t, int64_t>())
       .def("forward", &ConvRunner::forward, py::call_guard<py::gil_scoped_release>())

@@ -57,6 +57,18 @@ at::Tensor empty_bytes(uint64_t bytes, const at::Tensor &like) {
   return at::empty({(int64_t)bytes}, like.options().dtype(at::kByte).requires_grad(false));
 }
 
+// An [N, C, spatial...] tensor in torch's contiguous order as a channels-last one of another element type.
+at::Tensor turned_channels_last(const at::Tensor &t, at::ScalarType type, void *stream) {
+  const int nd = (int)t.dim() - 2;
+  at::Tensor out = at::empty(t.sizes(), t.options().dtype(type).requires_grad(false), nd == 2 ? at::MemoryFormat::ChannelsLast : at::MemoryFormat::ChannelsLast3d);
+  const int64_t pixels = t.numel() / (t.size(0) * t.size(1));
+  const int st = (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) ? WINOCONV_ERR_UNSUPPORTED
+                 : winoconv_to_channels_last(t.data_ptr(), code_of(t.scalar_type()), out.data_ptr(), code_of(type), (int)t.size(0), (int)t.size(1), pixels, (int)t.size(1), stream);
+  if (st == WINOCONV_ERR_UNSUPPORTED) out.copy_(t);
+  else check_abi(st, "winoconv_to_channels_last");
+  return out;
+}
+
 // The last dimension of a channels-last buffer zero-extended to `c` channels; the tensor itself where it has them.
 at::Tensor pad_channels(const at::Tensor &t, int64_t c) {
   const int nd = (int)t.dim();
@@ -107,6 +119,7 @@ ConvRunner::ConvRunner(int64_t nd, std::vector<int64_t> stride, std::vector<int6
 
 at::Tensor ConvRunner::channels_last(const at::Tensor &t, at::ScalarType type) const {
   if (t.scalar_type() == type && lies_channels_last(t)) return t;
+  if (t.is_contiguous() && t.size(1) > 1 && code_of(t.scalar_type()) >= 0 && t.size(0) <= 65535) return turned_channels_last(t, type, stream_of());
   return t.to(t.options().dtype(type), false, false, nd_ == 2 ? at::MemoryFormat::ChannelsLast : at::MemoryFormat::ChannelsLast3d);
 }
 
@@ -287,5 +300,82 @@ std::vector<std::tuple<std::vector<int64_t>, int64_t, int64_t, at::Tensor, int64
     for (int i = 4 - nd_; i < 5; ++i) shape.push_back(e->shape[i]);
     out.emplace_back(shape, e->dtype, e->device, e->u, e->serial, std::string(reinterpret_cast<const char *>(&e->info), sizeof e->info));
   }
+  return out;
+}
+
+std::optional<at::Tensor> conv_call(const at::Tensor &x_in, const at::Tensor &weight_in, const std::optional<at::Tensor> &bias,
+                                    std::vector<int64_t> stride, std::vector<int64_t> padding, int64_t compute, bool out_f32, int64_t tile_m) {
+  const int nd = (int)x_in.dim() - 2;
+  if (!x_in.is_cuda() || (nd != 2 && nd != 3) || weight_in.dim() != nd + 2 || x_in.size(1) != weight_in.size(1) || x_in.numel() == 0 ||
+      weight_in.numel() == 0 || (int)stride.size() != nd || (int)padding.size() != nd || (bias && bias->numel() != weight_in.size(0)))
+    return std::nullopt;
+  // bias with a graph: its gradient is the caller's addition
+  if (bias && at::GradMode::is_enabled() && bias->requires_grad()) return std::nullopt;
+  const int dtype = compute >= 0 ? (int)compute : code_of(x_in.scalar_type());
+  if (dtype < 0 || code_of(x_in.scalar_type()) < 0 || code_of(weight_in.scalar_type()) < 0) return std::nullopt;
+  at::AutoDispatchBelowADInplaceOrView no_graph;
+  c10::cuda::CUDAGuard guard(x_in.device());
+  const at::ScalarType type = type_of(dtype);
+  winoconv_desc_t d;
+  std::memset(&d, 0, sizeof d);
+  d.ndim = nd;
+  for (int64_t v : x_in.sizes())
+    if (v > 0x7fffffffLL) return std::nullopt;
+  d.batch = (int)x_in.size(0); d.c_in = (int)x_in.size(1); d.k_out = (int)weight_in.size(0);
+  for (int i = 0; i < 3; ++i) {
+    const int a = i - (3 - nd);
+    d.in_size[i] = a < 0 ? 1 : (int)x_in.size(2 + a);
+    d.ker_size[i] = a < 0 ? 1 : (int)weight_in.size(2 + a);
+    d.stride[i] = a < 0 ? 1 : (int)stride[a];
+    d.pad[i] = a < 0 ? 0 : (int)padding[a];
+  }
+  d.dtype = dtype;
+  const bool bias_after = bias && out_f32 && dtype != WINOCONV_F32;
+  d.epilogue = bias && !bias_after ? WINOCONV_EPI_BIAS : 0u;
+  // direct taps, unless F(2,r) does them in fewer multiplies than its traffic is worth (fp32, wide 3x3: see the planner)
+  winoconv_plan_info_t info;
+  const bool wide_f32 = dtype == WINOCONV_F32 && nd == 2 && d.ker_size[1] == 3 && d.ker_size[2] == 3 && d.stride[1] == 1 && d.stride[2] == 1 &&
+                        (int64_t)d.c_in * d.k_out > 128 * 128;
+  d.tile_m = 1;
+  if (tile_m != 2 || wide_f32 || winoconv_plan(&d, &info) != WINOCONV_OK) {
+    d.tile_m = (int)tile_m;
+    if (winoconv_plan(&d, &info) != WINOCONV_OK) return std::nullopt;
+  }
+  void *s = stream_of();
+  at::Tensor x = lies_channels_last(x_in) && x_in.scalar_type() == type ? x_in
+                 : x_in.is_contiguous() && x_in.size(0) <= 65535 ? turned_channels_last(x_in, type, s)
+                 : x_in.to(x_in.options().dtype(type), false, false, nd == 2 ? at::MemoryFormat::ChannelsLast : at::MemoryFormat::ChannelsLast3d);
+  at::Tensor w = weight_in.to(x.device()).contiguous();
+  at::Tensor u = empty_bytes(info.filter_bytes, x);
+  if (winoconv_filter_transform_from(&d, w.data_ptr(), code_of(w.scalar_type()), u.data_ptr(), s) != WINOCONV_OK) {
+    w = w.to(type);
+    check_abi(winoconv_filter_transform(&d, w.data_ptr(), u.data_ptr(), s), "winoconv_filter_transform");
+  }
+  at::Tensor b;
+  if (bias) b = bias->to(x.device(), bias_after ? at::kFloat : type).contiguous();
+  at::Tensor v, m;
+  if (!info.direct) {
+    if (info.input_ws_bytes) v = empty_bytes(info.input_ws_bytes, x);
+    if (info.product_ws_bytes) m = empty_bytes(info.product_ws_bytes, x);
+  }
+  int64_t sizes[5] = {d.batch, d.k_out, 0, 0, 0};
+  for (int i = 0; i < nd; ++i) sizes[2 + i] = info.out_size[3 - nd + i];
+  const at::IntArrayRef out_sizes(sizes, nd + 2);
+  at::Tensor y = at::empty(out_sizes, x.options().requires_grad(false), nd == 2 ? at::MemoryFormat::ChannelsLast : at::MemoryFormat::ChannelsLast3d);
+  check_abi(winoconv_forward(&d, x.data_ptr(), u.data_ptr(), d.epilogue ? b.data_ptr() : nullptr, y.data_ptr(), v.defined() ? v.data_ptr() : nullptr,
+                             info.input_ws_bytes, m.defined() ? m.data_ptr() : nullptr, info.product_ws_bytes, s),
+            "winoconv_forward");
+  const at::ScalarType out_type = out_f32 ? at::kFloat : type;
+  at::Tensor out = at::empty(out_sizes, x.options().dtype(out_type).requires_grad(false), at::MemoryFormat::Contiguous);
+  const int st = winoconv_to_channels_first(y.data_ptr(), dtype, out.data_ptr(), code_of(out_type), bias_after ? b.data_ptr<float>() : nullptr, d.batch, d.k_out,
+                                            y.numel() / ((int64_t)d.batch * d.k_out), s);
+  if (st == WINOCONV_ERR_UNSUPPORTED) {
+    out.copy_(y);
+    if (bias_after) {
+      std::vector<int64_t> shape(nd + 2, 1);
+      shape[1] = d.k_out;
+      out.add_(b.view(shape));
+    }
+  } else check_abi(st, "winoconv_to_channels_first");
   return out;
 }

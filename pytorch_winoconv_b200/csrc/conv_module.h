@@ -13,6 +13,13 @@
 
 #include "winoconv_b200.h"
 
+// One call of the reference's functional operators: x and weight in torch order, the filter transformed on the spot.  compute:
+// the dtype of operands and products' result (-1: x's own); the result is in torch order, in fp32 where out_f32 is set (bias
+// added in fp32 after the rounding to the compute dtype), else in the compute dtype.  tile_m as in winoconv_desc_t where the
+// direct-tap kernel does not take the layer.  Nothing where the caller's own path has to decide.
+std::optional<at::Tensor> conv_call(const at::Tensor &x, const at::Tensor &weight, const std::optional<at::Tensor> &bias,
+                                    std::vector<int64_t> stride, std::vector<int64_t> padding, int64_t compute, bool out_f32, int64_t tile_m);
+
 // One per module.  Every entry is the plan of an input shape with its transformed filters; they follow the weights (storage,
 // version, dtype), and the least recently used one goes when there are more than `max_plans`.
 class ConvRunner : public torch::CustomClassHolder {

@@ -120,7 +120,8 @@ int build_plan(const winoconv_desc_t *d, Plan *plan) {
   }
   int tile_m = d->tile_m;
   if (tile_m == 0) tile_m = (f43_ok && (!single_kernel_candidate || f43_wins)) ? 4 : 2;
-  if (tile_m != 2 && tile_m != 4 && tile_m != 6) return fail(WINOCONV_ERR_UNSUPPORTED, "tile_m must be 0, 2, 4 or 6");
+  if (tile_m == 1) tile_m = 2;     // direct taps; the plan's figures are those of 2-wide tiles
+  if (tile_m != 2 && tile_m != 4 && tile_m != 6) return fail(WINOCONV_ERR_UNSUPPORTED, "tile_m must be 0, 1, 2, 4 or 6");
   if (tile_m == 4 && !f43_ok) return fail(WINOCONV_ERR_UNSUPPORTED, "tile_m = 4 is F(4x4,3x3): 2-D, 3x3 kernel, stride 1 only");
   if (tile_m == 6 && !f43_ok) return fail(WINOCONV_ERR_UNSUPPORTED, "tile_m = 6 is F(6x6,3x3): 2-D, 3x3 kernel, stride 1 only");
   // F(6x6,3x3) with 16-bit or single-tf32 operands sits at 5e-2 of the output scale (measured), beyond the 2e-2 bound
@@ -256,14 +257,23 @@ int build_plan(const winoconv_desc_t *d, Plan *plan) {
     }
   }
 
-  // AUTO with no tile size asked for: the direct-tap kernel
+  // The direct-tap kernel: on request (tile_m = 1), or AUTO's choice where no tile size is asked for -- for every 16-bit layer
+  // that would otherwise run on the row-piece kernel (measured on B200, 1.1 to 3.6 times as fast on all shapes tried; the
+  // exception above keeps its staged F(4x4,3x3)), and for fp32 except 3x3 stride-1 layers whose quarter of the multiplies as
+  // F(4x4,3x3) outweighs the traffic of V and M: multiplies grow with C * K (K in whole 64-column blocks), V and M with C + K
+  // (measured, us direct / staged: 16 -> 16 at 112 x 112, N = 4: 12 / 22; 488 -> 24 at 63 x 95, N = 2: 83 / 53).
   plan->direct = false;
   static const int direct_env = [] { const char *v = getenv("WINOCONV_DIRECT"); return v && *v ? atoi(v) : 1; }();
-  if (d->algo == WINOCONV_ALGO_AUTO && d->tile_m == 0 && d->gemm_engine == WINOCONV_GEMM_AUTO && pdt == WINOCONV_F32 && direct_env != 0 &&
-      (plan->row || (d->dtype == WINOCONV_F32 && direct_env == 2))) {
+  const bool direct_ok = d->algo == WINOCONV_ALGO_AUTO && d->gemm_engine == WINOCONV_GEMM_AUTO && pdt == WINOCONV_F32;
+  const bool f32_f43_wins = d->dtype == WINOCONV_F32 && f43_ok && direct_env != 2 &&
+                            (long long)g.C * ((g.K + 63) / 64 * 64) > 32LL * (g.C + g.K);
+  if (d->tile_m == 1 && !direct_ok) return fail(WINOCONV_ERR_UNSUPPORTED, "tile_m = 1 (direct taps) goes with algo, engine and product dtype left to the planner");
+  if (direct_ok && (d->tile_m == 1 || (d->tile_m == 0 && direct_env != 0 && (d->dtype == WINOCONV_F32 ? !f32_f43_wins : plan->row)))) {
     DirectDesc &q = plan->dd;
     direct_forward_desc(&q, d->dtype, g.N, g.C, g.K, in, ks, st, pd, out, g.yH, g.yW, g.epilogue, g.weight_layout);
     plan->direct = direct_plan(q, &plan->dp);
+    if (d->tile_m == 1 && !plan->direct)
+      return fail(WINOCONV_ERR_UNSUPPORTED, "tile_m = 1 (direct taps) needs channels a multiple of 16 bytes and a slab that fits shared memory");
   }
 
   winoconv_plan_info_t &I = plan->info;
@@ -775,6 +785,30 @@ int winoconv_gemm_batched(int dtype, int product_dtype, int gemm_engine, int pos
   int st = winoconv_device_check();
   if (st != WINOCONV_OK) return st;
   return run_gemm(dtype, product_dtype, engine, positions, tiles, c_pad, k_out, v, u, m, (cudaStream_t)stream);
+}
+
+static int check_layout(const void *x, const void *y, int in_dtype, int out_dtype, int batch, int c, int64_t pixels) {
+  if (!x || !y) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "null tensor");
+  if (in_dtype < WINOCONV_F32 || in_dtype > WINOCONV_BF16 || out_dtype < WINOCONV_F32 || out_dtype > WINOCONV_BF16) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "bad dtype");
+  if (batch <= 0 || c <= 0 || pixels <= 0) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "sizes must be positive");
+  if (batch > 65535 || pixels > 0x3fffffff || c > 64 * 65535) return fail(WINOCONV_ERR_UNSUPPORTED, "tensor too large for the layout kernels");
+  if (!aligned16(x) || !aligned16(y)) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "tensors must be 16-byte aligned");
+  return winoconv_device_check();
+}
+
+int winoconv_to_channels_last(const void *x, int in_dtype, void *y, int out_dtype, int batch, int c, int64_t pixels, int c_stride, void *stream) {
+  int st = check_layout(x, y, in_dtype, out_dtype, batch, c, pixels);
+  if (st != WINOCONV_OK) return st;
+  if (c_stride < c) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "channel stride smaller than the channel count");
+  const cudaError_t e = launch_to_channels_last(in_dtype, out_dtype, x, y, batch, c, (int)pixels, c_stride, (cudaStream_t)stream);
+  return e == cudaSuccess ? WINOCONV_OK : cuda_fail(e, "layout kernel launch");
+}
+
+int winoconv_to_channels_first(const void *x, int in_dtype, void *y, int out_dtype, const float *bias, int batch, int c, int64_t pixels, void *stream) {
+  int st = check_layout(x, y, in_dtype, out_dtype, batch, c, pixels);
+  if (st != WINOCONV_OK) return st;
+  const cudaError_t e = launch_to_channels_first(in_dtype, out_dtype, x, y, bias, batch, c, (int)pixels, (cudaStream_t)stream);
+  return e == cudaSuccess ? WINOCONV_OK : cuda_fail(e, "layout kernel launch");
 }
 
 int winoconv_split(const float *x, float *out, int batch, int d, int h, int w, int c, int block_d, int block_h,

@@ -64,7 +64,7 @@ struct DGeom {
   int n_ph, n_var, org_h[4], org_w[4], taps[4], tap0[4], T_hw;   // parts of the taps: all of them per item, or one (variants)
   int n_chunks, ch_el, k_full, k_tail;   // channel chunks, channels per chunk, MMA K steps of a full and of the last chunk
   int units;                         // kD * T_hw * n_chunks: (tap, chunk) pairs of the whole reduction
-  int G, split;
+  int G, split, dual;                // taps per filter stage, CTAs (pairs) per item, whether both issuers have MMAs in every share
   unsigned epilogue;
   int y_tma, bias_vec;
   uint32_t a_hi, b_hi;               // high descriptor words
@@ -156,6 +156,13 @@ template <typename F> __device__ __forceinline__ bool for_steps(const DGeom &g, 
   return true;
 }
 
+// fp32: two threads take alternate K steps of a block into accumulators of their own (one thread issues an MMA every 60 to
+// 85 clocks, three products a step), and the products with a remainder go to another pair: the accumulator is cut off after
+// every MMA, so its error grows with the number of MMAs that went into it times its size -- small products in a small
+// accumulator cost nothing, and the large ones have a chain a sixth as long (64 -> 64 channels, 3x3: largest error 1.9e-5 of the
+// output scale with one accumulator for everything, under 1e-5 with four).  The epilogue adds them up.
+__host__ __device__ constexpr int accumulators_of_a_block(bool f32) { return f32 ? 4 : 1; }
+
 template <typename T, int BN, int MB, bool PAIR>
 __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
     direct_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_u,
@@ -163,8 +170,10 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
                   const __grid_constant__ DGeom g, const __grid_constant__ DSmem sl, uint32_t idesc) {
   constexpr bool F32 = std::is_same<T, float>::value;
   constexpr int COLS = OutWord<T>::COLS;            // output columns of one 128-byte staging row
-  constexpr int ACC = MB * BN;                      // accumulator columns of a buffer
-  constexpr int N_ISSUE = MB >= 2 ? 2 : 1;
+  constexpr int KS = F32 ? 2 : 1;                   // threads that share a block's K steps
+  constexpr int N_ACC = accumulators_of_a_block(F32);
+  constexpr int ACC = MB * BN * N_ACC;              // accumulator columns of a buffer
+  constexpr int N_ISSUE = MB >= 2 || KS == 2 ? 2 : 1;
   constexpr int BNH = PAIR ? BN / 2 : BN;           // filter rows this CTA loads
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
@@ -299,13 +308,13 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
         if (!mbar_wait_warp(acc_empty(buf), ((n_done >> 1) & 1u) ^ 1u, abort_word, err, ERR_ACC)) { alive = false; break; }
         tc_fence_after();
         const uint32_t d0 = tmem + (uint32_t)(buf * ACC + me * BN);
-        uint32_t acc = 0;
+        uint32_t acc = 0, cnt = 0;        // whether this thread's accumulators hold something; MMAs of the item so far (mod 2)
         const bool loaded = resident && n_done > 0;
         if (resident) { bs = 0; }
         alive = for_steps(g, g.n_var > 1 ? item / g.var_items : 0, u0, u1, [&](int kd, int p, int ch, int t0, int t1) -> bool {
           if (!mbar_wait_warp(F32 ? a_split(as) : a_full(as), a_ph, abort_word, err, ERR_A)) return false;
           tc_fence_after();
-          const uint32_t a_lo = desc_lo(base + (uint32_t)(as * sl.a_bytes)) + (uint32_t)(me * g.mb_off16);
+          const uint32_t a_lo = desc_lo(base + (uint32_t)(as * sl.a_bytes)) + (uint32_t)(KS == 2 ? 0 : me * g.mb_off16);
           const int nk = ch == g.n_chunks - 1 ? g.k_tail : g.k_full;
           const uint16_t *rows = g.tap_off + g.tap0[p];
           for (int t = t0; t < t1; t += g.G) {
@@ -321,31 +330,38 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
                 const uint32_t a_k = a_t + (uint32_t)(mb * g.mb_off16) + 2u * k, b_k = b_lo + 2u * k, d = d0 + (uint32_t)(mb * BN);
                 if (F32) {
                   const uint32_t al = a_k + (uint32_t)(sl.lo_off >> 4), bl = b_k + (uint32_t)(sl.b_lo >> 4);
-                  umma<PAIR, F32>(d, al, g.a_hi, b_k, g.b_hi, idesc, keep);
-                  umma<PAIR, F32>(d, a_k, g.a_hi, bl, g.b_hi, idesc, 1u);
-                  umma<PAIR, F32>(d, a_k, g.a_hi, b_k, g.b_hi, idesc, 1u);
+                  umma<PAIR, F32>(d + 2 * BN, al, g.a_hi, b_k, g.b_hi, idesc, keep);
+                  umma<PAIR, F32>(d, a_k, g.a_hi, b_k, g.b_hi, idesc, keep);
+                  umma<PAIR, F32>(d + 2 * BN, a_k, g.a_hi, bl, g.b_hi, idesc, 1u);
                 } else {
                   umma<PAIR, F32>(d, a_k, g.a_hi, b_k, g.b_hi, idesc, keep);
                 }
               }
             };
+            const bool whole = nk == 4 && (KS == 1 || g.dual);
             if (elect_one()) {
-              if (nk == 4) {     // whole 128-byte rows: straight-line code, the offset of the next tap read ahead
+              if (whole) {       // whole 128-byte rows: straight-line code, the offset of the next tap read ahead
                 uint32_t off = rows[t];
                 for (int j = 0; j < n; ++j, b_lo += (uint32_t)(sl.b_tile >> 4)) {
                   const uint32_t a_t = a_lo + off;
                   off = rows[t + j + 1];
-                  k_step(a_t, 0, acc); k_step(a_t, 1, 1u); k_step(a_t, 2, 1u); k_step(a_t, 3, 1u);
+                  if (KS == 1) { k_step(a_t, 0, acc); k_step(a_t, 1, 1u); k_step(a_t, 2, 1u); k_step(a_t, 3, 1u); }
+                  else { k_step(a_t, me, acc); k_step(a_t, me + 2, 1u); }
                   acc = 1u;
                 }
               } else {
+                uint32_t c = cnt;
                 for (int j = 0; j < n; ++j, b_lo += (uint32_t)(sl.b_tile >> 4)) {
                   const uint32_t a_t = a_lo + rows[t + j];
-                  for (int k = 0; k < nk; ++k, acc = 1u) k_step(a_t, k, acc);
+                  for (int k = 0; k < nk; ++k, ++c)
+                    if (KS == 1 || (g.dual ? (c & 1u) == (uint32_t)me : me == 0)) { k_step(a_t, k, acc); acc = 1u; }
                 }
               }
             }
-            acc = 1u;
+            // what the elected lane did, for the others (and the next election)
+            const uint32_t m = (uint32_t)(n * nk);
+            if (KS == 1 || whole || m + (((cnt ^ (uint32_t)me) & 1u) ^ 1u) >= 2u) acc = 1u;
+            cnt += m;
             if (!resident && elect_one()) umma_commit<PAIR>(b_empty(bs), pair_mask);
             if (++bs == sl.n_b) { bs = 0; b_ph ^= 1u; }
           }
@@ -418,6 +434,18 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
           if (COLS == 64) tmem_ld_x32(ta + 32u, r + 32 % COLS);
           tmem_wait_ld_x32(r);
           if (COLS == 64) tmem_wait_ld_x32(r + 32 % COLS);
+#pragma unroll
+          for (int a = 1; a < N_ACC; ++a)      // the block's other accumulators (1 and 3 are the second thread's)
+            if (g.dual || a == 2) {
+              uint32_t r2[32];
+#pragma unroll
+              for (int hc = 0; hc < COLS; hc += 32) {
+                tmem_ld_x32(ta + (uint32_t)(a * BN + hc), r2);
+                tmem_wait_ld_x32(r2);
+#pragma unroll
+                for (int i = 0; i < 32; ++i) r[hc + i] = __float_as_uint(__uint_as_float(r[hc + i]) + __uint_as_float(r2[i]));
+              }
+            }
         }
         if (ci + 2 >= N_CH) {      // this warp's last columns are in registers: its share of the hand-back
           tc_fence_before();
@@ -514,10 +542,19 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
       const int q = warp & 3, half = (warp - EPI_WARP0) >> 2;
       if (mbar_wait_warp(acc_full(0), 0u, abort_word, err, ERR_EPI)) {
         tc_fence_after();
-        for (int c0 = half * 32; c0 < ACC; c0 += 64) {
+        for (int c0 = half * 32; c0 < MB * BN; c0 += 64) {
           uint32_t r[32];
           tmem_ld_x32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
           tmem_wait_ld_x32(r);
+#pragma unroll
+          for (int a = 1; a < N_ACC; ++a)
+            if (g.dual || a == 2) {
+              uint32_t r2[32];
+              tmem_ld_x32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * BN + c0), r2);
+              tmem_wait_ld_x32(r2);
+#pragma unroll
+              for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(r2[i]));
+            }
           const int mb = c0 / BN;
           float4 *dst = reinterpret_cast<float4 *>(base_ptr) + ((mb * BM + q * 32 + lane) * ROW_F + (c0 - mb * BN)) / 4;
 #pragma unroll
@@ -661,7 +698,7 @@ static int clusters_at_once(int width) { return width == 1 ? 148 : width == 2 ? 
 // per clock, or its loads: about 28 B per clock and SM from L2 when all SMs load, at most 60 for one.  Set-up, first loads
 // and drain of a launch were measured at about 8000 clocks, 800 more for a pair, 4600 for a cluster's exchange of partial sums.
 static double estimate(const DirectPlan &p, double k_steps, int n_steps, int n_var, bool f32) {
-  const double t_mma = p.BN == 256 ? 130 : p.BN == 128 ? 66 : p.MB >= 2 ? 48 : 60;
+  const double t_mma = p.BN == 256 ? 130 : p.BN == 128 ? 66 : p.MB >= 2 || f32 ? 48 : 60;
   const int bn_own = p.pair ? p.BN / 2 : p.BN;
   const double mma = k_steps * p.MB * t_mma * (f32 ? 3 : 1);
   const double loads = n_steps * (double)p.slab_bytes + k_steps * bn_own * 32.0 * (f32 ? 2 : 1);
@@ -804,9 +841,9 @@ bool direct_plan(const DirectDesc &d, DirectPlan *out) {
 
   struct Cfg { int BN, MB, pair; };
   static const Cfg cfgs16[] = {{256, 1, 1}, {128, 2, 1}, {128, 1, 1}, {64, 2, 1}, {128, 1, 0}, {64, 1, 0}, {64, 2, 0}};
-  static const Cfg cfgs32[] = {{128, 1, 0}, {64, 1, 0}};
+  static const Cfg cfgs32[] = {{64, 1, 0}};
   const Cfg *cfgs = f32 ? cfgs32 : cfgs16;
-  const int n_cfgs = f32 ? 2 : 7;
+  const int n_cfgs = f32 ? 1 : 7;
   const int force = [] { const char *v = getenv("WINOCONV_DIRECT_CFG"); return v && *v ? atoi(v) : -1; }();
   const int force_split = [] { const char *v = getenv("WINOCONV_DIRECT_SPLIT"); return v && *v ? atoi(v) : 0; }();
   double best = 1e30;
@@ -1019,6 +1056,13 @@ cudaError_t launch_direct_forward(const DirectDesc &d, const DirectPlan &p, cons
     }
   }
   g.n_chunks = p.n_chunks; g.ch_el = p.ch_el; g.k_full = p.k_full; g.k_tail = p.k_tail; g.units = p.units;
+  {   // MMAs of the smallest share of an item
+    const int per_unit = p.n_chunks > 1 ? 1 : p.k_tail;
+    int least = p.units / p.split * per_unit;
+    if (d.variants)
+      for (int q = 0; q < d.n_parts; ++q) least = std::min(least, d.kD * p.taps[q] * p.n_chunks * per_unit);
+    g.dual = least >= 2;
+  }
   g.G = p.G; g.split = p.split; g.epilogue = d.epilogue;
   g.y_tma = y_tma; g.bias_vec = y_tma && (reinterpret_cast<uintptr_t>(bias) & 15u) == 0;
   g.a_hi = desc_hi((uint32_t)(p.PW * p.TI * p.rb), swz_code);
@@ -1048,7 +1092,6 @@ cudaError_t launch_direct_forward(const DirectDesc &d, const DirectPlan &p, cons
   } while (0)
   if (d.dtype == WINOCONV_F16) WINO_PICK(__half);
   if (d.dtype == WINOCONV_BF16) WINO_PICK(__nv_bfloat16);
-  if (p.BN == 128) WINO_GO(float, 128, 1, false);
   WINO_GO(float, 64, 1, false);
 #undef WINO_PICK
 #undef WINO_GO

@@ -16,6 +16,9 @@ cudaError_t launch_split(const float *x, float *out, int N, int D, int H, int W,
                          int oD, int oH, int oW, int nD, int nH, int nW, cudaStream_t s);
 cudaError_t launch_concat(const float *tiles, float *y, int N, int oD, int oH, int oW, int K, int mD, int mH, int mW,
                           cudaStream_t s);
+// [N, C, P] -> [N, P, Cs] (zeros from channel C on) and [N, P, C] -> [N, C, P] (+ bias), converting the element type
+cudaError_t launch_to_channels_last(int in_dtype, int out_dtype, const void *x, void *y, int N, int C, int P, int Cs, cudaStream_t s);
+cudaError_t launch_to_channels_first(int in_dtype, int out_dtype, const void *x, void *y, const float *bias, int N, int C, int P, cudaStream_t s);
 cudaError_t launch_add(const float *a, const float *b, float *c, long long n, cudaStream_t s);
 
 // m[p][t][k] = sum_c v[p][t][c] u[p][k][c]; fp32 accumulate.

@@ -66,8 +66,20 @@ def dwm3d_(x, w, stride=1):
     return _dwm(x, w, stride, 3)
 
 
+def _native(input, kernel, bias, stride, padding, nd):
+    """The whole call in one native function (layout in, filter, convolution with its padding and bias, layout out), or None
+    where the steps below have to decide: another output block asked for, a tensor to refuse."""
+    backend = _load()
+    if not input.is_cuda or backend.get_dwm_output_block() != 2:
+        return None
+    return backend.conv_call(input, kernel, bias, (_stride_int(stride, nd),) * nd, padding, -1, False, 2)
+
+
 def dwm2d(input, kernel, bias=None, stride=(1, 1), padding=0, groups=1):
     ph, pw = _pad_tuple(padding, 2)
+    out = _native(input, kernel, bias, stride, (ph, pw), 2)
+    if out is not None:
+        return out
     if ph or pw:
         input = torch.nn.functional.pad(input, (pw, pw, ph, ph))
     out = dwm2d_(input, kernel, _stride_int(stride, 2))
@@ -78,6 +90,9 @@ def dwm2d(input, kernel, bias=None, stride=(1, 1), padding=0, groups=1):
 
 def dwm3d(input, kernel, bias=None, stride=(1, 1, 1), padding=0, groups=1):
     pd, ph, pw = _pad_tuple(padding, 3)
+    out = _native(input, kernel, bias, stride, (pd, ph, pw), 3)
+    if out is not None:
+        return out
     if pd or ph or pw:
         input = torch.nn.functional.pad(input, (pw, pw, ph, ph, pd, pd))
     out = dwm3d_(input, kernel, _stride_int(stride, 3))

@@ -9,7 +9,8 @@ the engine too (the reference falls back to cuDNN, ``matrix_conv.py:71-75,93-95`
 import torch
 
 from . import matrix_convnd
-from .engine import conv_forward
+from ._backend import load as _load
+from .engine import conv_forward, dtype_code
 from .Split_and_Concat import wino_concat, wino_split
 
 USE_SPLIT_CHAIN = False
@@ -48,13 +49,18 @@ def _run(input, kernel, bias, stride, padding, output_block, fp16):
         input = input.cuda()
     kernel = kernel.to(input.device)
     strides = (stride,) * _ND if isinstance(stride, int) else tuple(stride)
+    ks = tuple(int(s) for s in kernel.shape[2:])
+    tile_m = output_block if (output_block == 2 or (ks == (3, 3) and all(s == 1 for s in strides))) else 2
     dt = torch.float16 if fp16 else torch.float32
+    if not (USE_SPLIT_CHAIN and all(s == 1 for s in strides)):
+        pads = (padding,) * _ND if isinstance(padding, int) else tuple(padding)
+        out = _load().conv_call(input, kernel, bias, strides, pads, dtype_code(dt), True, tile_m)     # the whole call, natively
+        if out is not None:
+            return out
     x, w = _pad(input, padding).to(dt), kernel.to(dt)
     if USE_SPLIT_CHAIN and all(s == 1 for s in strides):
         out = conv(x.float(), w.float(), output_block, strides, fp16)
     else:
-        ks = tuple(int(s) for s in kernel.shape[2:])
-        tile_m = output_block if (output_block == 2 or (ks == (3, 3) and all(s == 1 for s in strides))) else 2
         out = conv_forward(x, w, stride=strides, padding=0, tile_m=tile_m)
     out = out.float()
     if bias is not None:

@@ -2,7 +2,8 @@
 import torch
 
 from . import matrix_convnd
-from .engine import conv_forward
+from ._backend import load as _load
+from .engine import conv_forward, dtype_code
 from .Split_and_Concat import wino_concat, wino_split
 
 USE_SPLIT_CHAIN = False
@@ -33,6 +34,10 @@ def _run(input, kernel, bias, stride, padding, output_block, fp16):
     strides = (stride,) * _ND if isinstance(stride, int) else tuple(stride)
     pads = (padding,) * _ND if isinstance(padding, int) else tuple(padding)
     dt = torch.float16 if fp16 else torch.float32
+    if not (USE_SPLIT_CHAIN and all(s == 1 for s in strides)):
+        out = _load().conv_call(input, kernel, bias, strides, pads, dtype_code(dt), True, 2)     # the whole call, natively
+        if out is not None:
+            return out
     x, w = input.to(dt), kernel.to(dt)
     if any(pads):
         x = torch.nn.functional.pad(x, (pads[2], pads[2], pads[1], pads[1], pads[0], pads[0]))
