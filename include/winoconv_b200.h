@@ -99,7 +99,9 @@ typedef struct winoconv_desc {
   int32_t gemm_engine;   /* winoconv_gemm_t                                                  */
   int32_t product_dtype; /* dtype of the Winograd-domain products: F32 (default), F16, BF16  */
   int32_t algo;          /* winoconv_algo_t                                                  */
-  int32_t reserved[5];
+  int32_t bias_f32;      /* 1: the bias is f32 whatever dtype is (layers on the direct-tap kernel)   */
+  int32_t x_channels_first; /* 1: x is [N, C, D, H, W] (16-bit layers of few channels: kW * C <= 64)  */
+  int32_t reserved[3];
 } winoconv_desc_t;
 
 /* What winoconv_plan() derives from a descriptor. */
@@ -114,7 +116,8 @@ typedef struct winoconv_plan_info {
   int32_t gemm_engine;        /* engine AUTO resolves to                                      */
   int32_t algo;               /* algorithm AUTO resolves to (winoconv_algo_t)                 */
   int32_t direct;             /* 1: AUTO runs the layer on the direct-tap kernel: one launch, no     */
-                              /* scratch; algo, positions, n_pieces, tiles and gemm_flops are then   */
+                              /* scratch (2: after a copy of x with padded channels in v_ws); algo,  */
+                              /* positions, n_pieces, tiles and gemm_flops are then   */
                               /* those of the algorithm an explicit request would run                */
   int64_t tiles;              /* N * nD * nH * nW                                             */
   uint64_t filter_bytes;      /* size of the transformed filter U [positions][K][c_pad]       */

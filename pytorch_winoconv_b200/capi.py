@@ -38,7 +38,8 @@ class Desc(Structure):
     _fields_ = [("ndim", c_int32), ("batch", c_int32), ("c_in", c_int32), ("k_out", c_int32),
                 ("in_size", c_int32 * 3), ("ker_size", c_int32 * 3), ("stride", c_int32 * 3), ("pad", c_int32 * 3),
                 ("tile_m", c_int32), ("dtype", c_int32), ("weight_layout", c_int32), ("epilogue", c_uint32),
-                ("gemm_engine", c_int32), ("product_dtype", c_int32), ("algo", c_int32), ("reserved", c_int32 * 5)]
+                ("gemm_engine", c_int32), ("product_dtype", c_int32), ("algo", c_int32), ("bias_f32", c_int32),
+                ("x_channels_first", c_int32), ("reserved", c_int32 * 3)]
 
 
 class PlanInfo(Structure):

@@ -37,6 +37,7 @@ from typing import Optional, Tuple
 import torch
 import torch.nn as nn
 import torch.nn.functional as F
+from torch.nn.modules import module as _nn_module
 
 from . import _backend, capi, engine
 
@@ -72,6 +73,15 @@ class _WinoConvMixin:
     # and launch cost about 6 us a call where the same steps in Python cost 24.  What it does not take (an argument to
     # refuse, fp32 gradients) returns None and runs below.
     _CONFIG = frozenset(("compute_dtype", "activation", "pool", "tile_m", "algo", "stride", "padding"))
+
+    def __call__(self, *args, **kwargs):
+        """``torch.nn.Module.__call__`` without its 5 us of dispatch where there is no hook, tracer or compiled call to serve."""
+        d = self.__dict__
+        if (kwargs or len(args) != 1 or d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"]
+                or _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks or _nn_module._global_backward_hooks
+                or _nn_module._global_backward_pre_hooks or self._compiled_call_impl is not None or torch._C._get_tracing_state()):
+            return super().__call__(*args, **kwargs)
+        return self.forward(args[0])
 
     def _reset_plans(self):
         d = self.__dict__

@@ -124,14 +124,14 @@ at::Tensor ConvRunner::channels_last(const at::Tensor &t, at::ScalarType type) c
 }
 
 std::shared_ptr<ConvRunner::Entry> ConvRunner::entry_for(const at::Tensor &x, const at::Tensor &weight, const std::optional<at::Tensor> &bias,
-                                                         int dtype) {
+                                                         int dtype, bool first) {
   int64_t shape[5] = {x.size(0), 1, 1, 1, x.size(1)};
   for (int i = 0; i < nd_; ++i) shape[4 - nd_ + i] = x.size(2 + i);
-  const int device = x.get_device();
+  const int device = x.get_device(), bias_type = bias ? (int)bias->scalar_type() : -1;
   std::lock_guard<std::mutex> lock(mu_);
   for (size_t i = entries_.size(); i-- > 0;) {
     Entry &e = *entries_[i];
-    if (e.dtype == dtype && e.device == device && std::memcmp(e.shape, shape, sizeof shape) == 0) {
+    if (e.dtype == dtype && e.device == device && e.bias_type == bias_type && e.first == first && std::memcmp(e.shape, shape, sizeof shape) == 0) {
       auto hit = entries_[i];
       if (i + 1 != entries_.size()) {
         entries_.erase(entries_.begin() + i);
@@ -144,6 +144,8 @@ std::shared_ptr<ConvRunner::Entry> ConvRunner::entry_for(const at::Tensor &x, co
   std::memcpy(e->shape, shape, sizeof shape);
   e->dtype = dtype;
   e->device = device;
+  e->bias_type = bias_type;
+  e->first = first;
   winoconv_desc_t &d = e->desc;
   std::memset(&d, 0, sizeof d);
   d.ndim = nd_;
@@ -160,7 +162,12 @@ std::shared_ptr<ConvRunner::Entry> ConvRunner::entry_for(const at::Tensor &x, co
   d.dtype = dtype;
   d.epilogue = (bias ? WINOCONV_EPI_BIAS : 0u) | (relu_ ? WINOCONV_EPI_RELU : 0u) | (pool_ ? WINOCONV_EPI_POOL2 : 0u);
   d.algo = algo_;
-  if (winoconv_plan(&d, &e->info) != WINOCONV_OK) return nullptr;
+  d.x_channels_first = first ? 1 : 0;
+  d.bias_f32 = dtype != WINOCONV_F32 && bias && bias->scalar_type() == at::kFloat;      // read as it is where the kernel can
+  if (winoconv_plan(&d, &e->info) != WINOCONV_OK) {
+    d.bias_f32 = 0;
+    if (winoconv_plan(&d, &e->info) != WINOCONV_OK) return nullptr;
+  }
   entries_.push_back(e);
   while (entries_.size() > max_plans_) entries_.erase(entries_.begin());      // each entry holds its own transformed filter
   return e;
@@ -182,7 +189,7 @@ at::Tensor ConvRunner::run(Entry &e, const at::Tensor &x, const at::Tensor &weig
         w = w.to(type);
         check_abi(winoconv_filter_transform(&e.desc, w.data_ptr(), e.u.data_ptr(), s), "winoconv_filter_transform");
       }
-      e.bias = bias ? bias->to(type).contiguous() : at::Tensor();
+      e.bias = bias ? bias->detach().to(e.desc.bias_f32 ? at::kFloat : type).contiguous() : at::Tensor();
       e.stamp = now;
       e.serial = ++serial_;
       newest_ = now;
@@ -195,9 +202,9 @@ at::Tensor ConvRunner::run(Entry &e, const at::Tensor &x, const at::Tensor &weig
   at::Tensor y = at::empty(at::IntArrayRef(sizes, nd_ + 2), x.options().dtype(type).requires_grad(false),
                            nd_ == 2 ? at::MemoryFormat::ChannelsLast : at::MemoryFormat::ChannelsLast3d);
   at::Tensor v, m;
-  if (!e.info.direct) {
+  if (e.info.direct != 1) {
     if (e.info.input_ws_bytes) v = empty_bytes(e.info.input_ws_bytes, x);
-    if (e.info.product_ws_bytes) m = empty_bytes(e.info.product_ws_bytes, x);
+    if (!e.info.direct && e.info.product_ws_bytes) m = empty_bytes(e.info.product_ws_bytes, x);
   }
   check_abi(winoconv_forward(&e.desc, x.data_ptr(), u.data_ptr(), b.defined() ? b.data_ptr() : nullptr, y.data_ptr(),
                              v.defined() ? v.data_ptr() : nullptr, e.info.input_ws_bytes, m.defined() ? m.data_ptr() : nullptr,
@@ -215,7 +222,16 @@ std::optional<at::Tensor> ConvRunner::forward(const at::Tensor &x, const at::Ten
   const bool grad = at::GradMode::is_enabled() && (x.requires_grad() || (weight.requires_grad() && training));
   if (grad && (pool_ || dtype == WINOCONV_F32)) return std::nullopt;
   c10::cuda::CUDAGuard guard(x.device());
-  std::shared_ptr<Entry> e = entry_for(x, weight, bias, dtype);
+  std::shared_ptr<Entry> e;
+  if (!grad && dtype != WINOCONV_F32 && tile_m_ == 0 && algo_ == WINOCONV_ALGO_AUTO && x.scalar_type() == type_of(dtype) && x.is_contiguous() && x.size(1) * weight.size(-1) <= 64 && x.size(1) > 1 && !lies_channels_last(x)) {
+    // few channels in torch's contiguous order: the kernel gathers them as they lie
+    e = entry_for(x, weight, bias, dtype, true);
+    if (e) {
+      at::AutoDispatchBelowADInplaceOrView no_graph;
+      return run(*e, x, weight, bias);
+    }
+  }
+  e = entry_for(x, weight, bias, dtype, false);
   if (!e) return std::nullopt;
   if (!grad) {
     at::AutoDispatchBelowADInplaceOrView no_graph;
@@ -242,7 +258,7 @@ std::vector<at::Tensor> ConvRunner::backward(const at::Tensor &gy_in, const at::
   c10::cuda::CUDAGuard guard(x_in.device());
   const int dtype = compute_ >= 0 ? compute_ : code_of(x_in.scalar_type());
   const at::ScalarType type = type_of(dtype);
-  std::shared_ptr<Entry> e = entry_for(x_in, weight, bias, dtype);
+  std::shared_ptr<Entry> e = entry_for(x_in, weight, bias, dtype, false);
   TORCH_CHECK(e, "winoconv backward: no plan");
   void *s = stream_of();
   at::Tensor gy = gy_in;
@@ -354,9 +370,9 @@ std::optional<at::Tensor> conv_call(const at::Tensor &x_in, const at::Tensor &we
   at::Tensor b;
   if (bias) b = bias->to(x.device(), bias_after ? at::kFloat : type).contiguous();
   at::Tensor v, m;
-  if (!info.direct) {
+  if (info.direct != 1) {
     if (info.input_ws_bytes) v = empty_bytes(info.input_ws_bytes, x);
-    if (info.product_ws_bytes) m = empty_bytes(info.product_ws_bytes, x);
+    if (!info.direct && info.product_ws_bytes) m = empty_bytes(info.product_ws_bytes, x);
   }
   int64_t sizes[5] = {d.batch, d.k_out, 0, 0, 0};
   for (int i = 0; i < nd; ++i) sizes[2 + i] = info.out_size[3 - nd + i];

@@ -44,12 +44,13 @@ class ConvRunner : public torch::CustomClassHolder {
   };
   struct Entry {
     int64_t shape[5] = {0, 0, 0, 0, 0};      // N, D, H, W, C of the input
-    int dtype = -1, device = -1;
+    int dtype = -1, device = -1, bias_type = -1;   // bias_type: scalar type of the bias, -1 without one
     winoconv_desc_t desc;
     winoconv_plan_info_t info;
     at::Tensor u, bias;                      // transformed filter, bias in the compute dtype
     Stamp stamp;
     int64_t serial = 0;
+    bool first = false;                      // x in torch's contiguous order
     at::Tensor u_back;                       // filter of the data gradient
     Stamp back_stamp;
     bool back_known = false, back_ok = false;
@@ -61,7 +62,7 @@ class ConvRunner : public torch::CustomClassHolder {
                                    const std::optional<at::Tensor> &bias, bool need_x, bool need_w, bool need_b);
 
  private:
-  std::shared_ptr<Entry> entry_for(const at::Tensor &x, const at::Tensor &weight, const std::optional<at::Tensor> &bias, int dtype);
+  std::shared_ptr<Entry> entry_for(const at::Tensor &x, const at::Tensor &weight, const std::optional<at::Tensor> &bias, int dtype, bool first);
   at::Tensor channels_last(const at::Tensor &t, at::ScalarType type) const;
 
   int nd_, stride_[3], pad_[3], tile_m_, algo_, compute_;

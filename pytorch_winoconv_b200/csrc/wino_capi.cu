@@ -271,10 +271,26 @@ int build_plan(const winoconv_desc_t *d, Plan *plan) {
   if (direct_ok && (d->tile_m == 1 || (d->tile_m == 0 && direct_env != 0 && (d->dtype == WINOCONV_F32 ? !f32_f43_wins : plan->row)))) {
     DirectDesc &q = plan->dd;
     direct_forward_desc(&q, d->dtype, g.N, g.C, g.K, in, ks, st, pd, out, g.yH, g.yW, g.epilogue, g.weight_layout);
-    plan->direct = direct_plan(q, &plan->dp);
+    // few channels: folded, x gathered as it lies; otherwise channels that TMA cannot address go through a padded copy
+    const int vec = d->dtype == WINOCONV_F32 ? 4 : 8;
+    bool folded = false;
+    if (g.C % vec != 0 || d->x_channels_first) {
+      DirectDesc fd = q;
+      folded = direct_fold_desc(&fd, pd, d->x_channels_first) && direct_plan(fd, &plan->dp);
+      if (folded) q = fd;
+    }
+    if (folded) plan->direct = true;
+    else if (!d->x_channels_first) {
+      q.C = (g.C + vec - 1) / vec * vec;
+      plan->direct = direct_plan(q, &plan->dp);
+    }
     if (d->tile_m == 1 && !plan->direct)
-      return fail(WINOCONV_ERR_UNSUPPORTED, "tile_m = 1 (direct taps) needs channels a multiple of 16 bytes and a slab that fits shared memory");
+      return fail(WINOCONV_ERR_UNSUPPORTED, "tile_m = 1 (direct taps) needs a slab that fits shared memory");
   }
+
+  if (d->x_channels_first && !plan->direct) return fail(WINOCONV_ERR_UNSUPPORTED, "x_channels_first is for few-channel layers on the direct-tap kernel (kW * C <= 64, 16-bit)");
+  if (d->bias_f32 && !plan->direct) return fail(WINOCONV_ERR_UNSUPPORTED, "an f32 bias for a 16-bit layer needs the direct-tap kernel");
+  plan->dd.bias_f32 = d->bias_f32 && d->dtype != WINOCONV_F32;
 
   winoconv_plan_info_t &I = plan->info;
   for (int i = 0; i < 3; ++i) { I.conv_out_size[i] = out[i]; I.tile_m[i] = m[i]; I.tiles_per_dim[i] = nt[i]; }
@@ -318,7 +334,13 @@ int build_plan(const winoconv_desc_t *d, Plan *plan) {
     I.block_tiles = I.tiles;
   }
   if (plan->direct) {
-    I.direct = 1;
+    const DirectDesc &q = plan->dd;
+    I.direct = !q.fold && q.C != q.Cw ? 2 : 1;
+    if (I.direct == 2) {
+      const unsigned long long copy = (unsigned long long)g.N * g.D * g.H * g.W * q.C * esz;
+      I.input_ws_bytes = std::max<unsigned long long>(I.input_ws_bytes, copy);
+      I.input_ws_bytes_min = std::max<unsigned long long>(I.input_ws_bytes_min, copy);
+    }
     I.filter_bytes = std::max<unsigned long long>(I.filter_bytes, (unsigned long long)plan->dp.filter_elems * esz);
   }
   I.direct_flops = 2.0 * g.N * g.K * g.C * (double)ks[0] * ks[1] * ks[2] * (double)out[0] * out[1] * out[2];
@@ -366,7 +388,7 @@ struct BackPlan {
 };
 int build_back_plan(const winoconv_desc_t *d, BackPlan *b) {
   winoconv_desc_t f = *d;     // the forward layer's shape, whatever algorithm and epilogue it runs with
-  f.algo = WINOCONV_ALGO_AUTO; f.tile_m = 0; f.gemm_engine = WINOCONV_GEMM_AUTO; f.product_dtype = WINOCONV_F32; f.epilogue = 0;
+  f.algo = WINOCONV_ALGO_AUTO; f.tile_m = 0; f.gemm_engine = WINOCONV_GEMM_AUTO; f.product_dtype = WINOCONV_F32; f.epilogue = 0; f.bias_f32 = 0; f.x_channels_first = 0;
   const Plan *p = nullptr;
   const int st = plan_of<Plan>(&f, build_plan, &p);
   if (st != WINOCONV_OK) return st;
@@ -517,7 +539,7 @@ static int forward_impl(const winoconv_desc_t *desc, const void *x, const void *
   if (!x || !u || !y) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "null tensor pointer");
   if ((desc->epilogue & WINOCONV_EPI_BIAS) && !bias) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "EPI_BIAS set but bias is null");
   if (!aligned16(x) || !aligned16(u) || !aligned16(y)) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "tensors must be 16-byte aligned");
-  if (plan.row && !plan.direct && plan.info.input_ws_bytes_min > 0) {
+  if (plan.direct ? plan.info.direct == 2 : plan.row && plan.info.input_ws_bytes_min > 0) {
     if (!v_ws || !aligned16(v_ws)) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "channel-padding scratch (v_ws) must be a 16-byte aligned pointer");
     if (v_ws_bytes < plan.info.input_ws_bytes_min)
       return fail(WINOCONV_ERR_WORKSPACE, "v_ws holds " + std::to_string(v_ws_bytes) + " bytes; padding the input channels needs " +
@@ -539,11 +561,17 @@ static int forward_impl(const winoconv_desc_t *desc, const void *x, const void *
       if (e != cudaSuccess) return cuda_fail(e, "event record");
     }
     const char *detail = "";
+    if (plan.info.direct == 2) {     // channels padded to 16 bytes
+      const DirectDesc &q = plan.dd;
+      e = launch_pad_channels(plan.dtype, x, v_ws, (long long)q.N * q.D * q.H * q.W, q.Cw, q.C, fs);
+      if (e != cudaSuccess) return cuda_fail(e, "channel padding launch");
+      x = v_ws;
+    }
     e = plan.direct ? launch_direct_forward(plan.dd, plan.dp, x, u, bias, y, fs, &detail)
         : plan.row ? launch_rowfused_forward(plan.rd, plan.rp, plan.dtype, x, u, bias, y, v_ws, fs, &detail)
                  : launch_fused_forward(plan.fg, plan.dtype, x, u, bias, y, fs, &detail);
     if (e != cudaSuccess) return cuda_fail(e, "fused forward launch", detail);
-    if (launches) *launches = (plan.row && !plan.direct && plan.info.input_ws_bytes_min > 0) ? 2 : 1;
+    if (launches) *launches = (plan.direct ? plan.info.direct == 2 : plan.row && plan.info.input_ws_bytes_min > 0) ? 2 : 1;
     if (stage_ms) {
       stage_ms[0] = stage_ms[2] = 0.f;
       e = cudaEventRecord(e1, fs);

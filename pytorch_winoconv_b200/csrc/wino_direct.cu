@@ -19,6 +19,11 @@
 // tensor memory), warps 4-11 epilogue (lane quarter x alternate 128-byte column chunks: bias, ReLU, 2x2 pool, TMA stores),
 // for fp32 also warps 12-15, which split every landed slab into a tf32 part and its remainder (three products per multiply,
 // the filter comes split from its transform).
+// Few channels (an RGB stem) would leave most of a 16-channel step empty and cannot be loaded by TMA (16-byte pixels).  There
+// the taps along W are folded into the channels: a slab row is an input row, its entries the 8 output pixels, an entry the
+// kW * C values those pixels' taps see; only the taps along H remain.  7x7 at stride 2 over RGB is 7 x 2 K steps instead of 49.
+// Warps 12-15 gather the entries from a patch of raw rows of x as it lies (either layout) that warp 0 loads by TMA, or, where
+// rows are not 16-byte multiples, with plain loads (the latency of those is what it costs: 130 us against 45 for the stem).
 // Small problems run with one item per cluster of 2, 4 or 8 CTAs that share its reduction and add their accumulators through
 // distributed shared memory.  Every mbarrier wait is bounded and reports through the error word.
 //
@@ -47,6 +52,7 @@ constexpr int EPI_WARP0 = 4, EPI_WARPS = 8, SPLIT_WARP0 = 12, SPLIT_WARPS = 4;
 constexpr int STAGE_BYTES = 4096;      // epilogue staging per warp: 32 rows of 128 bytes
 constexpr int MAX_TAPS = 100;
 constexpr int BAR_BYTES = 512;
+constexpr unsigned RAW_BUFS = 4;       // raw patches in flight (few channels): small, and thousands of clocks away
 constexpr int FIXED_BYTES = 1024 /*alignment*/ + EPI_WARPS * STAGE_BYTES + BAR_BYTES;
 
 enum ErrCode : unsigned { ERR_A_EMPTY = 0x401, ERR_B_EMPTY = 0x402, ERR_ACC = 0x403, ERR_A = 0x404, ERR_B = 0x405, ERR_EPI = 0x406, ERR_SPLIT = 0x407 };
@@ -66,15 +72,20 @@ struct DGeom {
   int units;                         // kD * T_hw * n_chunks: (tap, chunk) pairs of the whole reduction
   int G, split, dual;                // taps per filter stage, CTAs (pairs) per item, whether both issuers have MMAs in every share
   unsigned epilogue;
-  int y_tma, bias_vec;
+  int y_tma, bias_vec, bias_f32;
   uint32_t a_hi, b_hi;               // high descriptor words
   int mb_off16;                      // slab offset of the second row block (16-byte units)
+  // fold: x's strides and extents, channels and taps of an entry, slab rows and how far apart the rows of neighbouring outputs are
+  long long fx_n, fx_d, fx_h;
+  int fx_w, fx_c, fD, fH, fW, fC, fkW, fold_rows;
+  // ... and the raw patch: by TMA or not, element strides of its rows, pixels and channels, elements before the first pixel
+  int raw_tma, raw_row, raw_w, raw_c, raw_rem;
   uint16_t tap_off[MAX_TAPS + 1];    // offset of each tap's first pixel in the slab (16-byte units), phase by phase
 };
 struct DSmem {
   int slab_bytes, a_bytes, lo_off;   // bytes TMA delivers, bytes of a stage, offset of the remainder copy (fp32)
   int b_tile, b_lo, b_bytes, n_a, n_b;   // bytes of one tap's filter tile (hi part, and lo part for fp32), of a stage
-  int off_b, off_stage, off_bars, total;
+  int off_b, off_stage, off_raw, raw_bytes, off_bars, total;   // raw_bytes: of a raw patch, a multiple of 128
 };
 
 template <typename T> struct OutWord {   // one 32-bit word of output: a 16-bit pair
@@ -86,20 +97,22 @@ template <> struct OutWord<float> {
   static __device__ __forceinline__ uint32_t max2(uint32_t a, uint32_t b) { return __float_as_uint(fmaxf(__uint_as_float(a), __uint_as_float(b))); }
 };
 
-// 8 (16-bit) or 4 (fp32) bias values from k on
-template <typename T> __device__ __forceinline__ void load_bias16(const T *bias, int k, int K, int vec, float *b) {
-  constexpr int V = 16 / (int)sizeof(T);
+// V bias values from k on, stored as T or as floats
+template <typename TB, int V> __device__ __forceinline__ void load_bias(const TB *bias, int k, int K, int vec, float *b) {
   if (vec && k + V <= K) {
-    const uint4 q = *reinterpret_cast<const uint4 *>(bias + k);
-    const uint32_t w[4] = {q.x, q.y, q.z, q.w};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      if constexpr (sizeof(T) == 4) b[i] = __uint_as_float(w[i]);
-      else { const float2 f = Pair16<T>::unpack(w[i]); b[2 * i] = f.x; b[2 * i + 1] = f.y; }
+    for (int i = 0; i < V * (int)sizeof(TB) / 16; ++i) {
+      const uint4 q = *reinterpret_cast<const uint4 *>(bias + k + i * (16 / (int)sizeof(TB)));
+      const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if constexpr (sizeof(TB) == 4) b[4 * i + j] = __uint_as_float(w[j]);
+        else { const float2 f = Pair16<TB>::unpack(w[j]); b[8 * i + 2 * j] = f.x; b[8 * i + 2 * j + 1] = f.y; }
+      }
     }
   } else {
 #pragma unroll
-    for (int i = 0; i < V; ++i) b[i] = k + i < K ? Elem<T>::load(bias + k + i) : 0.f;
+    for (int i = 0; i < V; ++i) b[i] = k + i < K ? Elem<TB>::load(bias + k + i) : 0.f;
   }
 }
 
@@ -163,10 +176,10 @@ template <typename F> __device__ __forceinline__ bool for_steps(const DGeom &g, 
 // output scale with one accumulator for everything, under 1e-5 with four).  The epilogue adds them up.
 __host__ __device__ constexpr int accumulators_of_a_block(bool f32) { return f32 ? 4 : 1; }
 
-template <typename T, int BN, int MB, bool PAIR>
-__global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
+template <typename T, int BN, int MB, bool PAIR, bool FOLD>
+__global__ void __launch_bounds__(std::is_same<T, float>::value || FOLD ? 512 : 384, 1)
     direct_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_u,
-                  const __grid_constant__ MapSet maps_y, T *__restrict__ y, const T *__restrict__ bias,
+                  const __grid_constant__ MapSet maps_y, const T *__restrict__ x, T *__restrict__ y, const T *__restrict__ bias,
                   const __grid_constant__ DGeom g, const __grid_constant__ DSmem sl, uint32_t idesc) {
   constexpr bool F32 = std::is_same<T, float>::value;
   constexpr int COLS = OutWord<T>::COLS;            // output columns of one 128-byte staging row
@@ -185,6 +198,7 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
   auto b_full = [&](int i) { return bars + 128u + 8u * i; };
   auto b_empty = [&](int i) { return bars + 192u + 8u * i; };
   auto a_split = [&](int i) { return bars + 256u + 8u * i; };
+  auto raw_empty = [&](int i) { return bars + 352u + 8u * i; };     // (raw_full: a_split)
   auto acc_full = [&](int i) { return bars + 320u + 8u * i; };
   auto acc_empty = [&](int i) { return bars + 336u + 8u * i; };
   volatile unsigned *abort_word = reinterpret_cast<volatile unsigned *>(base_ptr + sl.off_bars + 384);
@@ -197,12 +211,14 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
   if (warp == 1 && lane == 0) { prefetch_map(&map_x); prefetch_map(&map_u); prefetch_map(&maps_y.m[0]); }
   if (warp == 0) {
     if (lane < 8) {
-      mbar_init(a_full(lane), 1); mbar_init(a_empty(lane), N_ISSUE); mbar_init(a_split(lane), SPLIT_WARPS);
+      mbar_init(a_full(lane), FOLD ? SPLIT_WARPS : 1); mbar_init(a_empty(lane), N_ISSUE); mbar_init(a_split(lane), FOLD ? 1 : SPLIT_WARPS);
     } else if (lane < 16) {
       mbar_init(b_full(lane - 8), 1); mbar_init(b_empty(lane - 8), N_ISSUE);
     } else if (lane < 18) {
       mbar_init(acc_full(lane - 16), N_ISSUE); mbar_init(acc_empty(lane - 16), PAIR ? 2 * EPI_WARPS : EPI_WARPS);
-    } else if (lane == 18) {
+    } else if (lane < 22) {
+      mbar_init(raw_empty(lane - 18), SPLIT_WARPS);
+    } else if (lane == 22) {
       *abort_word = 0u;
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -236,7 +252,30 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
   const bool resident = g.n_kb == 1 && g.split == 1 && g.n_var == 1 && g.kD * g.n_ph * g.n_chunks * ((g.taps[0] + g.G - 1) / g.G) <= sl.n_b;
   bool alive = true;
 
-  if (warp == 0) {
+  if (warp == 0 && FOLD) {
+    // ---------------------------------------------------------------- raw patches, from which warps 12-15 gather the slabs
+    uint32_t it = 0;
+    for (int item = item0; item < g.n_items && alive && g.raw_tma; item += item_step) {
+      const Tile t = decode<MB, PAIR>(g, item, rank);
+      alive = for_steps(g, t.var, u0, u1, [&](int kd, int, int, int, int) -> bool {
+        const int s = (int)(it & (RAW_BUFS - 1u));
+        if (!mbar_wait_warp(raw_empty(s), ((it / RAW_BUFS) & 1u) ^ 1u, abort_word, err, ERR_A_EMPTY)) return false;
+        if (lane == 0) {
+          const uint32_t dst = base + (uint32_t)(sl.off_raw + s * sl.raw_bytes);
+          const int w = (g.sW * t.ow0 + g.org_w[0]) * g.raw_w - g.raw_rem, h = g.sH * t.oh0 + g.org_h[0], d = g.sD * t.od + kd - g.pD;
+          mbar_expect_tx(a_split(s), (uint32_t)sl.slab_bytes);
+          if (g.raw_c == 1) tma_load_5d(dst, &map_x, a_split(s), w, h, d, t.n0, 0);     // [W * C][H][D][N]
+          else tma_load_5d(dst, &map_x, a_split(s), w, h, d, 0, t.n0);                  // [W][H][D][C][N]
+        }
+        ++it;
+        return true;
+      });
+    }
+    if (*abort_word != 0u) {
+      const long long start = clock64();
+      while (clock64() - start < 2000000LL) { }
+    }
+  } else if (warp == 0) {
     // ---------------------------------------------------------------- slabs
     int s = 0;
     uint32_t ph = 1;
@@ -340,16 +379,27 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
             };
             const bool whole = nk == 4 && (KS == 1 || g.dual);
             if (elect_one()) {
-              if (whole) {       // whole 128-byte rows: straight-line code, the offset of the next tap read ahead
+              // straight-line code per tap for the usual numbers of K steps, the offset of the next tap read ahead: a loop over
+              // the steps costs this lone thread 180 clocks an MMA
+              auto taps_of = [&](auto steps) {
+                constexpr int NK = decltype(steps)::value;
                 uint32_t off = rows[t];
                 for (int j = 0; j < n; ++j, b_lo += (uint32_t)(sl.b_tile >> 4)) {
                   const uint32_t a_t = a_lo + off;
                   off = rows[t + j + 1];
-                  if (KS == 1) { k_step(a_t, 0, acc); k_step(a_t, 1, 1u); k_step(a_t, 2, 1u); k_step(a_t, 3, 1u); }
-                  else { k_step(a_t, me, acc); k_step(a_t, me + 2, 1u); }
+                  if (KS == 2) { k_step(a_t, me, acc); k_step(a_t, me + 2, 1u); }
+                  else {
+                    k_step(a_t, 0, acc);
+#pragma unroll
+                    for (int k = 1; k < NK; ++k) k_step(a_t, k, 1u);
+                  }
                   acc = 1u;
                 }
-              } else {
+              };
+              if (whole) taps_of(std::integral_constant<int, 4>());
+              else if (KS == 1 && nk == 2) taps_of(std::integral_constant<int, 2>());
+              else if (KS == 1 && nk == 1) taps_of(std::integral_constant<int, 1>());
+              else {
                 uint32_t c = cnt;
                 for (int j = 0; j < n; ++j, b_lo += (uint32_t)(sl.b_tile >> 4)) {
                   const uint32_t a_t = a_lo + rows[t + j];
@@ -372,6 +422,84 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
         if (resident) b_ph = 0;
         if (elect_one()) umma_commit<PAIR>(acc_full(buf), pair_mask);
       }
+    }
+  } else if (FOLD && warp >= SPLIT_WARP0) {
+    // ---------------------------------------------------------------- gathered slabs: a thread keeps one 16-byte vector of the entries
+    const int st = threadIdx.x - SPLIT_WARP0 * 32;
+    const int v_shift = g.k_full == 1 ? 1 : g.k_full == 2 ? 2 : 3, v = st & ((1 << v_shift) - 1);
+    const int rb_shift = v_shift + 4, swz_shift = 7 - rb_shift, swz_mask = (1 << v_shift) - 1;
+    int off[8], raw_off[8];        // element offsets of the vector's values in x and in a raw patch, -1 beyond the last
+    uint32_t taps_w[2] = {0, 0};   // their taps along W, four bits each
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int e = v * 8 + j, kw = e / g.fC, c = e - kw * g.fC;
+      off[j] = kw < g.fkW ? kw * g.fx_w + c * g.fx_c : -1;
+      raw_off[j] = kw < g.fkW ? kw * g.raw_w + c * g.raw_c + g.raw_rem : -1;
+      taps_w[j >> 2] |= (uint32_t)(kw & 15) << (8 * (j & 3));
+    }
+    int s = 0;
+    uint32_t ph = 1, it = 0;
+    for (int item = item0; item < g.n_items && alive; item += item_step) {
+      const Tile t = decode<MB, PAIR>(g, item, rank);
+      alive = for_steps(g, t.var, u0, u1, [&](int kd, int, int, int, int) -> bool {
+        if (!mbar_wait_warp(a_empty(s), ph, abort_word, err, ERR_A_EMPTY)) return false;
+        if (g.raw_tma) {
+          const int rs = (int)(it & (RAW_BUFS - 1u));
+          if (!mbar_wait_warp(a_split(rs), (it / RAW_BUFS) & 1u, abort_word, err, ERR_A)) return false;
+          const uint8_t *patch = base_ptr + sl.off_raw + rs * sl.raw_bytes;
+          const uint32_t slab_a = base + (uint32_t)(s * sl.a_bytes);
+          if (v < 2 * g.k_full) {
+            const int step_px = g.sW * g.raw_w;
+#pragma unroll 2
+            for (int i = st >> v_shift; i < g.fold_rows * 8; i += (SPLIT_WARPS * 32) >> v_shift) {
+              const unsigned short *src = reinterpret_cast<const unsigned short *>(patch) + (i >> 3) * g.raw_row + (i & 7) * step_px;
+              uint32_t e[8];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) e[j] = raw_off[j] >= 0 ? src[raw_off[j]] : 0u;
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(slab_a + (uint32_t)((i << rb_shift) + ((v ^ ((i >> swz_shift) & swz_mask)) << 4))),
+                           "r"(e[0] | (e[1] << 16)), "r"(e[2] | (e[3] << 16)), "r"(e[4] | (e[5] << 16)), "r"(e[6] | (e[7] << 16)) : "memory");
+            }
+          }
+          fence_async_smem();
+          __syncwarp();
+          if (lane == 0) { mbar_arrive(a_full(s)); mbar_arrive(raw_empty(rs)); }
+          ++it;
+          if (++s == sl.n_a) { s = 0; ph ^= 1u; }
+          return true;
+        }
+        uint8_t *slab = base_ptr + s * sl.a_bytes;
+        const int id = g.sD * t.od + kd - g.pD, ih0 = g.sH * t.oh0 + g.org_h[0], iw00 = g.sW * t.ow0 + g.org_w[0];
+        const bool plane = (unsigned)id < (unsigned)g.fD && t.n0 < g.N;
+        const unsigned short *xp = reinterpret_cast<const unsigned short *>(x) + t.n0 * g.fx_n + id * g.fx_d;
+        if (v < 2 * g.k_full) {
+#pragma unroll 2
+          for (int i = st >> v_shift; i < g.fold_rows * 8; i += (SPLIT_WARPS * 32) >> v_shift) {
+            const int ih = ih0 + (i >> 3), iw = iw00 + g.sW * (i & 7);
+            uint32_t e[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) e[j] = 0;
+            if (plane && (unsigned)ih < (unsigned)g.fH) {
+              const unsigned short *src = xp + ih * g.fx_h + (long long)iw * g.fx_w;
+              if (iw >= 0 && iw + g.fkW <= g.fW) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                  if (off[j] >= 0) e[j] = __ldg(src + off[j]);
+              } else {
+#pragma unroll
+                for (int j = 0; j < 8; ++j)
+                  if (off[j] >= 0 && (unsigned)(iw + (int)((taps_w[j >> 2] >> (8 * (j & 3))) & 15u)) < (unsigned)g.fW) e[j] = __ldg(src + off[j]);
+              }
+            }
+            *reinterpret_cast<uint4 *>(slab + (i << rb_shift) + ((v ^ ((i >> swz_shift) & swz_mask)) << 4)) =
+                make_uint4(e[0] | (e[1] << 16), e[2] | (e[3] << 16), e[4] | (e[5] << 16), e[6] | (e[7] << 16));
+          }
+        }
+        fence_async_smem();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(a_full(s));
+        if (++s == sl.n_a) { s = 0; ph ^= 1u; }
+        return true;
+      });
     }
   } else if (F32 && warp >= SPLIT_WARP0) {
     // ---------------------------------------------------------------- fp32: slab -> tf32 part in place, remainder beside it
@@ -427,71 +555,74 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
         const int k0 = kb * BN + c0;
         const int oh_b = t.oh0 + mb * g.TH;
         const bool wanted = k0 < g.K && t.valid && oh_b < g.oH;
-        uint32_t r[COLS];
-        if (wanted) {
-          const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * ACC + mb * BN + c0);
-          tmem_ld_x32(ta, r);
-          if (COLS == 64) tmem_ld_x32(ta + 32u, r + 32 % COLS);
-          tmem_wait_ld_x32(r);
-          if (COLS == 64) tmem_wait_ld_x32(r + 32 % COLS);
+        const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * ACC + mb * BN * N_ACC + c0);
+        // 32 columns at a time, in a loop: twice the code for 64 in one piece ran slower (an epilogue warp executes it once per
+        // item, mostly out of cold instruction caches)
+#pragma unroll 1
+        for (int hc = 0; hc < COLS; hc += 32) {
+          uint32_t r[32];
+          if (wanted) {
+            tmem_ld_x32(ta + (uint32_t)hc, r);
+            tmem_wait_ld_x32(r);
 #pragma unroll
-          for (int a = 1; a < N_ACC; ++a)      // the block's other accumulators (1 and 3 are the second thread's)
-            if (g.dual || a == 2) {
-              uint32_t r2[32];
-#pragma unroll
-              for (int hc = 0; hc < COLS; hc += 32) {
+            for (int a = 1; a < N_ACC; ++a)      // the block's other accumulators (1 and 3 are the second thread's)
+              if (g.dual || a == 2) {
+                uint32_t r2[32];
                 tmem_ld_x32(ta + (uint32_t)(a * BN + hc), r2);
                 tmem_wait_ld_x32(r2);
 #pragma unroll
-                for (int i = 0; i < 32; ++i) r[hc + i] = __float_as_uint(__uint_as_float(r[hc + i]) + __uint_as_float(r2[i]));
+                for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(r2[i]));
               }
+          }
+          if (ci + 2 >= N_CH && hc + 32 >= COLS) {      // this warp's last columns are in registers: its share of the hand-back
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) { if (PAIR) mbar_arrive_rank0(acc_empty(buf)); else mbar_arrive(acc_empty(buf)); }
+            handed = true;
+          }
+          if (!wanted) continue;
+          if (has_bias) {
+#pragma unroll
+            for (int v = 0; v < 4; ++v) {
+              float b[8];
+              if (!F32 && g.bias_f32) load_bias<float, 8>(reinterpret_cast<const float *>(bias), k0 + hc + 8 * v, g.K, g.bias_vec, b);
+              else load_bias<T, 8>(bias, k0 + hc + 8 * v, g.K, g.bias_vec, b);
+#pragma unroll
+              for (int i = 0; i < 8; ++i) r[8 * v + i] = __float_as_uint(__uint_as_float(r[8 * v + i]) + b[i]);
             }
-        }
-        if (ci + 2 >= N_CH) {      // this warp's last columns are in registers: its share of the hand-back
-          tc_fence_before();
-          __syncwarp();
-          if (lane == 0) { if (PAIR) mbar_arrive_rank0(acc_empty(buf)); else mbar_arrive(acc_empty(buf)); }
-          handed = true;
+          }
+          constexpr int OW = 32 * (int)sizeof(T) / 4;      // words of output: 16 pairs, or 32 floats
+          uint32_t o[OW];
+#pragma unroll
+          for (int i = 0; i < OW; ++i) {
+            if constexpr (F32) o[i] = r[i];
+            else o[i] = Pair16<T>::round(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+          }
+          if (pool) {
+#pragma unroll
+            for (int i = 0; i < OW; ++i) {
+              o[i] = OutWord<T>::max2(o[i], __shfl_xor_sync(0xffffffffu, o[i], g.TI));
+              o[i] = OutWord<T>::max2(o[i], __shfl_xor_sync(0xffffffffu, o[i], 8 << g.tn_shift));
+            }
+          }
+          if (relu) {
+#pragma unroll
+            for (int i = 0; i < OW; ++i) o[i] = OutWord<T>::max2(o[i], 0u);
+          }
+          if (hc == 0) {
+            if (lane == 0) bulk_wait_read();       // the previous store has read the staging rows
+            __syncwarp();
+          }
+          if (srow >= 0) {
+            const uint32_t dst = stage + (uint32_t)srow * 128u;
+            const int v0 = hc * (int)sizeof(T) / 16;
+#pragma unroll
+            for (int v = 0; v < OW / 4; ++v)
+              asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (uint32_t)(((v0 + v) ^ (srow & 7)) << 4)), "r"(o[4 * v]),
+                           "r"(o[4 * v + 1]), "r"(o[4 * v + 2]), "r"(o[4 * v + 3]) : "memory");
+          }
         }
         if (!wanted) continue;
-        uint32_t o[32];
-#pragma unroll
-        for (int v = 0; v < 8; ++v) {          // one 16-byte vector of output
-          constexpr int V = 16 / (int)sizeof(T);
-          float f[V], b[V];
-#pragma unroll
-          for (int i = 0; i < V; ++i) f[i] = __uint_as_float(r[v * V + i]);
-          if (has_bias) {
-            load_bias16<T>(bias, k0 + v * V, g.K, g.bias_vec, b);
-#pragma unroll
-            for (int i = 0; i < V; ++i) f[i] += b[i];
-          }
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            if constexpr (F32) o[v * 4 + i] = __float_as_uint(f[i]);
-            else o[v * 4 + i] = Pair16<T>::round(f[2 * i], f[2 * i + 1]);
-          }
-        }
-        if (pool) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            o[i] = OutWord<T>::max2(o[i], __shfl_xor_sync(0xffffffffu, o[i], g.TI));
-            o[i] = OutWord<T>::max2(o[i], __shfl_xor_sync(0xffffffffu, o[i], 8 << g.tn_shift));
-          }
-        }
-        if (relu) {
-#pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = OutWord<T>::max2(o[i], 0u);
-        }
-        if (lane == 0) bulk_wait_read();       // the previous store has read the staging rows
-        __syncwarp();
-        if (srow >= 0) {
-          const uint32_t dst = stage + (uint32_t)srow * 128u;
-#pragma unroll
-          for (int v = 0; v < 8; ++v)
-            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst + (uint32_t)((v ^ (srow & 7)) << 4)), "r"(o[4 * v]),
-                         "r"(o[4 * v + 1]), "r"(o[4 * v + 2]), "r"(o[4 * v + 3]) : "memory");
-        }
         // first pixel of this warp's rows
         const int g0 = q * 4, h0 = g0 >> g.tn_shift, n0 = (g0 & tnm) << g.ti_shift;
         if (g.y_tma) {
@@ -617,7 +748,8 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
         if (oh >= g.yH[t.var] || ow >= g.yW[t.var] || n >= g.N || !t.valid) continue;
         if (has_bias) {
 #pragma unroll
-          for (int v = 0; v < V; ++v) best[v] += k + v < g.K ? Elem<T>::load(bias + k + v) : 0.f;
+          for (int v = 0; v < V; ++v)
+            if (k + v < g.K) best[v] += g.bias_f32 ? reinterpret_cast<const float *>(bias)[k + v] : Elem<T>::load(bias + k + v);
         }
         if (relu) {
 #pragma unroll
@@ -646,8 +778,8 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value ? 512 : 384, 1)
 // U[tap][o][i] = w[o, i, tap] in the order the kernel walks the taps, rounded once to T; fp32 as [tap][tf32 part, remainder][o][i].
 // The weights are read through strides, so a data gradient's filter (channels exchanged, taps mirrored) is the same kernel.
 struct FGeomD {
-  int O, I, Ip, kD, n_hw;
-  long long s_o, s_i, s_d, off_d;
+  int O, I, Ip, kD, n_hw, fold;      // fold > 0: input i is tap i / fold along W of channel i % fold
+  long long s_o, s_i, s_d, off_d, s_w;
   int off_hw[MAX_TAPS];       // element offset of each (h, w) tap in walking order
 };
 template <typename TW, typename T>
@@ -656,7 +788,8 @@ __global__ void __launch_bounds__(256) direct_filter_kernel(const TW *__restrict
   const unsigned total = (unsigned)f.O * (unsigned)f.Ip;
   if (idx >= total) return;
   const int o = (int)(idx / (unsigned)f.Ip), i = (int)(idx - (unsigned)o * (unsigned)f.Ip);
-  const TW *src = w + o * f.s_o + i * f.s_i;
+  const int kw = f.fold ? i / f.fold : 0;
+  const TW *src = w + o * f.s_o + (i - kw * f.fold) * f.s_i + kw * f.s_w;
   const bool real = i < f.I;
   const int kd = blockIdx.y;
   for (int t = blockIdx.z; t < f.n_hw; t += gridDim.z) {
@@ -807,8 +940,66 @@ bool direct_grad_desc(DirectDesc *q, int dtype, int N, int C, int K, int Km, con
   return true;
 }
 
+bool direct_fold_desc(DirectDesc *q, const int pad[3], int x_first) {
+  if (q->dtype == WINOCONV_F32 || q->variants || q->transposed || q->Cw * q->kW_w > 64 || q->kW_w > 10) return false;
+  q->fold = 1;
+  q->x_first = x_first;
+  q->n_parts = 1;
+  DirectPart &p = q->parts[0];
+  std::memset(&p, 0, sizeof p);
+  p.th = q->kH_w; p.tw = 1; p.ts_h = 1; p.ts_w = 1;
+  p.org_h = -pad[1]; p.org_w = -pad[2];
+  return true;
+}
+
+// The folded kernel: 64 columns, one or two row blocks (two keep both halves of the epilogue warps busy), the filter resident
+// where one channel block covers K.
+static bool fold_plan(const DirectDesc &d, DirectPlan *out) {
+  DirectPlan p;
+  std::memset(&p, 0, sizeof p);
+  const int fold = d.Cw * d.kW_w, rows = d.parts[0].th;
+  p.k_full = p.k_tail = (fold + 15) / 16;
+  p.ch_el = p.k_full == 1 ? 16 : p.k_full == 2 ? 32 : 64;
+  p.rb = 2 * p.ch_el;
+  p.n_chunks = 1;
+  p.taps[0] = p.max_taps = p.n_taps = rows;
+  p.units = d.kD * rows;
+  p.filter_elems = (long long)d.kD * rows * d.K * p.ch_el;
+  p.BN = 64; p.split = 1; p.TN = 1; p.TH = 16; p.TI = 1; p.PW = 8;
+  p.n_kb = (d.K + 63) / 64;
+  p.n_wb = (d.oW + 7) / 8;
+  for (int mb = 2; mb >= 1; --mb) {
+    DirectPlan q = p;
+    q.MB = mb;
+    q.n_hb = (d.oH + 16 * mb - 1) / (16 * mb);
+    const long long tiles = (long long)q.n_wb * q.n_hb * d.oD * d.N;
+    if (tiles * p.n_kb > 0x3fffffffLL) continue;
+    if (mb == 2 && tiles * p.n_kb < 148) continue;       // not even one item per SM
+    q.n_tiles = (int)tiles; q.n_items = (int)(tiles * p.n_kb);
+    q.slab_rows_h = d.sH * (16 * mb - 1) + rows;
+    q.slab_bytes = q.slab_rows_h * 8 * q.rb;
+    q.a_bytes = q.lo_off = (q.slab_bytes + 1023) / 1024 * 1024;
+    q.b_lo = q.b_tile = 64 * q.rb;
+    // the raw patch (see launch): rows of (8 - 1) * stride + kW pixels of C channels from a multiple of eight elements on
+    const int px = d.sW * 7 + d.kW_w;
+    const bool first = d.x_first != 0;
+    const long long row = first ? d.W : (long long)d.W * d.Cw;
+    q.raw_rem = first ? ((d.parts[0].org_w % 8) + 8) % 8 : ((d.parts[0].org_w * d.Cw) % 8 + 8) % 8;
+    q.raw_el = ((first ? px : px * d.Cw) + q.raw_rem + 7) / 8 * 8;
+    q.raw_tma = row % 8 == 0 && q.raw_el <= 256 && q.slab_rows_h <= 256 && (!first || d.Cw <= 256);
+    q.raw_box = q.raw_tma ? q.slab_rows_h * q.raw_el * 2 * (first ? d.Cw : 1) : 0;
+    const int raws = (int)RAW_BUFS * ((q.raw_box + 127) / 128 * 128);
+    if (!ring_depths(q, rows, 227 * 1024 - FIXED_BYTES - raws)) continue;
+    q.smem = FIXED_BYTES + raws + q.n_a * q.a_bytes + q.n_b * q.b_bytes;
+    *out = q;
+    return true;
+  }
+  return false;
+}
+
 bool direct_plan(const DirectDesc &d, DirectPlan *out) {
   if (d.n_parts == 0) return false;
+  if (d.fold) return fold_plan(d, out);
   const bool f32 = d.dtype == WINOCONV_F32;
   const int esz = f32 ? 4 : 2, vec = 16 / esz;
   if (d.C % vec != 0) return false;
@@ -898,7 +1089,7 @@ bool direct_plan(const DirectDesc &d, DirectPlan *out) {
 cudaError_t launch_direct_filter_transform(const DirectDesc &d, const DirectPlan &p, int w_dtype, const void *w, void *u, cudaStream_t s) {
   FGeomD f;
   std::memset(&f, 0, sizeof f);
-  f.O = d.K; f.I = d.Cw; f.Ip = d.C; f.kD = d.kD; f.n_hw = p.n_taps;
+  f.O = d.K; f.I = d.fold ? d.Cw * d.kW_w : d.Cw; f.Ip = d.fold ? p.ch_el : d.C; f.kD = d.kD; f.n_hw = p.n_taps; f.fold = d.fold ? d.Cw : 0;
   // the weights' own channel counts: [Kw][Cw][taps] or [taps][Cw][Kw]
   const long long Kw = d.transposed ? d.Cw : d.K, Cw = d.transposed ? d.K : d.Cw;
   const bool kcrs = d.weight_layout == WINOCONV_W_KCRS;
@@ -906,6 +1097,7 @@ cudaError_t launch_direct_filter_transform(const DirectDesc &d, const DirectPlan
   const long long s_k = kcrs ? Cw * d.kD_w * hw : 1, s_c = kcrs ? d.kD_w * hw : Kw;
   f.s_o = d.transposed ? s_c : s_k;
   f.s_i = d.transposed ? s_k : s_c;
+  f.s_w = tap_stride;
   f.off_d = d.d0 * hw * tap_stride;
   f.s_d = d.ds * hw * tap_stride;
   for (int q = 0; q < d.n_parts; ++q) {
@@ -916,7 +1108,7 @@ cudaError_t launch_direct_filter_transform(const DirectDesc &d, const DirectPlan
     }
   }
   const unsigned blocks = (unsigned)(((long long)f.O * f.Ip + 255) / 256);
-  const dim3 grid(blocks, d.kD, blocks >= 296 ? 1 : std::min(p.n_taps, (int)(592 / blocks) + 1));
+  const dim3 grid(blocks, (unsigned)d.kD, blocks >= 296 ? 1 : std::min(p.n_taps, (int)(592 / blocks) + 1));
 #define WINO_FILT(TW, T) direct_filter_kernel<TW, T><<<grid, 256, 0, s>>>((const TW *)w, (T *)u, f)
   if (d.dtype == WINOCONV_F32) WINO_FILT(float, float);
   else if (d.dtype == WINOCONV_F16) { if (w_dtype == WINOCONV_F32) WINO_FILT(float, __half); else WINO_FILT(__half, __half); }
@@ -925,17 +1117,17 @@ cudaError_t launch_direct_filter_transform(const DirectDesc &d, const DirectPlan
   return cudaGetLastError();
 }
 
-template <typename T, int BN, int MB, bool PAIR>
-static cudaError_t launch_one(const DirectPlan &p, const CUtensorMap &mx, const CUtensorMap &mu, const MapSet &my, void *y,
+template <typename T, int BN, int MB, bool PAIR, bool FOLD = false>
+static cudaError_t launch_one(const DirectPlan &p, const CUtensorMap &mx, const CUtensorMap &mu, const MapSet &my, const void *x, void *y,
                               const void *bias, const DGeom &g, const DSmem &sl, uint32_t idesc, int sms, cudaStream_t s) {
-  auto kern = direct_kernel<T, BN, MB, PAIR>;
+  auto kern = direct_kernel<T, BN, MB, PAIR, FOLD>;
   static std::mutex mu_;
   static std::map<int, int> pairs_of;     // device -> resident CTA pairs (0: attribute set, not asked)
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(std::is_same<T, float>::value ? 512 : 384, 1, 1);
+  cfg.blockDim = dim3(std::is_same<T, float>::value || FOLD ? 512 : 384, 1, 1);
   cfg.dynamicSmemBytes = (size_t)p.smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[2];
@@ -967,7 +1159,7 @@ static cudaError_t launch_one(const DirectPlan &p, const CUtensorMap &mx, const 
   if (p.split > 1) cfg.gridDim = dim3((unsigned)(g.n_items * p.split) * (PAIR ? 2u : 1u), 1, 1);
   else if (PAIR) cfg.gridDim = dim3((unsigned)(2 * std::min(g.n_items, std::min(pairs, sms / 2))), 1, 1);
   else cfg.gridDim = dim3((unsigned)std::min(g.n_items, sms), 1, 1);
-  return cudaLaunchKernelEx(&cfg, kern, mx, mu, my, (T *)y, (const T *)bias, g, sl, idesc);
+  return cudaLaunchKernelEx(&cfg, kern, mx, mu, my, (const T *)x, (T *)y, (const T *)bias, g, sl, idesc);
 }
 
 cudaError_t launch_direct_forward(const DirectDesc &d, const DirectPlan &p, const void *x, const void *u, const void *bias, void *y,
@@ -982,6 +1174,7 @@ cudaError_t launch_direct_forward(const DirectDesc &d, const DirectPlan &p, cons
   const uint32_t swz_code = p.rb == 128 ? 2u : p.rb == 64 ? 4u : 6u;
   CUtensorMap mx, mu;
   MapSet my;
+  std::memset(&mx, 0, sizeof mx);
   // order of the dimensions (see tile_load): dims / strides / box / element strides of channel, W, image, H, depth
   const int mode = p.TI == 1 ? 0 : p.TN == 1 ? 1 : 2;
   auto tile_map = [&](CUtensorMap *m, const void *ptr, cuuint64_t C_, cuuint64_t W_, cuuint64_t H_, cuuint64_t D_, cuuint64_t sw_, cuuint64_t sh_,
@@ -1008,13 +1201,14 @@ cudaError_t launch_direct_forward(const DirectDesc &d, const DirectPlan &p, cons
                CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
   };
   const cuuint64_t xw = (cuuint64_t)d.C * esz, xh = xw * d.W, xd = xh * d.H, xn = xd * d.D;
-  if (!tile_map(&mx, x, d.C, d.W, d.H, d.D, xw, xh, xd, xn, p.ch_el, p.PW * d.sW, p.TN, p.slab_rows_h * d.sH, d.sW, d.sH, swz)) {
+  if (!d.fold && !tile_map(&mx, x, d.C, d.W, d.H, d.D, xw, xh, xd, xn, p.ch_el, p.PW * d.sW, p.TN, p.slab_rows_h * d.sH, d.sW, d.sH, swz)) {
     *detail = "cuTensorMapEncodeTiled failed for the input";
     return cudaErrorInvalidValue;
   }
   {   // filter tiles [tap][K][C] (fp32: two per tap)
-    const cuuint64_t dims[3] = {(cuuint64_t)d.C, (cuuint64_t)d.K, (cuuint64_t)d.kD * p.n_taps * (f32 ? 2 : 1)};
-    const cuuint64_t st[2] = {(cuuint64_t)d.C * esz, (cuuint64_t)d.C * esz * d.K};
+    const cuuint64_t row = d.fold ? (cuuint64_t)p.ch_el : (cuuint64_t)d.C;
+    const cuuint64_t dims[3] = {row, (cuuint64_t)d.K, (cuuint64_t)d.kD * p.n_taps * (f32 ? 2 : 1)};
+    const cuuint64_t st[2] = {row * esz, row * esz * d.K};
     const cuuint32_t box[3] = {(cuuint32_t)p.ch_el, (cuuint32_t)(p.pair ? p.BN / 2 : p.BN), 1u};
     const cuuint32_t es[3] = {1u, 1u, 1u};
     if (enc(&mu, dt, 3, const_cast<void *>(u), dims, st, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, swz, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
@@ -1055,6 +1249,33 @@ cudaError_t launch_direct_forward(const DirectDesc &d, const DirectPlan &p, cons
       g.tap_off[p.tap0[q] + t] = (uint16_t)((th * p.TN * p.PW + tw) * p.TI * (p.rb / 16));
     }
   }
+  if (d.fold) {
+    const long long C = d.Cw, plane = (long long)d.H * d.W;
+    g.raw_tma = p.raw_tma; g.raw_rem = p.raw_rem; g.raw_row = p.raw_el;
+    g.raw_w = d.x_first ? 1 : d.Cw; g.raw_c = d.x_first ? p.slab_rows_h * p.raw_el : 1;
+    if (p.raw_tma) {
+      cuuint64_t dims[5], st[4];
+      cuuint32_t box[5] = {(cuuint32_t)p.raw_el, (cuuint32_t)p.slab_rows_h, 1u, 1u, 1u};
+      const cuuint32_t es[5] = {1u, 1u, 1u, 1u, 1u};
+      const cuuint64_t row = d.x_first ? (cuuint64_t)d.W : (cuuint64_t)d.W * d.Cw;
+      dims[0] = row; dims[1] = (cuuint64_t)d.H; dims[2] = (cuuint64_t)d.D;
+      st[0] = row * 2; st[1] = st[0] * d.H; st[2] = st[1] * d.D;
+      if (d.x_first) {
+        dims[3] = (cuuint64_t)d.Cw; dims[4] = (cuuint64_t)d.N; st[3] = st[2] * d.Cw;
+        box[3] = (cuuint32_t)d.Cw;
+      } else {
+        dims[3] = (cuuint64_t)d.N; dims[4] = 1; st[3] = st[2] * d.N;
+      }
+      if (enc(&mx, dt, 5, const_cast<void *>(x), dims, st, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS) {
+        *detail = "cuTensorMapEncodeTiled failed for the few-channel input";
+        return cudaErrorInvalidValue;
+      }
+    }
+    if (d.x_first) { g.fx_c = (int)(plane * d.D); g.fx_w = 1; g.fx_h = d.W; g.fx_d = plane; g.fx_n = C * plane * d.D; }
+    else { g.fx_c = 1; g.fx_w = (int)C; g.fx_h = C * d.W; g.fx_d = C * plane; g.fx_n = C * plane * d.D; }
+    g.fD = d.D; g.fH = d.H; g.fW = d.W; g.fC = d.Cw; g.fkW = d.kW_w; g.fold_rows = p.slab_rows_h;
+  }
   g.n_chunks = p.n_chunks; g.ch_el = p.ch_el; g.k_full = p.k_full; g.k_tail = p.k_tail; g.units = p.units;
   {   // MMAs of the smallest share of an item
     const int per_unit = p.n_chunks > 1 ? 1 : p.k_tail;
@@ -1064,23 +1285,29 @@ cudaError_t launch_direct_forward(const DirectDesc &d, const DirectPlan &p, cons
     g.dual = least >= 2;
   }
   g.G = p.G; g.split = p.split; g.epilogue = d.epilogue;
-  g.y_tma = y_tma; g.bias_vec = y_tma && (reinterpret_cast<uintptr_t>(bias) & 15u) == 0;
-  g.a_hi = desc_hi((uint32_t)(p.PW * p.TI * p.rb), swz_code);
+  g.y_tma = y_tma; g.bias_f32 = d.bias_f32; g.bias_vec = y_tma && (reinterpret_cast<uintptr_t>(bias) & 15u) == 0;
+  const int row_step = d.fold ? d.sH : 1;      // slab rows between neighbouring output rows
+  g.a_hi = desc_hi((uint32_t)(row_step * p.PW * p.TI * p.rb), swz_code);
   g.b_hi = desc_hi((uint32_t)(8 * p.rb), swz_code);
-  g.mb_off16 = p.TH * p.TN * p.PW * p.TI * p.rb / 16;
+  g.mb_off16 = row_step * p.TH * p.TN * p.PW * p.TI * p.rb / 16;
   DSmem sl;
   sl.slab_bytes = p.slab_bytes; sl.a_bytes = p.a_bytes; sl.lo_off = p.lo_off;
   sl.b_tile = p.b_tile; sl.b_lo = p.b_lo; sl.b_bytes = p.b_bytes; sl.n_a = p.n_a; sl.n_b = p.n_b;
   sl.off_b = p.n_a * p.a_bytes; sl.off_stage = sl.off_b + p.n_b * p.b_bytes;
-  sl.off_bars = sl.off_stage + EPI_WARPS * STAGE_BYTES; sl.total = p.smem;
+  sl.off_raw = sl.off_stage + EPI_WARPS * STAGE_BYTES;
+  sl.raw_bytes = (p.raw_box + 127) / 128 * 128;
+  if (d.fold) sl.slab_bytes = p.raw_box;       // what TMA delivers
+  sl.off_bars = sl.off_raw + (int)RAW_BUFS * sl.raw_bytes; sl.total = p.smem;
   const int sms = sm_count_of_current_device();
   if (sms <= 0) { *detail = "no device"; return cudaErrorNoDevice; }
   const uint32_t fmt = f32 ? 2u : d.dtype == WINOCONV_F16 ? 0u : 1u;
   const uint32_t m_rows = p.pair ? 2u * BM : (uint32_t)BM;
   const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.BN >> 3) << 17) | ((m_rows >> 4) << 24);
-#define WINO_GO(T, BN_, MB_, P_) return launch_one<T, BN_, MB_, P_>(p, mx, mu, my, y, bias, g, sl, idesc, sms, s)
+#define WINO_GO(T, BN_, MB_, P_) return launch_one<T, BN_, MB_, P_>(p, mx, mu, my, x, y, bias, g, sl, idesc, sms, s)
+#define WINO_FOLD(T, MB_) return launch_one<T, 64, MB_, false, true>(p, mx, mu, my, x, y, bias, g, sl, idesc, sms, s)
 #define WINO_PICK(T)                                                             \
   do {                                                                           \
+    if (d.fold) { if (p.MB == 2) WINO_FOLD(T, 2); WINO_FOLD(T, 1); }             \
     if (p.pair) {                                                                \
       if (p.BN == 256) WINO_GO(T, 256, 1, true);                                 \
       if (p.BN == 128) { if (p.MB == 2) WINO_GO(T, 128, 2, true); WINO_GO(T, 128, 1, true); } \
@@ -1094,6 +1321,7 @@ cudaError_t launch_direct_forward(const DirectDesc &d, const DirectPlan &p, cons
   if (d.dtype == WINOCONV_BF16) WINO_PICK(__nv_bfloat16);
   WINO_GO(float, 64, 1, false);
 #undef WINO_PICK
+#undef WINO_FOLD
 #undef WINO_GO
 }
 

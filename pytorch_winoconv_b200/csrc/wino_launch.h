@@ -49,6 +49,9 @@ cudaError_t launch_fused_forward(const FGeom &g, int dtype, const void *x, const
                                  cudaStream_t s, const char **detail);
 cudaError_t read_and_clear_fused_error(cudaStream_t s, unsigned int *code);
 
+// x [pixels][C] -> xp [pixels][Cp], zeros from C on
+cudaError_t launch_pad_channels(int dtype, const void *x, void *xp, long long pixels, int C, int Cp, cudaStream_t s);
+
 // Row-piece DWM kernel (f16 / bf16, stride 1): 1 x 3 pieces, F(2,3) along W, taps along H / depth summed in TMEM.
 struct RowDesc {
   int N, C, K, D, H, W, oD, oH, oW, yH, yW;
@@ -98,6 +101,9 @@ struct DirectDesc {
   DirectPart parts[4];
   long long ys_n, ys_d, ys_h, ys_w;  // element strides of the output
   unsigned epilogue;
+  int bias_f32;                      // the bias is fp32 whatever dtype is
+  int fold;                          // few channels: the taps along W are folded into the channels and x is gathered by the kernel
+  int x_first;                       // (fold only) x is [N, C, D, H, W]
   int weight_layout, transposed;     // transposed: K and C exchanged in the weights (data gradient)
 };
 // A forward layer; and the part of a layer's data gradient with input depths of parity e (e < stride along depth).
@@ -112,10 +118,12 @@ struct DirectPlan {
   int taps[4], tap0[4], max_taps, n_taps, units;
   int n_wb, n_hb, n_tiles, n_kb, n_items;   // n_items: of one variant
   int slab_bytes, a_bytes, lo_off, b_tile, b_lo, b_bytes, G, n_a, n_b, smem;
+  int raw_tma, raw_rem, raw_el, raw_box;   // fold: the raw patch loaded by TMA, elements before its first pixel, of a row, bytes
   long long filter_elems;
   double estimate;                   // clocks
 };
 bool direct_plan(const DirectDesc &d, DirectPlan *out);
+bool direct_fold_desc(DirectDesc *q, const int pad[3], int x_first);   // turns a forward description into a folded one where it applies
 cudaError_t launch_direct_filter_transform(const DirectDesc &d, const DirectPlan &p, int w_dtype, const void *w, void *u, cudaStream_t s);
 cudaError_t launch_direct_forward(const DirectDesc &d, const DirectPlan &p, const void *x, const void *u, const void *bias, void *y,
                                   cudaStream_t s, const char **detail);

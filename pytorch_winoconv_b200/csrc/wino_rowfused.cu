@@ -886,19 +886,20 @@ __global__ void __launch_bounds__(256) rowfused_filter_kernel(const T *__restric
   for (int j = 0; j < 4; ++j) Elem<T>::store(u + ((slab0 + j) * K + k) * Cp + c, o[j]);
 }
 
-// zero-pads the channel dimension to a multiple of 8 so the input can be addressed by TMA; one thread writes one
-// 16-byte group of eight channels
+// zero-pads the channel dimension to a multiple of 16 bytes so the input can be addressed by TMA; one thread writes one
+// 16-byte group of channels
 template <typename T>
 __global__ void __launch_bounds__(256) pad_channels_kernel(const T *__restrict__ x, T *__restrict__ xp, long long pixels,
                                                            int C, int Cp) {
-  const int groups = Cp / 8;
+  constexpr int V = 16 / (int)sizeof(T);
+  const int groups = Cp / V;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= pixels * groups) return;
   const long long px = idx / groups;
-  const int c0 = (int)(idx - px * groups) * 8;
-  __align__(16) T v[8];
+  const int c0 = (int)(idx - px * groups) * V;
+  __align__(16) T v[V];
 #pragma unroll
-  for (int i = 0; i < 8; ++i) v[i] = (c0 + i < C) ? x[px * C + c0 + i] : T(0.f);
+  for (int i = 0; i < V; ++i) v[i] = (c0 + i < C) ? x[px * C + c0 + i] : T(0.f);
   *reinterpret_cast<uint4 *>(xp + px * Cp + c0) = *reinterpret_cast<const uint4 *>(v);
 }
 
@@ -1118,6 +1119,18 @@ bool rowfused_plan(const RowDesc &d, RowPlan *out) {
   return true;
 }
 
+template <typename T>
+static cudaError_t pad_channels_t(const void *x, void *xp, long long pixels, int C, int Cp, cudaStream_t s) {
+  const long long n = pixels * (Cp / (16 / (int)sizeof(T)));
+  rowf::pad_channels_kernel<T><<<(unsigned)((n + 255) / 256), 256, 0, s>>>((const T *)x, (T *)xp, pixels, C, Cp);
+  return cudaGetLastError();
+}
+cudaError_t launch_pad_channels(int dtype, const void *x, void *xp, long long pixels, int C, int Cp, cudaStream_t s) {
+  if (dtype == WINOCONV_F32) return pad_channels_t<float>(x, xp, pixels, C, Cp, s);
+  if (dtype == WINOCONV_F16) return pad_channels_t<__half>(x, xp, pixels, C, Cp, s);
+  return pad_channels_t<__nv_bfloat16>(x, xp, pixels, C, Cp, s);
+}
+
 cudaError_t launch_rowfused_filter_transform(const RowDesc &d, const RowPlan &p, int dtype, const void *w, void *u, cudaStream_t s) {
   const long long n = (long long)d.kD * d.kH * p.PW * p.Cp * d.K;
   const unsigned blocks = (unsigned)((n + 255) / 256);
@@ -1229,13 +1242,7 @@ cudaError_t launch_rowfused_forward(const RowDesc &d, const RowPlan &p, int dtyp
     xin = pad_ws;
   } else if (p.Cp != d.C && !p.raw_c && !p.s2_chunks) {   // channels not a multiple of 8: TMA needs 16-byte pixel strides, so pad into scratch first
     if (!pad_ws) { *detail = "channel padding scratch missing"; return cudaErrorInvalidValue; }
-    const long long pixels = (long long)d.N * d.D * d.H * d.W;
-    const unsigned blocks = (unsigned)((pixels * (p.Cp / 8) + 255) / 256);
-    if (dtype == WINOCONV_F16)
-      pad_channels_kernel<__half><<<blocks, 256, 0, s>>>((const __half *)x, (__half *)pad_ws, pixels, d.C, p.Cp);
-    else
-      pad_channels_kernel<__nv_bfloat16><<<blocks, 256, 0, s>>>((const __nv_bfloat16 *)x, (__nv_bfloat16 *)pad_ws, pixels, d.C, p.Cp);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_pad_channels(dtype, x, pad_ws, (long long)d.N * d.D * d.H * d.W, d.C, p.Cp, s);
     if (e != cudaSuccess) { *detail = "channel padding launch failed"; return e; }
     xin = pad_ws;
   }

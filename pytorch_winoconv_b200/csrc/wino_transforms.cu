@@ -587,9 +587,8 @@ __global__ void __launch_bounds__(256) add_kernel(const float *__restrict__ a, c
 // layout: [N, C, P] <-> [N, P, C] with a change of element type on the way (P: pixels of an image)
 // ------------------------------------------------------------------------------------------
 // Both directions are one read and one write of the tensor; a 64 x 64 tile is turned in shared memory so that either side moves
-// runs of 64 elements, two per lane where the run's alignment allows.  With fewer than 16 channels a thread takes a pixel: its
-// reads are coalesced per channel and a warp's writes are one run anyway (RGB at 224 x 224, N = 32: 4 us where torch's
-// strided copy takes 11).
+// runs of 64 elements, two per lane where the run's alignment allows.  With up to 16 channels a block takes 256 pixels, whose
+// values are one run of the output.
 constexpr int LT = 64;
 
 // y[n][p][0 .. Cs) = x[n][c][p], zeros from C on
@@ -632,16 +631,19 @@ __global__ void __launch_bounds__(256) to_channels_last_kernel(const TI *__restr
 }
 template <typename TI, typename TO>
 __global__ void __launch_bounds__(256) to_channels_last_few_kernel(const TI *__restrict__ x, TO *__restrict__ y, int C, int P, int Cs) {
-  const int p = blockIdx.x * 256 + threadIdx.x;
-  if (p >= P) return;
-  const TI *src = x + (long long)blockIdx.z * C * P + p;
-  TO *dst = y + ((long long)blockIdx.z * P + p) * Cs;
-  float v[16];
-#pragma unroll
-  for (int c = 0; c < 16; ++c) v[c] = c < C ? Elem<TI>::load(src + (long long)c * P) : 0.f;
-#pragma unroll
-  for (int c = 0; c < 16; ++c)
-    if (c < Cs) Elem<TO>::store(dst + c, v[c]);
+  __shared__ __align__(16) TO sm[256 * 16];
+  const int p0 = blockIdx.x * 256, tid = threadIdx.x, n_p = min(256, P - p0);
+  const TI *src = x + (long long)blockIdx.z * C * P + p0 + tid;
+  for (int c = 0; c < Cs; ++c) Elem<TO>::store(&sm[tid * Cs + c], tid < n_p && c < C ? Elem<TI>::load(src + (long long)c * P) : 0.f);
+  __syncthreads();
+  TO *dst = y + ((long long)blockIdx.z * P + p0) * Cs;
+  const int run = n_p * Cs;
+  constexpr int V = 16 / (int)sizeof(TO);
+  if ((reinterpret_cast<uintptr_t>(dst) & 15u) == 0 && run % V == 0) {
+    for (int i = tid; i < run / V; i += 256) reinterpret_cast<uint4 *>(dst)[i] = reinterpret_cast<const uint4 *>(sm)[i];
+  } else {
+    for (int i = tid; i < run; i += 256) dst[i] = sm[i];
+  }
 }
 
 // y[n][c][p] = x[n][p][c] (+ bias[c])

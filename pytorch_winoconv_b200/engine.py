@@ -140,7 +140,7 @@ class WinoConv:
 
     def _scratch(self):
         """V / M scratch for the staged algorithm; the fused kernel needs none."""
-        if self.info.algo == capi.ALGO_FUSED or (self.info.algo == capi.ALGO_ROW and self.info.input_ws_bytes == 0):
+        if self.info.direct == 1 or self.info.algo == capi.ALGO_FUSED or (self.info.algo == capi.ALGO_ROW and self.info.input_ws_bytes == 0):
             return _NO_SCRATCH, _NO_SCRATCH
         if self.info.algo == capi.ALGO_ROW:          # channel-padding buffer only
             v, _ = self.pool.get(self.device, int(self.info.input_ws_bytes), 16)
@@ -161,6 +161,8 @@ class WinoConv:
     @property
     def launches_per_call(self) -> int:
         """Kernels this forward launches: three per pass over a block of tiles."""
+        if self.info.direct:
+            return int(self.info.direct)
         if self.info.algo == capi.ALGO_FUSED:
             return 1
         if self.info.algo == capi.ALGO_ROW:
