@@ -77,7 +77,7 @@ class _WinoConvMixin:
     def __call__(self, *args, **kwargs):
         """``torch.nn.Module.__call__`` without its 5 us of dispatch where there is no hook, tracer or compiled call to serve."""
         d = self.__dict__
-        if (kwargs or len(args) != 1 or d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"]
+        if (kwargs or len(args) != 1 or type(args[0]) is not torch.Tensor or d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"]
                 or _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks or _nn_module._global_backward_hooks
                 or _nn_module._global_backward_pre_hooks or self._compiled_call_impl is not None or torch._C._get_tracing_state()):
             return super().__call__(*args, **kwargs)

@@ -27,12 +27,14 @@ void *stream_of() { return (void *)at::cuda::getCurrentCUDAStream().stream(); }
 
 ConvRunner::Stamp stamp_of(const at::Tensor &w, const std::optional<at::Tensor> &b) {
   ConvRunner::Stamp s;
+  s.w_ref = ConvRunner::Stamp::Ref(w.getIntrusivePtr());
   s.w = w.data_ptr();
-  s.w_version = w.is_inference() ? 0 : (int64_t)w._version();
+  s.w_version = (int64_t)w._version();
   s.w_dtype = (int)w.scalar_type();
   if (b) {
+    s.b_ref = ConvRunner::Stamp::Ref(b->getIntrusivePtr());
     s.b = b->data_ptr();
-    s.b_version = b->is_inference() ? 0 : (int64_t)b->_version();
+    s.b_version = (int64_t)b->_version();
   }
   return s;
 }
@@ -68,6 +70,9 @@ at::Tensor turned_channels_last(const at::Tensor &t, at::ScalarType type, void *
   else check_abi(st, "winoconv_to_channels_last");
   return out;
 }
+
+// The tensor itself where it starts on 16 bytes, as TMA and the C ABI want it; else a copy in the same order.
+at::Tensor aligned(const at::Tensor &t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) ? t.clone() : t; }
 
 // The last dimension of a channels-last buffer zero-extended to `c` channels; the tensor itself where it has them.
 at::Tensor pad_channels(const at::Tensor &t, int64_t c) {
@@ -217,13 +222,15 @@ std::optional<at::Tensor> ConvRunner::forward(const at::Tensor &x, const at::Ten
   if (!x.is_cuda() || x.dim() != nd_ + 2 || weight.dim() != nd_ + 2 || !weight.is_cuda() || weight.get_device() != x.get_device() ||
       x.size(1) != weight.size(1) || x.numel() == 0 || (bias && !bias->is_cuda()) || code_of(weight.scalar_type()) < 0)
     return std::nullopt;
+  if (weight.is_inference() || (bias && bias->is_inference())) return std::nullopt;      // no version to tell a new value by
   const int dtype = compute_ >= 0 ? compute_ : code_of(x.scalar_type());
   if (dtype < 0) return std::nullopt;
   const bool grad = at::GradMode::is_enabled() && (x.requires_grad() || (weight.requires_grad() && training));
   if (grad && (pool_ || dtype == WINOCONV_F32)) return std::nullopt;
   c10::cuda::CUDAGuard guard(x.device());
   std::shared_ptr<Entry> e;
-  if (!grad && dtype != WINOCONV_F32 && tile_m_ == 0 && algo_ == WINOCONV_ALGO_AUTO && x.scalar_type() == type_of(dtype) && x.is_contiguous() && x.size(1) * weight.size(-1) <= 64 && x.size(1) > 1 && !lies_channels_last(x)) {
+  if (!grad && dtype != WINOCONV_F32 && tile_m_ == 0 && algo_ == WINOCONV_ALGO_AUTO && x.scalar_type() == type_of(dtype) && x.is_contiguous() &&
+      x.size(1) * weight.size(-1) <= 64 && x.size(1) > 1 && !lies_channels_last(x) && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15u) == 0) {
     // few channels in torch's contiguous order: the kernel gathers them as they lie
     e = entry_for(x, weight, bias, dtype, true);
     if (e) {
@@ -240,6 +247,7 @@ std::optional<at::Tensor> ConvRunner::forward(const at::Tensor &x, const at::Ten
   if (!e->back_known) {
     winoconv_backward_info_t info;
     e->back_ok = winoconv_backward_plan(&e->desc, &info) == WINOCONV_OK && info.data_ok && info.weight_ok;
+    for (int i = 0; i < 3; ++i) e->back_ok = e->back_ok && pad_[i] < e->desc.ker_size[i];      // the Python path refuses the data gradient
     e->back_known = true;
   }
   if (!e->back_ok) return std::nullopt;
@@ -263,7 +271,7 @@ std::vector<at::Tensor> ConvRunner::backward(const at::Tensor &gy_in, const at::
   void *s = stream_of();
   at::Tensor gy = gy_in;
   if (y.defined()) gy = gy * (y > 0).to(gy.scalar_type());
-  gy = channels_last(gy, type);
+  gy = aligned(channels_last(gy, type));
   winoconv_desc_t d = e->desc;
   d.epilogue = need_b ? WINOCONV_EPI_BIAS : 0u;
   winoconv_backward_info_t info;
@@ -291,7 +299,7 @@ std::vector<at::Tensor> ConvRunner::backward(const at::Tensor &gy_in, const at::
     if (x_in.scalar_type() != type) gx = gx.to(x_in.scalar_type());
   }
   if (need_w) {
-    const at::Tensor xp = pad_channels(channels_last(x_in, type), info.c_stride);
+    const at::Tensor xp = aligned(pad_channels(channels_last(x_in, type), info.c_stride));
     gw = at::empty(weight.sizes(), weight.options().requires_grad(false));
     if (need_b) gb = at::empty({weight.size(0)}, weight.options().dtype(at::kFloat).requires_grad(false));
     const at::Tensor ws = empty_bytes(info.weight_ws_bytes, w);
@@ -361,6 +369,7 @@ std::optional<at::Tensor> conv_call(const at::Tensor &x_in, const at::Tensor &we
   at::Tensor x = lies_channels_last(x_in) && x_in.scalar_type() == type ? x_in
                  : x_in.is_contiguous() && x_in.size(0) <= 65535 ? turned_channels_last(x_in, type, s)
                  : x_in.to(x_in.options().dtype(type), false, false, nd == 2 ? at::MemoryFormat::ChannelsLast : at::MemoryFormat::ChannelsLast3d);
+  x = aligned(x);
   at::Tensor w = weight_in.to(x.device()).contiguous();
   at::Tensor u = empty_bytes(info.filter_bytes, x);
   if (winoconv_filter_transform_from(&d, w.data_ptr(), code_of(w.scalar_type()), u.data_ptr(), s) != WINOCONV_OK) {

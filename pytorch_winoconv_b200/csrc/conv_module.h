@@ -34,12 +34,16 @@ class ConvRunner : public torch::CustomClassHolder {
   // whose filter belongs to the newest weights, least recently used first
   std::vector<std::tuple<std::vector<int64_t>, int64_t, int64_t, at::Tensor, int64_t, std::string>> entries();
 
-  struct Stamp {        // what a transformed filter was made from
+  // What a transformed filter was made from.  The weak references keep the tensors' headers (not their memory) from being
+  // reused, so that a new tensor at an old one's address is another one: a parametrised module computes its weight per call.
+  struct Stamp {
+    using Ref = c10::weak_intrusive_ptr<c10::TensorImpl, c10::UndefinedTensorImpl>;
+    Ref w_ref{c10::intrusive_ptr<c10::TensorImpl, c10::UndefinedTensorImpl>()}, b_ref{c10::intrusive_ptr<c10::TensorImpl, c10::UndefinedTensorImpl>()};
     const void *w = nullptr, *b = nullptr;
     int64_t w_version = -1, b_version = -1;
     int w_dtype = -1;
     bool operator==(const Stamp &o) const {
-      return w == o.w && b == o.b && w_version == o.w_version && b_version == o.b_version && w_dtype == o.w_dtype;
+      return w_ref == o.w_ref && b_ref == o.b_ref && w == o.w && b == o.b && w_version == o.w_version && b_version == o.b_version && w_dtype == o.w_dtype;
     }
   };
   struct Entry {

@@ -263,12 +263,11 @@ int build_plan(const winoconv_desc_t *d, Plan *plan) {
   // F(4x4,3x3) outweighs the traffic of V and M: multiplies grow with C * K (K in whole 64-column blocks), V and M with C + K
   // (measured, us direct / staged: 16 -> 16 at 112 x 112, N = 4: 12 / 22; 488 -> 24 at 63 x 95, N = 2: 83 / 53).
   plan->direct = false;
-  static const int direct_env = [] { const char *v = getenv("WINOCONV_DIRECT"); return v && *v ? atoi(v) : 1; }();
   const bool direct_ok = d->algo == WINOCONV_ALGO_AUTO && d->gemm_engine == WINOCONV_GEMM_AUTO && pdt == WINOCONV_F32;
-  const bool f32_f43_wins = d->dtype == WINOCONV_F32 && f43_ok && direct_env != 2 &&
+  const bool f32_f43_wins = d->dtype == WINOCONV_F32 && f43_ok &&
                             (long long)g.C * ((g.K + 63) / 64 * 64) > 32LL * (g.C + g.K);
   if (d->tile_m == 1 && !direct_ok) return fail(WINOCONV_ERR_UNSUPPORTED, "tile_m = 1 (direct taps) goes with algo, engine and product dtype left to the planner");
-  if (direct_ok && (d->tile_m == 1 || (d->tile_m == 0 && direct_env != 0 && (d->dtype == WINOCONV_F32 ? !f32_f43_wins : plan->row)))) {
+  if (direct_ok && (d->tile_m == 1 || (d->tile_m == 0 && (d->dtype == WINOCONV_F32 ? !f32_f43_wins : plan->row)))) {
     DirectDesc &q = plan->dd;
     direct_forward_desc(&q, d->dtype, g.N, g.C, g.K, in, ks, st, pd, out, g.yH, g.yW, g.epilogue, g.weight_layout);
     // few channels: folded, x gathered as it lies; otherwise channels that TMA cannot address go through a padded copy
@@ -283,6 +282,13 @@ int build_plan(const winoconv_desc_t *d, Plan *plan) {
     else if (!d->x_channels_first) {
       q.C = (g.C + vec - 1) / vec * vec;
       plan->direct = direct_plan(q, &plan->dp);
+      // winoconv_forward_static pads into the built-in array, image by image: a layer that ran there without such a copy, or in
+      // blocks of tiles, keeps its algorithm where the copy would not fit
+      if (q.C != q.Cw && d->tile_m == 0) {
+        const unsigned long long image = (unsigned long long)q.D * q.H * q.W * q.C * (16 / vec);
+        const bool row_copies = plan->row && (plan->rd.phases > 1 || plan->rp.Cp != g.C) && !plan->rp.raw_c && !plan->rp.s2_chunks;
+        if (!row_copies && image * (plan->row ? (unsigned long long)g.N : 1ull) > WINOCONV_STATIC_SCRATCH_BYTES) plan->direct = false;
+      }
     }
     if (d->tile_m == 1 && !plan->direct)
       return fail(WINOCONV_ERR_UNSUPPORTED, "tile_m = 1 (direct taps) needs a slab that fits shared memory");
@@ -712,6 +718,33 @@ int winoconv_forward_static(const winoconv_desc_t *desc, const void *x, const vo
     unsigned char *pad = nullptr;
     if ((st = static_scratch_of_current_device(&pad)) != WINOCONV_OK) return st;
     return forward_impl(desc, x, u, bias, y, pad, WINOCONV_STATIC_SCRATCH_BYTES, nullptr, 0, stream, nullptr, nullptr);
+  }
+  if (I.direct == 2) {   // as many images at a time as the array holds with their channels padded
+    if (!x || !u || !y) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "null tensor pointer");
+    if ((desc->epilogue & WINOCONV_EPI_BIAS) && !bias) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "EPI_BIAS set but bias is null");
+    if (!aligned16(x) || !aligned16(u) || !aligned16(y)) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "tensors must be 16-byte aligned");
+    const DirectDesc q = plan.dd;        // (a plan of another batch may take this one's place)
+    const int dtype = plan.dtype;
+    const size_t esz = dtype == WINOCONV_F32 ? 4 : 2;
+    const long long pixels = (long long)q.D * q.H * q.W;
+    const long long fit = WINOCONV_STATIC_SCRATCH_BYTES / (long long)(pixels * q.C * esz);
+    if (fit < 1)
+      return fail(WINOCONV_ERR_WORKSPACE, "the channel-padded copy of one image needs " + std::to_string(pixels * q.C * esz) +
+                                              " bytes; the built-in array holds " + std::to_string(WINOCONV_STATIC_SCRATCH_BYTES));
+    unsigned char *pad = nullptr;
+    if ((st = static_scratch_of_current_device(&pad)) != WINOCONV_OK) return st;
+    for (int n0 = 0; n0 < q.N; n0 += (int)fit) {
+      winoconv_desc_t part = *desc;
+      part.batch = (int)std::min<long long>(fit, q.N - n0);
+      const Plan *pp = nullptr;
+      if ((st = plan_of<Plan>(&part, build_plan, &pp)) != WINOCONV_OK) return st;
+      if (!pp->direct || pp->info.direct != 2) return fail(WINOCONV_ERR_UNSUPPORTED, "no plan for a part of the batch");
+      cudaError_t e = launch_pad_channels(dtype, (const uint8_t *)x + n0 * pixels * q.Cw * esz, pad, part.batch * pixels, q.Cw, q.C, (cudaStream_t)stream);
+      const char *detail = "";
+      if (e == cudaSuccess) e = launch_direct_forward(pp->dd, pp->dp, pad, u, bias, (uint8_t *)y + n0 * q.ys_n * esz, (cudaStream_t)stream, &detail);
+      if (e != cudaSuccess) return cuda_fail(e, "forward from the built-in array", detail);
+    }
+    return WINOCONV_OK;
   }
   const unsigned long long tiles_min = (unsigned long long)std::min<long long>(128, I.tiles);
   const unsigned long long v_tile = I.input_ws_bytes_min / tiles_min, m_tile = I.product_ws_bytes_min / tiles_min;

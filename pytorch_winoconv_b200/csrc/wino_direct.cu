@@ -29,9 +29,7 @@
 //
 // Stands in for the chain of src/base_conv_launchers.cu:338-381 where no output tile larger than 1 is worth its transforms.
 #include <algorithm>
-#include <cstdlib>
 #include <cstring>
-#include <cstdio>
 #include <map>
 #include <mutex>
 #include <type_traits>
@@ -942,6 +940,7 @@ bool direct_grad_desc(DirectDesc *q, int dtype, int N, int C, int K, int Km, con
 
 bool direct_fold_desc(DirectDesc *q, const int pad[3], int x_first) {
   if (q->dtype == WINOCONV_F32 || q->variants || q->transposed || q->Cw * q->kW_w > 64 || q->kW_w > 10) return false;
+  if ((long long)q->D * q->H * q->W * q->Cw > 0x7fffffffLL) return false;      // offsets within an image are 32-bit
   q->fold = 1;
   q->x_first = x_first;
   q->n_parts = 1;
@@ -1035,14 +1034,11 @@ bool direct_plan(const DirectDesc &d, DirectPlan *out) {
   static const Cfg cfgs32[] = {{64, 1, 0}};
   const Cfg *cfgs = f32 ? cfgs32 : cfgs16;
   const int n_cfgs = f32 ? 1 : 7;
-  const int force = [] { const char *v = getenv("WINOCONV_DIRECT_CFG"); return v && *v ? atoi(v) : -1; }();
-  const int force_split = [] { const char *v = getenv("WINOCONV_DIRECT_SPLIT"); return v && *v ? atoi(v) : 0; }();
   double best = 1e30;
   bool found = false;
   for (int ci = 0; ci < n_cfgs; ++ci) {
     const Cfg &c = cfgs[ci];
-    if (!f32 && force >= 0 && force != ci) continue;
-    if (c.BN > 64 && d.K <= c.BN / 2 && force < 0) continue;
+    if (c.BN > 64 && d.K <= c.BN / 2) continue;
     const int n_kb = (d.K + c.BN - 1) / c.BN;
     for (int ti = 1; ti <= 8; ti *= 2)
     for (int tn = 1; tn <= 16; tn *= 2) {
@@ -1070,7 +1066,6 @@ bool direct_plan(const DirectDesc &d, DirectPlan *out) {
         const int width = split * (c.pair ? 2 : 1);
         if (split > 1 && (width > 8 || d.variants || q.n_items > clusters_at_once(width) || split > q.units)) break;
         if (split > 1 && pool && c.MB * BM / split < 16 * tn) break;
-        if (force_split > 0 && split != force_split) continue;
         q.split = split;
         if (!ring_depths(q, p.max_taps, 227 * 1024 - FIXED_BYTES)) continue;
         if (split > 1 && c.MB * BM * (c.BN + 4) * 4 > q.n_a * q.a_bytes + q.n_b * q.b_bytes) continue;
@@ -1080,7 +1075,6 @@ bool direct_plan(const DirectDesc &d, DirectPlan *out) {
     }
   }
   if (!found) return false;
-  if (getenv("WINOCONV_DIRECT_DEBUG")) fprintf(stderr, "[direct] BN%d MB%d pair%d split%d TI%d TN%d tiles%d items%d na%d nb%d G%d slab%d est %.1f us\n", out->BN, out->MB, out->pair, out->split, out->TI, out->TN, out->n_tiles, out->n_items, out->n_a, out->n_b, out->G, out->slab_bytes, best/1.9e3);
   out->estimate = best;
   out->smem = FIXED_BYTES + out->n_a * out->a_bytes + out->n_b * out->b_bytes;
   return true;

@@ -156,3 +156,69 @@ def test_conv3d_backward_and_pool_refusal():
         mp(torch.randn(1, 8, 8, 8, device="cuda"))                        # train mode: the fused pool has no gradient
     with torch.no_grad():
         assert tuple(mp(torch.randn(1, 8, 8, 8, device="cuda")).shape) == (1, 8, 4, 4)
+
+
+def _by_torch(m, x, dtype=torch.float16):
+    f = torch.nn.functional.conv2d if x.dim() == 4 else torch.nn.functional.conv3d
+    b = None if m.bias is None else m.bias.detach().cpu().double()
+    return f(x.cpu().to(dtype).double(), m.weight.detach().cpu().to(dtype).double(), b, m.stride, m.padding)
+
+
+@pytest.mark.gpu
+def test_inputs_and_gradients_that_do_not_start_on_16_bytes():
+    from pytorch_winoconv_b200 import dwm
+    torch.manual_seed(21)
+    m = wconv.Conv2d(3, 16, 3, padding=1).cuda().eval()
+    x = torch.randn(2 * 3 * 20 * 24 + 1, device="cuda").half()[1:].view(2, 3, 20, 24)      # few channels, read as they lie
+    assert wo.error_metrics(m(x).detach().cpu().double(), _by_torch(m, x))["E_B"] < 2e-2
+    w = torch.randn(8, 8, 3, 3, device="cuda") * 0.1
+    xl = torch.randn(2 * 8 * 12 * 12 + 1, device="cuda")[1:].view(2, 12, 12, 8).permute(0, 3, 1, 2)
+    ref = torch.nn.functional.conv2d(xl.cpu().double(), w.cpu().double(), None, 1, 1)
+    assert wo.error_metrics(dwm.dwm2d(xl, w, padding=1).cpu(), ref)["E_B"] < 1e-3
+    m = wconv.Conv2d(16, 16, 3, stride=2, padding=1).cuda().train()
+    x = torch.randn(2, 16, 16, 16, device="cuda").half().to(memory_format=torch.channels_last).requires_grad_(True)
+    gy = torch.randn(2 * 8 * 8 * 16 + 1, device="cuda").half()[1:].view(2, 8, 8, 16).permute(0, 3, 1, 2)
+    m(x).backward(gy)
+    got, got_w = x.grad.clone(), m.weight.grad.clone()
+    x.grad = m.weight.grad = None
+    m(x).backward(gy.clone(memory_format=torch.contiguous_format).contiguous(memory_format=torch.channels_last))
+    assert torch.equal(got, x.grad) and torch.equal(got_w, m.weight.grad)
+
+
+@pytest.mark.gpu
+def test_a_weight_computed_anew_at_an_old_address_is_not_mistaken_for_it():
+    torch.manual_seed(22)
+    m = wconv.Conv2d(16, 16, 3, padding=1, bias=False).cuda().eval()
+    x = torch.randn(1, 16, 10, 10, device="cuda").half()
+    seen = set()
+    for i in range(6):          # the allocator hands the freed weight's block to the next one
+        w = torch.randn(16, 16, 3, 3, device="cuda") * 0.1
+        m.weight = torch.nn.Parameter(w.clone())
+        seen.add(m.weight.data_ptr())
+        assert wo.error_metrics(m(x).detach().cpu().double(), _by_torch(m, x))["E_B"] < 2e-2
+        del m.weight
+        m.register_parameter("weight", None)
+        del w
+    assert len(seen) < 6
+
+
+@pytest.mark.gpu
+def test_inference_weights_and_wide_padding_are_refused_as_before():
+    m = wconv.Conv2d(8, 8, 3, padding=1, bias=False).cuda().eval()
+    with torch.inference_mode():
+        m.weight = torch.nn.Parameter(torch.randn(8, 8, 3, 3, device="cuda"), requires_grad=False)
+    with torch.no_grad(), pytest.raises(RuntimeError):
+        m(torch.randn(1, 8, 6, 6, device="cuda").half())
+    m = wconv.Conv2d(8, 8, 1, padding=1).cuda().train()
+    y = m(torch.randn(1, 8, 6, 6, device="cuda").half().requires_grad_(True))
+    with pytest.raises(NotImplementedError):
+        y.sum().backward()
+
+
+def test_a_tracer_sees_the_module_call():
+    class Leaf(torch.fx.Tracer):
+        def is_leaf_module(self, module, name):
+            return isinstance(module, wconv.Conv2d)
+
+    net = torch.nn.Sequential(wconv.Conv2d(8, 8, 3), torch.nn.ReLU())
+    assert [n.op for n in Leaf().trace(net).nodes][1] == "call_module"

@@ -64,6 +64,16 @@ def test_static_scratch_serves_the_single_kernel_paths():
     print("forward_static vs forward (row kernel), E_B:", errs)
 
 
+def test_static_scratch_pads_channels_a_part_of_the_batch_at_a_time():
+    # fp32, 3 channels padded to 4: 36 images of 256 x 256 are 36 MiB of copy, more than the array holds
+    xa, ca = _layer(7, 36, 3, 8, 256, 3, 1, torch.float32)
+    assert ca.info.direct == 2
+    _both(xa, ca)
+    xb, cb = _layer(8, 2, 7, 12, 33, 5, 2, torch.float32)         # copy of 278784 bytes: not a multiple of 256
+    assert cb.info.direct == 2
+    _both(xb, cb)
+
+
 def test_static_scratch_refuses_oversized_layers():
     # 3-D 3x3x3 with 1024 -> 1024 channels: 64 positions x (1024*2 + 1024*4) B x 128 tiles = 48 MiB > 32 MiB (512 tiles in all)
     d = capi.make_desc(ndim=3, batch=1, c_in=1024, k_out=1024, in_size=(16, 16, 16), ker_size=3, pad=1, algo=capi.ALGO_STAGED)
