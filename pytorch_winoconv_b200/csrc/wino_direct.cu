@@ -68,7 +68,7 @@ struct DGeom {
   int n_ph, n_var, org_h[4], org_w[4], taps[4], tap0[4], T_hw;   // parts of the taps: all of them per item, or one (variants)
   int n_chunks, ch_el, k_full, k_tail;   // channel chunks, channels per chunk, MMA K steps of a full and of the last chunk
   int units;                         // kD * T_hw * n_chunks: (tap, chunk) pairs of the whole reduction
-  int G, split, dual;                // taps per filter stage, CTAs (pairs) per item, whether both issuers have MMAs in every share
+  int G, split;                      // taps per filter stage, CTAs (pairs) per item
   unsigned epilogue;
   int y_tma, bias_vec, bias_f32;
   uint32_t a_hi, b_hi;               // high descriptor words
@@ -170,9 +170,13 @@ template <typename F> __device__ __forceinline__ bool for_steps(const DGeom &g, 
 // fp32: two threads take alternate K steps of a block into accumulators of their own (one thread issues an MMA every 60 to
 // 85 clocks, three products a step), and the products with a remainder go to another pair: the accumulator is cut off after
 // every MMA, so its error grows with the number of MMAs that went into it times its size -- small products in a small
-// accumulator cost nothing, and the large ones have a chain a sixth as long (64 -> 64 channels, 3x3: largest error 1.9e-5 of the
-// output scale with one accumulator for everything, under 1e-5 with four).  The epilogue adds them up.
+// accumulator cost nothing.  After ACC_STEPS K steps the accumulators are handed to the epilogue, which keeps the sum in
+// registers, rounded to nearest, while the next ones fill: no chain is longer than ACC_STEPS / 2 and a filter stage.  2-norm
+// errors against 64 bits over 8 layers of 8 to 512 channels, 1x1 to 9x9: 1.6e-7 to 2.2e-7 and 3.0e-7 (17836 products) with 16
+// steps, 1.6e-7 to 2.4e-7 with 8, 2.5e-7 to 7.9e-6 without handing over; one step of 16 costs 5 % (64 -> 64 5x5 at 56x56, N = 8:
+// 57 us; with 8 steps 63), which one MMA for both parts of the filter (N = 128 instead of two of 64) gives back.
 __host__ __device__ constexpr int accumulators_of_a_block(bool f32) { return f32 ? 4 : 1; }
+constexpr int ACC_STEPS = 16;
 
 template <typename T, int BN, int MB, bool PAIR, bool FOLD>
 __global__ void __launch_bounds__(std::is_same<T, float>::value || FOLD ? 512 : 384, 1)
@@ -223,7 +227,7 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value || FOLD ? 512 : 
   }
   const uint32_t crank = PAIR ? cluster_ctarank() : 0u, rank = crank & 1u;   // rank within the pair
   const bool leader = rank == 0;                   // issues the MMAs of the pair
-  const uint32_t tmem_cols = g.split > 1 ? ACC : 2 * ACC;      // a shared item needs one accumulator
+  const uint32_t tmem_cols = g.split > 1 && !F32 ? ACC : 2 * ACC;      // a shared item needs one accumulator
   if (warp == 2) tmem_alloc<PAIR>(tmem_slot, tmem_cols);
   tc_fence_before();
   __syncthreads();
@@ -249,6 +253,45 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value || FOLD ? 512 : 
   // one channel block whose whole filter fits the ring: loaded once, its stages are never handed back
   const bool resident = g.n_kb == 1 && g.split == 1 && g.n_var == 1 && g.kD * g.n_ph * g.n_chunks * ((g.taps[0] + g.G - 1) / g.G) <= sl.n_b;
   bool alive = true;
+
+  // fp32: how many times an item's accumulators change hands, the K steps of the last time, and an epilogue warp's sum of 32 columns
+  int n_hand = 1, last_steps = 0;
+  float sum[32];
+  uint32_t n_acc = 0;
+  auto sum_accumulators = [&]() -> bool {
+    if constexpr (F32) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) sum[i] = 0.f;
+      const uint32_t ta = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(((warp - EPI_WARP0) >> 2) * 32);
+      for (int f = 0; f < n_hand; ++f, ++n_acc) {
+        const int buf = (int)(n_acc & 1u);
+        if (!mbar_wait_warp(acc_full(buf), (n_acc >> 1) & 1u, abort_word, err, ERR_EPI) || *abort_word != 0u) return false;
+        tc_fence_after();
+        const bool both = f + 1 < n_hand || last_steps >= 2;      // a single step is the first thread's
+#pragma unroll 1
+        for (int a = 0; a < (both ? N_ACC : N_ACC / 2); ++a) {
+          uint32_t r[32];
+          tmem_ld_x32(ta + (uint32_t)(buf * ACC + a * BN), r);
+          tmem_wait_ld_x32(r);
+#pragma unroll
+          for (int i = 0; i < 32; ++i) sum[i] += __uint_as_float(r[i]);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(acc_empty(buf));
+      }
+    }
+    return true;
+  };
+  if (F32 && warp >= EPI_WARP0 && warp < EPI_WARP0 + EPI_WARPS)
+    for_steps(g, 0, u0, u1, [&](int, int, int ch, int t0, int t1) -> bool {
+      const int nk = ch == g.n_chunks - 1 ? g.k_tail : g.k_full;
+      for (int t = t0; t < t1; t += g.G) {
+        if (last_steps >= ACC_STEPS) { ++n_hand; last_steps = 0; }
+        last_steps += min(g.G, t1 - t) * nk;
+      }
+      return true;
+    });
 
   if (warp == 0 && FOLD) {
     // ---------------------------------------------------------------- raw patches, from which warps 12-15 gather the slabs
@@ -341,11 +384,18 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value || FOLD ? 512 : 
       int as = 0, bs = 0;
       uint32_t a_ph = 0, b_ph = 0, n_done = 0;
       for (int item = item0; item < g.n_items && alive; item += item_step, ++n_done) {
-        const int buf = (int)(n_done & 1u);
-        if (!mbar_wait_warp(acc_empty(buf), ((n_done >> 1) & 1u) ^ 1u, abort_word, err, ERR_ACC)) { alive = false; break; }
-        tc_fence_after();
-        const uint32_t d0 = tmem + (uint32_t)(buf * ACC + me * BN);
-        uint32_t acc = 0, cnt = 0;        // whether this thread's accumulators hold something; MMAs of the item so far (mod 2)
+        int buf = 0;
+        uint32_t d0 = 0, acc = 0, cnt = 0;        // whether this thread's accumulators hold something; K steps that went into them
+        auto take = [&]() -> bool {
+          buf = (int)(n_acc & 1u);
+          if (!mbar_wait_warp(acc_empty(buf), ((n_acc >> 1) & 1u) ^ 1u, abort_word, err, ERR_ACC)) return false;
+          tc_fence_after();
+          d0 = tmem + (uint32_t)(buf * ACC + me * BN * (F32 ? 2 : 1));
+          acc = cnt = 0;
+          ++n_acc;
+          return true;
+        };
+        if (!take()) { alive = false; break; }
         const bool loaded = resident && n_done > 0;
         if (resident) { bs = 0; }
         alive = for_steps(g, g.n_var > 1 ? item / g.var_items : 0, u0, u1, [&](int kd, int p, int ch, int t0, int t1) -> bool {
@@ -359,23 +409,25 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value || FOLD ? 512 : 
               if (!mbar_wait_warp(b_full(bs), b_ph, abort_word, err, ERR_B)) return false;
               tc_fence_after();
             }
+            if (F32 && cnt >= (uint32_t)ACC_STEPS) {
+              if (elect_one()) umma_commit<PAIR>(acc_full(buf), pair_mask);
+              if (!take()) return false;
+            }
             const int n = min(g.G, t1 - t);
             uint32_t b_lo = desc_lo(base + (uint32_t)(sl.off_b + bs * sl.b_bytes));
             auto k_step = [&](uint32_t a_t, int k, uint32_t keep) {
 #pragma unroll
               for (int mb = 0; mb < MB; mb += N_ISSUE) {   // blocks me, me + 2, ...
                 const uint32_t a_k = a_t + (uint32_t)(mb * g.mb_off16) + 2u * k, b_k = b_lo + 2u * k, d = d0 + (uint32_t)(mb * BN);
-                if (F32) {
-                  const uint32_t al = a_k + (uint32_t)(sl.lo_off >> 4), bl = b_k + (uint32_t)(sl.b_lo >> 4);
-                  umma<PAIR, F32>(d + 2 * BN, al, g.a_hi, b_k, g.b_hi, idesc, keep);
-                  umma<PAIR, F32>(d, a_k, g.a_hi, b_k, g.b_hi, idesc, keep);
-                  umma<PAIR, F32>(d + 2 * BN, a_k, g.a_hi, bl, g.b_hi, idesc, 1u);
+                if (F32) {     // the filter's remainders lie behind its tf32 parts: both against the slab's tf32 part in one MMA
+                  umma<PAIR, F32>(d, a_k, g.a_hi, b_k, g.b_hi, idesc + ((uint32_t)(BN >> 3) << 17), keep);
+                  umma<PAIR, F32>(d + BN, a_k + (uint32_t)(sl.lo_off >> 4), g.a_hi, b_k, g.b_hi, idesc, 1u);
                 } else {
                   umma<PAIR, F32>(d, a_k, g.a_hi, b_k, g.b_hi, idesc, keep);
                 }
               }
             };
-            const bool whole = nk == 4 && (KS == 1 || g.dual);
+            const bool whole = nk == 4;
             if (elect_one()) {
               // straight-line code per tap for the usual numbers of K steps, the offset of the next tap read ahead: a loop over
               // the steps costs this lone thread 180 clocks an MMA
@@ -402,7 +454,7 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value || FOLD ? 512 : 
                 for (int j = 0; j < n; ++j, b_lo += (uint32_t)(sl.b_tile >> 4)) {
                   const uint32_t a_t = a_lo + rows[t + j];
                   for (int k = 0; k < nk; ++k, ++c)
-                    if (KS == 1 || (g.dual ? (c & 1u) == (uint32_t)me : me == 0)) { k_step(a_t, k, acc); acc = 1u; }
+                    if (KS == 1 || (c & 1u) == (uint32_t)me) { k_step(a_t, k, acc); acc = 1u; }
                 }
               }
             }
@@ -516,7 +568,7 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value || FOLD ? 512 : 
           float4 h;
           h.x = tf32_round(v.x); h.y = tf32_round(v.y); h.z = tf32_round(v.z); h.w = tf32_round(v.w);
           hi[i] = h;
-          lo[i] = make_float4(v.x - h.x, v.y - h.y, v.z - h.z, v.w - h.w);
+          lo[i] = make_float4(tf32_round(v.x - h.x), tf32_round(v.y - h.y), tf32_round(v.z - h.z), tf32_round(v.w - h.w));
         }
         fence_async_smem();
         __syncwarp();
@@ -543,36 +595,34 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value || FOLD ? 512 : 
       const Tile t = decode<MB, PAIR>(g, item, rank);
       const int kb = t.kb, yH = g.yH[t.var], yW = g.yW[t.var];
       const int buf = (int)(n_done & 1u);
-      if (!mbar_wait_warp(acc_full(buf), (n_done >> 1) & 1u, abort_word, err, ERR_EPI)) { alive = false; break; }
-      if (*abort_word != 0u) { alive = false; break; }
-      tc_fence_after();
-      bool handed = false;
+      if constexpr (F32) {
+        if (!sum_accumulators()) { alive = false; break; }
+      } else {
+        if (!mbar_wait_warp(acc_full(buf), (n_done >> 1) & 1u, abort_word, err, ERR_EPI)) { alive = false; break; }
+        if (*abort_word != 0u) { alive = false; break; }
+        tc_fence_after();
+      }
+      bool handed = F32;
 #pragma unroll 1
       for (int ci = half; ci < N_CH; ci += 2) {
         const int mb = ci / CH_PER_MB, c0 = (ci - mb * CH_PER_MB) * COLS;
         const int k0 = kb * BN + c0;
         const int oh_b = t.oh0 + mb * g.TH;
         const bool wanted = k0 < g.K && t.valid && oh_b < g.oH;
-        const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * ACC + mb * BN * N_ACC + c0);
+        const uint32_t ta = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(buf * ACC + mb * BN + c0);
         // 32 columns at a time, in a loop: twice the code for 64 in one piece ran slower (an epilogue warp executes it once per
         // item, mostly out of cold instruction caches)
 #pragma unroll 1
         for (int hc = 0; hc < COLS; hc += 32) {
           uint32_t r[32];
-          if (wanted) {
+          if constexpr (F32) {
+#pragma unroll
+            for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(sum[i]);
+          } else if (wanted) {
             tmem_ld_x32(ta + (uint32_t)hc, r);
             tmem_wait_ld_x32(r);
-#pragma unroll
-            for (int a = 1; a < N_ACC; ++a)      // the block's other accumulators (1 and 3 are the second thread's)
-              if (g.dual || a == 2) {
-                uint32_t r2[32];
-                tmem_ld_x32(ta + (uint32_t)(a * BN + hc), r2);
-                tmem_wait_ld_x32(r2);
-#pragma unroll
-                for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(r2[i]));
-              }
           }
-          if (ci + 2 >= N_CH && hc + 32 >= COLS) {      // this warp's last columns are in registers: its share of the hand-back
+          if (!F32 && ci + 2 >= N_CH && hc + 32 >= COLS) {      // this warp's last columns are in registers: its share of the hand-back
             tc_fence_before();
             __syncwarp();
             if (lane == 0) { if (PAIR) mbar_arrive_rank0(acc_empty(buf)); else mbar_arrive(acc_empty(buf)); }
@@ -660,6 +710,7 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value || FOLD ? 512 : 
     }
     if (lane == 0) bulk_wait_read();     // the staging rows are read before the CTA's shared memory goes
   }
+  if (F32 && g.split > 1 && warp >= EPI_WARP0 && warp < EPI_WARP0 + EPI_WARPS && item0 < g.n_items) alive = sum_accumulators();
   if (g.split > 1) {
     // ---------------------------------------------------------------- the cluster's shares of one item added up
     // Every CTA puts its accumulator into its own shared memory (the operand rings are idle by then) and finishes 1 / split
@@ -669,21 +720,17 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value || FOLD ? 512 : 
     __syncthreads();
     if (epi && item0 < g.n_items) {
       const int q = warp & 3, half = (warp - EPI_WARP0) >> 2;
-      if (mbar_wait_warp(acc_full(0), 0u, abort_word, err, ERR_EPI)) {
+      if (F32 || mbar_wait_warp(acc_full(0), 0u, abort_word, err, ERR_EPI)) {
         tc_fence_after();
         for (int c0 = half * 32; c0 < MB * BN; c0 += 64) {
           uint32_t r[32];
-          tmem_ld_x32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
-          tmem_wait_ld_x32(r);
+          if constexpr (F32) {
 #pragma unroll
-          for (int a = 1; a < N_ACC; ++a)
-            if (g.dual || a == 2) {
-              uint32_t r2[32];
-              tmem_ld_x32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(a * BN + c0), r2);
-              tmem_wait_ld_x32(r2);
-#pragma unroll
-              for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) + __uint_as_float(r2[i]));
-            }
+            for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(sum[i]);
+          } else {
+            tmem_ld_x32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
+            tmem_wait_ld_x32(r);
+          }
           const int mb = c0 / BN;
           float4 *dst = reinterpret_cast<float4 *>(base_ptr) + ((mb * BM + q * 32 + lane) * ROW_F + (c0 - mb * BN)) / 4;
 #pragma unroll
@@ -796,7 +843,7 @@ __global__ void __launch_bounds__(256) direct_filter_kernel(const TW *__restrict
     if constexpr (std::is_same<T, float>::value) {
       const float h = tf32_round(v);
       u[2 * tap * total + idx] = h;
-      u[(2 * tap + 1) * total + idx] = v - h;
+      u[(2 * tap + 1) * total + idx] = tf32_round(v - h);      // the tensor core would cut it off
     } else {
       Elem<T>::store(u + tap * total + idx, v);
     }
@@ -1001,7 +1048,7 @@ bool direct_plan(const DirectDesc &d, DirectPlan *out) {
   if (d.fold) return fold_plan(d, out);
   const bool f32 = d.dtype == WINOCONV_F32;
   const int esz = f32 ? 4 : 2, vec = 16 / esz;
-  if (d.C % vec != 0) return false;
+  if (d.C % vec != 0 || (f32 && d.variants)) return false;
   const bool pool = (d.epilogue & WINOCONV_EPI_POOL2) != 0;
   DirectPlan p;
   std::memset(&p, 0, sizeof p);
@@ -1271,13 +1318,6 @@ cudaError_t launch_direct_forward(const DirectDesc &d, const DirectPlan &p, cons
     g.fD = d.D; g.fH = d.H; g.fW = d.W; g.fC = d.Cw; g.fkW = d.kW_w; g.fold_rows = p.slab_rows_h;
   }
   g.n_chunks = p.n_chunks; g.ch_el = p.ch_el; g.k_full = p.k_full; g.k_tail = p.k_tail; g.units = p.units;
-  {   // MMAs of the smallest share of an item
-    const int per_unit = p.n_chunks > 1 ? 1 : p.k_tail;
-    int least = p.units / p.split * per_unit;
-    if (d.variants)
-      for (int q = 0; q < d.n_parts; ++q) least = std::min(least, d.kD * p.taps[q] * p.n_chunks * per_unit);
-    g.dual = least >= 2;
-  }
   g.G = p.G; g.split = p.split; g.epilogue = d.epilogue;
   g.y_tma = y_tma; g.bias_f32 = d.bias_f32; g.bias_vec = y_tma && (reinterpret_cast<uintptr_t>(bias) & 15u) == 0;
   const int row_step = d.fold ? d.sH : 1;      // slab rows between neighbouring output rows

@@ -14,9 +14,10 @@
 // the weight's own order.  What bounds it: the shares.  Their number times dW is written and read once, 148 CTAs x up to
 // 256 KB, so small layers use fewer, longer shares (see wgrad_plan).
 //
-// The bias gradient rides along: one more accumulator whose (tap, channel) operand is all ones.
+// The bias gradient rides along: warps 4-7 add up the gy tiles as they lie in shared memory, in fp32 and in short chains (as
+// one more accumulator, against an operand of ones, the tensor core's cut-off sums had twice the error of an fp32 sum).
 //
-// Roles: warp 0 TMA (x slabs), warp 1 TMA (gy tiles), warps 2-3 MMA issue (alternate bundles); then all eight warps move the
+// Roles: warp 0 TMA (x slabs), warp 1 TMA (gy tiles), warps 2-3 MMA issue (alternate bundles), warps 4-7 bias sums; then all eight warps move the
 // accumulators to global memory, laid out so that a warp's store is 128 consecutive bytes: [share][channel block][bundle][k][row].
 // Every mbarrier wait is bounded and reports through the error word.
 #include <algorithm>
@@ -37,7 +38,7 @@ using namespace sm100;
 
 constexpr int N_THREADS = 256;
 constexpr int MAX_BUNDLES = 80, MAX_STEPS = 40, MAX_GROUPS = 24;
-constexpr int ONES_BYTES = 4096;       // two blocks of 16 pixels x 128 bytes
+constexpr int SUMS_BYTES = 4 * 128 * 4;       // bias sums of four warps
 constexpr int BAR_BYTES = 256;
 
 enum ErrCode : unsigned { ERR_X_EMPTY = 0x501, ERR_G_EMPTY = 0x502, ERR_X = 0x503, ERR_G = 0x504, ERR_EPI = 0x505 };
@@ -58,7 +59,7 @@ struct WGeom {
   uint32_t a_hi, b_hi, b_lead, b_tile;   // descriptor words; distance of gy's 64-channel blocks (16-byte units), bytes of one
   int n_gblk;                            // 64-channel blocks of a gy tile
   int bias_on;
-  int slab_bytes, x_bytes, g_bytes, n_x, n_g, off_g, off_ones, off_bars;
+  int slab_bytes, x_bytes, g_bytes, n_x, n_g, off_g, off_sums, off_bars;
   long long part_stride, bias_off;       // floats of one share, offset of the bias sums in it
   Step steps[MAX_STEPS];
   Bundle bundles[MAX_BUNDLES];
@@ -84,7 +85,7 @@ __device__ __forceinline__ void tile_load(const WGeom &g, uint32_t dst, const CU
 
 __global__ void __launch_bounds__(N_THREADS, 1)
     wgrad_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_g, float *__restrict__ part,
-                 uint32_t ones, const __grid_constant__ WGeom g, uint32_t idesc) {
+                 int bf16, const __grid_constant__ WGeom g, uint32_t idesc) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -99,29 +100,6 @@ __global__ void __launch_bounds__(N_THREADS, 1)
   unsigned *err = &g_wgrad_error;
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
 
-  if (warp == 1 && lane == 0) { prefetch_map(&map_x); prefetch_map(&map_g); }
-  if (warp == 0) {
-    if (lane < 4) { mbar_init(x_full(lane), 1); mbar_init(x_empty(lane), 2); }
-    else if (lane < 8) { mbar_init(g_full(lane - 4), 1); mbar_init(g_empty(lane - 4), 2); }
-    else if (lane == 8) mbar_init(done, 2);
-    else if (lane == 9) *abort_word = 0u;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  if (warp >= 4) {      // the operand of the bias sums
-    for (int i = threadIdx.x - 128; i < ONES_BYTES / 16; i += 128)
-      *reinterpret_cast<uint4 *>(base_ptr + g.off_ones + i * 16) = make_uint4(ones, ones, ones, ones);
-    fence_async_smem();
-  }
-  if (warp == 2) tmem_alloc<false>(tmem_slot, 512);
-  tc_fence_before();
-  __syncthreads();
-  tc_fence_after();
-  uint32_t tmem;
-  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot));
-  tmem = __shfl_sync(0xffffffffu, tmem, 0);
-  grid_launch_dependents();
-  grid_dependency_wait();
-
   // this CTA: share, bundle group, channel blocks
   unsigned q = blockIdx.x / (unsigned)g.n_kb;
   const int kb = (int)(blockIdx.x - q * (unsigned)g.n_kb);
@@ -133,6 +111,25 @@ __global__ void __launch_bounds__(N_THREADS, 1)
   const int blk0 = (int)((long long)g.n_blocks * share / g.split), blk1 = (int)((long long)g.n_blocks * (share + 1) / g.split);
   const int gb0 = g.g_b0[grp], gb1 = g.g_b0[grp + 1];            // bundles of the group
   const bool bias = g.bias_on && cb == 0 && grp == 0;
+
+  if (warp == 1 && lane == 0) { prefetch_map(&map_x); prefetch_map(&map_g); }
+  if (warp == 0) {
+    if (lane < 4) { mbar_init(x_full(lane), 1); mbar_init(x_empty(lane), 2); }
+    else if (lane < 8) { mbar_init(g_full(lane - 4), 1); mbar_init(g_empty(lane - 4), bias ? 6 : 2); }
+    else if (lane == 8) mbar_init(done, 2);
+    else if (lane == 9) *abort_word = 0u;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 2) tmem_alloc<false>(tmem_slot, 512);
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  uint32_t tmem;
+  asm volatile("ld.shared.b32 %0, [%1];" : "=r"(tmem) : "r"(tmem_slot));
+  tmem = __shfl_sync(0xffffffffu, tmem, 0);
+  grid_launch_dependents();
+  grid_dependency_wait();
+
   const int st0 = g.g_step0[grp];
   bool alive = true;
 
@@ -192,11 +189,6 @@ __global__ void __launch_bounds__(N_THREADS, 1)
       if (!mbar_wait_warp(g_full(gs), g_ph, abort_word, err, ERR_G)) { alive = false; break; }
       tc_fence_after();
       const uint32_t b_lo = (((base + (uint32_t)(g.off_g + gs * g.g_bytes)) & 0x3FFFFu) >> 4) | (g.b_lead << 16);
-      if (bias && me == 1 && elect_one()) {       // M = 128 rows of ones x this tile
-        const uint32_t a = desc_lo(base + g.off_ones, 2048), d = tmem + (uint32_t)((gb1 - gb0) * g.N_mma);
-#pragma unroll
-        for (int k = 0; k < 8; ++k) umma<false, false>(d, a, desc_hi(1024, 2), b_lo + (uint32_t)k * g_pair, g.b_hi, idesc, k == 0 ? acc : 1u);
-      }
       alive = for_steps([&](int st, int b0, int b1) -> bool {
         (void)st;
         if (!mbar_wait_warp(x_full(xs), x_ph, abort_word, err, ERR_X)) return false;
@@ -219,6 +211,41 @@ __global__ void __launch_bounds__(N_THREADS, 1)
       acc = 1u;
     }
     if (elect_one()) umma_commit<false>(done, 0);
+  } else if (bias) {
+    // a warp takes 32 pixels of every tile, a lane two neighbouring channels of each 64-channel block
+    int gs = 0;
+    uint32_t g_ph = 0;
+    float total[2][2] = {{0.f, 0.f}, {0.f, 0.f}};
+    for (int b = blk0; b < blk1; ++b) {
+      if (!mbar_wait_warp(g_full(gs), g_ph, abort_word, err, ERR_G)) break;
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        if (j >= g.n_gblk) break;
+        const uint8_t *tile = base_ptr + g.off_g + gs * g.g_bytes + j * (int)g.b_tile + (warp - 4) * 4096 + (lane & 3) * 4;
+        float a[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+          const uint32_t v = *reinterpret_cast<const uint32_t *>(tile + i * 128 + (((lane >> 2) ^ (i & 7)) << 4));
+          const float2 f = bf16 ? Pair16<__nv_bfloat16>::unpack(v) : Pair16<__half>::unpack(v);
+          a[2 * (i & 3)] += f.x;
+          a[2 * (i & 3) + 1] += f.y;
+        }
+        total[j][0] += (a[0] + a[2]) + (a[4] + a[6]);
+        total[j][1] += (a[1] + a[3]) + (a[5] + a[7]);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(g_empty(gs));
+      if (++gs == g.n_g) { gs = 0; g_ph ^= 1u; }
+    }
+    float *sums = reinterpret_cast<float *>(base_ptr + g.off_sums);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      sums[(warp - 4) * 128 + j * 64 + 2 * lane] = total[j][0];
+      sums[(warp - 4) * 128 + j * 64 + 2 * lane + 1] = total[j][1];
+    }
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    const int c = threadIdx.x - 128, k = kb * g.n_k + c;
+    if (c < g.n_k && k < g.K) part[(long long)share * g.part_stride + g.bias_off + k] = (sums[c] + sums[128 + c]) + (sums[256 + c] + sums[384 + c]);
   }
   __syncwarp();
   if (mbar_wait_warp(done, 0, abort_word, err, ERR_EPI) && *abort_word == 0u) {
@@ -236,18 +263,6 @@ __global__ void __launch_bounds__(N_THREADS, 1)
 #pragma unroll
       for (int j = 0; j < 32; ++j)
         if (k + j < g.K) dst[j * 128] = __uint_as_float(v[j]);
-    }
-    if (bias && warp == 0) {       // every row of the ones accumulator holds the sums: lane j writes column j
-      for (int k0 = 0; k0 < g.N_mma; k0 += 32) {
-        uint32_t v[32];
-        tmem_ld_x32(t_row + (uint32_t)(n_b * g.N_mma + k0), v);
-        tmem_wait_ld_x32(v);
-        uint32_t own = v[0];
-#pragma unroll
-        for (int j = 1; j < 32; ++j) own = lane == j ? v[j] : own;
-        const int k = kb * g.n_k + k0 + lane;
-        if (k < g.K) part[(long long)share * g.part_stride + g.bias_off + k] = __uint_as_float(own);
-      }
     }
     tc_fence_before();
   }
@@ -286,8 +301,7 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float *__restri
     float v[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) v[e] = src[(j + e) * g.part_stride];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) s += v[e];
+    s += ((v[0] + v[1]) + (v[2] + v[3])) + ((v[4] + v[5]) + (v[6] + v[7]));
   }
   for (; j < g.split; ++j) s += src[j * g.part_stride];
   if (is_bias) dbias[i - (int)g.bias_off] = s;
@@ -372,16 +386,12 @@ bool wgrad_plan(const WgradDesc &d, WgradPlan *out) {
         q.g_bytes = q.n_gblk * 16384;
         const int cap = (q.N_mma % 32 == 0 ? 512 : 496) / q.N_mma;
         if (cap < 2) continue;
-        const int virt = n_b + (d.bias ? 1 : 0);
-        q.n_groups = (virt + cap - 1) / cap;
+        q.n_groups = (n_b + cap - 1) / cap;
         if (q.n_groups > MAX_GROUPS) continue;
         int widest = 0, most_steps = 0;
-        for (int i = 0; i <= q.n_groups; ++i) {
-          const int e = (int)((long long)virt * i / q.n_groups) - (d.bias ? 1 : 0);
-          q.g_b0[i] = i == 0 ? 0 : e;
-        }
+        for (int i = 0; i <= q.n_groups; ++i) q.g_b0[i] = (int)((long long)n_b * i / q.n_groups);
         for (int i = 0; i < q.n_groups; ++i) {
-          widest = std::max(widest, q.g_b0[i + 1] - q.g_b0[i] + (i == 0 && d.bias ? 1 : 0));
+          widest = std::max(widest, q.g_b0[i + 1] - q.g_b0[i]);
           int s0 = 0, n = 0;
           while (g.steps[s0].b1 <= q.g_b0[i]) ++s0;
           q.g_step0[i] = s0;
@@ -389,7 +399,7 @@ bool wgrad_plan(const WgradDesc &d, WgradPlan *out) {
           most_steps = std::max(most_steps, n);
         }
         // rings: two gy tiles, then slabs, then more of both
-        const int budget = 227 * 1024 - 1024 - ONES_BYTES - BAR_BYTES - 1024;
+        const int budget = 227 * 1024 - 1024 - SUMS_BYTES - BAR_BYTES - 1024;
         q.n_g = 2; q.n_x = 1;
         if (q.n_g * q.g_bytes + q.n_x * q.x_bytes > budget) continue;
         while (q.n_x < 4 && q.n_g * q.g_bytes + (q.n_x + 1) * q.x_bytes <= budget) ++q.n_x;
@@ -424,8 +434,8 @@ bool wgrad_plan(const WgradDesc &d, WgradPlan *out) {
   g.a_hi = desc_hi((uint32_t)(g.PW * g.TI * rb), rb == 128 ? 2u : rb == 64 ? 4u : 6u);
   g.b_hi = desc_hi(1024, 2);
   g.off_g = g.n_x * g.x_bytes;
-  g.off_ones = g.off_g + g.n_g * g.g_bytes;
-  g.off_bars = g.off_ones + ONES_BYTES;
+  g.off_sums = g.off_g + g.n_g * g.g_bytes;
+  g.off_bars = g.off_sums + SUMS_BYTES;
   g.bias_off = (long long)g.n_cb * g.all_bundles * d.K * 128;
   g.part_stride = (g.bias_off + d.K + 31) / 32 * 32;
   out->smem = 1024 + g.off_bars + BAR_BYTES;
@@ -492,7 +502,6 @@ cudaError_t launch_wgrad(const WgradDesc &d, const WgradPlan &p, const void *x, 
   // A = B = f16 / bf16, both MN-major, D = f32, M = 128
   const uint32_t fmt = d.dtype == WINOCONV_F16 ? 0u : 1u;
   const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | (1u << 15) | (1u << 16) | ((uint32_t)(g.N_mma >> 3) << 17) | ((128u >> 4) << 24);
-  const uint32_t ones = d.dtype == WINOCONV_F16 ? 0x3C003C00u : 0x3F803F80u;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(g.split * g.n_groups * g.n_cb * g.n_kb)); cfg.blockDim = dim3(N_THREADS);
   cfg.dynamicSmemBytes = (size_t)p.smem; cfg.stream = s;
@@ -500,7 +509,7 @@ cudaError_t launch_wgrad(const WgradDesc &d, const WgradPlan &p, const void *x, 
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr; cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, wgrad_kernel, mx, mg, (float *)ws, ones, g, idesc);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, wgrad_kernel, mx, mg, (float *)ws, d.dtype == WINOCONV_BF16 ? 1 : 0, g, idesc);
   if (e != cudaSuccess) return e;
   RGeom r;
   std::memset(&r, 0, sizeof r);

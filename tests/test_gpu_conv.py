@@ -7,7 +7,7 @@ import pytest
 import torch
 
 from oracle import winograd_oracle as wo
-from pytorch_winoconv_b200 import capi
+from pytorch_winoconv_b200 import capi, engine
 from tests.gpu_util import TOL, check_against_oracle, run_engine, seeded
 
 pytestmark = pytest.mark.gpu
@@ -413,3 +413,30 @@ def test_translation_equivariance():
     y, _ = run_engine(x, w, padding=0)
     ys, _ = run_engine(x[:, :, 4:, 4:].contiguous(), w, padding=0)
     assert torch.equal(y[:, :, 4:, 4:], ys)
+
+
+@pytest.mark.parametrize("n,c,k,sp,ks", [(1, 64, 64, (56, 56), 3), (8, 8, 24, (20, 20), 9), (2, 12, 72, (9, 11), 7), (3, 96, 64, (4, 9, 9), 3)])
+def test_fp32_direct_taps_keep_short_accumulator_chains(n, c, k, sp, ks):
+    # three tf32 products of rounded halves: 2**-22 per operand at worst, a third of that in the 2-norm; chains of at most 16 MMAs add
+    # less than that again.  One chain for the whole sum sits above 6e-7 on each of these.
+    x, w = _rand(n, c, k, sp, ks, torch.float32)
+    y = _run_direct(x, w, ks // 2)
+    o = wo.direct_conv_f64(x, w, padding=ks // 2)
+    rel = float((y.double() - o).norm() / o.norm())
+    assert rel < 3e-7, rel
+
+
+def _rand(n, c, k, sp, ks, dtype):
+    g = torch.Generator().manual_seed(c * 1000 + ks)
+    x = torch.randn(n, c, *sp, generator=g).clamp_min(0).to(dtype)
+    w = (torch.randn(k, c, *([ks] * len(sp)), generator=g) * (2.0 / (c * ks ** len(sp))) ** 0.5).to(dtype)
+    return x, w
+
+
+def _run_direct(x, w, pad, tile_m=1):
+    nd = x.dim() - 2
+    xl = x.permute(0, *range(2, 2 + nd), 1).contiguous().cuda()
+    y = engine.WinoConv(xl.shape, w.cuda(), padding=pad, tile_m=tile_m)(xl)
+    torch.cuda.synchronize()
+    assert capi.read_device_error() == 0
+    return y.permute(0, nd + 1, *range(1, nd + 1)).cpu()

@@ -222,3 +222,15 @@ def test_a_tracer_sees_the_module_call():
 
     net = torch.nn.Sequential(wconv.Conv2d(8, 8, 3), torch.nn.ReLU())
     assert [n.op for n in Leaf().trace(net).nodes][1] == "call_module"
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("k", [8, 72, 136])
+def test_bias_gradient_is_an_fp32_sum(k):
+    # chains of 8 in a tile, then of tiles and shares: a handful of roundings of 2**-24 on partial sums of the same size
+    torch.manual_seed(23)
+    m = wconv.Conv2d(16, k, 1).cuda().train()
+    gy = torch.randn(16, k, 33, 35, device="cuda").half().to(memory_format=torch.channels_last)
+    m(torch.randn(16, 16, 33, 35, device="cuda").half()).backward(gy)
+    exact = gy.double().sum((0, 2, 3))
+    assert float((m.bias.grad.double() - exact).norm() / exact.norm()) < 4e-7
