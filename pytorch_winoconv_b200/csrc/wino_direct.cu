@@ -16,7 +16,8 @@
 // and spend an epilogue and a producer pass on the transforms.
 //
 // Roles of a CTA: warp 0 TMA slabs, warp 1 TMA filter tiles, warps 2-3 MMA issue (one per 128-row block; warp 2 owns the
-// tensor memory), warps 4-11 epilogue (lane quarter x alternate 128-byte column chunks: bias, ReLU, 2x2 pool, TMA stores),
+// tensor memory), warps 4-11 epilogue (lane quarter x alternate 128-byte column chunks: bias, ReLU, 2x2 pool, TMA stores; items of few
+// MMAs come with a second such set, warps 12-19, and the sets take items in turn),
 // for fp32 also warps 12-15, which split every landed slab into a tf32 part and its remainder (three products per multiply,
 // the filter comes split from its transform).
 // Few channels (an RGB stem) would leave most of a 16-channel step empty and cannot be loaded by TMA (16-byte pixels).  There
@@ -52,6 +53,8 @@ constexpr int MAX_TAPS = 100;
 constexpr int BAR_BYTES = 512;
 constexpr unsigned RAW_BUFS = 4;       // raw patches in flight (few channels): small, and thousands of clocks away
 constexpr int FIXED_BYTES = 1024 /*alignment*/ + EPI_WARPS * STAGE_BYTES + BAR_BYTES;
+constexpr int SET_BYTES = EPI_WARPS * STAGE_BYTES;     // staging of a second set of epilogue warps (warps 12-19)
+__host__ __device__ constexpr int threads_of(bool splits, int sets) { return 32 * (SPLIT_WARP0 + (splits ? SPLIT_WARPS : 0) + (sets - 1) * EPI_WARPS); }
 
 enum ErrCode : unsigned { ERR_A_EMPTY = 0x401, ERR_B_EMPTY = 0x402, ERR_ACC = 0x403, ERR_A = 0x404, ERR_B = 0x405, ERR_EPI = 0x406, ERR_SPLIT = 0x407 };
 
@@ -178,8 +181,8 @@ template <typename F> __device__ __forceinline__ bool for_steps(const DGeom &g, 
 __host__ __device__ constexpr int accumulators_of_a_block(bool f32) { return f32 ? 4 : 1; }
 constexpr int ACC_STEPS = 16;
 
-template <typename T, int BN, int MB, bool PAIR, bool FOLD>
-__global__ void __launch_bounds__(std::is_same<T, float>::value || FOLD ? 512 : 384, 1)
+template <typename T, int BN, int MB, bool PAIR, bool FOLD, int SETS>
+__global__ void __launch_bounds__(threads_of(std::is_same<T, float>::value || FOLD, SETS), 1)
     direct_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_u,
                   const __grid_constant__ MapSet maps_y, const T *__restrict__ x, T *__restrict__ y, const T *__restrict__ bias,
                   const __grid_constant__ DGeom g, const __grid_constant__ DSmem sl, uint32_t idesc) {
@@ -577,11 +580,14 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value || FOLD ? 512 : 
         return true;
       });
     }
-  } else if (warp >= EPI_WARP0 && warp < EPI_WARP0 + EPI_WARPS && g.split == 1) {
+  } else if (warp >= EPI_WARP0 && g.split == 1) {
     // ---------------------------------------------------------------- epilogue
-    const int q = warp & 3, half = (warp - EPI_WARP0) >> 2;
-    const uint32_t stage = base + (uint32_t)(sl.off_stage + (warp - EPI_WARP0) * STAGE_BYTES);
-    const uint8_t *stage_ptr = base_ptr + sl.off_stage + (warp - EPI_WARP0) * STAGE_BYTES;
+    // a set of eight warps per accumulator buffer, or one for both
+    const int set = SETS == 2 && warp >= EPI_WARP0 + EPI_WARPS ? 1 : 0;
+    const int ew = warp - EPI_WARP0 - set * EPI_WARPS;
+    const int q = warp & 3, half = ew >> 2;
+    const uint32_t stage = base + (uint32_t)(sl.off_stage + (set * EPI_WARPS + ew) * STAGE_BYTES);
+    const uint8_t *stage_ptr = base_ptr + sl.off_stage + (set * EPI_WARPS + ew) * STAGE_BYTES;
     const bool relu = (g.epilogue & WINOCONV_EPI_RELU) != 0, has_bias = (g.epilogue & WINOCONV_EPI_BIAS) != 0;
     const bool pool = (g.epilogue & WINOCONV_EPI_POOL2) != 0;
     constexpr int CH_PER_MB = BN / COLS, N_CH = MB * CH_PER_MB;
@@ -590,8 +596,8 @@ __global__ void __launch_bounds__(std::is_same<T, float>::value || FOLD ? 512 : 
     const int grp = q * 4 + (lane >> 3), h_l = grp >> g.tn_shift, w_l = (lane & 7) >> g.ti_shift, i_l = lane & (g.TI - 1);
     int srow = lane;
     if (pool) srow = ((h_l | w_l) & 1) ? -1 : ((g.TN == 1 ? lane >> 4 : grp & tnm) << 2) + ((w_l >> 1) << g.ti_shift) + i_l;
-    uint32_t n_done = 0;
-    for (int item = item0; item < g.n_items; item += item_step, ++n_done) {
+    uint32_t n_done = (uint32_t)set;
+    for (int item = item0 + set * item_step; item < g.n_items; item += SETS * item_step, n_done += (uint32_t)SETS) {
       const Tile t = decode<MB, PAIR>(g, item, rank);
       const int kb = t.kb, yH = g.yH[t.var], yW = g.yW[t.var];
       const int buf = (int)(n_done & 1u);
@@ -875,19 +881,22 @@ static int clusters_at_once(int width) { return width == 1 ? 148 : width == 2 ? 
 // instruction of 128 / 256 columns; of 64 columns 60 from one issuing thread, 48 from two), its shared-memory traffic at 128 B
 // per clock, or its loads: about 28 B per clock and SM from L2 when all SMs load, at most 60 for one.  Set-up, first loads
 // and drain of a launch were measured at about 8000 clocks, 800 more for a pair, 4600 for a cluster's exchange of partial sums.
-static double estimate(const DirectPlan &p, double k_steps, int n_steps, int n_var, bool f32) {
+static double item_clocks(const DirectPlan &p, double k_steps, int n_steps, int n_var, bool f32) {
   const double t_mma = p.BN == 256 ? 130 : p.BN == 128 ? 66 : p.MB >= 2 || f32 ? 48 : 60;
   const int bn_own = p.pair ? p.BN / 2 : p.BN;
   const double mma = k_steps * p.MB * t_mma * (f32 ? 3 : 1);
   const double loads = n_steps * (double)p.slab_bytes + k_steps * bn_own * 32.0 * (f32 ? 2 : 1);
   const double smem = k_steps * p.MB * (f32 ? 3 : 1) * (4096.0 + bn_own * 32.0) + loads + (f32 ? 3.0 * n_steps * p.slab_bytes : 0.0);
-  const int width = (p.pair ? 2 : 1) * p.split;
-  const int slots = clusters_at_once(width);
-  const int n_items = p.n_items * n_var;
-  const double waves = (n_items + slots - 1) / slots;
-  const double active = std::min(148.0, (double)n_items * width);
+  const double active = std::min(148.0, (double)p.n_items * n_var * (p.pair ? 2 : 1) * p.split);
   const double l2 = loads / std::min(60.0, 28.0 * 148 / active);
-  const double item = std::max(mma, std::max(smem / 128.0, l2));
+  return std::max(mma, std::max(smem / 128.0, l2));
+}
+static double waves_of(const DirectPlan &p, int n_var) {
+  const int slots = clusters_at_once((p.pair ? 2 : 1) * p.split);
+  return (p.n_items * n_var + slots - 1) / slots;
+}
+static double estimate(const DirectPlan &p, double k_steps, int n_steps, int n_var, bool f32) {
+  const double item = item_clocks(p, k_steps, n_steps, n_var, f32), waves = waves_of(p, n_var);
   const double epi = 400.0 + 350.0 * p.MB * p.BN / 64;
   const double tail = 1500.0 * ((p.MB * p.BN / (f32 ? 32 : 64) + 1) / 2 - 1);     // the last epilogue
   if (p.split > 1) return 8000.0 + (p.pair ? 800.0 : 0.0) + item / p.split + 4000.0 + 10.0 * p.BN * p.MB;
@@ -1035,6 +1044,7 @@ static bool fold_plan(const DirectDesc &d, DirectPlan *out) {
     q.raw_tma = row % 8 == 0 && q.raw_el <= 256 && q.slab_rows_h <= 256 && (!first || d.Cw <= 256);
     q.raw_box = q.raw_tma ? q.slab_rows_h * q.raw_el * 2 * (first ? d.Cw : 1) : 0;
     const int raws = (int)RAW_BUFS * ((q.raw_box + 127) / 128 * 128);
+    q.epi_sets = 1;
     if (!ring_depths(q, rows, 227 * 1024 - FIXED_BYTES - raws)) continue;
     q.smem = FIXED_BYTES + raws + q.n_a * q.a_bytes + q.n_b * q.b_bytes;
     *out = q;
@@ -1123,7 +1133,18 @@ bool direct_plan(const DirectDesc &d, DirectPlan *out) {
   }
   if (!found) return false;
   out->estimate = best;
-  out->smem = FIXED_BYTES + out->n_a * out->a_bytes + out->n_b * out->b_bytes;
+  out->epi_sets = 1;
+  // A second set of epilogue warps, where a CTA has several items and their epilogues (about 4000 clocks for two 64-column pieces,
+  // one each for the two halves of a set) take more than twice as long as their loads and MMAs.  us on B200, one set / two, N = 32:
+  // 1x1 64 -> 64 at 112x112 26.5 / 22.1, 64 -> 256 at 56x56 24.5 / 20.7; 3x3 16 -> 64 at 112x112 24.5 / 21.1, 8 -> 64 26.2 / 22.7.
+  // With more MMAs an item it loses ring depth and registers (640 threads: 80 each): 1x1 256 -> 64 at 56x56 13.0 / 13.9, 3x3
+  // 64 -> 64 at 112x112 30.5 / 31.3; the gathered stem (7x7 at stride 2, 768 threads, spills) 37.4 / 50.0.
+  if (!f32 && out->split == 1 && waves_of(*out, n_var) > 1 &&
+      2.0 * (item_clocks(*out, k_steps, n_steps, n_var, f32) + 200.0) < 4000.0 * ((out->MB * out->BN / 64 + 1) / 2)) {
+    DirectPlan q = *out;
+    if (ring_depths(q, p.max_taps, 227 * 1024 - FIXED_BYTES - SET_BYTES)) { *out = q; out->epi_sets = 2; }
+  }
+  out->smem = FIXED_BYTES + (out->epi_sets - 1) * SET_BYTES + out->n_a * out->a_bytes + out->n_b * out->b_bytes;
   return true;
 }
 
@@ -1158,17 +1179,17 @@ cudaError_t launch_direct_filter_transform(const DirectDesc &d, const DirectPlan
   return cudaGetLastError();
 }
 
-template <typename T, int BN, int MB, bool PAIR, bool FOLD = false>
+template <typename T, int BN, int MB, bool PAIR, bool FOLD = false, int SETS = 1>
 static cudaError_t launch_one(const DirectPlan &p, const CUtensorMap &mx, const CUtensorMap &mu, const MapSet &my, const void *x, void *y,
                               const void *bias, const DGeom &g, const DSmem &sl, uint32_t idesc, int sms, cudaStream_t s) {
-  auto kern = direct_kernel<T, BN, MB, PAIR, FOLD>;
+  auto kern = direct_kernel<T, BN, MB, PAIR, FOLD, SETS>;
   static std::mutex mu_;
   static std::map<int, int> pairs_of;     // device -> resident CTA pairs (0: attribute set, not asked)
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
-  cfg.blockDim = dim3(std::is_same<T, float>::value || FOLD ? 512 : 384, 1, 1);
+  cfg.blockDim = dim3(threads_of(std::is_same<T, float>::value || FOLD, SETS), 1, 1);
   cfg.dynamicSmemBytes = (size_t)p.smem;
   cfg.stream = s;
   cudaLaunchAttribute attr[2];
@@ -1328,7 +1349,7 @@ cudaError_t launch_direct_forward(const DirectDesc &d, const DirectPlan &p, cons
   sl.slab_bytes = p.slab_bytes; sl.a_bytes = p.a_bytes; sl.lo_off = p.lo_off;
   sl.b_tile = p.b_tile; sl.b_lo = p.b_lo; sl.b_bytes = p.b_bytes; sl.n_a = p.n_a; sl.n_b = p.n_b;
   sl.off_b = p.n_a * p.a_bytes; sl.off_stage = sl.off_b + p.n_b * p.b_bytes;
-  sl.off_raw = sl.off_stage + EPI_WARPS * STAGE_BYTES;
+  sl.off_raw = sl.off_stage + p.epi_sets * EPI_WARPS * STAGE_BYTES;
   sl.raw_bytes = (p.raw_box + 127) / 128 * 128;
   if (d.fold) sl.slab_bytes = p.raw_box;       // what TMA delivers
   sl.off_bars = sl.off_raw + (int)RAW_BUFS * sl.raw_bytes; sl.total = p.smem;
@@ -1337,7 +1358,9 @@ cudaError_t launch_direct_forward(const DirectDesc &d, const DirectPlan &p, cons
   const uint32_t fmt = f32 ? 2u : d.dtype == WINOCONV_F16 ? 0u : 1u;
   const uint32_t m_rows = p.pair ? 2u * BM : (uint32_t)BM;
   const uint32_t idesc = (1u << 4) | (fmt << 7) | (fmt << 10) | ((uint32_t)(p.BN >> 3) << 17) | ((m_rows >> 4) << 24);
-#define WINO_GO(T, BN_, MB_, P_) return launch_one<T, BN_, MB_, P_>(p, mx, mu, my, x, y, bias, g, sl, idesc, sms, s)
+#define WINO_GO(T, BN_, MB_, P_)                                                                                              \
+  return p.epi_sets == 2 ? launch_one<T, BN_, MB_, P_, false, 2>(p, mx, mu, my, x, y, bias, g, sl, idesc, sms, s)              \
+                         : launch_one<T, BN_, MB_, P_>(p, mx, mu, my, x, y, bias, g, sl, idesc, sms, s)
 #define WINO_FOLD(T, MB_) return launch_one<T, 64, MB_, false, true>(p, mx, mu, my, x, y, bias, g, sl, idesc, sms, s)
 #define WINO_PICK(T)                                                             \
   do {                                                                           \
@@ -1353,7 +1376,7 @@ cudaError_t launch_direct_forward(const DirectDesc &d, const DirectPlan &p, cons
   } while (0)
   if (d.dtype == WINOCONV_F16) WINO_PICK(__half);
   if (d.dtype == WINOCONV_BF16) WINO_PICK(__nv_bfloat16);
-  WINO_GO(float, 64, 1, false);
+  return launch_one<float, 64, 1, false>(p, mx, mu, my, x, y, bias, g, sl, idesc, sms, s);
 #undef WINO_PICK
 #undef WINO_FOLD
 #undef WINO_GO

@@ -113,6 +113,7 @@ bool direct_grad_desc(DirectDesc *q, int dtype, int N, int C, int K, int Km, con
                       const int pad[3], const int out[3], int weight_layout, int e, bool *zero_fill);
 struct DirectPlan {
   int BN, MB, pair, split;           // columns and row blocks of an item, CTA pairs, CTAs that share an item's reduction
+  int epi_sets;                      // sets of eight epilogue warps
   int TN, TH, TI, PW, slab_rows_h;   // a block's image groups and output rows, images within a group of 8 rows, pixels of a slab row, slab rows
   int ch_el, rb, n_chunks, k_full, k_tail;
   int taps[4], tap0[4], max_taps, n_taps, units;
