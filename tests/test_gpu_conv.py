@@ -7,7 +7,7 @@ import pytest
 import torch
 
 from oracle import winograd_oracle as wo
-from pytorch_winoconv_b200 import capi, engine
+from pytorch_winoconv_b200 import capi, conv, engine
 from tests.gpu_util import TOL, check_against_oracle, run_engine, seeded
 
 pytestmark = pytest.mark.gpu
@@ -440,3 +440,71 @@ def _run_direct(x, w, pad, tile_m=1):
     torch.cuda.synchronize()
     assert capi.read_device_error() == 0
     return y.permute(0, nd + 1, *range(1, nd + 1)).cpu()
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("n,c,k,sp,ks,stride,options", [
+    (8, 16, 64, (113, 112), 1, 1, {}),                      # many items of one K step: two sets of epilogue warps, an odd number of items
+    (3, 8, 40, (201, 67), 3, 1, {}),                        # a partial channel block
+    (5, 64, 60, (97, 59), 1, 1, {}),                        # rows of y that TMA cannot address
+    (4, 64, 256, (56, 58), 1, 1, {"activation": "relu"}),   # several channel blocks an item, CTA pairs
+    (6, 64, 64, (96, 90), 3, 1, {"activation": "relu", "pool": 2}),
+    (3, 32, 64, (90, 121), 3, 2, {}),
+    (1, 64, 64, (7, 7), 3, 1, {}),                          # fewer items than SMs: one cluster shares an item's reduction
+    (3, 3, 64, (120, 136), 7, 2, {"activation": "relu"}),   # taps along W folded into the channels, patches loaded by TMA
+    (3, 3, 64, (97, 131), 3, 1, {}),                        # the same, patches with plain loads
+    (7, 1, 24, (75, 90), 5, 1, {}),
+    (2, 24, 72, (5, 37, 41), 3, 1, {}),
+])
+def test_direct_taps_16_bit(n, c, k, sp, ks, stride, options, dtype):
+    nd = len(sp)
+    x, w = _rand(n, c, k, sp, ks, dtype)
+    b = torch.linspace(-1, 1, k)
+    layer = (conv.Conv2d if nd == 2 else conv.Conv3d)(c, k, ks, stride=stride, padding=ks // 2, device="cuda", compute_dtype=dtype, **options).eval()
+    with torch.no_grad():
+        layer.weight.copy_(w.float())
+        layer.bias.copy_(b)
+    f = torch.nn.functional
+    o = (f.conv2d if nd == 2 else f.conv3d)(x.double(), w.double(), b.double(), stride=stride, padding=ks // 2)
+    if "pool" in options:
+        o = f.max_pool2d(o, 2)
+    if "activation" in options:
+        o = o.relu()
+    # one rounding of an fp32 sum to the result's type: half a unit of its last place, in every element and so in the 2-norm
+    tol = (2.0 ** -11 if dtype == torch.float16 else 2.0 ** -8) * 1.02
+    for channels_last in (True, False):
+        xg = x.cuda()
+        if channels_last:
+            xg = xg.contiguous(memory_format=torch.channels_last if nd == 2 else torch.channels_last_3d)
+        with torch.no_grad():
+            y = layer(xg).double().cpu()
+        assert capi.read_device_error() == 0
+        assert y.shape == o.shape
+        assert float((y - o).norm() / o.norm()) < tol
+
+
+@pytest.mark.parametrize("n,c,k,sp,ks,stride", [
+    (2, 24, 40, (13, 19), 3, 1), (3, 64, 136, (9, 9), 3, 2), (1, 8, 8, (30, 31), 5, 1), (2, 72, 64, (7, 8), 1, 2),
+    (5, 128, 64, (28, 28), 3, 1), (2, 16, 24, (4, 9, 11), 3, 1), (1, 16, 32, (5, 8, 9), 3, 2),
+])
+def test_gradients_16_bit(n, c, k, sp, ks, stride):
+    nd = len(sp)
+    x, w = _rand(n, c, k, sp, ks, torch.float16)
+    layer = (conv.Conv2d if nd == 2 else conv.Conv3d)(c, k, ks, stride=stride, padding=ks // 2, device="cuda", compute_dtype=torch.float16)
+    with torch.no_grad():
+        layer.weight.copy_(w.float())
+        layer.bias.zero_()
+    fmt = torch.channels_last if nd == 2 else torch.channels_last_3d
+    xg = x.cuda().contiguous(memory_format=fmt).requires_grad_(True)
+    y = layer(xg)
+    gy = torch.randn(y.shape, generator=torch.Generator().manual_seed(7)).half()
+    y.backward(gy.cuda().contiguous(memory_format=fmt))
+    assert capi.read_device_error() == 0
+    xd, wd, bd = x.double().requires_grad_(True), w.double().requires_grad_(True), torch.zeros(k).double().requires_grad_(True)
+    f = torch.nn.functional
+    (f.conv2d if nd == 2 else f.conv3d)(xd, wd, bd, stride=stride, padding=ks // 2).backward(gy.double())
+    rel = lambda a, o: float((a.double().cpu() - o).norm() / o.norm())
+    assert rel(xg.grad, xd.grad) < 2.0 ** -11 * 1.02            # rounded to the type of x once
+    # fp32 sums of at most a few thousand exact products, cut off after every MMA: 2**-23 of the running sum each, far below 1e-5
+    assert rel(layer.weight.grad, wd.grad) < 1e-5
+    assert rel(layer.bias.grad, bd.grad) < 1e-6                 # plain fp32 sums
