@@ -346,7 +346,9 @@ def describe_algorithms(layers):
     out = []
     for c in layers:
         a = int(c.info.algo)
-        if a in text:
+        if getattr(c.info, "direct", 0):
+            d = "direct taps, one fused tcgen05 kernel per layer"
+        elif a in text:
             d = text[a]
         else:
             m = max(int(v) for v in c.info.tile_m)
@@ -753,7 +755,8 @@ def run_ours(args):
         cinfo, cname = contract_info(conv)
         t_ms = sum(st)
         mma_peak, mma_bound = product_peak(conv)
-        t_tc = info.gemm_flops / (mma_peak * 1e12) * 1e3
+        gemm_flops = info.direct_flops if info.direct else info.gemm_flops      # multiply-adds x 2 of what ran
+        t_tc = gemm_flops / (mma_peak * 1e12) * 1e3
         t_hbm = info.algorithmic_bytes / (peaks["hbm_gbs"] * 1e9) * 1e3
         t_tc_c = cinfo.gemm_flops / (mma_peak * 1e12) * 1e3
         # the configuration's compulsory bytes count the convolution's own output (before a fused pool), as its table does
@@ -762,9 +765,9 @@ def run_ours(args):
         t_hbm_c = b_contract / (peaks["hbm_gbs"] * 1e9) * 1e3
         per_layer.append({"layer": li + 1, "c": int(conv.desc.c_in), "k": int(conv.desc.k_out),
                           "hw": int(conv.in_shape[-2]), "ms": round(t_ms, 4), "stage_ms": [round(v, 4) for v in st],
-                          "launches": n_launch, "algo": ALGO_NAMES[int(info.algo)],
+                          "launches": n_launch, "algo": "direct" if info.direct else ALGO_NAMES[int(info.algo)],
                           "eff_tflops": round(info.direct_flops / (t_ms * 1e-3) / 1e12, 2),
-                          "gemm_tflops": round(info.gemm_flops / (st[1] * 1e-3) / 1e12, 2),
+                          "gemm_tflops": round(gemm_flops / (st[1] * 1e-3) / 1e12, 2),
                           "roof_ms": round(max(t_tc, t_hbm), 4), "roof_bound": mma_bound if t_tc >= t_hbm else "hbm",
                           "roof_frac": round(max(t_tc, t_hbm) / t_ms, 4),
                           "contract": cname, "roof_ms_contract": round(max(t_tc_c, t_hbm_c), 5),
@@ -773,7 +776,7 @@ def run_ours(args):
         h = out
     stage_tot = [sum(l["stage_ms"][i] for l in per_layer) for i in range(3)]
     # Time per kernel class over the step (a stack may mix algorithms: AUTO takes staged F(4x4,3x3) for some layers and
-    # the row-piece kernel for the rest): the dominant class is the one the roofline object describes.
+    # the direct-tap kernel for the rest): the dominant class is the one the roofline object describes.
     esz = x_host.element_size()
     classes = {}      # kernel -> [ms, launches, algorithmic flops, algorithmic bytes]
 
@@ -783,7 +786,9 @@ def run_ours(args):
 
     for l, conv in zip(per_layer, layers):
         a = int(conv.info.algo)
-        if a == capi.ALGO_ROW:
+        if conv.info.direct:
+            add("direct_kernel", l["stage_ms"][1], flops=conv.info.direct_flops)
+        elif a == capi.ALGO_ROW:
             add("rowfused_kernel", l["stage_ms"][1], flops=conv.info.gemm_flops)
         elif a == capi.ALGO_FUSED:
             add("fused23_kernel", l["stage_ms"][1], flops=conv.info.gemm_flops)
