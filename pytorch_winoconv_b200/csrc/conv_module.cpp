@@ -71,6 +71,15 @@ at::Tensor turned_channels_last(const at::Tensor &t, at::ScalarType type, void *
   return out;
 }
 
+// The tensor itself where it is of `type` and lies channels last without gaps, else a copy that does.  (Tensor::to would hand a
+// crop, a channel slice or the gradient behind a concatenation back as it is: it looks at the order of the strides only.)
+at::Tensor dense_channels_last(const at::Tensor &t, at::ScalarType type, void *stream) {
+  if (t.scalar_type() == type && lies_channels_last(t)) return t;
+  if (t.is_contiguous() && t.size(1) > 1 && code_of(t.scalar_type()) >= 0 && t.size(0) <= 65535) return turned_channels_last(t, type, stream);
+  at::Tensor out = at::empty(t.sizes(), t.options().dtype(type).requires_grad(false), t.dim() == 4 ? at::MemoryFormat::ChannelsLast : at::MemoryFormat::ChannelsLast3d);
+  return out.copy_(t);
+}
+
 // The tensor itself where it starts on 16 bytes, as TMA and the C ABI want it; else a copy in the same order.
 at::Tensor aligned(const at::Tensor &t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) ? t.clone() : t; }
 
@@ -120,12 +129,6 @@ ConvRunner::ConvRunner(int64_t nd, std::vector<int64_t> stride, std::vector<int6
   TORCH_CHECK((nd == 2 || nd == 3) && (int64_t)stride.size() == nd && (int64_t)padding.size() == nd, "ConvRunner: bad rank");
   for (int i = 0; i < 3; ++i) { stride_[i] = 1; pad_[i] = 0; }
   for (int i = 0; i < nd; ++i) { stride_[3 - nd + i] = (int)stride[i]; pad_[3 - nd + i] = (int)padding[i]; }
-}
-
-at::Tensor ConvRunner::channels_last(const at::Tensor &t, at::ScalarType type) const {
-  if (t.scalar_type() == type && lies_channels_last(t)) return t;
-  if (t.is_contiguous() && t.size(1) > 1 && code_of(t.scalar_type()) >= 0 && t.size(0) <= 65535) return turned_channels_last(t, type, stream_of());
-  return t.to(t.options().dtype(type), false, false, nd_ == 2 ? at::MemoryFormat::ChannelsLast : at::MemoryFormat::ChannelsLast3d);
 }
 
 std::shared_ptr<ConvRunner::Entry> ConvRunner::entry_for(const at::Tensor &x, const at::Tensor &weight, const std::optional<at::Tensor> &bias,
@@ -242,7 +245,7 @@ std::optional<at::Tensor> ConvRunner::forward(const at::Tensor &x, const at::Ten
   if (!e) return std::nullopt;
   if (!grad) {
     at::AutoDispatchBelowADInplaceOrView no_graph;
-    return run(*e, channels_last(x, type_of(dtype)), weight, bias);
+    return run(*e, dense_channels_last(x, type_of(dtype), stream_of()), weight, bias);
   }
   if (!e->back_known) {
     winoconv_backward_info_t info;
@@ -254,7 +257,7 @@ std::optional<at::Tensor> ConvRunner::forward(const at::Tensor &x, const at::Ten
   at::Tensor x_cl;
   {
     at::AutoDispatchBelowADInplaceOrView no_graph;
-    x_cl = channels_last(x, type_of(dtype));
+    x_cl = dense_channels_last(x, type_of(dtype), stream_of());
     if (x_cl.is_same(x)) x_cl = x.detach();
   }
   return ConvFn::apply(c10::intrusive_ptr<ConvRunner>::reclaim_copy(this), x, x_cl, e, weight, bias, relu_);
@@ -271,7 +274,7 @@ std::vector<at::Tensor> ConvRunner::backward(const at::Tensor &gy_in, const at::
   void *s = stream_of();
   at::Tensor gy = gy_in;
   if (y.defined()) gy = gy * (y > 0).to(gy.scalar_type());
-  gy = aligned(channels_last(gy, type));
+  gy = aligned(dense_channels_last(gy, type, s));
   winoconv_desc_t d = e->desc;
   d.epilogue = need_b ? WINOCONV_EPI_BIAS : 0u;
   winoconv_backward_info_t info;
@@ -299,7 +302,7 @@ std::vector<at::Tensor> ConvRunner::backward(const at::Tensor &gy_in, const at::
     if (x_in.scalar_type() != type) gx = gx.to(x_in.scalar_type());
   }
   if (need_w) {
-    const at::Tensor xp = aligned(pad_channels(channels_last(x_in, type), info.c_stride));
+    const at::Tensor xp = aligned(pad_channels(dense_channels_last(x_in, type, s), info.c_stride));
     gw = at::empty(weight.sizes(), weight.options().requires_grad(false));
     if (need_b) gb = at::empty({weight.size(0)}, weight.options().dtype(at::kFloat).requires_grad(false));
     const at::Tensor ws = empty_bytes(info.weight_ws_bytes, w);
@@ -366,10 +369,7 @@ std::optional<at::Tensor> conv_call(const at::Tensor &x_in, const at::Tensor &we
     if (winoconv_plan(&d, &info) != WINOCONV_OK) return std::nullopt;
   }
   void *s = stream_of();
-  at::Tensor x = lies_channels_last(x_in) && x_in.scalar_type() == type ? x_in
-                 : x_in.is_contiguous() && x_in.size(0) <= 65535 ? turned_channels_last(x_in, type, s)
-                 : x_in.to(x_in.options().dtype(type), false, false, nd == 2 ? at::MemoryFormat::ChannelsLast : at::MemoryFormat::ChannelsLast3d);
-  x = aligned(x);
+  at::Tensor x = aligned(dense_channels_last(x_in, type, s));
   at::Tensor w = weight_in.to(x.device()).contiguous();
   at::Tensor u = empty_bytes(info.filter_bytes, x);
   if (winoconv_filter_transform_from(&d, w.data_ptr(), code_of(w.scalar_type()), u.data_ptr(), s) != WINOCONV_OK) {

@@ -67,7 +67,6 @@ class ConvRunner : public torch::CustomClassHolder {
 
  private:
   std::shared_ptr<Entry> entry_for(const at::Tensor &x, const at::Tensor &weight, const std::optional<at::Tensor> &bias, int dtype, bool first);
-  at::Tensor channels_last(const at::Tensor &t, at::ScalarType type) const;
 
   int nd_, stride_[3], pad_[3], tile_m_, algo_, compute_;
   bool relu_, pool_;

@@ -234,3 +234,100 @@ def test_bias_gradient_is_an_fp32_sum(k):
     m(torch.randn(16, 16, 33, 35, device="cuda").half()).backward(gy)
     exact = gy.double().sum((0, 2, 3))
     assert float((m.bias.grad.double() - exact).norm() / exact.norm()) < 4e-7
+
+
+_VIEWS = {      # what a network hands on: channels last in the order of the strides, but with gaps
+    "crop": lambda b: b[:, :, 1:-1, 1:-1], "crop3d": lambda b: b[..., 2:, 1:-1], "channel slice": lambda b: b[:, 16:32],
+    "chunk": lambda b: b.chunk(2, 1)[1], "space by two": lambda b: b[:, :, ::2, ::2], "batch by two": lambda b: b[::2],
+}
+
+
+def _gappy(nd, dtype, view, requires_grad=False):
+    fmt = torch.channels_last if nd == 2 else torch.channels_last_3d
+    base = torch.randn((4, 48, 13, 18) if nd == 2 else (4, 48, 6, 9, 12), device="cuda").to(dtype).to(memory_format=fmt)
+    x = _VIEWS[view](base.requires_grad_(requires_grad))
+    assert not x.is_contiguous() and not x.is_contiguous(memory_format=fmt)
+    return base, x
+
+
+def _rel(a, o):
+    return float((a.detach().cpu().double() - o.detach()).norm() / o.detach().norm())
+
+
+# one rounding of a result is half a unit of its last place, in the 2-norm too; fp32: sums of some hundred products
+_ONE_ROUNDING = {torch.float16: 2.0 ** -11 * 1.02, torch.float32: 1e-5}
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nd", [2, 3])
+@pytest.mark.parametrize("dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("view", _VIEWS)
+def test_tensors_with_gaps_through_the_modules(nd, dtype, view):
+    torch.manual_seed(31)
+    base, x = _gappy(nd, dtype, view, requires_grad=True)
+    layer = (wconv.Conv2d if nd == 2 else wconv.Conv3d)(x.shape[1], 24, 3, padding=1, bias=False, compute_dtype=None).cuda()
+    with torch.no_grad():
+        layer.weight.copy_(layer.weight.to(dtype))
+        y = layer(x)
+    f = torch.nn.functional.conv2d if nd == 2 else torch.nn.functional.conv3d
+    bd = base.detach().cpu().double().requires_grad_(True)
+    wd = layer.weight.detach().cpu().double().requires_grad_(True)
+    o = f(_VIEWS[view](bd), wd, None, 1, 1)
+    assert _rel(y, o) < _ONE_ROUNDING[dtype]
+    gy = torch.randn_like(o).to(dtype)
+    layer(x).backward(gy.cuda())
+    o.backward(gy.double())
+    assert _rel(base.grad, bd.grad) < _ONE_ROUNDING[dtype]
+    # 16 bits: shares of the pixels, summed in fp32.  fp32: one chain of three products per 8 pixels, the accumulator cut off
+    # after each, by 2**-23 of the running sum at most
+    pixels = gy.numel() // gy.shape[1]
+    assert _rel(layer.weight.grad, wd.grad) < (1e-5 if dtype == torch.float16 else 3 * (pixels / 8) * 2.0 ** -23)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nd", [2, 3])
+@pytest.mark.parametrize("view", _VIEWS)
+def test_gradients_with_gaps(nd, view):
+    torch.manual_seed(32)
+    _, gy = _gappy(nd, torch.float16, view)
+    fmt = torch.channels_last if nd == 2 else torch.channels_last_3d
+    x = torch.randn(gy.shape[0], 16, *gy.shape[2:], device="cuda").half().to(memory_format=fmt).requires_grad_(True)
+    layer = (wconv.Conv2d if nd == 2 else wconv.Conv3d)(16, gy.shape[1], 3, padding=1).cuda()
+    with torch.no_grad():
+        layer.weight.copy_(layer.weight.half())
+    layer(x).backward(gy)
+    gx, gw, gb = _grads_f64(x.detach().cpu(), layer.weight.detach().cpu(), layer.bias.detach().cpu(), gy.cpu(), 1, 1, False)
+    assert _rel(x.grad, gx) < _ONE_ROUNDING[torch.float16]
+    assert _rel(layer.weight.grad, gw) < 1e-5 and _rel(layer.bias.grad, gb) < 1e-5
+
+
+@pytest.mark.gpu
+def test_gradients_behind_a_concatenation():
+    torch.manual_seed(33)
+    a, b = wconv.Conv2d(16, 8, 3, padding=1).cuda(), wconv.Conv2d(16, 24, 5, padding=2).cuda()
+    x = torch.randn(2, 16, 11, 12, device="cuda").half().to(memory_format=torch.channels_last).requires_grad_(True)
+    gy = torch.randn(2, 32, 11, 12, device="cuda").half().to(memory_format=torch.channels_last)
+    torch.cat([a(x), b(x)], 1).backward(gy)
+    xd = x.detach().cpu().double().requires_grad_(True)
+    wd = [m.weight.detach().cpu().half().double().requires_grad_(True) for m in (a, b)]
+    f = torch.nn.functional.conv2d
+    torch.cat([f(xd, wd[0], None, 1, 1), f(xd, wd[1], None, 1, 2)], 1).backward(gy.cpu().double())
+    # grad_x: two rounded results and their rounded sum
+    assert _rel(x.grad, xd.grad) < 3 * _ONE_ROUNDING[torch.float16]
+    assert _rel(a.weight.grad, wd[0].grad) < 1e-5 and _rel(b.weight.grad, wd[1].grad) < 1e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("nd", [2, 3])
+@pytest.mark.parametrize("view", _VIEWS)
+def test_tensors_with_gaps_through_the_functional_operators(nd, view):
+    from pytorch_winoconv_b200 import dwm, matrix_conv, matrix_conv3d
+    torch.manual_seed(34)
+    f = torch.nn.functional.conv2d if nd == 2 else torch.nn.functional.conv3d
+    ops = matrix_conv if nd == 2 else matrix_conv3d
+    for op, dtype in ((dwm.dwm2d if nd == 2 else dwm.dwm3d, torch.float32), (dwm.dwm2d if nd == 2 else dwm.dwm3d, torch.float16),
+                      (ops.conv32, torch.float32), (ops.conv16, torch.float16)):
+        _, x = _gappy(nd, dtype, view)
+        w = (torch.randn(24, x.shape[1], *[3] * nd, device="cuda") * 0.1).to(dtype)
+        y = op(x, w, padding=(1,) * nd)
+        assert _rel(y, f(x.cpu().double(), w.cpu().double(), None, 1, 1)) < _ONE_ROUNDING[dtype], op
