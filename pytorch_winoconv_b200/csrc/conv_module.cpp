@@ -135,11 +135,14 @@ std::shared_ptr<ConvRunner::Entry> ConvRunner::entry_for(const at::Tensor &x, co
                                                          int dtype, bool first) {
   int64_t shape[5] = {x.size(0), 1, 1, 1, x.size(1)};
   for (int i = 0; i < nd_; ++i) shape[4 - nd_ + i] = x.size(2 + i);
+  int64_t w_shape[4] = {weight.size(0), 1, 1, 1};
+  for (int i = 0; i < nd_; ++i) w_shape[4 - nd_ + i] = weight.size(2 + i);
   const int device = x.get_device(), bias_type = bias ? (int)bias->scalar_type() : -1;
   std::lock_guard<std::mutex> lock(mu_);
   for (size_t i = entries_.size(); i-- > 0;) {
     Entry &e = *entries_[i];
-    if (e.dtype == dtype && e.device == device && e.bias_type == bias_type && e.first == first && std::memcmp(e.shape, shape, sizeof shape) == 0) {
+    if (e.dtype == dtype && e.device == device && e.bias_type == bias_type && e.first == first && std::memcmp(e.shape, shape, sizeof shape) == 0 &&
+        std::memcmp(e.w_shape, w_shape, sizeof w_shape) == 0) {
       auto hit = entries_[i];
       if (i + 1 != entries_.size()) {
         entries_.erase(entries_.begin() + i);
@@ -150,6 +153,7 @@ std::shared_ptr<ConvRunner::Entry> ConvRunner::entry_for(const at::Tensor &x, co
   }
   auto e = std::make_shared<Entry>();
   std::memcpy(e->shape, shape, sizeof shape);
+  std::memcpy(e->w_shape, w_shape, sizeof w_shape);
   e->dtype = dtype;
   e->device = device;
   e->bias_type = bias_type;
@@ -157,12 +161,12 @@ std::shared_ptr<ConvRunner::Entry> ConvRunner::entry_for(const at::Tensor &x, co
   winoconv_desc_t &d = e->desc;
   std::memset(&d, 0, sizeof d);
   d.ndim = nd_;
-  for (int64_t s : {shape[0], shape[1], shape[2], shape[3], shape[4], weight.size(0)})
+  for (int64_t s : {shape[0], shape[1], shape[2], shape[3], shape[4], w_shape[0], w_shape[1], w_shape[2], w_shape[3]})
     if (s <= 0 || s > 0x7fffffffLL) return nullptr;
-  d.batch = (int)shape[0]; d.c_in = (int)shape[4]; d.k_out = (int)weight.size(0);
+  d.batch = (int)shape[0]; d.c_in = (int)shape[4]; d.k_out = (int)w_shape[0];
   for (int i = 0; i < 3; ++i) {
     d.in_size[i] = (int)shape[1 + i];
-    d.ker_size[i] = i < 3 - nd_ ? 1 : (int)weight.size(2 + i - (3 - nd_));
+    d.ker_size[i] = (int)w_shape[1 + i];
     d.stride[i] = stride_[i];
     d.pad[i] = pad_[i];
   }
@@ -223,7 +227,8 @@ at::Tensor ConvRunner::run(Entry &e, const at::Tensor &x, const at::Tensor &weig
 
 std::optional<at::Tensor> ConvRunner::forward(const at::Tensor &x, const at::Tensor &weight, const std::optional<at::Tensor> &bias, bool training) {
   if (!x.is_cuda() || x.dim() != nd_ + 2 || weight.dim() != nd_ + 2 || !weight.is_cuda() || weight.get_device() != x.get_device() ||
-      x.size(1) != weight.size(1) || x.numel() == 0 || (bias && !bias->is_cuda()) || code_of(weight.scalar_type()) < 0)
+      x.size(1) != weight.size(1) || x.numel() == 0 || code_of(weight.scalar_type()) < 0 ||
+      (bias && (!bias->is_cuda() || bias->get_device() != x.get_device() || bias->numel() != weight.size(0))))
     return std::nullopt;
   if (weight.is_inference() || (bias && bias->is_inference())) return std::nullopt;      // no version to tell a new value by
   const int dtype = compute_ >= 0 ? compute_ : code_of(x.scalar_type());

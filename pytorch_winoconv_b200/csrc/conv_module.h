@@ -20,8 +20,8 @@
 std::optional<at::Tensor> conv_call(const at::Tensor &x, const at::Tensor &weight, const std::optional<at::Tensor> &bias,
                                     std::vector<int64_t> stride, std::vector<int64_t> padding, int64_t compute, bool out_f32, int64_t tile_m);
 
-// One per module.  Every entry is the plan of an input shape with its transformed filters; they follow the weights (storage,
-// version, dtype), and the least recently used one goes when there are more than `max_plans`.
+// One per module.  Every entry is the plan of an input and a weight shape with its transformed filters; they follow the weights
+// (storage, version, dtype), and the least recently used one goes when there are more than `max_plans`.
 class ConvRunner : public torch::CustomClassHolder {
  public:
   ConvRunner(int64_t nd, std::vector<int64_t> stride, std::vector<int64_t> padding, int64_t tile_m, int64_t algo, bool relu, bool pool,
@@ -48,6 +48,7 @@ class ConvRunner : public torch::CustomClassHolder {
   };
   struct Entry {
     int64_t shape[5] = {0, 0, 0, 0, 0};      // N, D, H, W, C of the input
+    int64_t w_shape[4] = {0, 0, 0, 0};       // K, kD, kH, kW of the weight: a module's weight may be replaced by one of another shape
     int dtype = -1, device = -1, bias_type = -1;   // bias_type: scalar type of the bias, -1 without one
     winoconv_desc_t desc;
     winoconv_plan_info_t info;

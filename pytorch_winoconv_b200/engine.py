@@ -102,6 +102,8 @@ class WinoConv:
         k, c = int(weight.shape[0]), int(weight.shape[1])
         if self.in_shape[-1] != c:
             raise ValueError(f"input has {self.in_shape[-1]} channels, weight expects {c}")
+        if bias is not None and bias.numel() != k:
+            raise ValueError(f"bias has {bias.numel()} values, weight {k} output channels")
         epi = (capi.EPI_BIAS if bias is not None else 0) | (capi.EPI_RELU if relu else 0) | (capi.EPI_POOL2 if pool2 else 0)
         pdt = capi.F32 if product_dtype is None else dtype_code(product_dtype)
         self.desc = capi.make_desc(ndim=nd, batch=self.in_shape[0], c_in=c, k_out=k, in_size=self.in_shape[1:-1],

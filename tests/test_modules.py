@@ -331,3 +331,42 @@ def test_tensors_with_gaps_through_the_functional_operators(nd, view):
         w = (torch.randn(24, x.shape[1], *[3] * nd, device="cuda") * 0.1).to(dtype)
         y = op(x, w, padding=(1,) * nd)
         assert _rel(y, f(x.cpu().double(), w.cpu().double(), None, 1, 1)) < _ONE_ROUNDING[dtype], op
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("new", [(8, 16, 3, 3), (72, 16, 3, 3), (24, 16, 5, 5), (24, 16, 1, 1), (40, 16, 2, 3)])
+@pytest.mark.parametrize("bias", [False, True])
+def test_a_weight_of_another_shape_gets_a_plan_of_its_own(new, bias):
+    torch.manual_seed(35)
+    m = wconv.Conv2d(16, 24, 3, padding=0, bias=bias).cuda()
+    x = torch.randn(2, 16, 13, 14, device="cuda").half().to(memory_format=torch.channels_last)
+    with torch.no_grad():
+        m(x)
+    m(x.clone().requires_grad_(True)).sum().backward()
+    first = m.weight.detach().clone()
+    for shape in (new, tuple(first.shape)):              # and back again
+        m.weight = torch.nn.Parameter((torch.randn(shape, device="cuda") * 0.1).half().float())
+        if bias:
+            m.bias = torch.nn.Parameter(torch.randn(shape[0], device="cuda"))
+        with torch.no_grad():
+            y = m(x)
+        o = _by_torch(m, x)
+        assert y.shape == o.shape and _rel(y, o) < _ONE_ROUNDING[torch.float16]
+        xg = x.clone().requires_grad_(True)
+        gy = torch.randn(o.shape, device="cuda").half()
+        m(xg).backward(gy)
+        gx, gw, gb = (*_grads_f64(x.cpu(), m.weight.detach().cpu(), m.bias.detach().cpu() if bias else None, gy.cpu(), 1, 0, False), None)[:3]
+        assert _rel(xg.grad, gx) < _ONE_ROUNDING[torch.float16] and _rel(m.weight.grad, gw) < 1e-5
+        assert not bias or _rel(m.bias.grad, gb) < 1e-5
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("length", [8, 48])
+def test_a_bias_of_another_length_is_refused(length):
+    m = wconv.Conv2d(16, 24, 3, padding=1).cuda().eval()
+    x = torch.randn(1, 16, 8, 8, device="cuda").half()
+    with torch.no_grad():
+        m(x)
+        m.bias = torch.nn.Parameter(torch.zeros(length, device="cuda"))
+        with pytest.raises(ValueError, match="bias"):
+            m(x)
