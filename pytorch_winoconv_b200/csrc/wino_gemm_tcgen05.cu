@@ -635,11 +635,7 @@ __global__ void __launch_bounds__(YT_THREADS, 1) output_f43_tma_kernel(const __g
 #pragma unroll
         for (int cidx = 0; cidx < 4; ++cidx) Xf<4, 3>::template at2<4, 4>(&t1[cidx], &o[cidx]);   // along H
         uint64_t bv = f2_pack(0.f, 0.f);
-        if (has_bias) {
-          float bf[2];
-          VecIO<T, 2>::load(bias + k, bf);
-          bv = f2_pack(bf[0], bf[1]);
-        }
+        if (has_bias) bv = f2_pack(Elem<T>::load(bias + k), Elem<T>::load(bias + k + 1));      // a bias may start anywhere
         const unsigned t32 = (unsigned)tile;
         const unsigned tw = t32 % (unsigned)g.nW, r2 = t32 / (unsigned)g.nW;
         const unsigned th = r2 % (unsigned)g.nH, n = r2 / (unsigned)g.nH;

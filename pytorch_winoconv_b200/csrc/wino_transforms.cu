@@ -322,8 +322,7 @@ __global__ void __launch_bounds__(256) output_transform_kernel(const TM *__restr
   }
   float bv[VEC];
 #pragma unroll
-  for (int l = 0; l < VEC; ++l) bv[l] = 0.f;
-  if (g.epilogue & WINOCONV_EPI_BIAS) VecIO<T, VEC>::load(bias + k0, bv);
+  for (int l = 0; l < VEC; ++l) bv[l] = (g.epilogue & WINOCONV_EPI_BIAS) ? Elem<T>::load(bias + k0 + l) : 0.f;      // a bias may start anywhere
   const bool relu = (g.epilogue & WINOCONV_EPI_RELU) != 0;
   const TileCoord tc = decode_tile(g, t0 + row);
   if (g.epilogue & WINOCONV_EPI_POOL2) {

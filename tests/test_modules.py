@@ -370,3 +370,33 @@ def test_a_bias_of_another_length_is_refused(length):
         m.bias = torch.nn.Parameter(torch.zeros(length, device="cuda"))
         with pytest.raises(ValueError, match="bias"):
             m(x)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("c,k", [(16, 24), (136, 136)])          # fp32: direct taps, and F(2,3) / F(4x4,3x3) with an output transform
+def test_a_bias_that_starts_anywhere(c, k):
+    from pytorch_winoconv_b200 import dwm, engine, matrix_conv
+    torch.manual_seed(36)
+    whole = torch.randn(3 * k + 3, device="cuda")                # the biases of three layers in one buffer
+    f = torch.nn.functional
+    w = torch.randn(k, c, 3, 3, device="cuda") * 0.1
+    x = torch.randn(2, c, 12, 12, device="cuda")
+    ref = f.conv2d(x.cpu().double(), w.cpu().double(), None, 1, 1)
+    for start in (1, 2, 3):
+        b = whole[start:start + k]
+        o = ref + b.cpu().double().view(1, -1, 1, 1)
+        for y in (dwm.dwm2d(x, w, b, padding=1), matrix_conv.conv32(x, w, b, padding=1), matrix_conv.conv32(x, w, b, padding=1, output_block=4)):
+            assert _rel(y, o) < _ONE_ROUNDING[torch.float32]
+        m = wconv.Conv2d(c, k, 3, padding=1, compute_dtype=None).cuda().eval()
+        with torch.no_grad():
+            m.weight.copy_(w)
+            m.bias = torch.nn.Parameter(b)
+            assert m.bias.data_ptr() == b.data_ptr()
+            assert _rel(m(x), o) < _ONE_ROUNDING[torch.float32]
+            m.compute_dtype = torch.float16                      # an fp32 bias read as it is
+            assert _rel(m(x), f.conv2d(x.cpu().half().double(), w.cpu().half().double(), b.cpu().double(), 1, 1)) < _ONE_ROUNDING[torch.float16]
+        x16, w16, b16 = x.half().permute(0, 2, 3, 1).contiguous(), w.half(), whole.half()[start:start + k]
+        o16 = f.conv2d(x.cpu().half().double(), w16.cpu().double(), b16.cpu().double(), 1, 1)
+        for tile_m in (0, 2, 4):
+            y = engine.WinoConv(x16.shape, w16, padding=1, bias=b16, tile_m=tile_m)(x16)
+            assert wo.error_metrics(y.permute(0, 3, 1, 2).cpu(), o16)["E_B"] < 2e-2
