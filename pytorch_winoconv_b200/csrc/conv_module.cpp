@@ -252,13 +252,7 @@ std::optional<at::Tensor> ConvRunner::forward(const at::Tensor &x, const at::Ten
     at::AutoDispatchBelowADInplaceOrView no_graph;
     return run(*e, dense_channels_last(x, type_of(dtype), stream_of()), weight, bias);
   }
-  if (!e->back_known) {
-    winoconv_backward_info_t info;
-    e->back_ok = winoconv_backward_plan(&e->desc, &info) == WINOCONV_OK && info.data_ok && info.weight_ok;
-    for (int i = 0; i < 3; ++i) e->back_ok = e->back_ok && pad_[i] < e->desc.ker_size[i];      // the Python path refuses the data gradient
-    e->back_known = true;
-  }
-  if (!e->back_ok) return std::nullopt;
+  if (!backward_covered(*e)) return std::nullopt;
   at::Tensor x_cl;
   {
     at::AutoDispatchBelowADInplaceOrView no_graph;
@@ -266,6 +260,18 @@ std::optional<at::Tensor> ConvRunner::forward(const at::Tensor &x, const at::Ten
     if (x_cl.is_same(x)) x_cl = x.detach();
   }
   return ConvFn::apply(c10::intrusive_ptr<ConvRunner>::reclaim_copy(this), x, x_cl, e, weight, bias, relu_);
+}
+
+bool ConvRunner::backward_covered(Entry &e) {
+  std::lock_guard<std::mutex> lock(mu_);
+  if (!e.back_known) {
+    winoconv_backward_info_t info;
+    bool ok = winoconv_backward_plan(&e.desc, &info) == WINOCONV_OK && info.data_ok && info.weight_ok;
+    for (int i = 0; i < 3; ++i) ok = ok && pad_[i] < e.desc.ker_size[i];      // the Python path refuses the data gradient
+    e.back_ok = ok;
+    e.back_known = true;
+  }
+  return e.back_ok;
 }
 
 std::vector<at::Tensor> ConvRunner::backward(const at::Tensor &gy_in, const at::Tensor &x_in, const at::Tensor &y, const at::Tensor &weight,

@@ -68,6 +68,7 @@ class ConvRunner : public torch::CustomClassHolder {
 
  private:
   std::shared_ptr<Entry> entry_for(const at::Tensor &x, const at::Tensor &weight, const std::optional<at::Tensor> &bias, int dtype, bool first);
+  bool backward_covered(Entry &e);      // whether the native gradients take the layer
 
   int nd_, stride_[3], pad_[3], tile_m_, algo_, compute_;
   bool relu_, pool_;

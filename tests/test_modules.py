@@ -400,3 +400,23 @@ def test_a_bias_that_starts_anywhere(c, k):
         for tile_m in (0, 2, 4):
             y = engine.WinoConv(x16.shape, w16, padding=1, bias=b16, tile_m=tile_m)(x16)
             assert wo.error_metrics(y.permute(0, 3, 1, 2).cpu(), o16)["E_B"] < 2e-2
+
+
+@pytest.mark.gpu
+def test_threads_agree_on_what_the_gradients_cover():
+    # every thread's first call of a layer whose data gradient is refused (padding beyond kernel - 1)
+    import threading
+    x = torch.randn(1, 8, 6, 6, device="cuda").half()
+    names, n_threads = [], 8
+    for _ in range(100):
+        m = wconv.Conv2d(8, 8, 1, padding=1).cuda()
+        start = threading.Barrier(n_threads)
+
+        def call():
+            start.wait()
+            names.append(type(m(x).grad_fn).__name__)
+
+        threads = [threading.Thread(target=call) for _ in range(n_threads)]
+        [t.start() for t in threads]
+        [t.join() for t in threads]
+    assert len(names) == 100 * n_threads and set(names) == {"_WinoConvFnBackward"}, set(names)
