@@ -1,6 +1,7 @@
 #include "conv_module.h"
 
 #include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 
 #include <cstring>
@@ -89,6 +90,14 @@ at::Tensor pad_channels(const at::Tensor &t, int64_t c) {
   if (t.size(1) == c) return t;
   at::Tensor cl = t.movedim(1, nd - 1);
   return at::constant_pad_nd(cl, {0, c - t.size(1)}).contiguous().movedim(nd - 1, 1);
+}
+
+// The graph capture the stream takes part in, 0 outside of one.
+unsigned long long capture_of(cudaStream_t stream) {
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  C10_CUDA_CHECK(cudaStreamGetCaptureInfo(stream, &status, &id));
+  return status == cudaStreamCaptureStatusNone ? 0 : id;
 }
 
 struct ConvFn : public torch::autograd::Function<ConvFn> {
@@ -192,9 +201,9 @@ at::Tensor ConvRunner::run(Entry &e, const at::Tensor &x, const at::Tensor &weig
   at::Tensor u, b;
   {
     std::lock_guard<std::mutex> lock(mu_);
-    if (!(e.stamp == now) || !e.u.defined()) {
+    if (!(e.stamp == now) || !e.written.usable_here({e.u, e.bias})) {
       at::AutoDispatchBelowADInplaceOrView guard;
-      // a new buffer, not the old one: launches that read it may still be queued on another stream
+      // a new buffer, not the old one, which launches may still be queued to read (the allocator knows on which streams)
       e.u = empty_bytes(e.info.filter_bytes, weight);
       at::Tensor w = weight.is_contiguous() ? weight : weight.contiguous();
       if (winoconv_filter_transform_from(&e.desc, w.data_ptr(), code_of(w.scalar_type()), e.u.data_ptr(), s) != WINOCONV_OK) {
@@ -202,6 +211,7 @@ at::Tensor ConvRunner::run(Entry &e, const at::Tensor &x, const at::Tensor &weig
         check_abi(winoconv_filter_transform(&e.desc, w.data_ptr(), e.u.data_ptr(), s), "winoconv_filter_transform");
       }
       e.bias = bias ? bias->detach().to(e.desc.bias_f32 ? at::kFloat : type).contiguous() : at::Tensor();
+      e.written.here();
       e.stamp = now;
       e.serial = ++serial_;
       newest_ = now;
@@ -262,6 +272,33 @@ std::optional<at::Tensor> ConvRunner::forward(const at::Tensor &x, const at::Ten
   return ConvFn::apply(c10::intrusive_ptr<ConvRunner>::reclaim_copy(this), x, x_cl, e, weight, bias, relu_);
 }
 
+void ConvRunner::Written::here() {
+  stream = at::cuda::getCurrentCUDAStream();
+  capture = capture_of(*stream);
+  finished = false;
+  event.record(*stream);
+}
+
+bool ConvRunner::Written::usable_here(std::initializer_list<at::Tensor> buffers) {
+  const auto now = at::cuda::getCurrentCUDAStream();
+  if (!stream) return false;
+  if (capture == 0 && *stream == now) return true;
+  const unsigned long long current = capture_of(now);
+  if (capture != 0 && capture != current) return false;
+  if (*stream == now) return true;
+  if (capture == 0 && !finished) {
+    c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);      // a query is no part of anyone's capture
+    finished = event.query();
+  }
+  if (!finished) {
+    if (capture != current) return false;
+    event.block(now);
+  }
+  for (const at::Tensor &t : buffers)
+    if (t.defined()) t.record_stream(now);
+  return true;
+}
+
 bool ConvRunner::backward_covered(Entry &e) {
   std::lock_guard<std::mutex> lock(mu_);
   if (!e.back_known) {
@@ -298,12 +335,13 @@ std::vector<at::Tensor> ConvRunner::backward(const at::Tensor &gy_in, const at::
     const Stamp now = stamp_of(weight, std::nullopt);
     {
       std::lock_guard<std::mutex> lock(mu_);
-      if (!(e->back_stamp == now) || !e->u_back.defined()) {
+      if (!(e->back_stamp == now) || !e->back_written.usable_here({e->u_back})) {
         e->u_back = empty_bytes(std::max<uint64_t>(info.data_filter_bytes, 16), w);
         at::Tensor wt = w;
         if (code_of(w.scalar_type()) != WINOCONV_F32 && code_of(w.scalar_type()) != dtype) wt = w.to(type);
         check_abi(winoconv_backward_filter_transform(&d, wt.data_ptr(), code_of(wt.scalar_type()), e->u_back.data_ptr(), s),
                   "winoconv_backward_filter_transform");
+        e->back_written.here();
         e->back_stamp = now;
       }
       u = e->u_back;

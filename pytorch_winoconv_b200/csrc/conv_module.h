@@ -3,12 +3,14 @@
 #pragma once
 
 #include <cstdint>
+#include <initializer_list>
 #include <memory>
 #include <mutex>
 #include <optional>
 #include <string>
 #include <vector>
 
+#include <ATen/cuda/CUDAEvent.h>
 #include <torch/extension.h>
 
 #include "winoconv_b200.h"
@@ -46,6 +48,17 @@ class ConvRunner : public torch::CustomClassHolder {
       return w_ref == o.w_ref && b_ref == o.b_ref && w == o.w && b == o.b && w_version == o.w_version && b_version == o.b_version && w_dtype == o.w_dtype;
     }
   };
+  // Where an entry's buffers were written.  A call on another stream waits for that and tells the allocator that it reads them.
+  // A graph capture cannot wait for work outside of it: it uses them once that work has finished, else it makes its own; and what
+  // a capture writes holds its values only when the graph runs, so nobody outside of that capture uses it.
+  struct Written {
+    std::optional<c10::cuda::CUDAStream> stream;
+    at::cuda::CUDAEvent event;
+    bool finished = false;
+    unsigned long long capture = 0;
+    void here();                                                      // they are written by what is queued on the current stream so far
+    bool usable_here(std::initializer_list<at::Tensor> buffers);      // false: write them anew
+  };
   struct Entry {
     int64_t shape[5] = {0, 0, 0, 0, 0};      // N, D, H, W, C of the input
     int64_t w_shape[4] = {0, 0, 0, 0};       // K, kD, kH, kW of the weight: a module's weight may be replaced by one of another shape
@@ -54,10 +67,12 @@ class ConvRunner : public torch::CustomClassHolder {
     winoconv_plan_info_t info;
     at::Tensor u, bias;                      // transformed filter, bias in the compute dtype
     Stamp stamp;
+    Written written;
     int64_t serial = 0;
     bool first = false;                      // x in torch's contiguous order
     at::Tensor u_back;                       // filter of the data gradient
     Stamp back_stamp;
+    Written back_written;
     bool back_known = false, back_ok = false;
   };
 

@@ -420,3 +420,88 @@ def test_threads_agree_on_what_the_gradients_cover():
         [t.start() for t in threads]
         [t.join() for t in threads]
     assert len(names) == 100 * n_threads and set(names) == {"_WinoConvFnBackward"}, set(names)
+
+
+def _layer_and_input(seed, c=32):
+    torch.manual_seed(seed)
+    m = wconv.Conv2d(c, c, 3, padding=1).cuda()
+    with torch.no_grad():
+        m.weight.copy_(m.weight.half())
+    return m, torch.randn(2, c, 12, 12, device="cuda").half().to(memory_format=torch.channels_last)
+
+
+def _warm():        # every kernel of _layer_and_input's calls loaded
+    m, x = _layer_and_input(0)
+    m(x.clone().requires_grad_(True)).backward(x)
+    torch.cuda.synchronize()
+
+
+@pytest.mark.gpu
+def test_a_second_stream_waits_for_the_transformed_filters():
+    _warm()
+    m, x = _layer_and_input(41)
+    gy = torch.randn(x.shape, device="cuda").half().to(memory_format=torch.channels_last)
+    torch.cuda.synchronize()
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    grads = {}
+    with torch.cuda.stream(a):
+        torch.cuda._sleep(40_000_000)                  # the transforms are queued behind tens of milliseconds
+        xa = x.clone().requires_grad_(True)
+        ya = m(xa)
+        (grads["a"],) = torch.autograd.grad(ya, [xa], gy)
+    with torch.cuda.stream(b):
+        xb = x.clone().requires_grad_(True)
+        yb = m(xb)
+        (grads["b"],) = torch.autograd.grad(yb, [xb], gy)
+    torch.cuda.synchronize()
+    assert _rel(yb, _by_torch(m, x)) < _ONE_ROUNDING[torch.float16]
+    assert torch.equal(ya, yb) and torch.equal(grads["a"], grads["b"])
+
+
+@pytest.mark.gpu
+def test_an_outgrown_filter_lives_until_other_streams_have_read_it():
+    _warm()
+    m, x = _layer_and_input(42)
+    o = _by_torch(m, x)
+    with torch.no_grad():
+        m(x)
+        torch.cuda.synchronize()
+        old = next(iter(m._plans.values())).u
+        address, size = old.data_ptr(), old.numel()
+        del old
+        m.__dict__["_views"].clear()
+        b = torch.cuda.Stream()
+        with torch.cuda.stream(b):
+            torch.cuda._sleep(40_000_000)
+            y = m(x)
+        m.weight.zero_()
+        m(x)                                           # a new filter takes the old one's place in the cache
+        for _ in range(8):                             # whoever gets the old one's memory
+            t = torch.full((size,), 255, dtype=torch.uint8, device="cuda")
+            assert t.data_ptr() != address
+        torch.cuda.synchronize()
+    assert _rel(y, o) < _ONE_ROUNDING[torch.float16]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("warmed", ["not at all", "on another stream"])
+def test_filters_and_graph_captures(warmed):
+    _warm()
+    m, x = _layer_and_input(43)
+    with torch.no_grad():
+        if warmed == "on another stream":
+            m(x)
+        g, s = torch.cuda.CUDAGraph(), torch.cuda.Stream()
+        with torch.cuda.graph(g, stream=s):
+            y1, y2 = m(x), m(x)
+        y = m(x)                                       # before the graph has run
+        assert _rel(y, _by_torch(m, x)) < _ONE_ROUNDING[torch.float16]
+        g.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, y1) and torch.equal(y, y2)
+        g2 = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g2, stream=s):
+            y3 = m(x)
+        g2.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(y, y3)
