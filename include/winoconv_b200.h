@@ -115,10 +115,12 @@ typedef struct winoconv_plan_info {
   int32_t c_pad;              /* channel stride of the transformed operands (C rounded to 8)  */
   int32_t gemm_engine;        /* engine AUTO resolves to                                      */
   int32_t algo;               /* algorithm AUTO resolves to (winoconv_algo_t)                 */
-  int32_t direct;             /* 1: AUTO runs the layer on the direct-tap kernel: one launch, no     */
-                              /* scratch (2: after a copy of x with padded channels in v_ws); algo,  */
-                              /* positions, n_pieces, tiles and gemm_flops are then   */
-                              /* those of the algorithm an explicit request would run                */
+  int32_t direct;             /* 1: AUTO runs the layer on the direct-tap kernel: one launch that  */
+                              /* reads no scratch (null v_ws and m_ws will do); algo, positions,   */
+                              /* n_pieces, tiles, gemm_flops and the scratch sizes are those of    */
+                              /* the algorithm an explicit request would run.  2: the same after a */
+                              /* copy of x with padded channels: input_ws_bytes is that copy's     */
+                              /* size, product_ws_bytes 0                                          */
   int64_t tiles;              /* N * nD * nH * nW                                             */
   uint64_t filter_bytes;      /* size of the transformed filter U [positions][K][c_pad]       */
   uint64_t input_ws_bytes;    /* preferred size of the transformed-input scratch V            */

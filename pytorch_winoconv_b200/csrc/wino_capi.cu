@@ -342,10 +342,9 @@ int build_plan(const winoconv_desc_t *d, Plan *plan) {
   if (plan->direct) {
     const DirectDesc &q = plan->dd;
     I.direct = !q.fold && q.C != q.Cw ? 2 : 1;
-    if (I.direct == 2) {
-      const unsigned long long copy = (unsigned long long)g.N * g.D * g.H * g.W * q.C * esz;
-      I.input_ws_bytes = std::max<unsigned long long>(I.input_ws_bytes, copy);
-      I.input_ws_bytes_min = std::max<unsigned long long>(I.input_ws_bytes_min, copy);
+    if (I.direct == 2) {      // the copy with padded channels and nothing else
+      I.input_ws_bytes = I.input_ws_bytes_min = (unsigned long long)g.N * g.D * g.H * g.W * q.C * esz;
+      I.product_ws_bytes = I.product_ws_bytes_min = 0;
     }
     I.filter_bytes = std::max<unsigned long long>(I.filter_bytes, (unsigned long long)plan->dp.filter_elems * esz);
   }

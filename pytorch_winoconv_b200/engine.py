@@ -142,6 +142,9 @@ class WinoConv:
 
     def _scratch(self):
         """V / M scratch for the staged algorithm; the fused kernel needs none."""
+        if self.info.direct == 2:                    # a copy of the input with padded channels
+            v, _ = self.pool.get(self.device, int(self.info.input_ws_bytes), 16)
+            return v, _NO_SCRATCH
         if self.info.direct == 1 or self.info.algo == capi.ALGO_FUSED or (self.info.algo == capi.ALGO_ROW and self.info.input_ws_bytes == 0):
             return _NO_SCRATCH, _NO_SCRATCH
         if self.info.algo == capi.ALGO_ROW:          # channel-padding buffer only

@@ -246,3 +246,19 @@ def test_reference_named_modules_import():
             assert hasattr(mod, n), (mod.__name__, n)
     with pytest.raises(RuntimeError):
         dwm.dwm2d(torch.zeros(1, 4, 8, 8), torch.zeros(4, 4, 3, 3))     # CPU tensors: no CPU path
+
+
+@pytest.mark.parametrize("kw", [
+    dict(ndim=2, batch=32, c_in=3, k_out=64, in_size=(224, 224), ker_size=7, stride=2, pad=3, dtype=capi.F32),
+    dict(ndim=3, batch=2, c_in=7, k_out=24, in_size=(9, 10, 11), ker_size=3, pad=1, dtype=capi.F32),
+    dict(ndim=2, batch=3, c_in=42, k_out=16, in_size=(15, 17), ker_size=3, pad=1, dtype=capi.F16),
+])
+def test_a_layer_with_padded_channels_asks_for_that_copy_only(kw):
+    info = capi.plan(capi.make_desc(**kw))
+    vec = 4 if kw["dtype"] == capi.F32 else 8
+    pixels = kw["batch"]
+    for e in kw["in_size"]:
+        pixels *= e
+    assert info.direct == 2
+    assert info.input_ws_bytes == info.input_ws_bytes_min == pixels * (-(-kw["c_in"] // vec) * vec) * (16 // vec)
+    assert info.product_ws_bytes == info.product_ws_bytes_min == 0

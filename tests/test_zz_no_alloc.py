@@ -13,11 +13,11 @@ pytestmark = pytest.mark.gpu
 TOL = {torch.float16: 2e-2, torch.float32: 1e-3}     # the E_B bounds of tests/gpu_util.py
 
 
-def _layer(seed, n, c, k, hw, ks, pad, dtype, tile_m=0, stride=1):
+def _layer(seed, n, c, k, hw, ks, pad, dtype, tile_m=0, stride=1, algo=capi.ALGO_AUTO):
     g = torch.Generator().manual_seed(seed)
     x = torch.randn(n, hw, hw, c, generator=g).to(dtype).cuda()
     w = (torch.randn(k, c, ks, ks, generator=g) * (2.0 / (c * ks * ks)) ** 0.5).to(dtype).cuda()
-    conv = engine.WinoConv(x.shape, w, stride=stride, padding=pad, tile_m=tile_m)
+    conv = engine.WinoConv(x.shape, w, stride=stride, padding=pad, tile_m=tile_m, algo=algo)
     conv.test_w, conv.test_stride, conv.test_pad = w, stride, pad
     return x, conv
 
@@ -92,3 +92,11 @@ def test_static_scratch_refuses_an_oversized_row_layer_and_names_the_way_out():
         capi.forward_static(d, 256, 256, None, 256)
     assert ei.value.status == capi.ERR_WORKSPACE
     assert "WINOCONV_ALGO_FUSED" in str(ei.value) and "33554432" in str(ei.value)
+
+
+def test_padded_channels_cost_the_copy_and_no_more():
+    x, c = _layer(9, 4, 3, 16, 112, 7, 3, torch.float32, stride=2)
+    assert c.info.direct == 2
+    c.pool = engine.ScratchPool()
+    c(x)
+    assert c.pool.v.numel() == 4 * 112 * 112 * 4 * 4 and c.pool.m.numel() <= 16
