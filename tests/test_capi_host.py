@@ -262,3 +262,14 @@ def test_a_layer_with_padded_channels_asks_for_that_copy_only(kw):
     assert info.direct == 2
     assert info.input_ws_bytes == info.input_ws_bytes_min == pixels * (-(-kw["c_in"] // vec) * vec) * (16 // vec)
     assert info.product_ws_bytes == info.product_ws_bytes_min == 0
+
+
+@pytest.mark.parametrize("n,c,k,sp,ks,stride", [
+    (1, 64, 64, (56, 56), 3, 1), (8, 16, 64, (113, 112), 1, 1), (3, 8, 40, (201, 67), 3, 1), (4, 64, 256, (56, 58), 1, 1), (3, 32, 64, (90, 121), 3, 2),
+    (3, 3, 64, (120, 136), 7, 2), (7, 1, 24, (75, 90), 5, 1), (2, 24, 72, (5, 37, 41), 3, 1), (32, 128, 128, (56, 56), 5, 1)])
+def test_auto_runs_16_bit_layers_on_direct_taps(n, c, k, sp, ks, stride):
+    kw = dict(ndim=len(sp), batch=n, c_in=c, k_out=k, in_size=sp, ker_size=ks, stride=stride, pad=ks // 2)
+    assert capi.plan(capi.make_desc(**kw)).direct == 1
+    assert capi.plan(capi.make_desc(**kw, algo=capi.ALGO_ROW)).direct == 0         # an explicit algorithm is what runs
+    assert capi.plan(capi.make_desc(**kw, tile_m=2)).direct == 0
+    assert capi.plan(capi.make_desc(**kw, dtype=capi.F32, tile_m=1)).direct in (1, 2)

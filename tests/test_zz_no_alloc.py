@@ -94,6 +94,18 @@ def test_static_scratch_refuses_an_oversized_row_layer_and_names_the_way_out():
     assert "WINOCONV_ALGO_FUSED" in str(ei.value) and "33554432" in str(ei.value)
 
 
+def test_static_scratch_serves_the_row_kernel():
+    # on request, not by AUTO: channels padded (3 -> 8), and stride-2 phases gathered (4 x 3 -> 16 channels)
+    layers = []
+    for seed, ks, pad, stride in ((5, 3, 1, 1), (6, 7, 3, 2)):
+        x, c = _layer(seed, 4, 3, 32, 41, ks, pad, torch.float16, stride=stride, algo=capi.ALGO_ROW)
+        assert c.info.direct == 0 and c.info.algo == capi.ALGO_ROW
+        assert 0 < int(c.info.input_ws_bytes) <= capi.STATIC_SCRATCH_BYTES
+        layers.append((x, c))
+    for x, c in (*layers, layers[0]):
+        _both(x, c)
+
+
 def test_padded_channels_cost_the_copy_and_no_more():
     x, c = _layer(9, 4, 3, 16, 112, 7, 3, torch.float32, stride=2)
     assert c.info.direct == 2
