@@ -75,11 +75,13 @@ class _WinoConvMixin:
     _CONFIG = frozenset(("compute_dtype", "activation", "pool", "tile_m", "algo", "stride", "padding"))
 
     def __call__(self, *args, **kwargs):
-        """``torch.nn.Module.__call__`` without its 5 us of dispatch where there is no hook, tracer or compiled call to serve."""
+        """``torch.nn.Module.__call__`` without its 5 us of dispatch where there is no hook, tracer, compiled call or
+        patched ``torch.nn.Module.__call__`` to serve."""
         d = self.__dict__
         if (kwargs or len(args) != 1 or type(args[0]) is not torch.Tensor or d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"]
                 or _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks or _nn_module._global_backward_hooks
-                or _nn_module._global_backward_pre_hooks or self._compiled_call_impl is not None or torch._C._get_tracing_state()):
+                or _nn_module._global_backward_pre_hooks or self._compiled_call_impl is not None or torch._C._get_tracing_state()
+                or nn.Module.__call__ is not nn.Module._wrapped_call_impl):
             return super().__call__(*args, **kwargs)
         return self.forward(args[0])
 

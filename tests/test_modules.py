@@ -505,3 +505,15 @@ def test_filters_and_graph_captures(warmed):
         g2.replay()
         torch.cuda.synchronize()
         assert torch.equal(y, y3)
+
+
+def test_a_patched_module_call_sees_calls_with_tensors(monkeypatch):
+    seen = []
+    monkeypatch.setattr(torch.nn.Module, "__call__", lambda self, *args: seen.append(self) or args[0])
+    m = wconv.Conv2d(8, 8, 3)
+    x = torch.zeros(1, 8, 4, 4)
+    assert m(x) is x and seen == [m]
+    monkeypatch.undo()
+    with pytest.raises(RuntimeError, match="CUDA"):
+        m(x)
+    assert seen == [m]
