@@ -100,7 +100,8 @@ typedef struct winoconv_desc {
   int32_t product_dtype; /* dtype of the Winograd-domain products: F32 (default), F16, BF16  */
   int32_t algo;          /* winoconv_algo_t                                                  */
   int32_t bias_f32;      /* 1: the bias is f32 whatever dtype is (layers on the direct-tap kernel)   */
-  int32_t x_channels_first; /* 1: x is [N, C, D, H, W] (16-bit layers of few channels: kW * C <= 64)  */
+  int32_t x_channels_first; /* 1: x is [N, C, D, H, W] (16-bit layers of few channels: kW * C <= 64); 2: the same, refused where */
+                            /* turning x channels last and the layer on that are estimated to be faster */
   int32_t reserved[3];
 } winoconv_desc_t;
 

@@ -183,7 +183,7 @@ std::shared_ptr<ConvRunner::Entry> ConvRunner::entry_for(const at::Tensor &x, co
   d.dtype = dtype;
   d.epilogue = (bias ? WINOCONV_EPI_BIAS : 0u) | (relu_ ? WINOCONV_EPI_RELU : 0u) | (pool_ ? WINOCONV_EPI_POOL2 : 0u);
   d.algo = algo_;
-  d.x_channels_first = first ? 1 : 0;
+  d.x_channels_first = first ? 2 : 0;
   d.bias_f32 = dtype != WINOCONV_F32 && bias && bias->scalar_type() == at::kFloat;      // read as it is where the kernel can
   if (winoconv_plan(&d, &e->info) != WINOCONV_OK) {
     d.bias_f32 = 0;
@@ -249,7 +249,7 @@ std::optional<at::Tensor> ConvRunner::forward(const at::Tensor &x, const at::Ten
   std::shared_ptr<Entry> e;
   if (!grad && dtype != WINOCONV_F32 && tile_m_ == 0 && algo_ == WINOCONV_ALGO_AUTO && x.scalar_type() == type_of(dtype) && x.is_contiguous() &&
       x.size(1) * weight.size(-1) <= 64 && x.size(1) > 1 && !lies_channels_last(x) && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15u) == 0) {
-    // few channels in torch's contiguous order: the kernel gathers them as they lie
+    // few channels in torch's contiguous order: the kernel gathers them as they lie where that beats a copy
     e = entry_for(x, weight, bias, dtype, true);
     if (e) {
       at::AutoDispatchBelowADInplaceOrView no_graph;

@@ -46,6 +46,7 @@ struct Plan {
   bool row;      // row-piece kernel
   RowDesc rd;
   RowPlan rp;
+  unsigned long long row_ws;   // bytes of its copy of x with padded or gathered channels
   bool direct;   // AUTO: the direct-tap kernel runs the layer
   DirectDesc dd;
   DirectPlan dp;
@@ -270,31 +271,33 @@ int build_plan(const winoconv_desc_t *d, Plan *plan) {
   if (direct_ok && (d->tile_m == 1 || (d->tile_m == 0 && (d->dtype == WINOCONV_F32 ? !f32_f43_wins : plan->row)))) {
     DirectDesc &q = plan->dd;
     direct_forward_desc(&q, d->dtype, g.N, g.C, g.K, in, ks, st, pd, out, g.yH, g.yW, g.epilogue, g.weight_layout);
-    // few channels: folded, x gathered as it lies; otherwise channels that TMA cannot address go through a padded copy
+    // few channels: folded, x gathered as it lies, where that is the faster form; otherwise channels that TMA cannot address go
+    // through a padded copy
     const int vec = d->dtype == WINOCONV_F32 ? 4 : 8;
+    const int Cp = (g.C + vec - 1) / vec * vec;
+    // winoconv_forward_static pads into the built-in array, image by image: a layer that ran there without such a copy, or in
+    // blocks of tiles, keeps its algorithm where the copy would not fit
+    const unsigned long long image = (unsigned long long)g.D * g.H * g.W * Cp * (16 / vec);
+    const bool row_copies = plan->row && (plan->rd.phases > 1 || plan->rp.Cp != g.C) && !plan->rp.raw_c && !plan->rp.s2_chunks;
+    const bool may_pad = Cp == g.C || d->tile_m != 0 || row_copies || image * (plan->row ? (unsigned long long)g.N : 1ull) <= WINOCONV_STATIC_SCRATCH_BYTES;
     bool folded = false;
     if (g.C % vec != 0 || d->x_channels_first) {
-      DirectDesc fd = q;
-      folded = direct_fold_desc(&fd, pd, d->x_channels_first) && direct_plan(fd, &plan->dp);
+      DirectDesc fd = q, plain = q;
+      plain.C = Cp;
+      folded = direct_fold_desc(&fd, pd, d->x_channels_first) && direct_plan(fd, &plan->dp) &&
+               (d->x_channels_first == 1 || !may_pad || image > WINOCONV_STATIC_SCRATCH_BYTES || direct_fold_pays(fd, plan->dp, plain, pd));
       if (folded) q = fd;
     }
     if (folded) plan->direct = true;
     else if (!d->x_channels_first) {
-      q.C = (g.C + vec - 1) / vec * vec;
-      plan->direct = direct_plan(q, &plan->dp);
-      // winoconv_forward_static pads into the built-in array, image by image: a layer that ran there without such a copy, or in
-      // blocks of tiles, keeps its algorithm where the copy would not fit
-      if (q.C != q.Cw && d->tile_m == 0) {
-        const unsigned long long image = (unsigned long long)q.D * q.H * q.W * q.C * (16 / vec);
-        const bool row_copies = plan->row && (plan->rd.phases > 1 || plan->rp.Cp != g.C) && !plan->rp.raw_c && !plan->rp.s2_chunks;
-        if (!row_copies && image * (plan->row ? (unsigned long long)g.N : 1ull) > WINOCONV_STATIC_SCRATCH_BYTES) plan->direct = false;
-      }
+      q.C = Cp;
+      plan->direct = may_pad && direct_plan(q, &plan->dp);
     }
     if (d->tile_m == 1 && !plan->direct)
       return fail(WINOCONV_ERR_UNSUPPORTED, "tile_m = 1 (direct taps) needs a slab that fits shared memory");
   }
 
-  if (d->x_channels_first && !plan->direct) return fail(WINOCONV_ERR_UNSUPPORTED, "x_channels_first is for few-channel layers on the direct-tap kernel (kW * C <= 64, 16-bit)");
+  if (d->x_channels_first && !plan->direct) return fail(WINOCONV_ERR_UNSUPPORTED, "x_channels_first is for few-channel layers on the direct-tap kernel (kW * C <= 64, 16-bit; 2: where that is the faster form)");
   if (d->bias_f32 && !plan->direct) return fail(WINOCONV_ERR_UNSUPPORTED, "an f32 bias for a 16-bit layer needs the direct-tap kernel");
   plan->dd.bias_f32 = d->bias_f32 && d->dtype != WINOCONV_F32;
 
@@ -334,7 +337,7 @@ int build_plan(const winoconv_desc_t *d, Plan *plan) {
     // scratch only to zero-pad the channels of x to a multiple of 8 (TMA needs 16-byte pixel strides), or to hold
     // the input with its stride-2 phases gathered into channels
     const RowDesc &rd = plan->rd;
-    I.input_ws_bytes = I.input_ws_bytes_min =
+    I.input_ws_bytes = I.input_ws_bytes_min = plan->row_ws =
         ((rd.phases > 1 || rp.Cp != g.C) && !rp.raw_c && !rp.s2_chunks) ? (unsigned long long)rd.N * rd.D * rd.H * rd.W * rp.Cp * esz : 0ull;
     I.product_ws_bytes = I.product_ws_bytes_min = 0;
     I.block_tiles = I.tiles;
@@ -705,24 +708,17 @@ int winoconv_forward_static(const winoconv_desc_t *desc, const void *x, const vo
   const Plan &plan = *plan_p;
   if ((st = winoconv_device_check()) != WINOCONV_OK) return st;
   const winoconv_plan_info_t &I = plan.info;
-  if (plan.fused || (plan.row && I.input_ws_bytes_min == 0))
-    return forward_impl(desc, x, u, bias, y, nullptr, 0, nullptr, 0, stream, nullptr, nullptr);
-  if (plan.row) {   // the built-in array serves as the channel-padding buffer
-    if (I.input_ws_bytes_min > WINOCONV_STATIC_SCRATCH_BYTES)
-      return fail(WINOCONV_ERR_WORKSPACE, "the row kernel's channel-padded / phase-gathered copy of the input needs " +
-                                              std::to_string(I.input_ws_bytes_min) + " bytes; the built-in array holds " +
-                                              std::to_string(WINOCONV_STATIC_SCRATCH_BYTES) +
-                                              " (plan and filter-transform this layer with algo = WINOCONV_ALGO_FUSED, which needs"
-                                              " no scratch, or WINOCONV_ALGO_STAGED, and call again)");
-    unsigned char *pad = nullptr;
-    if ((st = static_scratch_of_current_device(&pad)) != WINOCONV_OK) return st;
-    return forward_impl(desc, x, u, bias, y, pad, WINOCONV_STATIC_SCRATCH_BYTES, nullptr, 0, stream, nullptr, nullptr);
-  }
+  if (plan.row && plan.row_ws > WINOCONV_STATIC_SCRATCH_BYTES)
+    return fail(WINOCONV_ERR_WORKSPACE, "the row kernel's channel-padded / phase-gathered copy of the input needs " +
+                                            std::to_string(plan.row_ws) + " bytes; the built-in array holds " +
+                                            std::to_string(WINOCONV_STATIC_SCRATCH_BYTES) +
+                                            " (plan and filter-transform this layer with algo = WINOCONV_ALGO_FUSED, which needs"
+                                            " no scratch, or WINOCONV_ALGO_STAGED, and call again)");
   if (I.direct == 2) {   // as many images at a time as the array holds with their channels padded
     if (!x || !u || !y) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "null tensor pointer");
     if ((desc->epilogue & WINOCONV_EPI_BIAS) && !bias) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "EPI_BIAS set but bias is null");
     if (!aligned16(x) || !aligned16(u) || !aligned16(y)) return fail(WINOCONV_ERR_INVALID_ARGUMENT, "tensors must be 16-byte aligned");
-    const DirectDesc q = plan.dd;        // (a plan of another batch may take this one's place)
+    const DirectDesc &q = plan.dd;
     const int dtype = plan.dtype;
     const size_t esz = dtype == WINOCONV_F32 ? 4 : 2;
     const long long pixels = (long long)q.D * q.H * q.W;
@@ -733,17 +729,23 @@ int winoconv_forward_static(const winoconv_desc_t *desc, const void *x, const vo
     unsigned char *pad = nullptr;
     if ((st = static_scratch_of_current_device(&pad)) != WINOCONV_OK) return st;
     for (int n0 = 0; n0 < q.N; n0 += (int)fit) {
-      winoconv_desc_t part = *desc;
-      part.batch = (int)std::min<long long>(fit, q.N - n0);
-      const Plan *pp = nullptr;
-      if ((st = plan_of<Plan>(&part, build_plan, &pp)) != WINOCONV_OK) return st;
-      if (!pp->direct || pp->info.direct != 2) return fail(WINOCONV_ERR_UNSUPPORTED, "no plan for a part of the batch");
-      cudaError_t e = launch_pad_channels(dtype, (const uint8_t *)x + n0 * pixels * q.Cw * esz, pad, part.batch * pixels, q.Cw, q.C, (cudaStream_t)stream);
+      DirectDesc part = q;          // the whole batch's filter: a plan of its own might fold the taps
+      part.N = (int)std::min<long long>(fit, q.N - n0);
+      DirectPlan pp;
+      if (!direct_plan(part, &pp)) return fail(WINOCONV_ERR_UNSUPPORTED, "no plan for a part of the batch");
+      cudaError_t e = launch_pad_channels(dtype, (const uint8_t *)x + n0 * pixels * q.Cw * esz, pad, part.N * pixels, q.Cw, q.C, (cudaStream_t)stream);
       const char *detail = "";
-      if (e == cudaSuccess) e = launch_direct_forward(pp->dd, pp->dp, pad, u, bias, (uint8_t *)y + n0 * q.ys_n * esz, (cudaStream_t)stream, &detail);
+      if (e == cudaSuccess) e = launch_direct_forward(part, pp, pad, u, bias, (uint8_t *)y + n0 * q.ys_n * esz, (cudaStream_t)stream, &detail);
       if (e != cudaSuccess) return cuda_fail(e, "forward from the built-in array", detail);
     }
     return WINOCONV_OK;
+  }
+  if (plan.fused || (plan.row && plan.row_ws == 0))
+    return forward_impl(desc, x, u, bias, y, nullptr, 0, nullptr, 0, stream, nullptr, nullptr);
+  if (plan.row) {   // the built-in array serves as the channel-padding buffer
+    unsigned char *pad = nullptr;
+    if ((st = static_scratch_of_current_device(&pad)) != WINOCONV_OK) return st;
+    return forward_impl(desc, x, u, bias, y, pad, WINOCONV_STATIC_SCRATCH_BYTES, nullptr, 0, stream, nullptr, nullptr);
   }
   const unsigned long long tiles_min = (unsigned long long)std::min<long long>(128, I.tiles);
   const unsigned long long v_tile = I.input_ws_bytes_min / tiles_min, m_tile = I.product_ws_bytes_min / tiles_min;

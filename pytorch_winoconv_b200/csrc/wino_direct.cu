@@ -30,6 +30,7 @@
 //
 // Stands in for the chain of src/base_conv_launchers.cu:338-381 where no output tile larger than 1 is worth its transforms.
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <map>
 #include <mutex>
@@ -1146,6 +1147,41 @@ bool direct_plan(const DirectDesc &d, DirectPlan *out) {
   }
   out->smem = FIXED_BYTES + (out->epi_sets - 1) * SET_BYTES + out->n_a * out->a_bytes + out->n_b * out->b_bytes;
   return true;
+}
+
+// Microseconds of a folded layer: what an item takes -- the gather (an iteration moves 128 vectors, from a TMA patch or by plain
+// loads), the MMAs or the epilogue -- times the rounds of items on 148 SMs.  Fitted to 1300 folded layers of 1 to 64 channels,
+// 1x1 to 9x9, K = 16 to 512, 2-D and 3-D, strides 1 and 2 on B200: rms 10 %, at most 45 % off.
+static double fold_us(const DirectDesc &d, const DirectPlan &p) {
+  const int lanes = p.k_full == 1 ? 2 : p.k_full == 2 ? 4 : 8;
+  const double gather = d.kD * (std::ceil(p.slab_rows_h * 8 * lanes / 128.0) * (p.raw_tma ? 230.0 : 725.0) + 950.0);
+  const double mma = 48.0 * d.kD * d.parts[0].th * p.k_full * p.MB;
+  return 7.0 + std::ceil(p.n_items / 148.0) * std::max(std::max(gather, 550.0 + 1580.0 * p.MB), mma) / 1900.0;
+}
+// ... and of the same layer on padded channels, its copy included (rms 13 %; `estimate` is half of what layers of so few
+// channels take).
+static double padded_us(const DirectDesc &d, const DirectPlan &p) {
+  const double copied = d.C == d.Cw ? 0.0 : 2.0 * d.N * d.D * d.H * d.W * (d.C + d.Cw);
+  return 1.2 + 1.98 * p.estimate / 1900.0 + copied / 5.25e6;
+}
+
+// Folding saves the copy and most K steps, but every 64 output channels gather x again: it loses where those are many, entries
+// long or rows not 16-byte multiples.  us folded / padded on B200: 3 -> 64 7x7 s2, N = 32, at 225x225 (plain loads) 101 / 58; 6 -> 328
+// 3x3x3 s2 at 24x34x41, N = 16: 369 / 69; 16 -> 96 1x1 at 99x99, N = 61, from torch's order 134 / 51 with the copy; 3 -> 64 3x3 at
+// 56x56, N = 16: 12 / 15.  Over 2849 layers of 1 to 64 channels the rule takes 0.79 of always folding; it folds where the two are
+// close, and is slower than folding by more than 5 % on 25 of them (at most 15 %).
+bool direct_fold_pays(const DirectDesc &fold, const DirectPlan &fp, const DirectDesc &plain, const int pad[3]) {
+  DirectPlan p;
+  if (!direct_plan(plain, &p)) return true;
+  double other = padded_us(plain, p);
+  if (!fold.x_first) return fold_us(fold, fp) < 1.25 * other;
+  if (plain.C != plain.Cw) {
+    DirectDesc last = plain;
+    last.C = last.Cw;
+    if (direct_fold_desc(&last, pad, 0) && direct_plan(last, &p)) other = std::min(other, fold_us(last, p));
+  }
+  const double turn = 2.3 + 4.0 * fold.N * fold.D * fold.H * fold.W * fold.Cw / 9.9e6;
+  return fold_us(fold, fp) < 1.15 * (turn + other);
 }
 
 cudaError_t launch_direct_filter_transform(const DirectDesc &d, const DirectPlan &p, int w_dtype, const void *w, void *u, cudaStream_t s) {

@@ -125,6 +125,8 @@ struct DirectPlan {
 };
 bool direct_plan(const DirectDesc &d, DirectPlan *out);
 bool direct_fold_desc(DirectDesc *q, const int pad[3], int x_first);   // turns a forward description into a folded one where it applies
+// Whether the folded form is the faster one; `plain` is the layer on (padded) channels-last channels.
+bool direct_fold_pays(const DirectDesc &fold, const DirectPlan &fp, const DirectDesc &plain, const int pad[3]);
 cudaError_t launch_direct_filter_transform(const DirectDesc &d, const DirectPlan &p, int w_dtype, const void *w, void *u, cudaStream_t s);
 cudaError_t launch_direct_forward(const DirectDesc &d, const DirectPlan &p, const void *x, const void *u, const void *bias, void *y,
                                   cudaStream_t s, const char **detail);

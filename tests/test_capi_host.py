@@ -273,3 +273,21 @@ def test_auto_runs_16_bit_layers_on_direct_taps(n, c, k, sp, ks, stride):
     assert capi.plan(capi.make_desc(**kw, algo=capi.ALGO_ROW)).direct == 0         # an explicit algorithm is what runs
     assert capi.plan(capi.make_desc(**kw, tile_m=2)).direct == 0
     assert capi.plan(capi.make_desc(**kw, dtype=capi.F32, tile_m=1)).direct in (1, 2)
+
+
+def test_few_channels_are_folded_where_that_is_the_faster_form():
+    def direct(first=0, **kw):
+        d = capi.make_desc(pad=kw["ker_size"] // 2, **kw)
+        d.x_channels_first = first
+        try:
+            return capi.plan(d).direct
+        except capi.WinoconvError as e:
+            assert e.status == capi.ERR_UNSUPPORTED
+            return None
+    stem = dict(ndim=2, batch=32, c_in=3, k_out=64, in_size=(224, 224), ker_size=7, stride=2)
+    odd_stem = dict(stem, in_size=(225, 225))                      # rows of x that TMA cannot address
+    many_out = dict(ndim=3, batch=16, c_in=6, k_out=328, in_size=(24, 34, 41), ker_size=3, stride=2)
+    pointwise = dict(ndim=2, batch=61, c_in=16, k_out=96, in_size=(99, 99), ker_size=1)
+    assert [direct(**kw) for kw in (stem, odd_stem, many_out, pointwise)] == [1, 2, 2, 1]
+    assert [direct(2, **kw) for kw in (stem, many_out, pointwise)] == [1, None, None]
+    assert [direct(1, **kw) for kw in (stem, odd_stem, many_out, pointwise)] == [1, 1, 1, 1]      # asked for without a condition

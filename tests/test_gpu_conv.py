@@ -508,3 +508,17 @@ def test_gradients_16_bit(n, c, k, sp, ks, stride):
     # fp32 sums of at most a few thousand exact products, cut off after every MMA: 2**-23 of the running sum each, far below 1e-5
     assert rel(layer.weight.grad, wd.grad) < 1e-5
     assert rel(layer.bias.grad, bd.grad) < 1e-6                 # plain fp32 sums
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("n,c,k,sp,ks,stride,options", [
+    (2, 6, 328, (5, 18, 21), 3, 2, {}),                       # folded or padded by their cost: both sides of the rule, both orders
+    (8, 3, 64, (113, 113), 7, 2, {"activation": "relu"}),
+    (3, 12, 130, (57, 57), 3, 1, {"pool": 2}),
+    (16, 16, 96, (57, 57), 1, 1, {}),
+    (2, 4, 16, (97, 95), 9, 2, {}),
+    (2, 64, 300, (56, 56), 1, 1, {"activation": "relu"}),
+    (1, 1, 500, (30, 31), 5, 1, {}),
+])
+def test_few_channels_folded_or_padded(n, c, k, sp, ks, stride, options, dtype):
+    test_direct_taps_16_bit(n, c, k, sp, ks, stride, options, dtype)
