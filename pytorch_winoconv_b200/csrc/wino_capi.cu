@@ -360,8 +360,13 @@ int build_plan(const winoconv_desc_t *d, Plan *plan) {
 }
 
 // Plans are functions of the descriptor alone; a caller runs the same few descriptors over and over, so each thread keeps the
-// last ones (direct mapped by a hash of the descriptor; a planner pass costs tens of microseconds).
-template <typename P> struct PlanSlot { winoconv_desc_t desc; std::unique_ptr<P> plan; };
+// last ones, refusals among them (direct mapped by a hash of the descriptor; a planner pass takes 2 to 7 us).
+template <typename P> struct PlanSlot {
+  winoconv_desc_t desc;
+  std::unique_ptr<P> plan;      // null where the descriptor was refused, with `status` and `why`
+  int status = WINOCONV_OK;
+  std::string why;
+};
 constexpr unsigned kPlanSlots = 64;
 template <typename P>
 int plan_of(const winoconv_desc_t *d, int (*build)(const winoconv_desc_t *, P *), const P **out) {
@@ -371,15 +376,15 @@ int plan_of(const winoconv_desc_t *d, int (*build)(const winoconv_desc_t *, P *)
   uint32_t h = 2166136261u;
   for (size_t i = 0; i < sizeof(*d) / 4; ++i) h = (h ^ w[i]) * 16777619u;
   PlanSlot<P> &s = slots[(h ^ (h >> 15)) % kPlanSlots];
-  if (!s.plan || std::memcmp(&s.desc, d, sizeof(*d)) != 0) {
+  if ((!s.plan && s.status == WINOCONV_OK) || std::memcmp(&s.desc, d, sizeof(*d)) != 0) {
     std::unique_ptr<P> fresh(new P());
-    const int st = build(d, fresh.get());
-    if (st != WINOCONV_OK) return st;
+    s.status = build(d, fresh.get());
+    s.why = s.status == WINOCONV_OK ? std::string() : t_last_error;
     s.desc = *d;
-    s.plan = std::move(fresh);
+    s.plan = s.status == WINOCONV_OK ? std::move(fresh) : nullptr;
   }
   *out = s.plan.get();
-  return WINOCONV_OK;
+  return s.status == WINOCONV_OK ? WINOCONV_OK : fail(s.status, s.why);
 }
 
 // Gradients of a 16-bit layer: the data gradient on the direct-tap kernel (a launch per depth parity), the weight gradient on

@@ -291,3 +291,32 @@ def test_few_channels_are_folded_where_that_is_the_faster_form():
     assert [direct(**kw) for kw in (stem, odd_stem, many_out, pointwise)] == [1, 2, 2, 1]
     assert [direct(2, **kw) for kw in (stem, many_out, pointwise)] == [1, None, None]
     assert [direct(1, **kw) for kw in (stem, odd_stem, many_out, pointwise)] == [1, 1, 1, 1]      # asked for without a condition
+
+
+def test_a_refusal_is_remembered():
+    import ctypes
+    import time
+    lib, info = capi.lib(), capi.PlanInfo()
+
+    def descs(batches):
+        out = [capi.make_desc(ndim=2, batch=n, c_in=16, k_out=256, in_size=(56, 56), ker_size=3, pad=1) for n in batches]
+        for d in out:
+            d.x_channels_first = 2
+        return out
+
+    def seconds(ds):
+        best = 1.0
+        for _ in range(7):
+            t = time.perf_counter()
+            for d in ds:
+                assert lib.winoconv_plan(ctypes.byref(d), ctypes.byref(info)) == capi.ERR_UNSUPPORTED
+            best = min(best, time.perf_counter() - t)
+        return best
+
+    assert seconds(descs([40] * 300)) < 0.5 * seconds(descs(range(20, 320)))        # one planner pass against 300 (more than are kept)
+    reasons = []
+    for d in descs([40, 40]) + [capi.make_desc(ndim=2, batch=1, c_in=8, k_out=8, in_size=(8, 8), ker_size=3, tile_m=5)] * 2:
+        with pytest.raises(capi.WinoconvError) as e:
+            capi.plan(d)
+        reasons.append(str(e.value))
+    assert reasons[0] == reasons[1] and reasons[2] == reasons[3] and "x_channels_first" in reasons[0] and "tile_m" in reasons[2]
