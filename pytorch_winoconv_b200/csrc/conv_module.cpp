@@ -275,8 +275,7 @@ std::optional<at::Tensor> ConvRunner::forward(const at::Tensor &x, const at::Ten
 void ConvRunner::Written::here() {
   stream = at::cuda::getCurrentCUDAStream();
   capture = capture_of(*stream);
-  finished = false;
-  event.record(*stream);
+  recorded = finished = false;
 }
 
 bool ConvRunner::Written::usable_here(std::initializer_list<at::Tensor> buffers) {
@@ -286,9 +285,14 @@ bool ConvRunner::Written::usable_here(std::initializer_list<at::Tensor> buffers)
   const unsigned long long current = capture_of(now);
   if (capture != 0 && capture != current) return false;
   if (*stream == now) return true;
-  if (capture == 0 && !finished) {
+  if (!finished) {
     c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);      // a query is no part of anyone's capture
-    finished = event.query();
+    if (!recorded && capture_of(*stream) != capture) return false;      // being captured now: it tells nothing of the work before that
+    finished = capture == 0 && (recorded ? event.query() : stream->query());
+    if (!finished && !recorded) {
+      event.record(*stream);
+      recorded = true;
+    }
   }
   if (!finished) {
     if (capture != current) return false;

@@ -48,13 +48,14 @@ class ConvRunner : public torch::CustomClassHolder {
       return w_ref == o.w_ref && b_ref == o.b_ref && w == o.w && b == o.b && w_version == o.w_version && b_version == o.b_version && w_dtype == o.w_dtype;
     }
   };
-  // Where an entry's buffers were written.  A call on another stream waits for that and tells the allocator that it reads them.
-  // A graph capture cannot wait for work outside of it: it uses them once that work has finished, else it makes its own; and what
-  // a capture writes holds its values only when the graph runs, so nobody outside of that capture uses it.
+  // Where an entry's buffers were written.  The first call on another stream records an event there (whoever stays on one stream
+  // pays for none), waits for it and tells the allocator that it reads them.  A graph capture cannot wait for work outside of it:
+  // it uses them once that work has finished, else it makes its own; and what a capture writes holds its values only when the
+  // graph runs, so nobody outside of that capture uses it.
   struct Written {
     std::optional<c10::cuda::CUDAStream> stream;
     at::cuda::CUDAEvent event;
-    bool finished = false;
+    bool recorded = false, finished = false;
     unsigned long long capture = 0;
     void here();                                                      // they are written by what is queued on the current stream so far
     bool usable_here(std::initializer_list<at::Tensor> buffers);      // false: write them anew

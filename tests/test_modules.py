@@ -472,13 +472,13 @@ def test_an_outgrown_filter_lives_until_other_streams_have_read_it():
         m.__dict__["_views"].clear()
         b = torch.cuda.Stream()
         with torch.cuda.stream(b):
-            torch.cuda._sleep(40_000_000)
+            torch.cuda._sleep(400_000_000)
             y = m(x)
         m.weight.zero_()
         m(x)                                           # a new filter takes the old one's place in the cache
-        for _ in range(8):                             # whoever gets the old one's memory
+        for _ in range(8):                             # whoever gets the old one's memory, gets it when b has read it
             t = torch.full((size,), 255, dtype=torch.uint8, device="cuda")
-            assert t.data_ptr() != address
+            assert t.data_ptr() != address or b.query()
         torch.cuda.synchronize()
     assert _rel(y, o) < _ONE_ROUNDING[torch.float16]
 
