@@ -522,3 +522,31 @@ def test_gradients_16_bit(n, c, k, sp, ks, stride):
 ])
 def test_few_channels_folded_or_padded(n, c, k, sp, ks, stride, options, dtype):
     test_direct_taps_16_bit(n, c, k, sp, ks, stride, options, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("n,c,k,sp,ks,pad,stride", [(2, 24, 40, (13, 19), 3, 1, 1), (2, 16, 24, (18, 11), 3, 0, 1), (1, 64, 72, (21, 23), 3, 1, 2), (2, 13, 8, (4, 7, 9), 3, 1, 1), (1, 8, 16, (16, 16), 3, 1, 1)])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_weight_gradient_with_a_pixel_that_is_not_finite(n, c, k, sp, ks, pad, stride, value, dtype):
+    # in the last row and column, which blocks of pixels reach beyond: only taps that read it may lose their value
+    nd = len(sp)
+    x, w = _rand(n, c, k, sp, ks, dtype)
+    x[0, 1, ..., -1, -1] = value
+    x[-1, 2, ..., -1, 3] = value
+    layer = (conv.Conv2d if nd == 2 else conv.Conv3d)(c, k, ks, stride=stride, padding=pad, device="cuda", compute_dtype=dtype)
+    with torch.no_grad():
+        layer.weight.copy_(w.float())
+    y = layer(x.cuda())
+    gy = torch.randn(y.shape, generator=torch.Generator().manual_seed(8)).to(dtype)
+    y.backward(gy.cuda())
+    assert capi.read_device_error() == 0
+    xp = torch.nn.functional.pad(x.double(), (pad, pad) * nd)
+    o = torch.empty(w.shape, dtype=torch.float64)
+    for tap in torch.cartesian_prod(*[torch.arange(ks)] * nd).tolist():
+        win = xp[(slice(None), slice(None), *[slice(t, t + (e - 1) * stride + 1, stride) for t, e in zip(tap, gy.shape[2:])])]
+        o[(slice(None), slice(None), *tap)] = torch.einsum("nko,nco->kc", gy.double().flatten(2), win.flatten(2))
+    got = layer.weight.grad.cpu().double()
+    assert 0 < int((~o.isfinite()).sum()) < o.numel()
+    assert torch.equal(got.isfinite(), o.isfinite())
+    fine = o.isfinite()
+    assert float((got[fine] - o[fine]).norm() / o[fine].norm()) < 1e-5
