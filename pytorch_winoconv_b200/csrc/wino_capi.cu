@@ -489,6 +489,14 @@ int winoconv_device_check(void) {
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) { cudaGetLastError(); return fail(WINOCONV_ERR_NO_DEVICE, std::string("cudaGetDevice: ") + cudaGetErrorString(e)); }
+  // A thread that has launched nothing yet has no context, and without one the driver's tensor map encoder refuses: an autograd
+  // thread, or a caller's new thread, may come here first.
+  static thread_local int bound = -1;
+  if (bound != dev) {
+    e = cudaSetDevice(dev);
+    if (e != cudaSuccess) { cudaGetLastError(); return fail(WINOCONV_ERR_NO_DEVICE, std::string("cudaSetDevice: ") + cudaGetErrorString(e)); }
+    bound = dev;
+  }
   int major = 0;
   e = cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev);
   if (e != cudaSuccess) { cudaGetLastError(); return fail(WINOCONV_ERR_NO_DEVICE, std::string("cudaDeviceGetAttribute: ") + cudaGetErrorString(e)); }

@@ -517,3 +517,42 @@ def test_a_patched_module_call_sees_calls_with_tensors(monkeypatch):
     with pytest.raises(RuntimeError, match="CUDA"):
         m(x)
     assert seen == [m]
+
+
+@pytest.mark.gpu
+def test_threads_that_have_made_no_cuda_call():
+    import threading
+    m, x = _layer_and_input(51)
+    out = []
+    with torch.no_grad():
+        out.append(m(x))
+
+        def call():
+            with torch.no_grad():
+                out.append(m(x))
+
+        for _ in range(3):
+            t = threading.Thread(target=call)
+            t.start()
+            t.join()
+    assert len(out) == 4 and all(torch.equal(y, out[0]) for y in out)
+
+
+@pytest.mark.gpu
+def test_a_first_layer_trains_in_a_process_of_its_own():
+    # no data gradient and nothing to convert: the weight gradient is the first thing autograd's thread does
+    import subprocess
+    import sys
+    code = """
+import torch
+from pytorch_winoconv_b200 import conv
+m = conv.Conv2d(16, 24, 3, padding=1).cuda()
+x = torch.randn(2, 16, 19, 21, device="cuda").half().to(memory_format=torch.channels_last)
+y = m(x)
+gy = torch.randn(y.shape, device="cuda").half().to(memory_format=torch.channels_last)
+y.backward(gy)
+o = torch.nn.grad.conv2d_weight(x.cpu().double(), m.weight.shape, gy.cpu().double(), 1, 1)
+assert float((m.weight.grad.cpu().double() - o).norm() / o.norm()) < 1e-5
+"""
+    done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0, done.stderr[-2000:]
