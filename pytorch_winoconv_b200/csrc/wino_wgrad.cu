@@ -283,15 +283,16 @@ struct RGeom {
   long long part_stride, bias_off;
   Bundle bundles[MAX_BUNDLES];
   uint16_t tap_of[400];         // position in the weight of each walked tap
-  // blocks that reach beyond the output (see pixel_sum), and what that function reads
-  int ragged, bf16, N, D, H, W, oD, oH, oW, sD, sH, sW, pD, pH, pW, kH, kW, Cm, Km;
+  // what pixel_sum reads
+  int bf16, N, D, H, W, oD, oH, oW, sD, sH, sW, pD, pH, pW, kH, kW, Cm, Km;
 };
 
 // A block that reaches beyond the output multiplies zeros of gy by pixels of x which another tap has a use for.  Where such a pixel
 // is infinite or not a number, so is the sum: a sum that is not a number is done again over the output's own pixels.  It ends
-// where it has become one by rights.  One such pixel costs a 64 -> 64 3x3 layer at 114x114, N = 64, 74 ms where the gradient takes 0.14
-// (16 loads in flight; 361 ms with one).
-__device__ __noinline__ float pixel_sum(const unsigned short *__restrict__ x, const unsigned short *__restrict__ gy, const RGeom &g, int k, int c, int tap) {
+// where it has become one by rights.  Layers without such blocks run the kernel without this code; in it, it costs the others about 5 %
+// of their time (128 -> 128 3x3 at 57x57, N = 32: 41.1 -> 43.1 us with the first kernel's; 32 registers as before).  One infinite pixel
+// at the edge costs 64 -> 64 at 114x114, N = 64, 0.37 s.
+__device__ __forceinline__ float pixel_sum(const unsigned short *__restrict__ x, const unsigned short *__restrict__ gy, const RGeom &g, int k, int c, int tap) {
   const int tw = tap % g.kW, th = tap / g.kW % g.kH, td = tap / (g.kW * g.kH);
   auto value = [&](unsigned short v) { return g.bf16 ? __uint_as_float((uint32_t)v << 16) : Pair16<__half>::unpack(v).x; };
   float total = 0.f;
@@ -303,24 +304,24 @@ __device__ __noinline__ float pixel_sum(const unsigned short *__restrict__ x, co
         const unsigned short *gr = gy + (((long long)n * g.oD + od) * g.oH + oh) * g.oW * g.Km + k;
         const unsigned short *xr = x + (((long long)n * g.D + id) * g.H + ih) * g.W * g.Cm + c;
         float row = 0.f;
-        for (int o0 = 0; o0 < g.oW; o0 += 16) {      // sixteen pixels' loads in flight: a thread has nothing else to wait with
-          unsigned short a[16], b[16];
+        for (int o0 = 0; o0 < g.oW; o0 += 8) {      // eight pixels' loads in flight: a thread has nothing else to wait with
+          unsigned short a[8], b[8];
 #pragma unroll
-          for (int i = 0; i < 16; ++i) {
+          for (int i = 0; i < 8; ++i) {
             const int ow = o0 + i, iw = g.sW * ow + tw - g.pW;
             a[i] = ow < g.oW ? gr[(long long)ow * g.Km] : 0;
             b[i] = ow < g.oW && row_in && (unsigned)iw < (unsigned)g.W ? xr[(long long)iw * g.Cm] : 0;
           }
 #pragma unroll
-          for (int i = 0; i < 16; ++i) row = fmaf(value(a[i]), value(b[i]), row);
+          for (int i = 0; i < 8; ++i) row = fmaf(value(a[i]), value(b[i]), row);
         }
         total += row;
         if (total != total) return total;
       }
   return total;
 }
-template <typename T>
-__global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float *__restrict__ part, T *__restrict__ dw, float *__restrict__ dbias,
+template <typename T, bool REDO>
+__global__ void __launch_bounds__(256, 8) wgrad_reduce_kernel(const float *__restrict__ part, T *__restrict__ dw, float *__restrict__ dbias,
                                                            const unsigned short *__restrict__ x, const unsigned short *__restrict__ gy,
                                                            const __grid_constant__ RGeom g, int n_values) {
   grid_dependency_wait();
@@ -342,7 +343,7 @@ __global__ void __launch_bounds__(256) wgrad_reduce_kernel(const float *__restri
   for (; j < g.split; ++j) s += src[j * g.part_stride];
   if (is_bias) { dbias[i - (int)g.bias_off] = s; return; }
   const int tap = g.tap_of[g.bundles[bu].tap + tl];
-  if (s != s && g.ragged) s = pixel_sum(x, gy, g, k, c, tap);
+  if constexpr (REDO) { if (s != s) s = pixel_sum(x, gy, g, k, c, tap); }
   Elem<T>::store(dw + ((long long)k * g.C + c) * g.taps + tap, s);
 }
 
@@ -483,14 +484,16 @@ bool wgrad_plan(const WgradDesc &d, WgradPlan *out) {
 }
 
 template <typename T>
-static cudaError_t launch_reduce(const RGeom &r, const float *part, void *dw, float *db, const void *x, const void *gy, int n, cudaStream_t s) {
+static cudaError_t launch_reduce(const RGeom &r, bool redo, const float *part, void *dw, float *db, const void *x, const void *gy, int n, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)((n + 255) / 256)); cfg.blockDim = dim3(256); cfg.stream = s;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr; cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, wgrad_reduce_kernel<T>, part, (T *)dw, db, (const unsigned short *)x, (const unsigned short *)gy, r, n);
+  const auto *xs = (const unsigned short *)x, *gs = (const unsigned short *)gy;
+  return redo ? cudaLaunchKernelEx(&cfg, wgrad_reduce_kernel<T, true>, part, (T *)dw, db, xs, gs, r, n)
+              : cudaLaunchKernelEx(&cfg, wgrad_reduce_kernel<T, false>, part, (T *)dw, db, xs, gs, r, n);
 }
 
 cudaError_t launch_wgrad(const WgradDesc &d, const WgradPlan &p, const void *x, const void *gy, void *dw, int dw_dtype, float *dbias,
@@ -553,7 +556,6 @@ cudaError_t launch_wgrad(const WgradDesc &d, const WgradPlan &p, const void *x, 
   std::memset(&r, 0, sizeof r);
   r.K = d.K; r.C = d.C; r.taps = g.taps; r.split = g.split; r.part_stride = g.part_stride; r.bias_off = g.bias_off;
   r.n_bundles = g.all_bundles; r.ch_el = g.ch_el;
-  r.ragged = g.n_wb * (8 / g.TI) != d.oW || g.n_hb * g.TH != d.oH;
   r.bf16 = d.dtype == WINOCONV_BF16;
   r.N = d.N; r.D = d.D; r.H = d.H; r.W = d.W; r.oD = d.oD; r.oH = d.oH; r.oW = d.oW; r.Cm = d.Cm; r.Km = d.Km;
   r.sD = d.sD; r.sH = d.sH; r.sW = d.sW; r.pD = d.pD; r.pH = d.pH; r.pW = d.pW; r.kH = d.kH; r.kW = d.kW;
@@ -565,9 +567,10 @@ cudaError_t launch_wgrad(const WgradDesc &d, const WgradPlan &p, const void *x, 
         for (int th = a; th < d.kH; th += d.sH)
           for (int tw = b; tw < d.kW; tw += d.sW) r.tap_of[nt++] = (uint16_t)((kd * d.kH + th) * d.kW + tw);
   const int n = (int)g.bias_off + (g.bias_on ? d.K : 0);
-  if (dw_dtype == WINOCONV_F32) return launch_reduce<float>(r, (const float *)ws, dw, dbias, x, gy, n, s);
-  if (dw_dtype == WINOCONV_F16) return launch_reduce<__half>(r, (const float *)ws, dw, dbias, x, gy, n, s);
-  return launch_reduce<__nv_bfloat16>(r, (const float *)ws, dw, dbias, x, gy, n, s);
+  const bool redo = g.n_wb * (8 / g.TI) != d.oW || g.n_hb * g.TH != d.oH;      // blocks that reach beyond the output
+  if (dw_dtype == WINOCONV_F32) return launch_reduce<float>(r, redo, (const float *)ws, dw, dbias, x, gy, n, s);
+  if (dw_dtype == WINOCONV_F16) return launch_reduce<__half>(r, redo, (const float *)ws, dw, dbias, x, gy, n, s);
+  return launch_reduce<__nv_bfloat16>(r, redo, (const float *)ws, dw, dbias, x, gy, n, s);
 }
 
 cudaError_t read_and_clear_wgrad_error(cudaStream_t s, unsigned int *code) {
