@@ -58,10 +58,11 @@ typedef enum winoconv_gemm {
 } winoconv_gemm_t;
 
 typedef enum winoconv_algo {
-  WINOCONV_ALGO_AUTO = 0,   /* ROW where it applies, else FUSED where it applies, else STAGED; with      */
-                            /* tile_m = 0 a 16-bit 3x3 stride-1 layer of >= 512 input and output channels */
-                            /* whose 4-wide tiles cover the output exactly (>= 4096 of them) runs as       */
-                            /* STAGED F(4x4,3x3) instead (measured faster; needs the V / M scratch)        */
+  WINOCONV_ALGO_AUTO = 0,   /* with tile_m = 0 or 1 the direct-tap kernel (winoconv_plan_info_t.direct), except with */
+                            /* tile_m = 0 a 16-bit 3x3 stride-1 layer of >= 512 input and output channels  */
+                            /* whose 4-wide tiles cover the output exactly (>= 4096 of them) and fp32 3x3  */
+                            /* stride-1 layers of many channels: STAGED F(4x4,3x3), with V / M scratch.    */
+                            /* With another tile_m: ROW where it applies, else FUSED, else STAGED          */
   WINOCONV_ALGO_STAGED = 1, /* input transform -> batched GEMM -> output transform through V / M scratch  */
   WINOCONV_ALGO_FUSED = 2,  /* one tcgen05 kernel, 3x3 pieces as F(2x2,3x3); f16 / bf16, any stride       */
   WINOCONV_ALGO_ROW = 3     /* one tcgen05 kernel, 1x3 pieces: F(2,3) along W, taps along H / depth summed */
@@ -172,7 +173,9 @@ WINOCONV_API int winoconv_filter_transform(const winoconv_desc_t *desc, const vo
 WINOCONV_API int winoconv_filter_transform_from(const winoconv_desc_t *desc, const void *weights, int w_dtype, void *u, void *stream);
 
 /*
- * y = conv(x, w) by the algorithm the plan names (winoconv_plan_info_t.algo):
+ * y = conv(x, w) by the algorithm the plan names (winoconv_plan_info_t.direct, then .algo):
+ *   direct taps  one kernel, every kernel tap a slice of the reduction read from one halo slab in shared memory;
+ *                v_ws holds the copy of x with padded channels where direct is 2, else no scratch is used.
  *   ROW / FUSED  one kernel: input tiles are transformed in shared memory, multiplied on the tensor
  *                cores with the DWM pieces summed in the accumulator, and written through the output
  *                transform with the bias / ReLU / 2x2 max-pool epilogue; v_ws and m_ws are not used

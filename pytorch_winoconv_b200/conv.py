@@ -18,11 +18,12 @@ stride 2 included, no cuDNN branch.  What the reference pays per call and these 
 Backward (the reference left only traces of one: ``include/splitstrideone/split_functions_grad.h:1-7``,
 ``backwardAssign`` at ``src/back/utils.cu:16``) runs on the engine's kernels too:
 
-* data gradient: the forward engine on the flipped, transposed filter -- ``grad_x = conv(grad_y, flip(w)^T)``
-  with padding ``k - 1 - p``; a stride-2 layer first spreads ``grad_y`` onto the stride grid (zeros between);
-* weight gradient: one tensor-core GEMM per filter tap, ``dW[:, :, tap] = grad_y^T  x_shifted(tap)`` with the
-  batch and output pixels as the reduction (``winoconv_gemm_batched``, fp32 accumulate);
-* bias gradient: a sum.
+* 16-bit layers: native (``csrc/conv_module.cpp``) -- the data gradient on the direct-tap kernel with the taps mirrored and
+  the channels exchanged (a strided layer is a part per residue of the input's pixels), the weight gradient on a kernel that
+  reduces over pixels as they lie (``csrc/wino_wgrad.cu``), the bias gradient summed beside it in fp32;
+* fp32 layers, kernels of more than 400 taps: from Python -- the data gradient by the forward engine on the flipped, transposed
+  filter, ``grad_x = conv(grad_y, flip(w)^T)`` with padding ``k - 1 - p`` (a stride-2 layer first spreads ``grad_y`` onto the
+  stride grid), the weight gradient by one tensor-core GEMM per filter tap (``winoconv_gemm_batched``), the bias gradient a sum.
 
 A fused ReLU is differentiated through the stored output; the fused max-pool is forward only.
 ``groups != 1`` and dilation raise (the reference accepts ``groups`` and silently computes groups = 1).
@@ -271,7 +272,8 @@ class _WinoConvMixin:
 
     @property
     def planned_algorithms(self):
-        """Algorithm the engine chose for every input shape seen so far: {shape: 'row' | 'fused' | 'staged'}."""
+        """Algorithm of every input shape seen so far: {shape: 'row' | 'fused' | 'staged'}.  A layer that AUTO runs on the
+        direct-tap kernel (``plan.info.direct``) has the name of the algorithm that its tile size stands for otherwise."""
         names = {capi.ALGO_ROW: "row", capi.ALGO_FUSED: "fused", capi.ALGO_STAGED: "staged"}
         return {shape: names.get(int(p.info.algo), str(p.info.algo)) for shape, p in self._plans.items()}
 
@@ -314,7 +316,7 @@ class Conv2d(_WinoConvMixin, nn.Conv2d):
 
     Extra keyword arguments: ``compute_dtype`` (default ``torch.float16`` as upstream, ``None`` keeps the
     input's dtype; fp32 runs its products as three tf32 tensor-core products of a hi / lo split), ``activation`` (``None`` / ``"relu"``),
-    ``pool`` (``None`` / ``2``), ``tile_m`` (0 auto, 2, 4; 6 for fp32 layers) and ``algo`` (``capi.ALGO_*``).
+    ``pool`` (``None`` / ``2``), ``tile_m`` (0 auto, 1 direct taps, 2, 4; 6 for fp32 layers) and ``algo`` (``capi.ALGO_*``).
     """
 
     _nd = 2

@@ -412,7 +412,9 @@ std::optional<at::Tensor> conv_call(const at::Tensor &x_in, const at::Tensor &we
   d.dtype = dtype;
   const bool bias_after = bias && out_f32 && dtype != WINOCONV_F32;
   d.epilogue = bias && !bias_after ? WINOCONV_EPI_BIAS : 0u;
-  // direct taps, unless F(2,r) does them in fewer multiplies than its traffic is worth (fp32, wide 3x3: see the planner)
+  // direct taps, unless the tile asked for does the layer in fewer multiplies than its traffic is worth: F(2,3) of wide fp32 3x3 layers
+  // (us direct / F(2,3) on B200 at 28 x 28, N = 8: 128 -> 256 36 / 35, 416 -> 256 103 / 86, 128 -> 96 21 / 27; F(4x4,3x3), which AUTO
+  // weighs for the modules, crosses earlier)
   winoconv_plan_info_t info;
   const bool wide_f32 = dtype == WINOCONV_F32 && nd == 2 && d.ker_size[1] == 3 && d.ker_size[2] == 3 && d.stride[1] == 1 && d.stride[2] == 1 &&
                         (int64_t)d.c_in * d.k_out > 128 * 128;

@@ -100,10 +100,11 @@ int build_plan(const winoconv_desc_t *d, Plan *plan) {
     st[i] = unused ? 1 : d->stride[i];
     pd[i] = unused ? 0 : d->pad[i];
   }
-  // F(4x4,3x3): 2-D, 3x3, stride 1.  With tile_m = 0 it is chosen where the staged flow runs anyway (fp32, the
-  // SIMT engine, 16-bit products, algo = STAGED); a 16-bit layer that one of the single-kernel paths can take gets
-  // 2-wide tiles instead: measured on B200 the row-piece kernel runs the 256 -> 256 layer at 28 x 28, N = 32 in
-  // 35 us against 58 us for staged F(4x4,3x3), and its fp16 error is four times smaller.
+  // F(4x4,3x3): 2-D, 3x3, stride 1.  With tile_m = 0 it is the tile where the staged flow runs (the SIMT engine, 16-bit
+  // products, algo = STAGED; fp32 layers that the direct-tap kernel below does not take); a 16-bit layer that one of the
+  // single-kernel paths can take gets 2-wide tiles, which the direct-tap kernel then replaces: measured on B200 the 256 -> 256
+  // layer at 28 x 28, N = 32 takes 58 us as staged F(4x4,3x3), 35 us on the row-piece kernel and 31 us by direct taps, whose
+  // fp16 error is the smallest.
   const bool f43_ok = ks[0] == 1 && in[0] == 1 && ks[1] == 3 && ks[2] == 3 && st[1] == 1 && st[2] == 1;
   const bool single_kernel_candidate = d->dtype != WINOCONV_F32 && d->algo != WINOCONV_ALGO_STAGED &&
                                        d->gemm_engine != WINOCONV_GEMM_SIMT && d->product_dtype == WINOCONV_F32;
@@ -111,7 +112,7 @@ int build_plan(const winoconv_desc_t *d, Plan *plan) {
   // and with the tiles covering the output exactly and enough of them to fill the GPU the staged flow beats the
   // row-piece kernel (measured on B200, 512 -> 512 at 28 x 28, N = 256: 0.60 ms against 0.70 ms; at 14 x 14, where 4-wide
   // tiles cover 16 x 16, 0.23 against 0.18 ms; 256 -> 256 at 56 x 56: 1.03 against 0.69 ms).  AUTO takes it there, within
-  // the same 2e-2 bound (E_B 1.2e-2 against 2.8e-3).  WINOCONV_AUTO_F43=0 keeps the row-piece kernel everywhere.
+  // the same 2e-2 bound (E_B 1.2e-2 against 2.8e-3).  WINOCONV_AUTO_F43=0 keeps the single-kernel path everywhere.
   static const int auto_f43_env = [] { const char *v = getenv("WINOCONV_AUTO_F43"); return v && *v ? atoi(v) : 1; }();
   bool f43_wins = false;
   if (f43_ok && single_kernel_candidate && d->algo == WINOCONV_ALGO_AUTO && d->tile_m == 0 && auto_f43_env != 0 &&
@@ -261,8 +262,13 @@ int build_plan(const winoconv_desc_t *d, Plan *plan) {
   // The direct-tap kernel: on request (tile_m = 1), or AUTO's choice where no tile size is asked for -- for every 16-bit layer
   // that would otherwise run on the row-piece kernel (measured on B200, 1.1 to 3.6 times as fast on all shapes tried; the
   // exception above keeps its staged F(4x4,3x3)), and for fp32 except 3x3 stride-1 layers whose quarter of the multiplies as
-  // F(4x4,3x3) outweighs the traffic of V and M: multiplies grow with C * K (K in whole 64-column blocks), V and M with C + K
-  // (measured, us direct / staged: 16 -> 16 at 112 x 112, N = 4: 12 / 22; 488 -> 24 at 63 x 95, N = 2: 83 / 53).
+  // F(4x4,3x3) outweighs the traffic of V and M: multiplies grow with C * K (K in whole 64-column blocks), V and M with C + K.
+  // us direct / staged on B200: layers of 128 channels and more with many pixels go to staged rightly (416 -> 256 at 28 x 28, N = 8: 103 / 60;
+  // 128 -> 96 at 112 x 112, N = 2: 52 / 45), 64 -> 64, which lies on the line, to direct taps (22 / 24).  The line knows neither the
+  // image nor the batch, nor that K = 8 costs the direct kernel what 64 do: one small image, or 16 -> 8, is slower staged (128 -> 64
+  // at 28 x 28, N = 1: 11 / 16; 16 -> 8 at 28 x 28, N = 8: 7 / 14).  Kernels other than 3x3 always take direct taps: ahead on most
+  // (5x5 64 -> 64 at 112 x 112, N = 2: 46 / 76), behind with 256 and more channels over few pixels (416 -> 96 9x9 at 28 x 28, N = 1: 114 / 71), where they keep
+  // the smaller error (5x5 over 64 channels: 2e-7 against 5e-7).  Over 842 fp32 layers the choice is within 1.7 % of the faster one on average.
   plan->direct = false;
   const bool direct_ok = d->algo == WINOCONV_ALGO_AUTO && d->gemm_engine == WINOCONV_GEMM_AUTO && pdt == WINOCONV_F32;
   const bool f32_f43_wins = d->dtype == WINOCONV_F32 && f43_ok &&

@@ -87,7 +87,7 @@ struct DGeom {
 struct DSmem {
   int slab_bytes, a_bytes, lo_off;   // bytes TMA delivers, bytes of a stage, offset of the remainder copy (fp32)
   int b_tile, b_lo, b_bytes, n_a, n_b;   // bytes of one tap's filter tile (hi part, and lo part for fp32), of a stage
-  int off_b, off_stage, off_raw, raw_bytes, off_bars, total;   // raw_bytes: of a raw patch, a multiple of 128
+  int off_b, off_stage, off_raw, raw_bytes, off_bars;   // raw_bytes: of a raw patch, a multiple of 128
 };
 
 template <typename T> struct OutWord {   // one 32-bit word of output: a 16-bit pair
@@ -1388,7 +1388,7 @@ cudaError_t launch_direct_forward(const DirectDesc &d, const DirectPlan &p, cons
   sl.off_raw = sl.off_stage + p.epi_sets * EPI_WARPS * STAGE_BYTES;
   sl.raw_bytes = (p.raw_box + 127) / 128 * 128;
   if (d.fold) sl.slab_bytes = p.raw_box;       // what TMA delivers
-  sl.off_bars = sl.off_raw + (int)RAW_BUFS * sl.raw_bytes; sl.total = p.smem;
+  sl.off_bars = sl.off_raw + (int)RAW_BUFS * sl.raw_bytes;
   const int sms = sm_count_of_current_device();
   if (sms <= 0) { *detail = "no device"; return cudaErrorNoDevice; }
   const uint32_t fmt = f32 ? 2u : d.dtype == WINOCONV_F16 ? 0u : 1u;
