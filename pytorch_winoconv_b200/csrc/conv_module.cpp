@@ -104,7 +104,7 @@ struct ConvFn : public torch::autograd::Function<ConvFn> {
   static at::Tensor forward(torch::autograd::AutogradContext *ctx, const c10::intrusive_ptr<ConvRunner> &runner, const at::Tensor &x,
                             const at::Tensor &x_cl, const std::shared_ptr<ConvRunner::Entry> &entry, const at::Tensor &weight,
                             const std::optional<at::Tensor> &bias, bool relu) {
-    at::Tensor y = runner->run(*entry, x_cl, weight, bias);
+    at::Tensor y = runner->run(*entry, x_cl, weight, bias, weight.requires_grad());
     ctx->save_for_backward({x, relu ? y : at::Tensor()});
     ctx->saved_data["runner"] = c10::IValue::make_capsule(runner);
     ctx->saved_data["weight"] = weight;
@@ -194,22 +194,23 @@ std::shared_ptr<ConvRunner::Entry> ConvRunner::entry_for(const at::Tensor &x, co
   return e;
 }
 
-at::Tensor ConvRunner::run(Entry &e, const at::Tensor &x, const at::Tensor &weight, const std::optional<at::Tensor> &bias) {
+at::Tensor ConvRunner::run(Entry &e, const at::Tensor &x, const at::Tensor &weight, const std::optional<at::Tensor> &bias, bool learns) {
   const at::ScalarType type = type_of(e.dtype);
   void *s = stream_of();
   const Stamp now = stamp_of(weight, bias);
   at::Tensor u, b;
   {
     std::lock_guard<std::mutex> lock(mu_);
-    if (!(e.stamp == now) || !e.written.usable_here({e.u, e.bias})) {
+    if (!(e.stamp == now) || !e.written.usable_here({e.u, e.bias}, learns)) {
       at::AutoDispatchBelowADInplaceOrView guard;
       // a new buffer, not the old one, which launches may still be queued to read (the allocator knows on which streams)
-      e.u = empty_bytes(e.info.filter_bytes, weight);
+      const at::Tensor fresh = empty_bytes(e.info.filter_bytes, weight);
       at::Tensor w = weight.is_contiguous() ? weight : weight.contiguous();
-      if (winoconv_filter_transform_from(&e.desc, w.data_ptr(), code_of(w.scalar_type()), e.u.data_ptr(), s) != WINOCONV_OK) {
+      if (winoconv_filter_transform_from(&e.desc, w.data_ptr(), code_of(w.scalar_type()), fresh.data_ptr(), s) != WINOCONV_OK) {
         w = w.to(type);
-        check_abi(winoconv_filter_transform(&e.desc, w.data_ptr(), e.u.data_ptr(), s), "winoconv_filter_transform");
+        check_abi(winoconv_filter_transform(&e.desc, w.data_ptr(), fresh.data_ptr(), s), "winoconv_filter_transform");
       }
+      e.u = fresh;
       e.bias = bias ? bias->detach().to(e.desc.bias_f32 ? at::kFloat : type).contiguous() : at::Tensor();
       e.written.here();
       e.stamp = now;
@@ -253,14 +254,14 @@ std::optional<at::Tensor> ConvRunner::forward(const at::Tensor &x, const at::Ten
     e = entry_for(x, weight, bias, dtype, true);
     if (e) {
       at::AutoDispatchBelowADInplaceOrView no_graph;
-      return run(*e, x, weight, bias);
+      return run(*e, x, weight, bias, false);
     }
   }
   e = entry_for(x, weight, bias, dtype, false);
   if (!e) return std::nullopt;
   if (!grad) {
     at::AutoDispatchBelowADInplaceOrView no_graph;
-    return run(*e, dense_channels_last(x, type_of(dtype), stream_of()), weight, bias);
+    return run(*e, dense_channels_last(x, type_of(dtype), stream_of()), weight, bias, false);
   }
   if (!backward_covered(*e)) return std::nullopt;
   at::Tensor x_cl;
@@ -278,12 +279,12 @@ void ConvRunner::Written::here() {
   recorded = finished = false;
 }
 
-bool ConvRunner::Written::usable_here(std::initializer_list<at::Tensor> buffers) {
+bool ConvRunner::Written::usable_here(std::initializer_list<at::Tensor> buffers, bool learns) {
   const auto now = at::cuda::getCurrentCUDAStream();
   if (!stream) return false;
-  if (capture == 0 && *stream == now) return true;
+  if (capture == 0 && *stream == now && !learns) return true;
   const unsigned long long current = capture_of(now);
-  if (capture != 0 && capture != current) return false;
+  if ((capture != 0 || learns) && capture != current) return false;
   if (*stream == now) return true;
   if (!finished) {
     c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);      // a query is no part of anyone's capture
@@ -339,12 +340,13 @@ std::vector<at::Tensor> ConvRunner::backward(const at::Tensor &gy_in, const at::
     const Stamp now = stamp_of(weight, std::nullopt);
     {
       std::lock_guard<std::mutex> lock(mu_);
-      if (!(e->back_stamp == now) || !e->back_written.usable_here({e->u_back})) {
-        e->u_back = empty_bytes(std::max<uint64_t>(info.data_filter_bytes, 16), w);
+      if (!(e->back_stamp == now) || !e->back_written.usable_here({e->u_back}, weight.requires_grad())) {
+        const at::Tensor fresh = empty_bytes(std::max<uint64_t>(info.data_filter_bytes, 16), w);
         at::Tensor wt = w;
         if (code_of(w.scalar_type()) != WINOCONV_F32 && code_of(w.scalar_type()) != dtype) wt = w.to(type);
-        check_abi(winoconv_backward_filter_transform(&d, wt.data_ptr(), code_of(wt.scalar_type()), e->u_back.data_ptr(), s),
+        check_abi(winoconv_backward_filter_transform(&d, wt.data_ptr(), code_of(wt.scalar_type()), fresh.data_ptr(), s),
                   "winoconv_backward_filter_transform");
+        e->u_back = fresh;
         e->back_written.here();
         e->back_stamp = now;
       }

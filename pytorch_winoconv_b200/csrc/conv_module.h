@@ -58,7 +58,8 @@ class ConvRunner : public torch::CustomClassHolder {
     bool recorded = false, finished = false;
     unsigned long long capture = 0;
     void here();                                                      // they are written by what is queued on the current stream so far
-    bool usable_here(std::initializer_list<at::Tensor> buffers);      // false: write them anew
+    // false: write them anew; learns: of weights that change between two runs of a graph, which then writes them itself
+    bool usable_here(std::initializer_list<at::Tensor> buffers, bool learns);
   };
   struct Entry {
     int64_t shape[5] = {0, 0, 0, 0, 0};      // N, D, H, W, C of the input
@@ -77,7 +78,7 @@ class ConvRunner : public torch::CustomClassHolder {
     bool back_known = false, back_ok = false;
   };
 
-  at::Tensor run(Entry &e, const at::Tensor &x_cl, const at::Tensor &weight, const std::optional<at::Tensor> &bias);
+  at::Tensor run(Entry &e, const at::Tensor &x_cl, const at::Tensor &weight, const std::optional<at::Tensor> &bias, bool learns);
   // Gradients of one layer call; undefined where not asked for.
   std::vector<at::Tensor> backward(const at::Tensor &gy, const at::Tensor &x, const at::Tensor &y, const at::Tensor &weight,
                                    const std::optional<at::Tensor> &bias, bool need_x, bool need_w, bool need_b);

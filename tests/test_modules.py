@@ -556,3 +556,27 @@ assert float((m.weight.grad.cpu().double() - o).norm() / o.norm()) < 1e-5
 """
     done = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
     assert done.returncode == 0, done.stderr[-2000:]
+
+
+@pytest.mark.gpu
+def test_a_captured_training_step_follows_its_weights():
+    _warm()
+    m, x = _layer_and_input(61)
+    n = wconv.Conv2d(32, 32, 3, padding=1).cuda()
+    n.load_state_dict(m.state_dict())
+    graphed = torch.cuda.make_graphed_callables(n, (x.detach().clone().requires_grad_(True),))
+    for _ in range(3):
+        a, b = (x.detach().clone().requires_grad_(True) for _ in range(2))
+        m.zero_grad()
+        n.zero_grad()
+        ya, yb = m(a), graphed(b)
+        ya.backward(x)
+        yb.backward(x)
+        assert torch.equal(ya, yb) and torch.equal(a.grad, b.grad)
+        for p, q in zip(m.parameters(), n.parameters()):
+            assert torch.equal(p.grad, q.grad)
+            with torch.no_grad():
+                p.sub_(p.grad * 1e-3)
+                q.sub_(q.grad * 1e-3)
+    with torch.no_grad():
+        assert torch.equal(m(x), n(x))
