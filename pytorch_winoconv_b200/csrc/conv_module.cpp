@@ -4,6 +4,7 @@
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 
+#include <algorithm>
 #include <cstring>
 
 namespace {
@@ -219,6 +220,9 @@ at::Tensor ConvRunner::run(Entry &e, const at::Tensor &x, const at::Tensor &weig
     }
     u = e.u;
     b = e.bias;
+    if (e.written.capture == 0 && capture_of(at::cuda::getCurrentCUDAStream()) != 0 &&
+        std::none_of(in_graphs_.begin(), in_graphs_.end(), [&](const auto &t) { return t.first.is_same(u); }))
+      in_graphs_.emplace_back(u, b);
   }
   int64_t sizes[5] = {e.shape[0], (int64_t)e.desc.k_out, 0, 0, 0};
   for (int i = 0; i < nd_; ++i) sizes[2 + i] = e.info.out_size[3 - nd_ + i];

@@ -8,6 +8,7 @@
 #include <mutex>
 #include <optional>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include <ATen/cuda/CUDAEvent.h>
@@ -92,6 +93,7 @@ class ConvRunner : public torch::CustomClassHolder {
   size_t max_plans_;
   std::mutex mu_;
   std::vector<std::shared_ptr<Entry>> entries_;     // most recently used last
+  std::vector<std::pair<at::Tensor, at::Tensor>> in_graphs_;      // filters and biases that a captured graph reads: kept as long as the module
   Stamp newest_;
   int64_t serial_ = 0;
 };

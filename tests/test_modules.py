@@ -580,3 +580,32 @@ def test_a_captured_training_step_follows_its_weights():
                 q.sub_(q.grad * 1e-3)
     with torch.no_grad():
         assert torch.equal(m(x), n(x))
+
+
+@pytest.mark.gpu
+def test_a_graph_keeps_the_filters_it_was_captured_with():
+    _warm()
+    m, x = _layer_and_input(62)
+    with torch.no_grad():
+        m(x)
+        torch.cuda.synchronize()
+        size = next(iter(m._plans.values())).u.numel()
+        m.__dict__["_views"].clear()
+        g = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(g):
+            y = m(x)
+        g.replay()
+        torch.cuda.synchronize()
+        before = y.clone()
+        m.weight.mul_(2.0)
+        m.bias.add_(1.0)
+        z = m(x)                                       # new filters: the old ones are the graph's alone
+        spoil = [torch.full((size,), 255, dtype=torch.uint8, device="cuda") for _ in range(8)]
+        g.replay()
+        torch.cuda.synchronize()
+        o = torch.nn.functional.conv2d(x.cpu().double(), m.weight.cpu().double() / 2, None, 1, 1)
+        b = m.bias.cpu().double().view(1, -1, 1, 1) - 1        # an fp32 bias is read as it lies, in the graph too
+        assert _rel(before, o + b) < _ONE_ROUNDING[torch.float16]
+        assert _rel(y, o + b + 1) < _ONE_ROUNDING[torch.float16]
+        assert _rel(z, _by_torch(m, x)) < _ONE_ROUNDING[torch.float16]
+        del spoil
