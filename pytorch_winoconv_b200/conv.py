@@ -44,6 +44,8 @@ from . import _backend, capi, engine
 
 __all__ = ["Conv2d", "Conv3d"]
 
+_Module, _stock_call = nn.Module, nn.Module._wrapped_call_impl
+
 
 class _WinoConvMixin:
     """Shared forward of :class:`Conv2d` and :class:`Conv3d` (``self`` is a ``torch.nn._ConvNd``)."""
@@ -82,7 +84,7 @@ class _WinoConvMixin:
         if (kwargs or len(args) != 1 or type(args[0]) is not torch.Tensor or d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"]
                 or _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks or _nn_module._global_backward_hooks
                 or _nn_module._global_backward_pre_hooks or self._compiled_call_impl is not None or torch._C._get_tracing_state()
-                or nn.Module.__call__ is not nn.Module._wrapped_call_impl):
+                or _Module.__call__ is not _stock_call):
             return super().__call__(*args, **kwargs)
         return self.forward(args[0])
 

@@ -93,8 +93,9 @@ at::Tensor pad_channels(const at::Tensor &t, int64_t c) {
   return at::constant_pad_nd(cl, {0, c - t.size(1)}).contiguous().movedim(nd - 1, 1);
 }
 
-// The graph capture the stream takes part in, 0 outside of one.
+// The graph capture the stream takes part in, 0 outside of one.  (The default stream takes part in none, and needs no query.)
 unsigned long long capture_of(cudaStream_t stream) {
+  if (stream == nullptr) return 0;
   cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
   unsigned long long id = 0;
   C10_CUDA_CHECK(cudaStreamGetCaptureInfo(stream, &status, &id));
@@ -197,12 +198,13 @@ std::shared_ptr<ConvRunner::Entry> ConvRunner::entry_for(const at::Tensor &x, co
 
 at::Tensor ConvRunner::run(Entry &e, const at::Tensor &x, const at::Tensor &weight, const std::optional<at::Tensor> &bias, bool learns) {
   const at::ScalarType type = type_of(e.dtype);
-  void *s = stream_of();
+  const auto here = at::cuda::getCurrentCUDAStream();
+  void *s = (void *)here.stream();
   const Stamp now = stamp_of(weight, bias);
   at::Tensor u, b;
   {
     std::lock_guard<std::mutex> lock(mu_);
-    if (!(e.stamp == now) || !e.written.usable_here({e.u, e.bias}, learns)) {
+    if (!(e.stamp == now) || !e.written.usable_on(here, learns, e.u, e.bias)) {
       at::AutoDispatchBelowADInplaceOrView guard;
       // a new buffer, not the old one, which launches may still be queued to read (the allocator knows on which streams)
       const at::Tensor fresh = empty_bytes(e.info.filter_bytes, weight);
@@ -213,14 +215,14 @@ at::Tensor ConvRunner::run(Entry &e, const at::Tensor &x, const at::Tensor &weig
       }
       e.u = fresh;
       e.bias = bias ? bias->detach().to(e.desc.bias_f32 ? at::kFloat : type).contiguous() : at::Tensor();
-      e.written.here();
+      e.written.on(here);
       e.stamp = now;
       e.serial = ++serial_;
       newest_ = now;
     }
     u = e.u;
     b = e.bias;
-    if (e.written.capture == 0 && capture_of(at::cuda::getCurrentCUDAStream()) != 0 &&
+    if (e.written.capture == 0 && capture_of(here) != 0 &&
         std::none_of(in_graphs_.begin(), in_graphs_.end(), [&](const auto &t) { return t.first.is_same(u); }))
       in_graphs_.emplace_back(u, b);
   }
@@ -277,19 +279,18 @@ std::optional<at::Tensor> ConvRunner::forward(const at::Tensor &x, const at::Ten
   return ConvFn::apply(c10::intrusive_ptr<ConvRunner>::reclaim_copy(this), x, x_cl, e, weight, bias, relu_);
 }
 
-void ConvRunner::Written::here() {
-  stream = at::cuda::getCurrentCUDAStream();
-  capture = capture_of(*stream);
+void ConvRunner::Written::on(const c10::cuda::CUDAStream &here) {
+  stream = here;
+  capture = capture_of(here);
   recorded = finished = false;
 }
 
-bool ConvRunner::Written::usable_here(std::initializer_list<at::Tensor> buffers, bool learns) {
-  const auto now = at::cuda::getCurrentCUDAStream();
+bool ConvRunner::Written::usable_on(const c10::cuda::CUDAStream &here, bool learns, const at::Tensor &a, const at::Tensor &b) {
   if (!stream) return false;
-  if (capture == 0 && *stream == now && !learns) return true;
-  const unsigned long long current = capture_of(now);
+  if (capture == 0 && *stream == here && !learns) return true;
+  const unsigned long long current = capture_of(here);
   if ((capture != 0 || learns) && capture != current) return false;
-  if (*stream == now) return true;
+  if (*stream == here) return true;
   if (!finished) {
     c10::cuda::CUDAStreamCaptureModeGuard relaxed(cudaStreamCaptureModeRelaxed);      // a query is no part of anyone's capture
     if (!recorded && capture_of(*stream) != capture) return false;      // being captured now: it tells nothing of the work before that
@@ -301,10 +302,10 @@ bool ConvRunner::Written::usable_here(std::initializer_list<at::Tensor> buffers,
   }
   if (!finished) {
     if (capture != current) return false;
-    event.block(now);
+    event.block(here);
   }
-  for (const at::Tensor &t : buffers)
-    if (t.defined()) t.record_stream(now);
+  for (const at::Tensor *t : {&a, &b})
+    if (t->defined()) t->record_stream(here);
   return true;
 }
 
@@ -328,7 +329,8 @@ std::vector<at::Tensor> ConvRunner::backward(const at::Tensor &gy_in, const at::
   const at::ScalarType type = type_of(dtype);
   std::shared_ptr<Entry> e = entry_for(x_in, weight, bias, dtype, false);
   TORCH_CHECK(e, "winoconv backward: no plan");
-  void *s = stream_of();
+  const auto here = at::cuda::getCurrentCUDAStream();
+  void *s = (void *)here.stream();
   at::Tensor gy = gy_in;
   if (y.defined()) gy = gy * (y > 0).to(gy.scalar_type());
   gy = aligned(dense_channels_last(gy, type, s));
@@ -344,14 +346,14 @@ std::vector<at::Tensor> ConvRunner::backward(const at::Tensor &gy_in, const at::
     const Stamp now = stamp_of(weight, std::nullopt);
     {
       std::lock_guard<std::mutex> lock(mu_);
-      if (!(e->back_stamp == now) || !e->back_written.usable_here({e->u_back}, weight.requires_grad())) {
+      if (!(e->back_stamp == now) || !e->back_written.usable_on(here, weight.requires_grad(), e->u_back, at::Tensor())) {
         const at::Tensor fresh = empty_bytes(std::max<uint64_t>(info.data_filter_bytes, 16), w);
         at::Tensor wt = w;
         if (code_of(w.scalar_type()) != WINOCONV_F32 && code_of(w.scalar_type()) != dtype) wt = w.to(type);
         check_abi(winoconv_backward_filter_transform(&d, wt.data_ptr(), code_of(wt.scalar_type()), fresh.data_ptr(), s),
                   "winoconv_backward_filter_transform");
         e->u_back = fresh;
-        e->back_written.here();
+        e->back_written.on(here);
         e->back_stamp = now;
       }
       u = e->u_back;

@@ -3,7 +3,6 @@
 #pragma once
 
 #include <cstdint>
-#include <initializer_list>
 #include <memory>
 #include <mutex>
 #include <optional>
@@ -58,9 +57,9 @@ class ConvRunner : public torch::CustomClassHolder {
     at::cuda::CUDAEvent event;
     bool recorded = false, finished = false;
     unsigned long long capture = 0;
-    void here();                                                      // they are written by what is queued on the current stream so far
+    void on(const c10::cuda::CUDAStream &here);      // they are written by what is queued on that stream so far
     // false: write them anew; learns: of weights that change between two runs of a graph, which then writes them itself
-    bool usable_here(std::initializer_list<at::Tensor> buffers, bool learns);
+    bool usable_on(const c10::cuda::CUDAStream &here, bool learns, const at::Tensor &a, const at::Tensor &b);
   };
   struct Entry {
     int64_t shape[5] = {0, 0, 0, 0, 0};      // N, D, H, W, C of the input
