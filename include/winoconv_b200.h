@@ -220,6 +220,8 @@ WINOCONV_API int winoconv_forward_timed(const winoconv_desc_t *desc, const void 
  *     7x7 stride-2 stem on 225 x 225 RGB images, whose rows cannot be read as they lie, passes 32 MiB from batch 78 on) and is refused the same way beyond that:
  *     the transformed filter is laid out per algorithm, so re-plan that layer with algo =
  *     WINOCONV_ALGO_FUSED (no scratch at all) or WINOCONV_ALGO_STAGED, transform its filter again and call.
+ *     A direct-tap layer with padded channels (winoconv_plan: direct = 2) is padded a part of the batch at a time; one
+ *     whose algo is ROW is refused where that kernel's copy would be.
  *   - The first call on each device looks up the array's device address (with that device current) and
  *     keeps it; make that first call before starting any stream capture.
  *   - All calls on a device share the one array, and it keeps whatever the previous call left.  Nothing
